@@ -134,6 +134,11 @@ struct SceneDev {
     int enabled;          // 0: left out of resolve calls (candidates pass through)
     int strain_e0, strain_ne;  // its strain edges
     int nt;               // triangles (its first nt elements)
+    // schedule of its strain sweeps in shared memory (cc_sweep_plan.h): first
+    // level offset, levels, first epoch, epochs, levels per epoch, elements
+    // of the widest level, slots, records staged in shared memory, first
+    // element and elements; whether it fits
+    int sw_lev0, sw_levels, sw_ep0, sw_epochs, sw_k, sw_width, sw_slots, sw_ring, sw_e0, sw_ne, sw_fits;
 };
 
 // Per-pass state of a scene (written by the host before a pass, except

@@ -419,50 +419,78 @@ void finalize_positions(const uint8_t* in_elem, const double4_32a* xo, double4_3
                         const double* x_cand, double* x_out, int nv, const int* vscene, const SceneDev* scenes,
                         const uint8_t* fixed, const uint8_t* mask, cudaStream_t s);
 // reduceSuperelast: up to 10 Gauss-Seidel passes over each scene's strain
-// edges, one CTA per scene.
+// edges (cc_strain.cu).
 struct StrainEdge {
     int p0, p1;
     double len0;
-    int s0, s1;  // shared-memory slots of p0, p1 in the scene's window sweep
+    int s0, s1;  // slots of p0, p1 in the edge schedule (cc_strain_plan.h)
 };
-// Strain schedule of all scenes: the edges of a scene are contiguous and
-// sorted by dependency level; its levels are hdr[2*(hdr0 + l)] =
-// (edge begin, end, copy-in begin, end) and hdr[2*(hdr0 + l) + 1] =
-// (write-back begin, end, 0, 0) for l < levels, with (point, slot) entries
-// in load_list / wb_list; the write-backs after its last level are
-// wb_list[wb_final0 .. wb_final1) (SceneDev).
+// An element of the strain sweeps: a triangle with its edges p0p1, p1p2,
+// p2p0 in that order, or a bond with one edge (p[2] = p[0]), the slots of
+// its points in the shared-memory sweep, and its edges' rest lengths.
+struct SweepElem {
+    int p[3];
+    unsigned s01;  // slots of p[0] and p[1], 16 bits each
+    unsigned s2n;  // slot of p[2] and the number of edges
+    int pad;
+    double len0[3];
+    int np() const { return (s2n >> 16) == 1 ? 2 : 3; }
+    void set_slots(int a, int b, int c) {
+        s01 = ((unsigned)a & 0xffffu) | ((unsigned)b << 16);
+        s2n = (s2n & 0xffff0000u) | ((unsigned)c & 0xffffu);
+    }
+};
+// The shared-memory sweep's sizes: a slot (FP64 and FP32 velocity), an
+// element's record of the step, levels of records staged ahead.
+constexpr int kSweepSlotBytes = 48, kSweepRecBytes = 80, kSweepRing = 8;
+constexpr int kSweepMaxEpoch = 4;
+constexpr size_t kSweepMaxBytes = 224 * 1024;    // within the 227 KB a CTA may hold
+constexpr size_t kSweepSharedBytes = 110 * 1024;  // lets two CTAs share an SM
+inline size_t sweep_smem(int slots, int width, int ring) {
+    return (size_t)slots * kSweepSlotBytes + (ring ? (size_t)kSweepRing * width * kSweepRecBytes : 0);
+}
+
+// The strain schedules on the device. The sweep arrays are cc_sweep_plan.h's
+// (scenes' ranges in SceneDev::sw_*). The edge arrays are the schedule of
+// k_strain, for scenes whose sweep does not fit in shared memory or with
+// `window` off; null until one is needed.
+struct StrainBufs {
+    const SweepElem* elems = nullptr;
+    const int* lev = nullptr;
+    const int4* epoch = nullptr;
+    const int* need = nullptr;
+    const int2 *load = nullptr, *wb = nullptr;
+    int nelems = 0;
+    void* recs = nullptr;         // kSweepRecBytes per element
+    int* state = nullptr;         // strain_state_ints(nscenes)
+    const int2* chunks = nullptr; // (scene, first element) of every run of at most 256 elements of one scene
+    int nchunks = 0;
+    const int* order = nullptr;   // scenes by levels, most first
+    int* flags = nullptr;         // 2 per scene
+    int* passes_out = nullptr;    // 3 per scene: passes (-1: the sweeps timed out), averaged edges, exact tests
+    // k_strain's
+    const StrainEdge* edges = nullptr;
+    int nedges = 0;
+    const int4* hdr = nullptr;
+    void* edge_steps = nullptr;   // strain_edge_step_bytes(nedges)
+};
+// How the strain loop runs.
 struct StrainPlan {
-    bool window;           // sweep in shared memory where the scene's slots fit
-    int max_window_slots;  // largest slot count among the scenes that fit
-    bool any_global;       // some scene needs more slots than fit
-    int block;             // threads per sweep CTA
-    bool warp;             // one warp per scene with staged levels (k_strain_warp)
-    int ecap, lcap, wcap;  // most edges, copy-ins, write-backs of one level (scenes that fit)
-    size_t warp_smem;      // its dynamic shared memory
-    const int* order;      // device: scene of each sweep CTA, most levels first
-    // window sweep: first thread of the copy-in and the write-back roles (a
-    // level's edges on threads [0, cbase)); 0, 0: every thread takes all three
-    int cbase, wbase;
+    bool window;       // sweep in shared memory where the scene fits
+    bool any_global;   // some scene is swept by k_strain
+    int workers;       // warps taking a level's elements
+    size_t smem;       // dynamic shared memory of a sweep CTA
 };
-// Dynamic shared memory of the one-warp sweep for these sizes.
-size_t strain_warp_smem(int max_slots, int ecap, int lcap, int wcap);
-int strain_window_slot_cap();
+size_t strain_edge_step_bytes(int nedges);
+int strain_state_ints(int nscenes);
 // Once per device before any strain_limit (not a stream operation, so it
 // stays out of captured graphs).
 void strain_configure();
-// step_buf holds strain_step_bytes(nedges); passes_out holds 3 ints per
-// scene (passes, averaged edges, exact tests).
-size_t strain_step_bytes(int nedges);
-// chunks: (scene, first edge) of every run of at most 256 edges of one
-// scene; flags: 2 ints per scene.
-// Per step, before any strain_limit: each edge's records from x_old.
-void strain_setup(const StrainEdge* edges, int nedges, const SceneDev* scenes, const StrainPlan& plan,
-                  const double4_32a* xo, void* step_buf, const int* vscene, cudaStream_t s);
+// Per step, before any strain_limit: the elements' records from x_old.
+void strain_setup(const StrainBufs& b, const StrainPlan& plan, const double4_32a* xo, cudaStream_t s);
 // The strain loop of the scenes in mask (per scene, nonzero: in; null: all).
-void strain_limit(const StrainEdge* edges, int nedges, const int4* hdr, const int2* load_list, const int2* wb_list,
-                  const int2* chunks, int nchunks, const SceneDev* scenes, int nscenes, const StrainPlan& plan,
-                  const double4_32a* xo, double4_32a* av, void* step_buf, int* flags, int* passes_out,
-                  const uint8_t* mask, cudaStream_t s);
+void strain_limit(const StrainBufs& b, const SceneDev* scenes, int nscenes, const StrainPlan& plan,
+                  const double4_32a* xo, double4_32a* av, const uint8_t* mask, cudaStream_t s);
 // Correctly rounded cos/sin/acos/pow (fn 0..3) on device arrays, for self-tests.
 void math_selftest(int fn, const double* a, const double* b, double* out, int n, cudaStream_t s);
 // updateFinalVelocity.

@@ -1,10 +1,9 @@
 // Per-point stages around the detection passes: average velocity, applying
 // a pass's impulses, impact-zone rigid motion, the domain clamp, final
-// positions, strain limiting and final velocities (dcollid.cpp:116-220,
-// 290-310, 486-624, 677-751; dcollid3d.cpp:70-200).
+// positions and final velocities (dcollid.cpp:116-220, 290-310, 562-624,
+// 677-751; dcollid3d.cpp:70-200).
 #include "cc_launch.h"
 #include "cc_narrow.cuh"
-#include "cc_strain_plan.h"
 
 namespace ccg {
 
@@ -520,777 +519,6 @@ __global__ void k_finalize(const uint8_t* __restrict__ in_elem, const double4_32
     for (int j = 0; j < 3; ++j) x_out[3 * p + j] = xs[j] + v[j] * dt;
 }
 
-// One edge's strain test, reduceSuperelastOnce (dcollid.cpp:496-539),
-// evaluated as the reference does.
-__device__ __forceinline__ bool strain_flag_exact(int p0, int p1, double len0, const double4_32a* xo,
-                                                  const double4_32a* av, double dt) {
-    double x0[3], x1[3], v0[3], v1[3], c0[3], c1[3];
-    load3(xo, p0, x0);
-    load3(xo, p1, x1);
-    load3(av, p0, v0);
-    load3(av, p1, v1);
-    for (int k = 0; k < 3; ++k) {
-        c0[k] = x0[k] + dt * v0[k];
-        c1[k] = x1[k] + dt * v1[k];
-    }
-    double sn = 0.0, so = 0.0;
-    for (int k = 0; k < 3; ++k) sn += sqr(c0[k] - c1[k]);
-    for (int k = 0; k < 3; ++k) so += sqr(x0[k] - x1[k]);
-    double len_new = sqrt(sn), len_old = sqrt(so);
-    if (len_old > kRoundEps && len_new > kRoundEps) {
-        double strain_rate = (len_new - len_old) / len_old;
-        double strain = (len_new - len0) / len0;
-        return fabs(strain) > kStrainTol || fabs(strain_rate) > kStrainTol;
-    }
-    return true;
-}
-
-// Squared-length bounds that decide |(sqrt(s) - L)/L| > 0.1 without the
-// square root and the division: outside [lo_no, hi_no] the answer is "over",
-// inside [lo_def, hi_def] ... see strain_quick. The bounds sit 1e-9 (relative)
-// inside and outside the exact thresholds L*(1 -+ 0.1); the reference's own
-// rounding of sqrt, subtraction and division is below 1e-15, so a decision
-// taken here equals the reference's.
-struct StrainBounds {
-    double hi_def, hi_no, lo_no, lo_def;
-};
-__device__ __forceinline__ StrainBounds strain_bounds(double L) {
-    StrainBounds b;
-    double a = L * (1.1 * (1.0 + 1e-9)), c = L * (1.1 * (1.0 - 1e-9));
-    double d = L * (0.9 * (1.0 + 1e-9)), e = L * (0.9 * (1.0 - 1e-9));
-    b.hi_def = a * a;  // s above: over-stretched for sure
-    b.hi_no = c * c;   // s below (and above lo_no): not over-stretched
-    b.lo_no = d * d;
-    b.lo_def = e * e;  // s below: over-compressed for sure
-    return b;
-}
-// The same bounds from the squared length L2 = L*L, without the square root:
-// each differs from the one above by a few ulps, far inside the 1e-9 margin.
-__device__ __forceinline__ StrainBounds strain_bounds_sq(double L2) {
-    const double ka = (1.1 * (1.0 + 1e-9)) * (1.1 * (1.0 + 1e-9)), kc = (1.1 * (1.0 - 1e-9)) * (1.1 * (1.0 - 1e-9));
-    const double kd = (0.9 * (1.0 + 1e-9)) * (0.9 * (1.0 + 1e-9)), ke = (0.9 * (1.0 - 1e-9)) * (0.9 * (1.0 - 1e-9));
-    StrainBounds b;
-    b.hi_def = L2 * ka;
-    b.hi_no = L2 * kc;
-    b.lo_no = L2 * kd;
-    b.lo_def = L2 * ke;
-    return b;
-}
-// 1: over the limit, 0: within it, -1: too close to tell without the exact test.
-__device__ __forceinline__ int strain_quick(double s, const StrainBounds& b) {
-    if (s > b.hi_def || s < b.lo_def) return 1;
-    if (s < b.hi_no && s > b.lo_no) return 0;
-    return -1;
-}
-
-struct __align__(16) StrainEdgeStep {
-    int p0, p1;
-    double len0;
-    StrainBounds rest;  // from the rest length
-    StrainBounds prev;  // from the start-of-step length (strain rate)
-    double x0[3], x1[3];  // x_old of both points (constant through the sweep)
-    int exact_only;       // degenerate lengths: always take the exact test
-    int s0, s1;           // shared-memory slots of both points (window sweep)
-    int pad;
-    // FP32 view for the window sweep's first decision: x_old(p0) - x_old(p1)
-    // and the four squared-length bounds rounded outward (see k_strain_window)
-    float dx[3];
-    float over_hi, under_hi, under_lo, over_lo;
-    float pad2[2];
-};
-
-// The part of an edge record the window sweep reads for every edge: the
-// slots, x_old(p0) - x_old(p1) and the four bounds in FP32 (48 bytes).
-struct __align__(16) StrainEdgeHot {
-    int s0, s1;
-    float dx[3];
-    float over_hi, under_hi, under_lo, over_lo;
-    int pad[3];
-};
-
-// Per-step set-up of the strain sweep: the start-of-step length of every
-// edge (x_old does not change during the sweep) and both sets of bounds.
-// An edge's full record for the step, from its endpoints' x_old: the
-// exact test's inputs and the FP32 view of the window sweep.
-__device__ __forceinline__ StrainEdgeStep strain_step(const StrainEdge& ed, const double4_32a* __restrict__ xo) {
-    double x0[3], x1[3];
-    load3(xo, ed.p0, x0);
-    load3(xo, ed.p1, x1);
-    double so = 0.0;
-    for (int k = 0; k < 3; ++k) so += sqr(x0[k] - x1[k]);
-    StrainEdgeStep r;
-    r.p0 = ed.p0;
-    r.p1 = ed.p1;
-    r.len0 = ed.len0;
-    r.rest = strain_bounds(ed.len0);
-    r.prev = strain_bounds_sq(so);
-    for (int k = 0; k < 3; ++k) {
-        r.x0[k] = x0[k];
-        r.x1[k] = x1[k];
-    }
-    // tiny or non-positive lengths: leave every decision to the exact test
-    r.exact_only = !(so > 1e-12 && ed.len0 > 1e-6);
-    r.s0 = ed.s0;
-    r.s1 = ed.s1;
-    r.pad = 0;
-    for (int k = 0; k < 3; ++k) r.dx[k] = (float)(x0[k] - x1[k]);
-    // strain flags when s > hi_def (either bound) or s < lo_def; it is clear
-    // when lo_no < s < hi_no for both; FP32 thresholds rounded outward
-    double hdef = fmin(r.rest.hi_def, r.prev.hi_def), ldef = fmax(r.rest.lo_def, r.prev.lo_def);
-    double hno = fmin(r.rest.hi_no, r.prev.hi_no), lno = fmax(r.rest.lo_no, r.prev.lo_no);
-    r.over_hi = __double2float_ru(hdef);
-    r.over_lo = __double2float_rd(ldef);
-    r.under_hi = __double2float_rd(hno);
-    r.under_lo = __double2float_ru(lno);
-    r.pad2[0] = r.pad2[1] = 0.f;
-    return r;
-}
-
-// Per step: every edge's 48-byte hot record; the full record only for the
-// edges of scenes swept by k_strain (too many slots for shared memory) - the
-// shared-memory sweeps rebuild it for their rare exact tests.
-__global__ void k_strain_setup(const StrainEdge* __restrict__ edges, int m, const double4_32a* __restrict__ xo,
-                               StrainEdgeStep* out, StrainEdgeHot* hot, const int* __restrict__ vscene,
-                               const SceneDev* __restrict__ scenes, int slot_cap) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= m) return;
-    const StrainEdge ed = edges[e];
-    const StrainEdgeStep r = strain_step(ed, xo);
-    if (slot_cap < 0 || scenes[vscene[ed.p0]].strain_slots > slot_cap) out[e] = r;
-    StrainEdgeHot hh;
-    hh.s0 = r.s0;
-    hh.s1 = r.s1;
-    for (int k = 0; k < 3; ++k) hh.dx[k] = r.dx[k];
-    hh.over_hi = r.over_hi;
-    hh.under_hi = r.under_hi;
-    hh.under_lo = r.under_lo;
-    hh.over_lo = r.over_lo;
-    hh.pad[0] = hh.pad[1] = hh.pad[2] = 0;
-    hot[e] = hh;
-}
-
-// The strain decision for given end velocities v0, v1 (bounds first, the
-// exact test of dcollid.cpp:525-530 only inside the bounds' margin).
-__device__ __forceinline__ bool strain_flag_vals(const StrainEdgeStep& ed, const double* v0, const double* v1,
-                                                 double dt, int* n_exact) {
-    double c0[3], c1[3];
-    for (int k = 0; k < 3; ++k) {
-        c0[k] = ed.x0[k] + dt * v0[k];
-        c1[k] = ed.x1[k] + dt * v1[k];
-    }
-    double sn = 0.0;
-    for (int k = 0; k < 3; ++k) sn += sqr(c0[k] - c1[k]);
-    if (!ed.exact_only && sn > 1e-18) {
-        int q0 = strain_quick(sn, ed.rest), q1 = strain_quick(sn, ed.prev);
-        if (q0 == 1 || q1 == 1) return true;
-        if (q0 == 0 && q1 == 0) return false;
-    }
-    ++*n_exact;
-    double so = 0.0;
-    for (int k = 0; k < 3; ++k) so += sqr(ed.x0[k] - ed.x1[k]);
-    double len_new = sqrt(sn), len_old = sqrt(so);
-    if (len_old > kRoundEps && len_new > kRoundEps) {
-        double strain_rate = (len_new - len_old) / len_old;
-        double strain = (len_new - ed.len0) / ed.len0;
-        return fabs(strain) > kStrainTol || fabs(strain_rate) > kStrainTol;
-    }
-    return true;
-}
-
-// 0.5 * x, the averaging of the strain sweep: one less in the exponent field
-// (in the high 32 bits) when that field is 2..2046, where the halving is
-// exact; x itself for +-0; the FP64 multiply otherwise. GB300 issues a
-// warp's FP64 multiply in ~64 cycles whatever its active lanes, and the
-// averaging lies on the sweep's per-level critical path; these are a few
-// 32-bit integer instructions with the same result.
-__device__ __forceinline__ double half_of(double x) {
-    const int hi = __double2hiint(x), lo = __double2loint(x);
-    const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-    if (e - 2u < 0x7fdu) return __hiloint2double(hi - 0x00100000, lo);
-    if ((((unsigned)hi << 1) | (unsigned)lo) == 0u) return x;
-    return 0.5 * x;
-}
-
-// reduceSuperelast, dcollid.cpp:586-596: up to 10 Gauss-Seidel passes over
-// the edges in element order, each averaging the two end velocities of an
-// over-strained edge before the next edge is tested (one pass per launch). The edges arrive sorted
-// by dependency level (an edge's level is one more than the level of the
-// last earlier edge at either of its points), so the edges of one level share
-// no point and see exactly the values the sequential sweep gives them: the
-// level-by-level walk below is the reference's sweep, reordered only where
-// the order cannot matter.
-// Per scene and step, flags[2s] ("some edge would average": set by
-// k_strain_check) and flags[2s+1] (the sweep is over); passes_out[3s ..] the
-// sweeps run, edges averaged, exact tests. One launch is one pass: a scene
-// whose check found nothing to average is done - its sweep would change
-// nothing, which is how the reference's loop ends (dcollid.cpp:588-595) -
-// and counts that sweep; otherwise it sweeps once.
-__device__ __forceinline__ bool sweep_gate(int pass, int s, int* flags, int* passes_out_all) {
-    __shared__ int s_go;
-    if (threadIdx.x == 0) {
-        int go = 0;
-        if (!flags[2 * s + 1]) {
-            if (!flags[2 * s]) {
-                flags[2 * s + 1] = 1;
-                passes_out_all[3 * s] = pass + 1;
-            } else {
-                flags[2 * s] = 0;
-                go = 1;
-            }
-        }
-        s_go = go;
-    }
-    __syncthreads();
-    return s_go != 0;
-}
-
-__device__ __forceinline__ void sweep_done(int pass, int s, int n_avg, int n_exact, int* flags, int* passes_out_all) {
-    __shared__ int s_avg, s_exact;
-    if (threadIdx.x == 0) s_avg = s_exact = 0;
-    __syncthreads();
-    atomicAdd(&s_avg, n_avg);
-    atomicAdd(&s_exact, n_exact);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        passes_out_all[3 * s] = pass + 1;
-        passes_out_all[3 * s + 1] += s_avg;
-        passes_out_all[3 * s + 2] += s_exact;
-        if (pass + 1 >= kStrainMaxIter) flags[2 * s + 1] = 1;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_strain(const StrainEdgeStep* __restrict__ edges,
-                                                const int4* __restrict__ hdr_all,
-                                                const SceneDev* __restrict__ scenes, int slot_cap,
-                                                double4_32a* av, int pass, int* flags, int* passes_out_all,
-                                                const int* __restrict__ order) {
-    const int sc = order[blockIdx.x];
-    const SceneDev& sd = scenes[sc];
-    if ((slot_cap >= 0 && sd.strain_slots <= slot_cap) || !sd.enabled) return;  // k_strain_window's, or left out
-    if (!sweep_gate(pass, sc, flags, passes_out_all)) return;
-    const int4* hdr = hdr_all + 2 * sd.strain_hdr0;
-    const int nlevels = sd.strain_levels;
-    const double dt = sd.p.dt;
-    int n_avg = 0, n_exact = 0;
-    // the records of the next level are loaded before the barrier that ends
-    // the current one: they do not depend on the velocities
-    int e = 0, e1 = 0;
-    if (nlevels > 0) {
-        int4 h = hdr[0];
-        e = h.x + threadIdx.x;
-        e1 = h.y;
-    }
-    StrainEdgeStep cur;
-    bool have = e < e1;
-    if (have) cur = edges[e];
-    for (int l = 0; l < nlevels; ++l) {
-        int ne = 0, ne1 = 0;
-        if (l + 1 < nlevels) {
-            int4 h = hdr[2 * (l + 1)];
-            ne = h.x + threadIdx.x;
-            ne1 = h.y;
-        }
-        bool nhave = ne < ne1;
-        StrainEdgeStep nxt;
-        if (nhave) nxt = edges[ne];
-        while (have) {
-            double4_32a a0 = av[cur.p0], a1 = av[cur.p1];
-            double v0[3] = {a0.x, a0.y, a0.z}, v1[3] = {a1.x, a1.y, a1.z};
-            if (strain_flag_vals(cur, v0, v1, dt, &n_exact)) {
-                ++n_avg;
-                double t0 = a0.x + a1.x, t1 = a0.y + a1.y, t2 = a0.z + a1.z;
-                t0 = half_of(t0); t1 = half_of(t1); t2 = half_of(t2);
-                double4_32a nv4 = make_double4_32a(t0, t1, t2, 0.0);
-                av[cur.p0] = nv4;
-                av[cur.p1] = nv4;
-            }
-            e += blockDim.x;
-            have = e < e1;
-            if (have) cur = edges[e];
-        }
-        __syncthreads();
-        e = ne;
-        e1 = ne1;
-        have = nhave;
-        cur = nxt;
-    }
-    sweep_done(pass, sc, n_avg, n_exact, flags, passes_out_all);
-}
-
-// The same sweep with each point's velocity in shared memory while the
-// sweep uses it. Levels advance along the mesh like a wavefront, so a point
-// is live for only a few levels: at assembly every point gets a shared-memory
-// slot for its live interval (interval colouring; 418 slots for a 129x129
-// cloth). Its velocity is copied in with cp.async kWindowAhead levels before
-// its first edge and written back the level after its last one.
-//
-// FP64 runs at a small fraction of the FP32 rate on this GPU and the sweep
-// runs on one SM, so each slot also keeps an FP32 copy of the velocity and
-// an edge is first decided in FP32: s32 = |dx + dt (v0 - v1)|^2 from the
-// FP32 copies carries an error below 32 * 2^-24 * bnd^2 (bnd: sum of the
-// magnitudes entering it), and only when s32 +- that error straddles one of
-// the outward-rounded bounds does the FP64 decision (bounds, then the exact
-// test) run. The averaging itself is FP64, as in the reference.
-constexpr int kWindowAhead = 8;
-static_assert(kWindowAhead == kStrainAhead, "copy-ins are scheduled for the sweep's look-ahead");
-// dynamic shared memory of one sweep CTA at most: with the kernel's 2 KB of
-// static shared memory, within the 227 KB a CTA may hold (3,584 slots; a
-// 1025x1025 cloth needs 3,330)
-constexpr size_t kStrainWindowBytes = 224 * 1024;
-constexpr size_t kStrainWarpBytes = 200 * 1024;
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
-}
-
-// slot layout: [x y] [z -] as double2, then [x y z -] as float4
-struct WinSlot {
-    double2 a, b;
-    float4 f;
-    float4 pad;
-};
-
-__device__ __forceinline__ int strain_decide32(const StrainEdgeHot& ed, float4 f0, float4 f1, float dt32) {
-    float u[3], bnd = 0.f;
-    float v0[3] = {f0.x, f0.y, f0.z}, v1[3] = {f1.x, f1.y, f1.z};
-    float s32 = 0.f;
-    for (int k = 0; k < 3; ++k) {
-        float dv = __fsub_rn(v0[k], v1[k]);
-        u[k] = __fadd_rn(ed.dx[k], __fmul_rn(dt32, dv));
-        bnd = __fadd_ru(bnd, __fadd_ru(fabsf(ed.dx[k]), __fmul_ru(dt32, __fadd_ru(fabsf(v0[k]), fabsf(v1[k])))));
-        s32 = __fadd_rn(s32, __fmul_rn(u[k], u[k]));
-    }
-    float err = __fmul_ru(__fmul_ru(bnd, bnd), 32.0f * 5.9604645e-8f);
-    float lo = __fsub_rd(s32, err), hi = __fadd_ru(s32, err);
-    if (lo > ed.over_hi || hi < ed.over_lo) return 1;
-    if (hi < ed.under_hi && lo > ed.under_lo) return 0;
-    return -1;
-}
-
-__device__ __forceinline__ void strain_window_edge(const StrainEdgeHot& h, int e,
-                                                   const StrainEdge* __restrict__ edges,
-                                                   const double4_32a* __restrict__ xo, WinSlot* s_win,
-                                                   float dt32, double dt, int* n_avg, int* n_exact, bool* has) {
-    WinSlot& w0 = s_win[h.s0];
-    WinSlot& w1 = s_win[h.s1];
-    int q = strain_decide32(h, w0.f, w1.f, dt32);
-    if (q == 0) return;
-    double2 a0 = w0.a, a1 = w0.b, b0 = w1.a, b1 = w1.b;
-    double v0[3] = {a0.x, a0.y, a1.x}, v1[3] = {b0.x, b0.y, b1.x};
-    if (q < 0) {
-        const StrainEdgeStep full = strain_step(edges[e], xo);
-        if (!strain_flag_vals(full, v0, v1, dt, n_exact)) return;
-    }
-    ++*n_avg;
-    double t[3];
-    for (int k = 0; k < 3; ++k) {
-        t[k] = v0[k] + v1[k];
-        t[k] = half_of(t[k]);
-    }
-    double2 na = make_double2(t[0], t[1]), nb = make_double2(t[2], 0.0);
-    float4 nf = make_float4((float)t[0], (float)t[1], (float)t[2], 0.f);
-    w0.a = na; w0.b = nb; w0.f = nf;
-    w1.a = na; w1.b = nb; w1.f = nf;
-    *has = true;
-}
-
-// Everything a thread needs for a level arrives kRing levels early in a
-// register ring: the level's ranges, and the thread's first edge record,
-// copy-in entry and write-back entry. Entries beyond the first per thread
-// (levels wider than the block) are read when needed. The level loop is
-// unrolled by kWindowAhead (a multiple of kRing) so that every ring slot has
-// a fixed register name and nothing is shifted from level to level.
-constexpr int kRing = 4;
-
-struct WinRing {
-    int4 h0[kRing], h1[kRing];
-    StrainEdgeHot hot[kRing];
-    int2 ld[kRing], wb[kRing];
-    int lslot[kWindowAhead];  // slot this thread copied in, per recent level (-1: none)
-};
-
-// The level headers come from a shared-memory ring of kHdrRing levels,
-// filled kHdrAhead levels ahead with cp.async, so that the record loads that
-// depend on a header are issued without waiting on a global load.
-constexpr int kHdrRing = 64;
-constexpr int kHdrChunk = 16;                  // levels per refill, issued at levels l = 0 mod kHdrChunk
-constexpr int kHdrAhead = kHdrRing - kHdrChunk;  // a refill at level l brings levels [l + kHdrAhead, l + kHdrRing)
-
-// tid: this thread's edge of the level; tc, tw: its copy-in and write-back
-// (negative: none first-hand)
-__device__ __forceinline__ void win_fetch(WinRing& r, int j, int lk, int nlevels, int tid, int tc, int tw,
-                                          const int4* s_hdr, const StrainEdgeHot* __restrict__ hot,
-                                          const int2* __restrict__ load_list, const int2* __restrict__ wb_list) {
-    if (lk < nlevels) {
-        const int q = 2 * (lk % kHdrRing);
-        int4 a = s_hdr[q], b = s_hdr[q + 1];
-        r.h0[j] = a;
-        r.h1[j] = b;
-        if (a.x + tid < a.y) r.hot[j] = hot[a.x + tid];
-        if (tc >= 0 && a.z + tc < a.w) r.ld[j] = load_list[a.z + tc];
-        if (tw >= 0 && b.x + tw < b.y) r.wb[j] = wb_list[b.x + tw];
-    }
-}
-
-struct WinArgs {
-    const StrainEdge* edges;
-    const double4_32a* xo;
-    const StrainEdgeHot* hot;
-    const int4* hdr;
-    int4* s_hdr;  // the header ring
-    int nlevels;
-    const int2* load_list;
-    const int2* wb_list;
-    double4_32a* av;
-    double dt;
-    float dt32;
-    int multi_ld;  // some level has more copy-ins than the block has threads
-    // first thread of the copy-in and write-back roles; both 0 when every
-    // thread takes all three roles (edge, copy-in, write-back number tid)
-    int cbase, wbase;
-};
-
-// A thread's second and third edge records of the next level, for levels
-// wider than the block (WIDE sweeps): loaded a level early, so that they do
-// not wait on a global load inside their level.
-struct WideNext {
-    StrainEdgeHot x1, x2;
-};
-__device__ __forceinline__ void wide_fetch(WideNext& w, const int4& h, const StrainEdgeHot* __restrict__ hot,
-                                           int tid) {
-    const int e1 = h.x + tid + (int)blockDim.x, e2 = e1 + (int)blockDim.x;
-    if (e1 < h.y) w.x1 = hot[e1];
-    if (e2 < h.y) w.x2 = hot[e2];
-}
-
-// One level of the window sweep; J = level mod kWindowAhead.
-template <int J, bool WIDE>
-__device__ __forceinline__ void win_level(const WinArgs& A, WinRing& r, WideNext& wn, WinSlot* s_win, int l, int tid,
-                                          int* n_avg, int* n_exact, bool* has) {
-    constexpr int R = J % kRing;
-    const int4 h0 = r.h0[R], h1 = r.h1[R];
-    const StrainEdgeHot cur = r.hot[R];
-    const int2 ld = r.ld[R], wb = r.wb[R];
-    const int tc = tid - A.cbase, tw = tid - A.wbase;
-    StrainEdgeHot c1, c2;
-    if (WIDE) {
-        c1 = wn.x1;
-        c2 = wn.x2;
-        if (l + 1 < A.nlevels) wide_fetch(wn, r.h0[(J + 1) % kRing], A.hot, tid);
-    }
-    win_fetch(r, R, l + kRing, A.nlevels, tid, tc, tw, A.s_hdr, A.hot, A.load_list, A.wb_list);
-    if (J % kHdrChunk == 0 && l % kHdrChunk == 0 && l > 0) {
-        // headers of levels [l + kHdrAhead, l + kHdrRing) into the slots of
-        // levels [l - kHdrChunk, l), whose records were fetched kRing levels
-        // early and a barrier ago; they land in this level's copy group
-        const int m = l + kHdrAhead + (tid >> 1);
-        if (tid < 2 * kHdrChunk && m < A.nlevels)
-            cp_async16(&A.s_hdr[2 * (m % kHdrRing) + (tid & 1)], &A.hdr[2 * m + (tid & 1)]);
-    }
-    // copy in the points whose slot opens now
-    int my_slot = -1;
-    if (tc >= 0 && h0.z + tc < h0.w) {
-        my_slot = ld.y;
-        cp_async16(&s_win[ld.y].a, &A.av[ld.x]);
-        cp_async16(&s_win[ld.y].b, reinterpret_cast<const double2*>(&A.av[ld.x]) + 1);
-        for (int i = h0.z + tc + (int)blockDim.x; i < h0.w; i += blockDim.x) {
-            int2 ps = A.load_list[i];
-            cp_async16(&s_win[ps.y].a, &A.av[ps.x]);
-            cp_async16(&s_win[ps.y].b, reinterpret_cast<const double2*>(&A.av[ps.x]) + 1);
-        }
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-    // FP32 copies of the points whose copy has now landed (each by the thread
-    // that issued it): all of level 0's at once, then those issued
-    // kWindowAhead levels ago, before their first edge
-    const int old_slot = r.lslot[J];
-    r.lslot[J] = my_slot;
-    int cl = -1, cslot = -1;
-    if (l == 0) {
-        asm volatile("cp.async.wait_group 0;\n" ::);
-        cl = 0;
-        cslot = my_slot;
-    } else if (l < kWindowAhead) {
-        asm volatile("cp.async.wait_group 0;\n" ::);
-    } else {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(kWindowAhead));
-        if (l - kWindowAhead >= 1) {
-            cl = l - kWindowAhead;
-            cslot = old_slot;
-        }
-    }
-    if (cl >= 0 && cslot >= 0) {
-        WinSlot& w = s_win[cslot];
-        w.f = make_float4((float)w.a.x, (float)w.a.y, (float)w.b.x, 0.f);
-        if (A.multi_ld) {  // the copy-ins past the first per thread (a dependent load: only when needed)
-            int4 hc = A.hdr[2 * cl];
-            for (int i = hc.z + tc + (int)blockDim.x; i < hc.w; i += blockDim.x) {
-                WinSlot& w2 = s_win[A.load_list[i].y];
-                w2.f = make_float4((float)w2.a.x, (float)w2.a.y, (float)w2.b.x, 0.f);
-            }
-        }
-    }
-    __syncthreads();
-    // write back the points last used at the previous level
-    if (tw >= 0 && h1.x + tw < h1.y) {
-        double2 a = s_win[wb.y].a, b = s_win[wb.y].b;
-        A.av[wb.x] = make_double4_32a(a.x, a.y, b.x, 0.0);
-        for (int i = h1.x + tw + (int)blockDim.x; i < h1.y; i += blockDim.x) {
-            int2 ps = A.wb_list[i];
-            double2 a2 = s_win[ps.y].a, b2 = s_win[ps.y].b;
-            A.av[ps.x] = make_double4_32a(a2.x, a2.y, b2.x, 0.0);
-        }
-    }
-    const int bd = (int)blockDim.x;
-    int e = h0.x + tid;
-    if (e < h0.y) {
-        strain_window_edge(cur, e, A.edges, A.xo, s_win, A.dt32, A.dt, n_avg, n_exact, has);
-        if (WIDE) {
-            if (e + bd < h0.y) strain_window_edge(c1, e + bd, A.edges, A.xo, s_win, A.dt32, A.dt, n_avg, n_exact, has);
-            if (e + 2 * bd < h0.y)
-                strain_window_edge(c2, e + 2 * bd, A.edges, A.xo, s_win, A.dt32, A.dt, n_avg, n_exact, has);
-            e += 2 * bd;
-        }
-        for (e += bd; e < h0.y; e += bd)
-            strain_window_edge(A.hot[e], e, A.edges, A.xo, s_win, A.dt32, A.dt, n_avg, n_exact, has);
-    }
-}
-
-// WIDE: levels up to three times the block's width take their second and
-// third edges from registers loaded a level early (WideNext).
-template <bool WIDE>
-__global__ void __launch_bounds__(256) k_strain_window(const StrainEdge* __restrict__ edges,
-                                                       const double4_32a* __restrict__ xo,
-                                                       const StrainEdgeHot* __restrict__ hot,
-                                                       const int4* __restrict__ hdr_all,
-                                                       const SceneDev* __restrict__ scenes, int slot_cap,
-                                                       const int2* __restrict__ load_list,
-                                                       const int2* __restrict__ wb_list,
-                                                       double4_32a* av, int pass, int* flags,
-                                                       int* passes_out_all, int multi_ld,
-                                                       const int* __restrict__ order, int cbase, int wbase) {
-    extern __shared__ WinSlot s_win[];
-    const int sc = order[blockIdx.x];
-    const SceneDev& sd = scenes[sc];
-    if (sd.strain_slots > slot_cap || !sd.enabled) return;  // k_strain's, or left out
-    if (!sweep_gate(pass, sc, flags, passes_out_all)) return;
-    const int4* hdr = hdr_all + 2 * sd.strain_hdr0;
-    const int nlevels = sd.strain_levels;
-    const int2 wb_final = make_int2(sd.wb_final0, sd.wb_final1);
-    const double dt = sd.p.dt;
-    const int tid = threadIdx.x;
-    __shared__ int4 s_hdr[2 * kHdrRing];
-    for (int i = tid; i < 2 * kHdrRing && i < 2 * nlevels; i += blockDim.x) s_hdr[i] = hdr[i];
-    __syncthreads();
-    WinArgs A{edges, xo, hot, hdr, s_hdr, nlevels, load_list, wb_list, av, dt, __double2float_ru(dt), multi_ld,
-              cbase, wbase};
-    int n_avg = 0, n_exact = 0;
-    bool has = false;
-    WinRing r;
-#pragma unroll
-    for (int j = 0; j < kWindowAhead; ++j) r.lslot[j] = -1;
-#pragma unroll
-    for (int j = 0; j < kRing; ++j)
-        win_fetch(r, j, j, nlevels, tid, tid - cbase, tid - wbase, s_hdr, hot, load_list, wb_list);
-    WideNext wn;
-    if (WIDE && nlevels > 0) wide_fetch(wn, r.h0[0], hot, tid);
-    for (int lb = 0; lb < nlevels; lb += kWindowAhead) {
-        win_level<0, WIDE>(A, r, wn, s_win, lb + 0, tid, &n_avg, &n_exact, &has);
-        if (lb + 1 < nlevels) win_level<1, WIDE>(A, r, wn, s_win, lb + 1, tid, &n_avg, &n_exact, &has);
-        if (lb + 2 < nlevels) win_level<2, WIDE>(A, r, wn, s_win, lb + 2, tid, &n_avg, &n_exact, &has);
-        if (lb + 3 < nlevels) win_level<3, WIDE>(A, r, wn, s_win, lb + 3, tid, &n_avg, &n_exact, &has);
-        if (lb + 4 < nlevels) win_level<4, WIDE>(A, r, wn, s_win, lb + 4, tid, &n_avg, &n_exact, &has);
-        if (lb + 5 < nlevels) win_level<5, WIDE>(A, r, wn, s_win, lb + 5, tid, &n_avg, &n_exact, &has);
-        if (lb + 6 < nlevels) win_level<6, WIDE>(A, r, wn, s_win, lb + 6, tid, &n_avg, &n_exact, &has);
-        if (lb + 7 < nlevels) win_level<7, WIDE>(A, r, wn, s_win, lb + 7, tid, &n_avg, &n_exact, &has);
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();
-    for (int i = wb_final.x + tid; i < wb_final.y; i += blockDim.x) {
-        int2 ps = wb_list[i];
-        double2 a = s_win[ps.y].a, b = s_win[ps.y].b;
-        av[ps.x] = make_double4_32a(a.x, a.y, b.x, 0.0);
-    }
-    sweep_done(pass, sc, n_avg, n_exact, flags, passes_out_all);
-}
-
-// The sweep of one scene by a single warp. The block barrier of
-// k_strain_window costs most of a level there; here a level needs only
-// __syncwarp. Each level's edge records and its copy-in and write-back
-// lists are staged into a shared-memory ring kWarpAhead levels ahead with
-// cp.async, and velocities are copied into their slots (the same interval
-// schedule) kWindowAhead levels before their first edge, so a level touches
-// only shared memory. Slots hold the FP64 velocities; the FP32 values of the
-// first decision are converted from them as needed.
-constexpr int kWarpAhead = kWindowAhead;   // the copy-in distance of the schedule
-constexpr int kWarpRing = kWarpAhead + 1;  // level L+K goes where level L-1 was
-
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
-}
-
-struct WarpSlot {
-    double2 a, b;  // x y | z -
-};
-
-__global__ void __launch_bounds__(32) k_strain_warp(const StrainEdge* __restrict__ edges,
-                                                    const double4_32a* __restrict__ xo,
-                                                    const StrainEdgeHot* __restrict__ hot,
-                                                    const int4* __restrict__ hdr_all,
-                                                    const SceneDev* __restrict__ scenes, int slot_cap,
-                                                    const int2* __restrict__ load_list,
-                                                    const int2* __restrict__ wb_list, double4_32a* av, int pass,
-                                                    int* flags, int* passes_out_all, int max_slots, int ecap,
-                                                    int lcap, int wcap, const int* __restrict__ order) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int sc = order[blockIdx.x];
-    const SceneDev& sd = scenes[sc];
-    if (sd.strain_slots > slot_cap || !sd.enabled) return;  // k_strain's, or left out
-    if (!sweep_gate(pass, sc, flags, passes_out_all)) return;
-    WarpSlot* s_win = reinterpret_cast<WarpSlot*>(smem_raw);
-    size_t off = (size_t)max_slots * sizeof(WarpSlot);
-    StrainEdgeHot* s_hot = reinterpret_cast<StrainEdgeHot*>(smem_raw + off);
-    off += (size_t)kWarpRing * ecap * sizeof(StrainEdgeHot);
-    int2* s_ld = reinterpret_cast<int2*>(smem_raw + off);
-    off += (size_t)kWarpRing * lcap * 8;
-    int2* s_wb = reinterpret_cast<int2*>(smem_raw + off);
-    off += (size_t)kWarpRing * wcap * 8;
-    off = (off + 15) & ~(size_t)15;  // the headers are int4
-    int4* s_h = reinterpret_cast<int4*>(smem_raw + off);
-    const int lane = threadIdx.x;
-    const int4* hdr = hdr_all + 2 * sd.strain_hdr0;
-    const int nlevels = sd.strain_levels;
-    const double dt = sd.p.dt;
-    const float dt32 = __double2float_ru(dt);
-    // level L's records and lists into ring slot L % kWarpRing
-    auto stage = [&](int L) {
-        if (L >= nlevels) return;
-        const int r = L % kWarpRing;
-        const int4 h0 = hdr[2 * L], h1 = hdr[2 * L + 1];
-        if (lane == 0) {
-            s_h[2 * r] = h0;
-            s_h[2 * r + 1] = h1;
-        }
-        const float4* src = reinterpret_cast<const float4*>(hot + h0.x);
-        float4* dst = reinterpret_cast<float4*>(s_hot + (size_t)r * ecap);
-        const int nchunk = 3 * (h0.y - h0.x);  // 48-byte records, three 16-byte chunks each
-        for (int c = lane; c < nchunk; c += 32) cp_async16(dst + c, src + c);
-        for (int c = lane; c < h0.w - h0.z; c += 32) cp_async8(s_ld + (size_t)r * lcap + c, load_list + h0.z + c);
-        for (int c = lane; c < h1.y - h1.x; c += 32) cp_async8(s_wb + (size_t)r * wcap + c, wb_list + h1.x + c);
-    };
-    for (int L = 0; L < kWarpAhead; ++L) {
-        stage(L);
-        asm volatile("cp.async.commit_group;\n" ::);
-    }
-    int n_avg = 0, n_exact = 0;
-    for (int L = 0; L < nlevels; ++L) {
-        // level L's stage: the (L+1)-th group committed
-        if (L < kWarpAhead)
-            asm volatile("cp.async.wait_group 0;\n" ::);
-        else
-            asm volatile("cp.async.wait_group %0;\n" ::"n"(kWarpAhead - 1));
-        __syncwarp();
-        const int r = L % kWarpRing;
-        const int4 h0 = s_h[2 * r], h1 = s_h[2 * r + 1];
-        // velocities whose slots open now (first used kWindowAhead levels on)
-        for (int c = lane; c < h0.w - h0.z; c += 32) {
-            const int2 ps = s_ld[(size_t)r * lcap + c];
-            cp_async16(&s_win[ps.y].a, &av[ps.x]);
-            cp_async16(&s_win[ps.y].b, reinterpret_cast<const double2*>(&av[ps.x]) + 1);
-        }
-        stage(L + kWarpAhead);
-        asm volatile("cp.async.commit_group;\n" ::);
-        if (L < kWarpAhead) asm volatile("cp.async.wait_group 0;\n" ::);  // first levels use them at once
-        __syncwarp();
-        // write back the points last used at the previous level
-        for (int c = lane; c < h1.y - h1.x; c += 32) {
-            const int2 ps = s_wb[(size_t)r * wcap + c];
-            const double2 a = s_win[ps.y].a, b = s_win[ps.y].b;
-            av[ps.x] = make_double4_32a(a.x, a.y, b.x, 0.0);
-        }
-        for (int i = lane; i < h0.y - h0.x; i += 32) {
-            const StrainEdgeHot h = s_hot[(size_t)r * ecap + i];
-            WarpSlot& w0 = s_win[h.s0];
-            WarpSlot& w1 = s_win[h.s1];
-            const double2 a0 = w0.a, a1 = w0.b, b0 = w1.a, b1 = w1.b;
-            int q = strain_decide32(h, make_float4((float)a0.x, (float)a0.y, (float)a1.x, 0.f),
-                                    make_float4((float)b0.x, (float)b0.y, (float)b1.x, 0.f), dt32);
-            if (q == 0) continue;
-            double v0[3] = {a0.x, a0.y, a1.x}, v1[3] = {b0.x, b0.y, b1.x};
-            if (q < 0 && !strain_flag_vals(strain_step(edges[h0.x + i], xo), v0, v1, dt, &n_exact)) continue;
-            ++n_avg;
-            double t[3];
-            for (int k = 0; k < 3; ++k) {
-                t[k] = v0[k] + v1[k];
-                t[k] = half_of(t[k]);
-            }
-            const double2 na = make_double2(t[0], t[1]), nb = make_double2(t[2], 0.0);
-            w0.a = na; w0.b = nb;
-            w1.a = na; w1.b = nb;
-        }
-        __syncwarp();
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncwarp();
-    for (int i = sd.wb_final0 + lane; i < sd.wb_final1; i += 32) {
-        const int2 ps = wb_list[i];
-        const double2 a = s_win[ps.y].a, b = s_win[ps.y].b;
-        av[ps.x] = make_double4_32a(a.x, a.y, b.x, 0.0);
-    }
-    sweep_done(pass, sc, n_avg, n_exact, flags, passes_out_all);
-}
-
-// Would any edge of the chunk average on the current velocities? (A block
-// per chunk of at most 256 edges of one scene, the grid striding over the
-// chunks; chunks of finished scenes, or of scenes where an averaging edge is
-// already found, are skipped.) If none of a scene's
-// edges would, its sweep changes nothing: before the first edge that
-// averages every edge sees the start-of-pass velocities.
-__global__ void __launch_bounds__(256) k_strain_check(const StrainEdge* __restrict__ edges,
-                                                      const double4_32a* __restrict__ xo,
-                                                      const StrainEdgeHot* __restrict__ hot,
-                                                      const int2* __restrict__ chunks, int nchunks,
-                                                      const SceneDev* __restrict__ scenes,
-                                                      const double4_32a* __restrict__ av, int* flags) {
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const int2 ch = chunks[c];  // (scene, first edge)
-        const SceneDev& sd = scenes[ch.x];
-        // done scenes, and scenes where an edge that averages is already found
-        if (!sd.enabled || flags[2 * ch.x + 1] || *(volatile int*)&flags[2 * ch.x]) continue;
-        const int end = sd.strain_e0 + sd.strain_ne;
-        const int e = ch.y + threadIdx.x;
-        if (e >= end) continue;
-        const StrainEdgeHot h = hot[e];
-        const int2 pp = *reinterpret_cast<const int2*>(&edges[e]);  // p0, p1
-        const double4_32a a0 = av[pp.x], a1 = av[pp.y];
-        const float dt32 = __double2float_ru(sd.p.dt);
-        int q = strain_decide32(h, make_float4((float)a0.x, (float)a0.y, (float)a0.z, 0.f),
-                                make_float4((float)a1.x, (float)a1.y, (float)a1.z, 0.f), dt32);
-        if (q < 0) {
-            double v0[3] = {a0.x, a0.y, a0.z}, v1[3] = {a1.x, a1.y, a1.z};
-            int n_exact = 0;
-            q = strain_flag_vals(strain_step(edges[e], xo), v0, v1, sd.p.dt, &n_exact) ? 1 : 0;
-        }
-        if (q > 0 && !flags[2 * ch.x]) atomicOr(&flags[2 * ch.x], 1);
-    }
-}
-
-// Start of a strain loop for the scenes in mask (all: mask null): their
-// flags and counters cleared; the others marked finished, so that every
-// kernel of this loop leaves them and their counters alone.
-__global__ void k_strain_init(const uint8_t* __restrict__ mask, int nscenes, int* flags, int* passes_out) {
-    int sc = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sc >= nscenes) return;
-    if (mask && !mask[sc]) {
-        flags[2 * sc + 1] = 1;
-        return;
-    }
-    flags[2 * sc] = flags[2 * sc + 1] = 0;
-    passes_out[3 * sc] = passes_out[3 * sc + 1] = passes_out[3 * sc + 2] = 0;
-}
-
 __global__ void k_final_velocity(const uint8_t* __restrict__ in_elem, const uint8_t* __restrict__ has_collsn,
                                  const double4_32a* __restrict__ av, const int* __restrict__ vscene,
                                  const SceneDev* __restrict__ scenes, double* vel, int nv,
@@ -1338,12 +566,6 @@ __global__ void k_final_rg(const int* __restrict__ visit, const int* __restrict_
 }
 
 }  // namespace
-
-size_t strain_warp_smem(int max_slots, int ecap, int lcap, int wcap) {
-    size_t b = (size_t)max_slots * sizeof(WarpSlot) +
-               (size_t)kWarpRing * ((size_t)ecap * sizeof(StrainEdgeHot) + (size_t)lcap * 8 + (size_t)wcap * 8);
-    return ((b + 15) & ~(size_t)15) + (size_t)kWarpRing * 32;
-}
 
 void math_selftest(int fn, const double* a, const double* b, double* out, int n, cudaStream_t s) {
     if (n > 0) count_launch(), k_math_selftest<<<nblk(n, 128), 128, 0, s>>>(fn, a, b, out, n);
@@ -1419,61 +641,6 @@ void finalize_positions(const uint8_t* in_elem, const double4_32a* xo, double4_3
     if (nv > 0)
         count_launch(), k_finalize<<<nblk(nv, 256), 256, 0, s>>>(in_elem, xo, av, has_collsn, x_cand, x_out, nv,
                                                                  vscene, scenes, fixed, mask);
-}
-
-size_t strain_step_bytes(int nedges) {
-    size_t n = (size_t)(nedges > 0 ? nedges : 1);
-    return sizeof(StrainEdgeStep) * n + sizeof(StrainEdgeHot) * n;
-}
-
-int strain_window_slot_cap() { return (int)(kStrainWindowBytes / sizeof(WinSlot)); }
-
-void strain_configure() {
-    cudaFuncSetAttribute(k_strain_window<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStrainWindowBytes);
-    cudaFuncSetAttribute(k_strain_window<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStrainWindowBytes);
-    cudaFuncSetAttribute(k_strain_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStrainWarpBytes);
-}
-
-void strain_setup(const StrainEdge* edges, int nedges, const SceneDev* scenes, const StrainPlan& plan,
-                  const double4_32a* xo, void* step_buf, const int* vscene, cudaStream_t s) {
-    if (nedges <= 0) return;
-    StrainEdgeStep* se = (StrainEdgeStep*)step_buf;
-    StrainEdgeHot* hot = (StrainEdgeHot*)(se + nedges);
-    const int cap = plan.window ? strain_window_slot_cap() : -1;
-    count_launch(), k_strain_setup<<<nblk(nedges, 256), 256, 0, s>>>(edges, nedges, xo, se, hot, vscene, scenes, cap);
-}
-
-void strain_limit(const StrainEdge* edges, int nedges, const int4* hdr, const int2* load_list, const int2* wb_list,
-                  const int2* chunks, int nchunks, const SceneDev* scenes, int nscenes, const StrainPlan& plan,
-                  const double4_32a* xo, double4_32a* av, void* step_buf, int* flags, int* passes_out,
-                  const uint8_t* mask, cudaStream_t s) {
-    if (nscenes <= 0) return;
-    StrainEdgeStep* se = (StrainEdgeStep*)step_buf;
-    StrainEdgeHot* hot = (StrainEdgeHot*)(se + (nedges > 0 ? nedges : 1));
-    count_launch(), k_strain_init<<<nblk(nscenes, 128), 128, 0, s>>>(mask, nscenes, flags, passes_out);
-    // scenes with at most `cap` slots are swept in shared memory (cap -1: none)
-    int cap = plan.window ? strain_window_slot_cap() : -1;
-    size_t smem = (size_t)plan.max_window_slots * sizeof(WinSlot);
-    for (int pass = 0; pass < kStrainMaxIter; ++pass) {
-        if (nchunks > 0)
-            count_launch(), k_strain_check<<<nchunks < 152 * 8 ? nchunks : 152 * 8, 256, 0, s>>>(
-                edges, xo, hot, chunks, nchunks, scenes, av, flags);
-        if (plan.window && plan.warp)
-            count_launch(), k_strain_warp<<<nscenes, 32, plan.warp_smem, s>>>(
-                edges, xo, hot, hdr, scenes, cap, load_list, wb_list, av, pass, flags, passes_out, plan.max_window_slots,
-                plan.ecap, plan.lcap, plan.wcap, plan.order);
-        else if (plan.window && plan.ecap > plan.block)
-            count_launch(), k_strain_window<true><<<nscenes, plan.block, smem, s>>>(
-                edges, xo, hot, hdr, scenes, cap, load_list, wb_list, av, pass, flags, passes_out, plan.lcap > plan.block,
-                plan.order, plan.cbase, plan.wbase);
-        else if (plan.window)
-            count_launch(), k_strain_window<false><<<nscenes, plan.block, smem, s>>>(
-                edges, xo, hot, hdr, scenes, cap, load_list, wb_list, av, pass, flags, passes_out, plan.lcap > plan.block,
-                plan.order, plan.cbase, plan.wbase);
-        if (!plan.window || plan.any_global)
-            count_launch(), k_strain<<<nscenes, 256, 0, s>>>(se, hdr, scenes, cap, av, pass, flags, passes_out,
-                                                             plan.order);
-    }
 }
 
 void final_velocity(const uint8_t* in_elem, const uint8_t* has_collsn, const double4_32a* av, const int* vscene,

@@ -26,6 +26,7 @@
 
 #include "cc_launch.h"
 #include "cc_strain_plan.h"
+#include "cc_sweep_plan.h"
 #include "cc_tree_order.h"
 #include "cc_vtk.h"
 
@@ -135,7 +136,6 @@ struct SceneHost {
     bool built[2] = {false, false};
     double volume = 0.0;  // shared by both trees (dcollid.cpp:381, 422)
     int strain_edges = 0, strain_points = 0;
-    int strain_caps[3] = {0, 0, 0};
     bool enabled = true;
     int status = CC_OK;  // of the last resolve call
     int state = kHsDone;
@@ -169,17 +169,21 @@ struct cc_solver {
     uint8_t* d_erigid = nullptr;
     uint8_t* d_fixed = nullptr;
     uint8_t* d_in_elem = nullptr;
+    // strain limiting: the elements and their sweep schedules, and, once a
+    // step needs k_strain, its edge schedule (ensure_edge_schedule)
+    std::vector<SweepElem> h_strain_elems;  // in the reference's order, by scene
+    std::vector<int> h_strain_first;        // each scene's first, and the end
+    SweepElem* d_sw_elems = nullptr;
+    int *d_sw_lev = nullptr, *d_sw_need = nullptr, *d_sw_state = nullptr;
+    int4* d_sw_epoch = nullptr;
+    int2 *d_sw_load = nullptr, *d_sw_wb = nullptr, *d_strain_chunks = nullptr;
+    char *d_sw_recs = nullptr, *d_edge_steps = nullptr;
     StrainEdge* d_edges = nullptr;
-    int nedges = 0;
     int4* d_strain_hdr = nullptr;
-    int2* d_strain_load = nullptr;
-    int2* d_strain_wb = nullptr;
-    void* d_strain_step = nullptr;
     int* d_strain_passes = nullptr;  // 3 per scene
     int* d_strain_flags = nullptr;   // 2 per scene
-    int2* d_strain_chunks = nullptr; // (scene, first edge) per run of <= 256 edges
-    int* d_strain_order = nullptr;   // scenes by strain levels, most first (one sweep CTA each)
-    int n_strain_chunks = 0;
+    int* d_strain_order = nullptr;   // scenes by strain levels, most first
+    StrainBufs strain_bufs;
     std::vector<int> h_strain_passes;
 
     // state
@@ -432,8 +436,8 @@ struct cc_solver {
     int mode = 0;  // 0 plain FP64, 1 mixed precision
     bool strain_window = true;
     bool split_narrow = true;  // two-stage narrow phase for mixed passes
-    bool strain_warp = false;  // one-warp strain sweep with staged levels
-    bool strain_roles = true;  // window sweep: edges, copy-ins and write-backs on separate threads
+    bool strain_warp = false;  // a sweep CTA's elements on one warp
+    bool strain_roles = true;  // CC_TUNE_STRAIN_ROLES, without effect
     LaunchTuning tune;
     int host_threads = 0;  // tree emulation threads (0: hardware concurrency)
     const bool pass_log = std::getenv("CC_PASS_LOG") != nullptr;
@@ -482,11 +486,13 @@ struct cc_solver {
     void release_mesh() {
         clear_tail_graphs();
         dfree(d_ev); dfree(d_esurf); dfree(d_erigid); dfree(d_fixed); dfree(d_in_elem); dfree(d_edges);
-        dfree(d_strain_hdr); dfree(d_strain_load); dfree(d_strain_wb); dfree(d_strain_passes);
+        dfree(d_strain_hdr); dfree(d_edge_steps); dfree(d_strain_passes);
         dfree(d_strain_flags); dfree(d_strain_chunks); dfree(d_strain_order);
-        n_strain_chunks = 0;
-        if (d_strain_step) cudaFree(d_strain_step);
-        d_strain_step = nullptr;
+        dfree(d_sw_elems); dfree(d_sw_lev); dfree(d_sw_need); dfree(d_sw_state); dfree(d_sw_epoch);
+        dfree(d_sw_load); dfree(d_sw_wb); dfree(d_sw_recs);
+        strain_bufs = StrainBufs{};
+        h_strain_elems.clear();
+        h_strain_first.clear();
         dfree(d_scenes); dfree(d_run); dfree(d_vscene); dfree(d_escene); dfree(d_tail_mask);
         if (h_tail_masks) cudaFreeHost(h_tail_masks);
         h_tail_masks = nullptr;
@@ -550,7 +556,7 @@ struct cc_solver {
         h_sel = nullptr;
         sel_prev.clear();
         pair_cap = contrib_cap = rec_cap = 0;
-        nv = ne = nedges = 0;
+        nv = ne = 0;
         nscenes = 0;
         scenes.clear();
         h_scenes.clear();
@@ -749,9 +755,7 @@ struct cc_solver {
     void tail(const double* x_cand, double* x_out, double* vel) {
         finalize_positions(d_in_elem, d_xo, d_av, d_hc, x_cand, x_out, nv, d_vscene, d_scenes, d_fixed, d_tail_mask,
                            tail_stream);
-        strain_limit(d_edges, nedges, d_strain_hdr, d_strain_load, d_strain_wb, d_strain_chunks, n_strain_chunks,
-                     d_scenes, nscenes, strain_plan(), d_xo, d_av, d_strain_step, d_strain_flags, d_strain_passes,
-                     d_tail_mask, tail_stream);
+        strain_limit(strain_bufs, d_scenes, nscenes, strain_plan(), d_xo, d_av, d_tail_mask, tail_stream);
         final_velocity(d_in_elem, d_hc, d_av, d_vscene, d_scenes, vel, nv, d_tail_mask, tail_stream);
     }
     // Tail streams: the ends of steps of the scenes that have finished their
@@ -800,7 +804,7 @@ struct cc_solver {
     // strain settings, then replayed.
     struct TailGraph {
         const void* key[4];
-        int block, window, warp, roles;
+        int block, window, warp;
         cudaGraphExec_t exec;
         long long launches;
     };
@@ -815,7 +819,7 @@ struct cc_solver {
         TailGraph* hit = nullptr;
         for (auto& g : tail_graphs)
             if (std::equal(key, key + 4, g.key) && g.block == tune.strain_block && g.window == (int)strain_window &&
-                g.warp == (int)strain_warp && g.roles == (int)strain_roles) {
+                g.warp == (int)strain_warp) {
                 hit = &g;
                 break;
             }
@@ -838,7 +842,6 @@ struct cc_solver {
             tg.block = tune.strain_block;
             tg.window = (int)strain_window;
             tg.warp = (int)strain_warp;
-            tg.roles = (int)strain_roles;
             tg.launches = n;
             e = cudaGraphInstantiate(&tg.exec, g, 0);
             cudaGraphDestroy(g);
@@ -900,32 +903,51 @@ struct cc_solver {
     }
 
     StrainPlan strain_plan() const {
-        StrainPlan pl{strain_window, 0, false, tune.strain_block, false, 0, 0, 0, 0, d_strain_order};
-        int cap = strain_window_slot_cap();
+        StrainPlan pl{strain_window, false, 1, 0};
+        int width = 1;
         for (int s = 0; s < nscenes; ++s) {
             const SceneDev& sd = h_scenes[s];
-            if (strain_window && sd.strain_slots <= cap) {
-                pl.max_window_slots = std::max(pl.max_window_slots, sd.strain_slots);
-                pl.ecap = std::max(pl.ecap, scenes[s].strain_caps[0]);
-                pl.lcap = std::max(pl.lcap, scenes[s].strain_caps[1]);
-                pl.wcap = std::max(pl.wcap, scenes[s].strain_caps[2]);
+            if (strain_window && sd.sw_fits) {
+                pl.smem = std::max(pl.smem, sweep_smem(sd.sw_slots, sd.sw_width, sd.sw_ring));
+                width = std::max(width, sd.sw_width);
             } else {
                 pl.any_global = true;
             }
         }
-        pl.warp_smem = strain_warp_smem(pl.max_window_slots, pl.ecap, pl.lcap, pl.wcap);
-        // separate threads for a level's edges, copy-ins and write-backs,
-        // each role from a warp boundary, where they fit in the block
-        pl.cbase = pl.wbase = 0;
-        if (strain_roles) {
-            const int cb = (pl.ecap + 31) / 32 * 32, wb = cb + (pl.lcap + 31) / 32 * 32;
-            if (pl.ecap > 0 && wb + pl.wcap <= pl.block) {
-                pl.cbase = cb;
-                pl.wbase = wb;
-            }
-        }
-        pl.warp = strain_window && strain_warp && pl.warp_smem <= 200 * 1024;
+        pl.workers = strain_warp ? 1 : std::min((width + 7) / 8, tune.strain_block / 16);
         return pl;
+    }
+    // The edge schedule of k_strain, built when a step first needs it (a
+    // scene too large for the shared-memory sweeps, or those turned off).
+    cc_status ensure_edge_schedule() {
+        if (d_edges || h_strain_elems.empty() || !strain_plan().any_global) return CC_OK;
+        std::vector<StrainEdge> all;
+        std::vector<int4> hdr;
+        std::vector<int2> load, wb;
+        for (int s = 0; s < nscenes; ++s) {
+            std::vector<StrainEdge> edges;
+            for (int i = h_strain_first[s]; i < h_strain_first[s + 1]; ++i) {
+                const SweepElem& el = h_strain_elems[i];
+                const int n = el.np() == 2 ? 1 : 3;
+                for (int j = 0; j < n; ++j)
+                    edges.push_back(StrainEdge{el.p[j], el.p[(j + 1) % 3], el.len0[j], 0, 0});
+            }
+            int caps[3];
+            append_strain_schedule(edges, scenes[s].v0, scenes[s].nv, all, hdr, load, wb, h_scenes[s], caps);
+        }
+        if (dalloc(&d_edges, all.size()) != cudaSuccess || dalloc(&d_strain_hdr, hdr.size()) != cudaSuccess ||
+            dalloc(&d_edge_steps, strain_edge_step_bytes((int)all.size())) != cudaSuccess)
+            return fail(CC_NO_MEMORY, "strain edge schedule");
+        cudaMemcpyAsync(d_edges, all.data(), sizeof(StrainEdge) * all.size(), cudaMemcpyHostToDevice, stream);
+        cudaMemcpyAsync(d_strain_hdr, hdr.data(), sizeof(int4) * hdr.size(), cudaMemcpyHostToDevice, stream);
+        strain_bufs.edges = d_edges;
+        strain_bufs.nedges = (int)all.size();
+        strain_bufs.hdr = d_strain_hdr;
+        strain_bufs.edge_steps = d_edge_steps;
+        scenes_dirty = true;  // strain_hdr0, strain_levels
+        clear_tail_graphs();
+        cudaStreamSynchronize(stream);  // the vectors are pageable
+        return cuda_check("strain edge schedule");
     }
     void set_scene_params(int i, const cc_params& p) {
         h_scenes[i].p = Params{p.dt, p.thickness, p.eps, p.k, p.m, p.lambda, p.cr};
@@ -981,9 +1003,8 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     h_scenes.assign((size_t)n, SceneDev{});
     std::vector<int> ev((size_t)ne * 3, -1), esurf((size_t)ne, -1), vscene((size_t)nv), escene((size_t)ne);
     std::vector<uint8_t> fixed((size_t)nv, 0), in_elem((size_t)nv, 0), erigid((size_t)ne, 0);
-    std::vector<StrainEdge> all_edges;
-    std::vector<int4> hdr;
-    std::vector<int2> load, wb, chunks;
+    SweepArrays sweep;
+    std::vector<int2> chunks;
     int v0 = 0, e0 = 0;
     for (int si = 0; si < n; ++si) {
         const cc_mesh* m = &meshes[si];
@@ -1022,8 +1043,8 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
                 ev[3 * (size_t)(e0 + nt + b) + k] = v0 + v;
             }
         }
-        std::vector<StrainEdge> edges;
-        edges.reserve((size_t)3 * nt + nb);
+        std::vector<SweepElem> elems;
+        elems.reserve((size_t)sne);
         for (int e = 0; e < sne; ++e) {
             const int* E = &ev[3 * (size_t)(e0 + e)];
             int np = e < nt ? 3 : 2;
@@ -1035,24 +1056,23 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
             }
             erigid[e0 + e] = rigid ? 1 : 0;
             if (rigid) continue;  // isRigidBody(hse), dcollid.cpp:495
-            if (np == 3) {
-                for (int j = 0; j < 3; ++j)
-                    edges.push_back(StrainEdge{E[j], E[(j + 1) % 3], m->tri_rest_len[3 * e + j], 0, 0});
-            } else {
-                edges.push_back(StrainEdge{E[0], E[1], m->bond_rest_len[e - nt], 0, 0});
+            SweepElem el{};
+            for (int j = 0; j < 3; ++j) {
+                el.p[j] = E[j < np ? j : 0];
+                el.len0[j] = np == 3 ? m->tri_rest_len[3 * e + j] : m->bond_rest_len[e - nt];
             }
+            el.s2n = (np == 3 ? 3u : 1u) << 16;
+            elems.push_back(el);
+            sh.strain_edges += np == 3 ? 3 : 1;
         }
-        size_t nload = load.size();
-        sd.strain_e0 = (int)all_edges.size();
-        sd.strain_ne = (int)edges.size();
-        for (int c = 0; c < sd.strain_ne; c += 256) chunks.push_back(int2{si, sd.strain_e0 + c});
-        append_strain_schedule(edges, v0, snv, all_edges, hdr, load, wb, sd, sh.strain_caps);
-        sh.strain_edges = (int)edges.size();
-        sh.strain_points = (int)(load.size() - nload);
+        sh.strain_points = append_sweep_plan(elems, v0, snv, sweep, sd);
+        for (int c = 0; c < sd.sw_ne; c += 256) chunks.push_back(int2{si, sd.sw_e0 + c});
+        h_strain_first.push_back((int)h_strain_elems.size());
+        h_strain_elems.insert(h_strain_elems.end(), elems.begin(), elems.end());
         v0 += snv;
         e0 += sne;
     }
-    nedges = (int)all_edges.size();
+    h_strain_first.push_back((int)h_strain_elems.size());
 
     // Movable rigid bodies: a surface (run of equal tri_surface) whose first
     // point is movable (dcollid3d.cpp:62). Its points must all be movable and
@@ -1130,16 +1150,18 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     ok &= dalloc(&d_erigid, (size_t)ne) == cudaSuccess;
     ok &= dalloc(&d_fixed, (size_t)nv) == cudaSuccess;
     ok &= dalloc(&d_in_elem, (size_t)nv) == cudaSuccess;
-    ok &= dalloc(&d_edges, (size_t)nedges) == cudaSuccess;
-    ok &= dalloc(&d_strain_hdr, hdr.size()) == cudaSuccess;
-    ok &= dalloc(&d_strain_load, load.size()) == cudaSuccess;
-    ok &= dalloc(&d_strain_wb, wb.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_elems, sweep.elems.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_recs, (size_t)kSweepRecBytes * sweep.elems.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_lev, sweep.lev.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_epoch, sweep.epoch.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_need, sweep.need.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_load, sweep.load.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_wb, sweep.wb.size()) == cudaSuccess;
+    ok &= dalloc(&d_sw_state, (size_t)strain_state_ints(n)) == cudaSuccess;
     ok &= dalloc(&d_strain_passes, 3 * (size_t)n) == cudaSuccess;
     ok &= dalloc(&d_strain_flags, 2 * (size_t)n) == cudaSuccess;
     ok &= dalloc(&d_strain_chunks, chunks.size()) == cudaSuccess;
     ok &= dalloc(&d_strain_order, (size_t)n) == cudaSuccess;
-    n_strain_chunks = (int)chunks.size();
-    ok &= cudaMalloc(&d_strain_step, strain_step_bytes(nedges)) == cudaSuccess;
     ok &= dalloc(&d_xo, (size_t)nv) == cudaSuccess;
     ok &= dalloc(&d_av, (size_t)nv) == cudaSuccess;
 
@@ -1230,26 +1252,40 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     cudaMemcpyAsync(d_erigid, erigid.data(), erigid.size(), cudaMemcpyHostToDevice, stream);
     cudaMemcpyAsync(d_fixed, fixed.data(), fixed.size(), cudaMemcpyHostToDevice, stream);
     cudaMemcpyAsync(d_in_elem, in_elem.data(), in_elem.size(), cudaMemcpyHostToDevice, stream);
-    if (nedges)
-        cudaMemcpyAsync(d_edges, all_edges.data(), sizeof(StrainEdge) * all_edges.size(), cudaMemcpyHostToDevice,
-                        stream);
-    if (!hdr.empty())
-        cudaMemcpyAsync(d_strain_hdr, hdr.data(), sizeof(int4) * hdr.size(), cudaMemcpyHostToDevice, stream);
+    auto up = [&](void* d, const void* h, size_t bytes) {
+        if (bytes) cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, stream);
+    };
+    up(d_sw_elems, sweep.elems.data(), sizeof(SweepElem) * sweep.elems.size());
+    up(d_sw_lev, sweep.lev.data(), sizeof(int) * sweep.lev.size());
+    up(d_sw_epoch, sweep.epoch.data(), sizeof(int4) * sweep.epoch.size());
+    up(d_sw_need, sweep.need.data(), sizeof(int) * sweep.need.size());
+    up(d_sw_load, sweep.load.data(), sizeof(int2) * sweep.load.size());
+    up(d_sw_wb, sweep.wb.data(), sizeof(int2) * sweep.wb.size());
     if (!chunks.empty())
         cudaMemcpyAsync(d_strain_chunks, chunks.data(), sizeof(int2) * chunks.size(), cudaMemcpyHostToDevice, stream);
     {
-        // the sweep of a scene is a chain of its levels: the longest chains
-        // start first, so none waits for a second wave of CTAs
+        // the sweeps of a scene are a chain of its levels: the longest chains
+        // start first, so that none is left for a last wave of CTAs
         std::vector<int> order((size_t)n);
         for (int i = 0; i < n; ++i) order[i] = i;
         std::stable_sort(order.begin(), order.end(),
-                         [&](int a, int b) { return h_scenes[a].strain_levels > h_scenes[b].strain_levels; });
+                         [&](int a, int b) { return h_scenes[a].sw_levels > h_scenes[b].sw_levels; });
         cudaMemcpy(d_strain_order, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice);
     }
-    if (!load.empty()) {
-        cudaMemcpyAsync(d_strain_load, load.data(), sizeof(int2) * load.size(), cudaMemcpyHostToDevice, stream);
-        cudaMemcpyAsync(d_strain_wb, wb.data(), sizeof(int2) * wb.size(), cudaMemcpyHostToDevice, stream);
-    }
+    strain_bufs.elems = d_sw_elems;
+    strain_bufs.nelems = (int)sweep.elems.size();
+    strain_bufs.lev = d_sw_lev;
+    strain_bufs.epoch = d_sw_epoch;
+    strain_bufs.need = d_sw_need;
+    strain_bufs.load = d_sw_load;
+    strain_bufs.wb = d_sw_wb;
+    strain_bufs.recs = d_sw_recs;
+    strain_bufs.state = d_sw_state;
+    strain_bufs.chunks = d_strain_chunks;
+    strain_bufs.nchunks = (int)chunks.size();
+    strain_bufs.order = d_strain_order;
+    strain_bufs.flags = d_strain_flags;
+    strain_bufs.passes_out = d_strain_passes;
     cudaMemsetAsync(d_av, 0, sizeof(double4_32a) * (size_t)(nv > 0 ? nv : 1), stream);
     cudaMemsetAsync(d_run, 0, sizeof(SceneRun) * (size_t)n, stream);
     cudaMemsetAsync(d_rank[0], 0, sizeof(int) * (size_t)(ne > 0 ? ne : 1), stream);
@@ -2014,6 +2050,7 @@ cc_status cc_solver::resolve_impl(const double* x_old, const double* x_cand, dou
         cudaStreamSynchronize(stream);
         return cuda_check("empty mesh");
     }
+    if (cc_status st = ensure_edge_schedule()) return st;
     upload_scenes();
     // d_hc doubles as the device copy of has_collsn
     if (hc != d_hc) cudaMemcpyAsync(d_hc, hc, (size_t)nv, cudaMemcpyDeviceToDevice, stream);
@@ -2023,7 +2060,7 @@ cc_status cc_solver::resolve_impl(const double* x_old, const double* x_cand, dou
     prof(kStInit, true);
     step_init(x_old, x_cand, nv, d_in_elem, d_vscene, d_scenes, d_xo, d_av, d_ctr, stream);
     // the strain records depend on x_old only
-    strain_setup(d_edges, nedges, d_scenes, strain_plan(), d_xo, d_strain_step, d_vscene, stream);
+    strain_setup(strain_bufs, strain_plan(), d_xo, stream);
     tail_done.assign((size_t)nscenes, 0);
     tails_this_step = 0;
     start_zones();
@@ -2146,6 +2183,8 @@ cc_status cc_solver::resolve_impl(const double* x_old, const double* x_cand, dou
         }
         std::copy(B.com, B.com + 3, B.mrg_com);
     }
+    for (int s = 0; s < nscenes; ++s)
+        if (h_strain_passes[3 * s] < 0) return fail(CC_CUDA_ERROR, "strain sweeps gave up waiting for one another");
     for (int s = 0; s < nscenes; ++s) {
         // algorithmic bytes of the sweep: per pass, each edge's 48-byte
         // record and one 32-byte read and write of each point it touches

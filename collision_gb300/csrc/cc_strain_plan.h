@@ -1,5 +1,6 @@
-// Strain-limiting schedule of one scene: dependency levels of its edges and
-// the shared-memory slots of its points (host side of the window sweep).
+// Strain-limiting schedule of one scene by edges (host side): the dependency
+// levels that k_strain follows on global memory (cc_strain.cu), with a slot,
+// a copy-in and a write-back per point for a sweep that holds them closer.
 #pragma once
 
 #include <vector>
@@ -8,8 +9,7 @@
 
 namespace ccg {
 
-// Copy-ins run this many levels before a point's first edge (kWindowAhead of
-// the window sweep in cc_post.cu).
+// Copy-ins run this many levels before a point's first edge.
 constexpr int kStrainAhead = 8;
 
 // Appends one scene's strain schedule to the batch arrays. `edges` are the
@@ -20,7 +20,7 @@ constexpr int kStrainAhead = 8;
 // Level of an edge = 1 + the level of the last earlier edge at either of
 // its points: edges of one level share no point, so sweeping level by level
 // is the reference's sequential sweep (dcollid.cpp:586-596) reordered only
-// where the order cannot matter. For the shared-memory sweep each point gets
+// where the order cannot matter. Each point gets
 // a slot for its live interval - from kAhead levels before its first edge to
 // the level after its last one - by interval colouring.
 void append_strain_schedule(const std::vector<StrainEdge>& edges, int v0, int nv, std::vector<StrainEdge>& all_edges,

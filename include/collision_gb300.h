@@ -201,7 +201,8 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *   CC_TUNE_TRAVERSE_BLOCK  threads per block of the BVH traversal (32..1024)
  *   CC_TUNE_NARROW_BLOCK    threads per block of the per-pair filter stage
  *                           of split passes (32..512)
- *   CC_TUNE_STRAIN_BLOCK    threads of each scene's strain-sweep CTA (32..256)
+ *   CC_TUNE_STRAIN_BLOCK    32..256 (default): a strain-sweep CTA takes half
+ *                           as many elements of a level side by side
  *   CC_TUNE_TAIL_GRAPH      1 (default): the end of a step (domain clamp and
  *                           final positions, the strain-limiting loop, whose
  *                           end is decided on the device, final velocities)
@@ -212,11 +213,9 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           overlap, and the first CCD pass reuses them when
  *                           the proximity pass applied no impulse; 0: a
  *                           broad phase per pass
- *   CC_TUNE_STRAIN_WARP     1: each scene's strain sweep runs on one warp
- *                           with its levels staged in shared memory;
- *                           0 (default): on a CTA of CC_TUNE_STRAIN_BLOCK
- *                           threads. Same results; the CTA sweep is faster
- *                           for sheets whose levels hold more than ~32 edges
+ *   CC_TUNE_STRAIN_WARP     1: a strain-sweep CTA's elements on one warp,
+ *                           eight side by side; 0 (default): on
+ *                           CC_TUNE_STRAIN_BLOCK's warps. Same results
  *   CC_TUNE_PACKET_TRAVERSE 1: each warp walks the hierarchy as one packet of
  *                           32 Morton-consecutive queries with a shared-memory
  *                           stack; 0 (default): a stack per thread. Same
@@ -240,10 +239,9 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           hierarchy over all of them, refits that hierarchy
  *                           over its scenes' leaves; 0: it sorts and builds a
  *                           hierarchy of its own. Same pairs
- *   CC_TUNE_STRAIN_ROLES    1 (default): in the shared-memory strain sweep a
- *                           level's edges, copy-ins and write-backs run on
- *                           separate threads (when they fit in the block);
- *                           0: every thread takes one of each
+ *   CC_TUNE_STRAIN_ROLES    kept for callers that set it: the strain sweeps'
+ *                           copy-ins and write-backs always run on warps of
+ *                           their own
  *   CC_TUNE_TRAVERSE_REFILL 1..32 (default 8): the stackless traversal runs
  *                           on resident warps whose lanes take new queries
  *                           from a counter once this many of them have
