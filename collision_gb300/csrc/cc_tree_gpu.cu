@@ -8,21 +8,20 @@
 // root volume are needed (cc_tree_order.h says why).
 //
 // The insertions are sequential in the reference, but their descents can
-// overlap: insertion e reads, at depth d, only boxes at depth d+1 and the
-// child pointers at depth d, and every earlier insertion writes those while
-// it is at depth d. So one CTA runs up to blockDim.x insertions as a
-// pipeline, every active insertion one level per step with a block barrier
-// between steps, and at most one insertion starting per step. Insertion e
-// then reaches every depth at least one step after insertion e-1 and sees
-// exactly the tree the reference's insertion e sees; in one step no two
-// insertions touch the same depth. Boxes are widened on the way down (the
-// union with the new leaf's box), which gives the same box as the
-// reference's bottom-up union of the children: min and max are exact.
+// overlap: insertion e, at a node of depth d, reads and writes only that
+// node's record (its children's ids and boxes) and, splitting a leaf, makes
+// the record below it. So one CTA runs the insertions as a pipeline, every
+// active insertion one level per step with a block barrier between steps,
+// and at most one insertion starting per step. Insertion e then reaches
+// every depth at least one step after insertion e-1 and sees exactly the
+// tree the reference's insertion e sees; in one step no two insertions touch
+// the same record. Boxes are widened on the way down (the union with the new
+// leaf's box), which gives the same box as the reference's bottom-up union
+// of the children: min and max are exact.
 //
-// Leaves are nodes 0..n-1 and insertion e (e >= 1) creates node n+e-1, so
-// whether a node is a leaf needs no load. Each insertion also keeps parent
-// links and leaf counts, from which k_tree_ranks gives each leaf its inorder
-// rank by walking to the root.
+// Leaves are ids 0..n-1 and insertion e (e >= 1) creates the internal node
+// n+e-1. Each insertion also keeps parent links and leaf counts, from which
+// k_tree_ranks gives each leaf its inorder rank by walking to the root.
 #include "cc_launch.h"
 
 namespace ccg {
@@ -30,18 +29,27 @@ namespace ccg {
 namespace {
 
 constexpr int kTreeThreads = 1024;
+constexpr int kTreeGroups = kTreeThreads / 4;  // insertions in flight
 
 // Box coordinates are kept as order-preserving integer keys: key(a) <
 // key(b) exactly when a < b for doubles that are not NaN, except that -0
 // orders below +0. So min and max run on the integer pipe (GB300's FP64
-// rate is a small fraction of its integer rate), and containment is six
-// integer compares. Where the reference's std::min/std::max would keep +0
-// and the key order keeps -0, the difference is only the sign of a zero
-// coordinate, which changes no box extent, volume comparison or decision.
-struct __align__(16) TreeNode {
-    long long lo[3], hi[3];  // keys
-    double vol;              // AABB::volume of the box (AABB.cpp:51-54), kept with it
-    int left, right;
+// rate is a small fraction of its integer rate). Where the reference's
+// std::min/std::max would keep +0 and the key order keeps -0, the difference
+// is only the sign of a zero coordinate, which changes no box extent, volume
+// comparison or decision.
+//
+// A child as its parent's record holds it, in the halves that two lanes load:
+// the keys of x and y, then those of z, the volume (AABB::volume of the box,
+// AABB.cpp:51-54) and the child's id.
+struct __align__(16) TreeChild {
+    long long xlo, xhi, ylo, yhi;
+    long long zlo, zhi;
+    double vol;
+    long long id;
+};
+struct TreeNode {
+    TreeChild child[2];  // left, right
 };
 
 __device__ __forceinline__ long long okey(double d) {
@@ -55,187 +63,182 @@ __device__ __forceinline__ long long kmin(long long a, long long b) { return b <
 __device__ __forceinline__ long long kmax(long long a, long long b) { return a < b ? b : a; }
 
 // (hi - lo) products in the reference's order, never contracted
-__device__ __forceinline__ double volume_k(const long long* lo, const long long* hi) {
-    return __dmul_rn(__dmul_rn(__dsub_rn(odec(hi[0]), odec(lo[0])), __dsub_rn(odec(hi[1]), odec(lo[1]))),
-                     __dsub_rn(odec(hi[2]), odec(lo[2])));
-}
-// the volume of the union of two boxes
-__device__ __forceinline__ double volume_union(const long long* alo, const long long* ahi, const long long* blo,
-                                               const long long* bhi) {
-    long long lo[3], hi[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        lo[d] = kmin(alo[d], blo[d]);
-        hi[d] = kmax(ahi[d], bhi[d]);
-    }
-    return volume_k(lo, hi);
-}
-__device__ __forceinline__ bool contains(const long long* olo, const long long* ohi, const long long* ilo,
-                                         const long long* ihi) {
-    return olo[0] <= ilo[0] && olo[1] <= ilo[1] && olo[2] <= ilo[2] && ihi[0] <= ohi[0] && ihi[1] <= ohi[1] &&
-           ihi[2] <= ohi[2];
+__device__ __forceinline__ double volume_k(const TreeChild& c) {
+    return __dmul_rn(__dmul_rn(__dsub_rn(odec(c.xhi), odec(c.xlo)), __dsub_rn(odec(c.yhi), odec(c.ylo))),
+                     __dsub_rn(odec(c.zhi), odec(c.zlo)));
 }
 
-__device__ __forceinline__ void load_node(const TreeNode* t, long long* lo, long long* hi, double& vol) {
-    const longlong2* p = reinterpret_cast<const longlong2*>(t);
-    const longlong2 a = p[0], b = p[1], c = p[2];
-    lo[0] = a.x; lo[1] = a.y; lo[2] = b.x;
-    hi[0] = b.y; hi[1] = c.x; hi[2] = c.y;
-    vol = reinterpret_cast<const double*>(t)[6];
+// One lane's half of a child: lane h = 0 xlo, xhi, ylo, yhi; h = 1 zlo, zhi,
+// the volume's bits, the id.
+struct Half {
+    long long a, b, c, d;
+};
+__device__ __forceinline__ Half load_half(const TreeChild* p, int h) {
+    const longlong2* q = reinterpret_cast<const longlong2*>(p) + 2 * h;
+    const longlong2 u = q[0], v = q[1];
+    return Half{u.x, u.y, v.x, v.y};
+}
+__device__ __forceinline__ void store_half(TreeChild* p, int h, const Half& x) {
+    longlong2* q = reinterpret_cast<longlong2*>(p) + 2 * h;
+    q[0] = make_longlong2(x.a, x.b);
+    q[1] = make_longlong2(x.c, x.d);
 }
 
+// One CTA per tree, four lanes per insertion (lane 2 s + h: half h of child
+// s). What bounds a build is the time of a step, one level of every
+// insertion in flight: with a thread per insertion it was ~14 FP64
+// instructions of each warp (GB300 takes ~64 cycles for one however many
+// lanes it serves, and 32 insertions' lanes rarely all skip them), two
+// dependent loads (the child ids, then the children) and the barrier. Here
+// both children's unions are formed side by side, x and z too, which leaves
+// five FP64 instructions; a node's record holds both children, so a level is
+// one round of loads; a new leaf's record is loaded an insertion ahead; and
+// the leaf counts are adds that nothing waits for.
 __global__ void __launch_bounds__(kTreeThreads) k_tree_build(const Box6* __restrict__ boxes, const int* __restrict__ jobs,
-                                                            TreeNode* nodes_all, int* parent_all, int* count_all,
-                                                            int* root_out, double* vol_out) {
+                                                            TreeNode* nodes_all, TreeChild* leaves_all, int* parent_all,
+                                                            int* extra_all, int* root_out, double* vol_out) {
     const int e0 = jobs[3 * blockIdx.x + 1], n = jobs[3 * blockIdx.x + 2];
-    TreeNode* nd = nodes_all + 2 * (size_t)e0;
+    TreeNode* nd = nodes_all + e0;         // internal node q is nd[q - n]
+    TreeChild* leaf = leaves_all + e0;
     int* parent = parent_all + 2 * (size_t)e0;
-    int* count = count_all + 2 * (size_t)e0;
-    const int tid = threadIdx.x, T = blockDim.x;
-    for (int e = tid; e < n; e += T) {
+    int* extra = extra_all + e0;           // node q has 2 + extra[q - n] leaves
+    const int tid = threadIdx.x;
+    for (int e = tid; e < n; e += kTreeThreads) {
         const Box6 b = boxes[e0 + e];
-        TreeNode& L = nd[e];
-        for (int d = 0; d < 3; ++d) {
-            L.lo[d] = okey(b.lo[d]);
-            L.hi[d] = okey(b.hi[d]);
-        }
-        L.vol = __dmul_rn(__dmul_rn(__dsub_rn(b.hi[0], b.lo[0]), __dsub_rn(b.hi[1], b.lo[1])),
-                          __dsub_rn(b.hi[2], b.lo[2]));
-        L.left = L.right = -1;
+        TreeChild L;
+        L.xlo = okey(b.lo[0]); L.xhi = okey(b.hi[0]);
+        L.ylo = okey(b.lo[1]); L.yhi = okey(b.hi[1]);
+        L.zlo = okey(b.lo[2]); L.zhi = okey(b.hi[2]);
+        L.vol = volume_k(L);
+        L.id = e;
+        leaf[e] = L;
         parent[e] = -1;
-        count[e] = 1;
+        extra[e] = 0;
     }
     __syncthreads();
     if (n < 2) {
         if (tid == 0) {
             root_out[blockIdx.x] = n - 1;
-            vol_out[blockIdx.x] = n == 1 ? nd[0].vol : 0.0;
+            vol_out[blockIdx.x] = n == 1 ? leaf[0].vol : 0.0;
         }
         return;
     }
-    const int root = n;  // insertion 1 splits the root leaf 0 into node n
-    if (tid == 0) {
-        TreeNode& q = nd[n];
-        for (int d = 0; d < 3; ++d) {
-            q.lo[d] = kmin(nd[1].lo[d], nd[0].lo[d]);
-            q.hi[d] = kmax(nd[1].hi[d], nd[0].hi[d]);
-        }
-        q.vol = volume_k(q.lo, q.hi);
-        q.left = 1;
-        q.right = 0;
+    if (tid == 0) {  // insertion 1 splits the root leaf 0 into node n
+        nd[0].child[0] = leaf[1];
+        nd[0].child[1] = leaf[0];
         parent[n] = -1;
         parent[0] = parent[1] = n;
-        count[n] = 2;
     }
-    __syncthreads();
-
-    int my_e = -1, p = -1;
-    long long nlo[3], nhi[3];
+    const int g = tid >> 2, side = (tid >> 1) & 1, h = tid & 1;
+    const int lane = tid & 31, base = lane & ~3;  // the group's first lane in its warp
+    const Half none{0, 0, 0, 0};
+    int my_e = -1, p = n;
+    Half mine = none;
+    int ahead = g < 2 ? g + kTreeGroups : g;  // this group's next insertion, and its leaf
+    Half next_leaf = ahead < n ? load_half(&leaf[ahead], h) : none;
     int next = 2;  // the next insertion to start; the same in every thread
+    __syncthreads();
     for (;;) {
-        const bool start = next < n && my_e < 0 && next % T == tid;
+        const bool start = next < n && my_e < 0 && next == ahead;
         if (start) {
-            // the root's box is widened here; its volume is formed at the end
             my_e = next;
-            p = root;
-            double v;
-            load_node(&nd[my_e], nlo, nhi, v);
-            TreeNode& R = nd[root];
-            for (int d = 0; d < 3; ++d) {
-                R.lo[d] = kmin(R.lo[d], nlo[d]);
-                R.hi[d] = kmax(R.hi[d], nhi[d]);
-            }
-            ++count[root];
+            p = n;
+            mine = next_leaf;
+            ahead += kTreeGroups;
+            if (ahead < n) next_leaf = load_half(&leaf[ahead], h);
         }
-        if (my_e >= 0) {
-            // one level: p is an internal node on the path, its box already widened
-            const int l = nd[p].left, r = nd[p].right;
-            long long llo[3], lhi[3], rlo[3], rhi[3];
-            double lv, rv;
-            load_node(&nd[l], llo, lhi, lv);
-            load_node(&nd[r], rlo, rhi, rv);
+        if (__any_sync(0xffffffffu, my_e >= 0)) {
+            const bool on = my_e >= 0;
+            // one level: p is an internal node on the path
+            const Half old = on ? load_half(&nd[p - n].child[side], h) : none;
+            Half u = old;  // the child's half with the new leaf
+            u.a = kmin(old.a, mine.a);
+            u.b = kmax(old.b, mine.b);
+            if (h == 0) {
+                u.c = kmin(old.c, mine.c);
+                u.d = kmax(old.d, mine.d);
+            }
             // the volume growth of each child's box by the new leaf's
-            // (AABB::merge, AABB.cpp:38-49); a box that holds the new leaf's
-            // does not grow (the same doubles), and a growth is never below 0
-            bool go_left, grows;
-            double gc;  // the chosen child's new volume
-            if (contains(rlo, rhi, nlo, nhi)) {
-                go_left = false;  // vdiff2 = 0 <= vdiff1
-                grows = false;
-                gc = rv;
-            } else {
-                const double gr = volume_union(rlo, rhi, nlo, nhi);
-                if (contains(llo, lhi, nlo, nhi)) {
-                    go_left = 0.0 < __dsub_rn(gr, rv);  // vdiff1 = 0
-                    grows = !go_left;
-                    gc = go_left ? lv : gr;
-                } else {
-                    const double gl = volume_union(llo, lhi, nlo, nhi);
-                    go_left = __dsub_rn(gl, lv) < __dsub_rn(gr, rv);
-                    grows = true;
-                    gc = go_left ? gl : gr;
+            // (AABB::merge, AABB.cpp:38-49), in the lanes h = 0; ties go
+            // right. A box that holds the new leaf's gives its own volume
+            // again, and no growth: if every right child of the warp's does,
+            // there is nothing to form.
+            const bool same = u.a == old.a && u.b == old.b && u.c == old.c && u.d == old.d;
+            const unsigned holds = __ballot_sync(0xffffffffu, same) >> base;
+            const bool right_holds = (holds & 12u) == 12u;
+            bool go_left = false;
+            double vol = __longlong_as_double(__shfl_sync(0xffffffffu, old.c, lane | 1));
+            if (__any_sync(0xffffffffu, on && !right_holds)) {
+                const double e_a = __dsub_rn(odec(u.b), odec(u.a));
+                const double e_b = __dsub_rn(odec(u.d), odec(u.c));  // h = 1: not used
+                const double e_z = __shfl_sync(0xffffffffu, e_a, lane | 1);
+                const double grown = __dmul_rn(__dmul_rn(e_a, e_b), e_z);
+                const double growth = __dsub_rn(grown, vol);
+                const double gl = __shfl_sync(0xffffffffu, growth, base);
+                const double gr = __shfl_sync(0xffffffffu, growth, base + 2);
+                go_left = gl < gr;
+                vol = __shfl_sync(0xffffffffu, grown, lane & ~1);
+            }
+            const int chosen = go_left ? 0 : 1;
+            const int c = (int)__shfl_sync(0xffffffffu, old.d, base + 2 * chosen + 1);
+            const bool split = on && c < n;
+            const int q = n + my_e - 1;
+            if (on && side == chosen && (split || !((holds >> (2 * chosen) & 3u) == 3u))) {
+                Half w = u;
+                if (h == 1) {
+                    w.c = __double_as_longlong(vol);
+                    if (split) w.d = q;
+                }
+                store_half(&nd[p - n].child[side], h, w);
+            }
+            if (__any_sync(0xffffffffu, split)) {
+                Half was;  // the leaf's half, in both lanes h
+                was.a = __shfl_sync(0xffffffffu, old.a, base + 2 * chosen + h);
+                was.b = __shfl_sync(0xffffffffu, old.b, base + 2 * chosen + h);
+                was.c = __shfl_sync(0xffffffffu, old.c, base + 2 * chosen + h);
+                was.d = __shfl_sync(0xffffffffu, old.d, base + 2 * chosen + h);
+                if (split) {
+                    // new leaf left, old leaf right
+                    store_half(&nd[q - n].child[side], h, side == 0 ? mine : was);
+                    const int l4 = lane & 3;
+                    if (l4 == 0) parent[q] = p;
+                    if (l4 == 1) parent[my_e] = q;
+                    if (l4 == 2) parent[c] = q;
                 }
             }
-            const int c = go_left ? l : r;
-            long long clo[3], chi[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                clo[d] = go_left ? llo[d] : rlo[d];
-                chi[d] = go_left ? lhi[d] : rhi[d];
-            }
-            if (c >= n) {
-                if (grows) {
-                    TreeNode& C = nd[c];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        C.lo[d] = kmin(clo[d], nlo[d]);
-                        C.hi[d] = kmax(chi[d], nhi[d]);
-                    }
-                    C.vol = gc;
-                }
-                ++count[c];
-                p = c;
-            } else {
-                const int q = n + my_e - 1;
-                TreeNode& Q = nd[q];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    Q.lo[d] = kmin(nlo[d], clo[d]);
-                    Q.hi[d] = kmax(nhi[d], chi[d]);
-                }
-                Q.vol = gc;  // the union of the leaf's box and the new one's
-                Q.left = my_e;
-                Q.right = c;
-                parent[q] = p;
-                parent[my_e] = q;
-                parent[c] = q;
-                count[q] = 2;
-                if (go_left) nd[p].left = q;
-                else nd[p].right = q;
+            if (split) {
                 my_e = -1;
+            } else if (on) {
+                p = c;
+                if ((lane & 3) == 3) atomicAdd(&extra[c - n], 1);
             }
         }
         next += __syncthreads_or(start) ? 1 : 0;
         if (next >= n && !__syncthreads_or(my_e >= 0)) break;
     }
     if (tid == 0) {
-        root_out[blockIdx.x] = root;
-        vol_out[blockIdx.x] = volume_k(nd[root].lo, nd[root].hi);
+        const TreeChild a = nd[0].child[0], b = nd[0].child[1];
+        TreeChild r;
+        r.xlo = kmin(a.xlo, b.xlo); r.xhi = kmax(a.xhi, b.xhi);
+        r.ylo = kmin(a.ylo, b.ylo); r.yhi = kmax(a.yhi, b.yhi);
+        r.zlo = kmin(a.zlo, b.zlo); r.zhi = kmax(a.zhi, b.zhi);
+        root_out[blockIdx.x] = n;
+        vol_out[blockIdx.x] = volume_k(r);
     }
 }
 
 // Inorder rank of each leaf: the leaves of every left sibling on its path.
 __global__ void k_tree_ranks(const int* __restrict__ jobs, const TreeNode* __restrict__ nodes_all,
-                             const int* __restrict__ parent_all, const int* __restrict__ count_all, int* rank) {
+                             const int* __restrict__ parent_all, const int* __restrict__ extra_all, int* rank) {
     const int e0 = jobs[3 * blockIdx.y + 1], n = jobs[3 * blockIdx.y + 2];
-    const TreeNode* nd = nodes_all + 2 * (size_t)e0;
+    const TreeNode* nd = nodes_all + e0;
     const int* parent = parent_all + 2 * (size_t)e0;
-    const int* count = count_all + 2 * (size_t)e0;
+    const int* extra = extra_all + e0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         int r = 0, x = e;
         for (int a = parent[x]; a >= 0; x = a, a = parent[a]) {
-            const int lft = nd[a].left;
-            if (lft != x) r += count[lft];
+            const int lft = (int)nd[a - n].child[0].id;
+            if (lft != x) r += lft < n ? 1 : 2 + extra[lft - n];
         }
         rank[e0 + e] = r;
     }
@@ -244,18 +247,19 @@ __global__ void k_tree_ranks(const int* __restrict__ jobs, const TreeNode* __res
 }  // namespace
 
 size_t tree_scratch_bytes(long long ne) {
-    return (size_t)(2 * ne + 1) * (sizeof(TreeNode) + 2 * sizeof(int));
+    return (size_t)(ne + 1) * (sizeof(TreeNode) + sizeof(TreeChild) + 3 * sizeof(int));
 }
 
 void tree_order_gpu(const Box6* boxes, const int* jobs, int njobs, int max_ne, void* scratch, long long ne_total,
                     int* rank, int* root_out, double* vol_out, cudaStream_t s) {
     if (njobs <= 0) return;
     TreeNode* nodes = static_cast<TreeNode*>(scratch);
-    int* parent = reinterpret_cast<int*>(nodes + 2 * ne_total + 1);
-    int* count = parent + 2 * ne_total + 1;
-    k_tree_build<<<njobs, kTreeThreads, 0, s>>>(boxes, jobs, nodes, parent, count, root_out, vol_out);
+    TreeChild* leaves = reinterpret_cast<TreeChild*>(nodes + ne_total + 1);
+    int* parent = reinterpret_cast<int*>(leaves + ne_total + 1);
+    int* extra = parent + 2 * (ne_total + 1);
+    k_tree_build<<<njobs, kTreeThreads, 0, s>>>(boxes, jobs, nodes, leaves, parent, extra, root_out, vol_out);
     const int bx = std::max(1, std::min((max_ne + 255) / 256, 1024));
-    k_tree_ranks<<<dim3(bx, njobs), 256, 0, s>>>(jobs, nodes, parent, count, rank);
+    k_tree_ranks<<<dim3(bx, njobs), 256, 0, s>>>(jobs, nodes, parent, extra, rank);
 }
 
 }  // namespace ccg
