@@ -236,6 +236,18 @@ __device__ __forceinline__ int aggregated_add(int* p, int n) {
     base = g.shfl(base, g.size() - 1);
     return base + incl - n;
 }
+
+// x in FP32 by cutting the mantissa (error below 2^-23 |x|): the double's
+// bits re-biased and shifted on the integer pipe, where a conversion takes
+// the FP64 pipe's 64 cycles. Zeros keep their sign; values outside FP32's
+// normal range take the conversion.
+__device__ __forceinline__ float cut32(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned m = (hi & 0x7fffffffu) - 0x38000000u;  // exponent bias 1023 -> 127
+    if (m - 0x00100000u < 0x0fe00000u) return __uint_as_float((hi & 0x80000000u) | __funnelshift_l(lo, m, 3));
+    if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);
+    return (float)x;
+}
 #endif
 
 __device__ __forceinline__ double dot3(const double* a, const double* b) {

@@ -223,9 +223,8 @@ struct NarrowArgs {
     const float4* p32;      // x_old in FP32 (with pbox_lo)
     const float4* v32;      // avgVel in FP32 (with pbox_lo, moving passes)
     int check;              // hit decisions only (no impulses, contacts, zones)
-    // split pass (mixed precision, no zones, no recording): the sub-tests
-    // that pass the FP32 filters, point-triangle and edge-edge apart, and a
-    // hit flag per candidate pair
+    // split pass (no recording): the sub-tests that pass the filters,
+    // point-triangle and edge-edge apart, and a hit flag per candidate pair
     SubRec* sub_pt;
     SubRec* sub_ee;
     int sub_cap;
@@ -239,6 +238,7 @@ struct NarrowArgs {
     // 1: both sub-test lists in one launch, a warp per sub-test in small
     // passes (k_subtests_all); 0: one launch per list, a thread per sub-test
     int sub_merge = 1;
+    int sub_counted = 0;  // the filter has counted the sub-tests evaluated in FP64 (plain passes)
     // movable rigid bodies: the body of each point (-1 none), each body's
     // mass, and the contribution slot of body 0 (the point count)
     const int* vbody;
@@ -246,8 +246,9 @@ struct NarrowArgs {
     int body_slot0;
 };
 void narrow_pass(const NarrowArgs& a, int moving, int max_pairs, cudaStream_t s, int block = 128);
-// The same pass in stages (mixed precision only, no recording): FP32
-// filters per pair, then the FP64 sub-tests that pass them, one thread
+// The same pass in stages (no recording): the filters - FP32 ones per pair
+// with the point data of mode 1, else, for moving passes, each sub-test's
+// coplanarity cubic in FP64 - then the FP64 sub-tests that pass them, one thread
 // each, then - for scenes in impact-zone mode - the createImpZone calls of
 // every pair that hit. parts selects the filters (kSplitFilter), the rest
 // (kSplitSubtests) or both, so that the two can be timed apart.

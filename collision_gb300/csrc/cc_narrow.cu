@@ -168,7 +168,7 @@ struct OrientedPair {
     unsigned long long keybase;
 };
 __device__ __forceinline__ bool orient_pair(const NarrowArgs& a, int2 pr, OrientedPair& o) {
-    int ri = a.rank[pr.x], rj = a.rank[pr.y];
+    int ri = a.rank ? a.rank[pr.x] : pr.x, rj = a.rank ? a.rank[pr.y] : pr.y;
     int ea = ri > rj ? pr.x : pr.y;  // found leaf
     int eb = ri > rj ? pr.y : pr.x;  // query leaf
     int ra = ri > rj ? ri : rj, rb = ri > rj ? rj : ri;
@@ -253,6 +253,106 @@ __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pai
     if ((threadIdx.x & 31) == 0 && t_visits) atomicAdd(&a.ctr->nvisits, t_visits);
 }
 
+// The points of sub-test `sub` of a moving pair (for_each_subtest<true>'s
+// numbering) and whether it is edge-edge; false past the pair's last.
+__device__ __forceinline__ bool moving_subtest(const OrientedPair& o, int sub, int* pts, bool& ee) {
+    const int npt = o.kind == 0 ? 6 : o.kind == 1 ? 2 : 0;
+    const int n = o.kind == 0 ? 15 : o.kind == 1 ? 5 : 1;
+    ee = sub >= npt;
+    if (sub >= n) return false;
+    if (!ee) {
+        const bool first = sub < 3;  // the triangle is A, the point B's; then the reverse
+        const int i = first ? sub : sub - 3;
+        for (int k = 0; k < 3; ++k) pts[k] = first ? o.A[k] : o.B[k];
+        const int *P = first ? o.B : o.A;
+        pts[3] = i == 0 ? P[0] : i == 1 ? P[1] : P[2];
+        return true;
+    }
+    const int e = sub - npt;
+    const int i = o.kind == 2 ? 0 : o.kind == 1 ? e : e / 3, j = o.kind == 0 ? e - 3 * i : 0;
+    pts[0] = i == 0 ? o.A[0] : i == 1 ? o.A[1] : o.A[2];
+    pts[1] = i == 0 ? o.A[1] : i == 1 ? o.A[2] : o.A[0];
+    pts[2] = j == 0 ? o.B[0] : j == 1 ? o.B[1] : o.B[2];
+    pts[3] = j == 0 ? o.B[1] : j == 1 ? o.B[2] : o.B[0];
+    return true;
+}
+
+// Stage 1 of a plain FP64 moving pass: the coplanarity cubic of every
+// sub-test in FP64, sixteen threads per pair; a sub-test whose cubic can
+// have no root in the time window (may_be_coplanar) is done, the others are
+// queued for the full test. With one thread per pair taking its up to 15
+// sub-tests in turn (k_narrow), a warp waited for every lane's roots - a
+// correctly rounded one takes thousands of FP64 instructions - and a pass of
+// a few thousand pairs left most of the chip idle.
+constexpr int kPlainBlock = 128;
+__global__ void __launch_bounds__(kPlainBlock) k_plain_filter(NarrowArgs a, int max_pairs) {
+    int np = a.ctr->npairs;
+    if (np > max_pairs) np = max_pairs;
+    const int sub = threadIdx.x & 15, group = (threadIdx.x & 31) & ~15;
+    int t_visits = 0, t_sub = 0;
+    const int groups = (int)(gridDim.x * (kPlainBlock / 16));
+    const int g0 = (int)(blockIdx.x * (kPlainBlock / 16) + (threadIdx.x >> 4));
+    for (int base = 0; base < np; base += groups) {
+        const int idx = base + g0;
+        bool queue = false, ee = false;
+        int pts[4] = {0, 0, 0, 0}, sc = 0;
+        OrientedPair o;
+        o.keybase = 0;
+        if (idx < np) {
+            int2 pr = a.pairs[idx];
+            pr.y &= kPairIdMask;
+            if (orient_pair(a, pr, o)) {
+                t_visits += sub == 0;
+                bool shared = false;  // a shared point makes every test of the pair return false
+                for (int i = 0; i < o.n1; ++i)
+                    for (int j = 0; j < o.n2; ++j) shared |= o.A[i] == o.B[j];
+                sc = a.escene[pr.x];
+                if (!shared && moving_subtest(o, sub, pts, ee)) {
+                    double xo4[4][3], av4[4][3];
+                    for (int q = 0; q < 4; ++q) {
+                        load3(a.xo, pts[q], xo4[q]);
+                        load3(a.av, pts[q], av4[q]);
+                    }
+                    ++t_sub;
+                    queue = may_be_coplanar(xo4, av4, a.scenes[sc].p.dt);
+                }
+            }
+        }
+        const unsigned in_pair = __ballot_sync(0xffffffffu, queue) >> group & 0xffffu;
+        if (queue) {
+            int slot;  // (the lanes that add together share one counter)
+            if (ee)
+                slot = aggregated_add(&a.ctr->nsub_ee, 1);
+            else
+                slot = aggregated_add(&a.ctr->nsub_pt, 1);
+            if (slot >= a.sub_cap) {
+                atomicOr(&a.ctr->err, kErrSubOverflow);
+            } else {
+                SubRec r;
+                r.keybase = o.keybase;
+                r.pair = idx;
+                r.scene = sc;
+                for (int i = 0; i < 4; ++i) r.p[i] = pts[i];
+                r.sub = sub;
+                r.pad = 0;
+                (ee ? a.sub_ee : a.sub_pt)[slot] = r;
+            }
+            if ((in_pair & ((1u << sub) - 1u)) == 0) {  // the pair's first
+                a.pair_hit[idx] = 0;
+                a.pairq[aggregated_add(&a.ctr->npairq, 1)] = idx;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        t_visits += __shfl_xor_sync(0xffffffffu, t_visits, o);
+        t_sub += __shfl_xor_sync(0xffffffffu, t_sub, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (t_visits) atomicAdd(&a.ctr->nvisits, t_visits);
+        if (t_sub) atomicAdd(&a.ctr->nsub, t_sub);
+    }
+}
+
 // Stage 3 (impact-zone scenes): createImpZone for every sub-test of a pair
 // from its first hit on, in sub-test order - the reference's status stays
 // true after the first hit (dcollid3d.cpp:300-321), whether or not the
@@ -298,7 +398,7 @@ __device__ __forceinline__ NarrowCtx subtest_ctx(const NarrowArgs& a) {
     c.contrib = a.contrib; c.contrib_cap = a.contrib_cap; c.ctr = a.ctr; c.urec = nullptr; c.urec_cap = 0;
     c.rec = nullptr; c.rec_cap = 0;
     c.pbox_lo = nullptr; c.pbox_hi = nullptr; c.p32 = nullptr; c.v32 = nullptr;
-    c.check = 0;
+    c.check = a.check;
     c.robust_roots = a.robust_roots;
     c.zone = 0;
     return c;
@@ -341,7 +441,7 @@ __device__ __forceinline__ void subtest_counts(const NarrowArgs& a, SubTally t) 
         if (t.hits) atomicAdd(&a.ctr->nhit_pairs, t.hits);
         if (t.cr) atomicAdd(&a.ctr->ncr, t.cr);
         if (t.contacts) atomicAdd(&a.ctr->ncontacts, t.contacts);
-        if (t.sub) atomicAdd(&a.ctr->nsub, t.sub);
+        if (t.sub && !a.sub_counted) atomicAdd(&a.ctr->nsub, t.sub);
     }
 }
 
@@ -467,13 +567,16 @@ void narrow_pass(const NarrowArgs& a, int moving, int max_pairs, cudaStream_t s,
         count_launch(), k_narrow<false><<<blocks, threads, 0, s>>>(a, max_pairs);
 }
 
-void narrow_pass_split(const NarrowArgs& a, int moving, int max_pairs, cudaStream_t s, int block, bool zone,
+void narrow_pass_split(const NarrowArgs& args, int moving, int max_pairs, cudaStream_t s, int block, bool zone,
                        int parts) {
     if (max_pairs <= 0) return;
-    if (!a.pbox_lo || !a.p32 || (moving && !a.v32)) {  // the filters need the FP32 point data (mode 1)
-        if (parts & kSplitFilter) narrow_pass(a, moving, max_pairs, s, block);
+    const bool mixed = args.pbox_lo && args.p32 && (!moving || args.v32);  // the FP32 filters' point data (mode 1)
+    if (!mixed && !moving) {
+        if (parts & kSplitFilter) narrow_pass(args, moving, max_pairs, s, block);
         return;
     }
+    NarrowArgs a = args;
+    a.sub_counted = mixed ? 0 : 1;
     const int cap_blocks = 152 * 16 * 128 / block;
     int blocks = (max_pairs + block - 1) / block;
     if (blocks > cap_blocks) blocks = cap_blocks;
@@ -486,7 +589,15 @@ void narrow_pass_split(const NarrowArgs& a, int moving, int max_pairs, cudaStrea
     if (mb < (kSubSparse + 3) / 4) mb = (kSubSparse + 3) / 4;
     const int mblocks = (int)mb;
     if (moving) {
-        if (parts & kSplitFilter) count_launch(), k_narrow_filter<true><<<blocks, block, 0, s>>>(a, max_pairs);
+        if (parts & kSplitFilter) {
+            if (mixed) {
+                count_launch(), k_narrow_filter<true><<<blocks, block, 0, s>>>(a, max_pairs);
+            } else {
+                long long pb = (16ll * max_pairs + kPlainBlock - 1) / kPlainBlock;
+                if (pb > 152 * 16) pb = 152 * 16;
+                count_launch(), k_plain_filter<<<(int)pb, kPlainBlock, 0, s>>>(a, max_pairs);
+            }
+        }
         if (parts & kSplitSubtests) {
             if (a.sub_merge) count_launch(), k_subtests_all<true><<<mblocks, 128, 0, s>>>(a);
             count_launch(), k_subtests<true, false><<<sblocks, 128, 0, s>>>(a, a.sub_merge);

@@ -496,6 +496,120 @@ __device__ __forceinline__ bool root_misses(const double (*xo4)[3], const double
     return gap - 2.0 * dp - xmax * 0x1p-44 > h * 1.001;
 }
 
+// The coplanarity cubic a t^3 + b t^2 + c t + d of four points
+// (dcollid3d.cpp:371-408).
+struct Cubic {
+    double a, b, c, d;
+};
+__device__ __forceinline__ Cubic coplanarity_cubic(const double (*xo4)[3], const double (*av4)[3]) {
+    Cubic q;
+    double v[4][3], x[4][3];
+    for (int j = 0; j < 3; ++j) {
+        v[0][j] = av4[0][j];
+        x[0][j] = xo4[0][j];
+    }
+    for (int i = 1; i < 4; ++i)
+        for (int j = 0; j < 3; ++j) {
+            v[i][j] = av4[i][j] - av4[0][j];
+            x[i][j] = xo4[i][j] - xo4[0][j];
+        }
+    double vv[3], vx[3], xx[3];
+    vv[0] = v[1][1] * v[2][2] - v[1][2] * v[2][1];
+    vv[1] = v[1][0] * v[2][2] - v[1][2] * v[2][0];
+    vv[2] = v[1][0] * v[2][1] - v[1][1] * v[2][0];
+    vx[0] = v[1][1] * x[2][2] - v[1][2] * x[2][1] - v[2][1] * x[1][2] + v[2][2] * x[1][1];
+    vx[1] = v[1][0] * x[2][2] - v[1][2] * x[2][0] - v[2][0] * x[1][2] + v[2][2] * x[1][0];
+    vx[2] = v[1][0] * x[2][1] - v[1][1] * x[2][0] - v[2][0] * x[1][1] + v[2][1] * x[1][0];
+    xx[0] = x[1][1] * x[2][2] - x[1][2] * x[2][1];
+    xx[1] = x[1][0] * x[2][2] - x[1][2] * x[2][0];
+    xx[2] = x[1][0] * x[2][1] - x[1][1] * x[2][0];
+    q.a = v[3][0] * vv[0] - v[3][1] * vv[1] + v[3][2] * vv[2];
+    q.b = x[3][0] * vv[0] - x[3][1] * vv[1] + x[3][2] * vv[2] + v[3][0] * vx[0] - v[3][1] * vx[1] + v[3][2] * vx[2];
+    q.c = x[3][0] * vx[0] - x[3][1] * vx[1] + x[3][2] * vx[2] + v[3][0] * xx[0] - v[3][1] * xx[1] + v[3][2] * xx[2];
+    q.d = x[3][0] * xx[0] - x[3][1] * xx[1] + x[3][2] * xx[2];
+    return q;
+}
+
+// Whether isCoplanar can find no root in its window [0, dt + 2 MACH_EPS],
+// for |a| > MACH_EPS, from the coefficients alone: true only when it is
+// certain, so that acos, cos and pow need not run. (They are most of a
+// sub-test: ~400 of its ~500 FP64 instructions.)
+//
+// isCoplanar forms the roots of p(x) = x^3 + A x^2 + B x + C with A = b/a,
+// B = c/a, C = d/a. Let u = 2^-53 and T >= max(|A|, sqrt|B|, cbrt|C|), so
+// that |Q| <= 4/9 T^2, |R| <= 0.71 T^3 and Cardano's |A'| <= 1.2 T.
+//  - The rounding of Q and R, of z, and of R^2 - Q^3 is that of exact
+//    arithmetic on a cubic whose B and C are off by at most 16 u (A^2 + |B|)
+//    <= 32 u T^2 and 32 u (|A|^3 + |A B| + |C|) <= 96 u T^3.
+//  - The functions and the last operations move a root by at most
+//    2^-44 (2 sqrt Q + 2 |A'| + |A|) <= 2560 u T (pow's exponent 1/3 is
+//    rounded, which costs up to 120 u), and where |A'| < ROUND_EPS drops
+//    Q / A' every root taken lies within 4e-10 of the real one.
+//  - The double root taken when |A' - B'| < ROUND_EPS is the real part of
+//    two roots at most 0.87e-10 away, where |p| <= 3 |A'| 0.75e-20.
+// So if a root falls in the window, |p(x)| <= 32 u T^2 |x| + 96 u T^3 +
+// 2e-19 T for some x within E = 2560 u T + 5e-10 of it. The Bernstein
+// coefficients of the cubic on [0, dt] bound it there from below when they
+// have one sign; outside [0, dt] it changes by at most E (|c| + 2 |b| X + 3
+// |a| X^2). All terms are formed in FP32 from coefficients cut to FP32
+// (errors below 2^-20 of the sum of the terms' magnitudes in all; 2^-19
+// is taken).
+__device__ __forceinline__ bool no_root_in_window(const Cubic& q, double dt) {
+    const float a = cut32(q.a), b = cut32(q.b), c = cut32(q.c), d = cut32(q.d), w = (float)dt;
+    const float fa = fabsf(a), fb = fabsf(b), fc = fabsf(c), fd = fabsf(d);
+    const float w2 = w * w, w3 = w2 * w;
+    const float third = 1.0f / 3.0f;
+    const float b1 = d + c * w * third, b2 = d + (2.0f * c * w + b * w2) * third, b3 = d + c * w + b * w2 + a * w3;
+    const float lo = fminf(fminf(d, b1), fminf(b2, b3)), hi = fmaxf(fmaxf(d, b1), fmaxf(b2, b3));
+    const float low = fmaxf(lo, -hi);  // positive when the four have one sign: the least magnitude
+    if (!(low > 0.f)) return false;
+    const float ra = 1.0f / fa;
+    const float T = 1.01f * fmaxf(fb * ra, fmaxf(sqrtf(fc * ra), exp2f(log2f(fd * ra) * third)));
+    const float E = 3e-13f * T + 5e-10f;
+    const float X = w + E;
+    const float slope = fc + 2.0f * fb * X + 3.0f * fa * X * X;
+    const float mag = fd + fc * w + fb * w2 + fa * w3;
+    const float need = 0x1p-19f * mag + 1.01f * E * slope +
+                       1.1f * fa * T * (4e-15f * T * X + 1.1e-14f * T * T + 2e-19f) + 1e-30f;
+    return low > need;
+}
+
+// The roots where |a| <= MACH_EPS: quadratic or linear (dcollid3d.cpp:459-472).
+__device__ __forceinline__ void low_degree_roots(double a, double b, double c, double* roots) {
+    double delta = b * b - 4.0 * a * c;
+    if (fabs(a) > kRoundEps && delta > 0) {
+        double ds = sqrt(delta);
+        roots[0] = (-b + ds) / (2.0 * a);
+        roots[1] = (-b - ds) / (2.0 * a);
+    } else if (fabs(a) < kRoundEps && fabs(b) > kRoundEps) {
+        roots[0] = -c / b;
+    }
+}
+
+// Roots outside [0, dt] dropped after the shift by MACH_EPS, the rest
+// sorted; whether one is past MACH_EPS (dcollid3d.cpp:473-482).
+__device__ __forceinline__ bool window_roots(double* roots, double dt) {
+    for (int i = 0; i < 3; ++i) {
+        roots[i] = roots[i] - kMachEps;
+        if (roots[i] < 0 || roots[i] > dt) roots[i] = -1;
+    }
+    double t;
+    if (roots[0] > roots[1]) { t = roots[0]; roots[0] = roots[1]; roots[1] = t; }
+    if (roots[0] > roots[2]) { t = roots[0]; roots[0] = roots[2]; roots[2] = t; }
+    if (roots[1] > roots[2]) { t = roots[1]; roots[1] = roots[2]; roots[2] = t; }
+    return roots[0] > kMachEps || roots[1] > kMachEps || roots[2] > kMachEps;
+}
+
+// Whether a moving sub-test on these points can pass isCoplanar: false only
+// when isCoplanar returns false.
+__device__ __forceinline__ bool may_be_coplanar(const double (*xo4)[3], const double (*av4)[3], double dt) {
+    const Cubic q = coplanarity_cubic(xo4, av4);
+    if (fabs(q.a) > kMachEps) return !no_root_in_window(q, dt);
+    double roots[3] = {-1, -1, -1};
+    low_degree_roots(q.b, q.c, q.d, roots);
+    return window_roots(roots, dt);
+}
+
 // isCoplanar, dcollid3d.cpp:371-482: roots of the coplanarity cubic in
 // [0, dt], shifted by -MACH_EPS and sorted; roots[3] holds dt.
 //
@@ -512,32 +626,10 @@ __device__ __forceinline__ bool root_misses(const double (*xo4)[3], const double
 template <bool EE>
 static __device__ bool is_coplanar(const double (*xo4)[3], const double (*av4)[3], double dt, double* roots,
                                    int* ncr, bool rb = false, double h = 0.0, double eps = 0.0) {
-    double v[4][3], x[4][3];
-    for (int j = 0; j < 3; ++j) {
-        v[0][j] = av4[0][j];
-        x[0][j] = xo4[0][j];
-    }
-    for (int i = 1; i < 4; ++i)
-        for (int j = 0; j < 3; ++j) {
-            v[i][j] = av4[i][j] - av4[0][j];
-            x[i][j] = xo4[i][j] - xo4[0][j];
-        }
-    double a, b, c, d;
-    double vv[3], vx[3], xx[3];
-    vv[0] = v[1][1] * v[2][2] - v[1][2] * v[2][1];
-    vv[1] = v[1][0] * v[2][2] - v[1][2] * v[2][0];
-    vv[2] = v[1][0] * v[2][1] - v[1][1] * v[2][0];
-    vx[0] = v[1][1] * x[2][2] - v[1][2] * x[2][1] - v[2][1] * x[1][2] + v[2][2] * x[1][1];
-    vx[1] = v[1][0] * x[2][2] - v[1][2] * x[2][0] - v[2][0] * x[1][2] + v[2][2] * x[1][0];
-    vx[2] = v[1][0] * x[2][1] - v[1][1] * x[2][0] - v[2][0] * x[1][1] + v[2][1] * x[1][0];
-    xx[0] = x[1][1] * x[2][2] - x[1][2] * x[2][1];
-    xx[1] = x[1][0] * x[2][2] - x[1][2] * x[2][0];
-    xx[2] = x[1][0] * x[2][1] - x[1][1] * x[2][0];
-    a = v[3][0] * vv[0] - v[3][1] * vv[1] + v[3][2] * vv[2];
-    b = x[3][0] * vv[0] - x[3][1] * vv[1] + x[3][2] * vv[2] + v[3][0] * vx[0] - v[3][1] * vx[1] + v[3][2] * vx[2];
-    c = x[3][0] * vx[0] - x[3][1] * vx[1] + x[3][2] * vx[2] + v[3][0] * xx[0] - v[3][1] * xx[1] + v[3][2] * xx[2];
-    d = x[3][0] * xx[0] - x[3][1] * xx[1] + x[3][2] * xx[2];
+    const Cubic q = coplanarity_cubic(xo4, av4);
+    double a = q.a, b = q.b, c = q.c, d = q.d;
     if (fabs(a) > kMachEps) {
+        if (no_root_in_window(q, dt)) return false;
         b /= a; c /= a; d /= a;
         a = b; b = c; c = d;
         double Q = (a * a - 3 * b) / 9;
@@ -640,25 +732,9 @@ static __device__ bool is_coplanar(const double (*xo4)[3], const double (*av4)[3
             if (fabs(A - B) < kRoundEps) roots[1] = roots[2] = f1;
         }
     } else {
-        a = b; b = c; c = d;
-        double delta = b * b - 4.0 * a * c;
-        if (fabs(a) > kRoundEps && delta > 0) {
-            double ds = sqrt(delta);
-            roots[0] = (-b + ds) / (2.0 * a);
-            roots[1] = (-b - ds) / (2.0 * a);
-        } else if (fabs(a) < kRoundEps && fabs(b) > kRoundEps) {
-            roots[0] = -c / b;
-        }
+        low_degree_roots(b, c, d, roots);
     }
-    for (int i = 0; i < 3; ++i) {
-        roots[i] = roots[i] - kMachEps;
-        if (roots[i] < 0 || roots[i] > dt) roots[i] = -1;
-    }
-    double t;
-    if (roots[0] > roots[1]) { t = roots[0]; roots[0] = roots[1]; roots[1] = t; }
-    if (roots[0] > roots[2]) { t = roots[0]; roots[0] = roots[2]; roots[2] = t; }
-    if (roots[1] > roots[2]) { t = roots[1]; roots[1] = roots[2]; roots[2] = t; }
-    return roots[0] > kMachEps || roots[1] > kMachEps || roots[2] > kMachEps;
+    return window_roots(roots, dt);
 }
 
 // MovingPointToTri / MovingEdgeToEdge, dcollid3d.cpp:327-369: the static

@@ -435,7 +435,7 @@ struct cc_solver {
     int zone_cap = 10000;
     int mode = 0;  // 0 plain FP64, 1 mixed precision
     bool strain_window = true;
-    bool split_narrow = true;  // two-stage narrow phase for mixed passes
+    bool split_narrow = true;  // staged narrow phase
     bool strain_warp = false;  // a sweep CTA's elements on one warp
     bool strain_roles = true;  // CC_TUNE_STRAIN_ROLES, without effect
     LaunchTuning tune;
@@ -1611,7 +1611,7 @@ cc_status cc_solver::build_loop_graph(int n_hier) {
     mark(kStLoopPruned - m0, cs);
     NarrowArgs a = narrow_args(1, false);
     a.ps = loop_stamp();
-    if (mode == 1 && split_narrow) {
+    if (split_narrow) {
         narrow_pass_split(a, 1, pair_cap, cs, tune.narrow_block, true, kSplitFilter);
         mark(kStLoopFilter - m0, cs);
         narrow_pass_split(a, 1, pair_cap, cs, tune.narrow_block, true, kSplitSubtests);
@@ -1907,9 +1907,9 @@ cc_status cc_solver::detect_pass(int moving, bool any_zone) {
         a.pair_hit = d_pair_hit;
         a.pairq = d_pairq;
         a.static_only = combined ? 1 : 0;
-        // mixed passes without recording run in stages: per-pair FP32
-        // filters, the surviving FP64 sub-tests densely, then the zone unions
-        const bool split = mode == 1 && !record && split_narrow;
+        // passes without recording run in stages: the filters, the surviving
+        // FP64 sub-tests densely, then the zone unions
+        const bool split = !record && split_narrow;
         if (split && moving && profiling) {
             prof(kStNarrowCcd, true);
             narrow_pass_split(a, moving, pair_cap, stream, tune.narrow_block, any_zone, kSplitFilter);
@@ -2248,12 +2248,25 @@ cc_status cc_solver::check_ccd(const double* x_old, const double* x_new, long lo
         a.urec = nullptr; a.urec_cap = 0;
         a.rec = nullptr; a.rec_cap = 0; a.pbox_lo = nullptr; a.pbox_hi = nullptr;
         a.check = 1;
-        narrow_pass(a, 1, pair_cap, stream);
+        a.sub_pt = d_sub_pt;
+        a.sub_ee = d_sub_ee;
+        a.sub_cap = sub_cap;
+        a.pair_hit = d_pair_hit;
+        a.pairq = d_pairq;
+        if (split_narrow)  // in FP64 throughout: no FP32 point data
+            narrow_pass_split(a, 1, pair_cap, stream);
+        else
+            narrow_pass(a, 1, pair_cap, stream);
         cudaMemcpyAsync(h_ctr, d_ctr, sizeof(PassCounters), cudaMemcpyDeviceToHost, stream);
         cudaMemcpyAsync(h_run, d_run, sizeof(SceneRun) * (size_t)nscenes, cudaMemcpyDeviceToHost, stream);
         if (cudaStreamSynchronize(stream) != cudaSuccess) return cuda_check("ccd check");
         if (h_ctr->err & kErrPairOverflow) {
             cc_status st = grow_pairs(2 * h_ctr->npairs + 1024);
+            if (st) return st;
+            continue;
+        }
+        if (h_ctr->err & kErrSubOverflow) {
+            cc_status st = grow_subs(2 * std::max(h_ctr->nsub_pt, h_ctr->nsub_ee) + 1024);
             if (st) return st;
             continue;
         }
@@ -2369,7 +2382,7 @@ cc_status cc_solver::autotune(double* best_ms) {
         return CC_OK;
     };
     LaunchTuning best_t = tune;
-    bool best_split = split_narrow && mode == 1;  // the staged pass needs the FP32 point data of mode 1
+    bool best_split = split_narrow;
     float best = 1e30f;
     cc_status st = time_it(best_t, best_split, &best);  // the current setting, which also sizes the buffers
     const int tb[] = {64, 128, 256, 512};

@@ -260,18 +260,7 @@ struct __align__(16) SweepSlot {
 };
 static_assert(sizeof(SweepSlot) == kSweepSlotBytes, "slot size");
 
-// x in FP32 by cutting the mantissa (error below 2^-23 |x|): the double's
-// bits re-biased and shifted on the integer pipe, where a conversion takes
-// the FP64 pipe's 64 cycles. Zeros keep their sign; values outside FP32's
-// normal range take the conversion.
-__device__ __forceinline__ float cut32(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const unsigned m = (hi & 0x7fffffffu) - 0x38000000u;  // exponent bias 1023 -> 127
-    if (m - 0x00100000u < 0x0fe00000u) return __uint_as_float((hi & 0x80000000u) | __funnelshift_l(lo, m, 3));
-    if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);
-    return (float)x;
-}
-__device__ __forceinline__ float4 cut32(double x, double y, double z) {
+__device__ __forceinline__ float4 cut32x3(double x, double y, double z) {
     const float fx = cut32(x), fy = cut32(y), fz = cut32(z);
     return make_float4(fx, fy, fz, fabsf(fx) + fabsf(fy) + fabsf(fz));
 }
@@ -379,7 +368,7 @@ __global__ void __launch_bounds__(256) k_sweep_check(const SweepElem* __restrict
         float4 f[3];
         for (int k = 0; k < 3; ++k) {
             load3(av, el.p[k], v[k]);
-            f[k] = cut32(v[k][0], v[k][1], v[k][2]);
+            f[k] = cut32x3(v[k][0], v[k][1], v[k][2]);
         }
         const int ne = (int)(r.s2n >> 16);
         bool over = false;
@@ -772,7 +761,7 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
             for (int i = in1.x + h; i < in1.y; i += HT) {
                 const int2 ps = i == in1.x + h ? ld1 : A.load[i];
                 SweepSlot& w = win[ps.y];
-                *reinterpret_cast<float4*>(w.f) = cut32(w.d[0], w.d[1], w.d[2]);
+                *reinterpret_cast<float4*>(w.f) = cut32x3(w.d[0], w.d[1], w.d[2]);
             }
             if (h == 0) s_stop[t & 1] = seen >= kSweepStop ? 1 : 0;
             bar_sync(2, stepped);

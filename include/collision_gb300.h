@@ -194,8 +194,10 @@ cc_status cc_get_scene_status(cc_solver* s, int* out);
 cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
 
 /* Tuning knobs (none changes results):
- *   CC_TUNE_SPLIT_NARROW    1 (default): mixed passes without impact zones
- *                           or recording filter per pair, then run the FP64
+ *   CC_TUNE_SPLIT_NARROW    1 (default): passes without recording filter
+ *                           first (mixed: in FP32 per pair; plain moving
+ *                           passes and cc_check_ccd: each sub-test's
+ *                           coplanarity cubic in FP64), then run the FP64
  *                           sub-tests that pass, one thread each; 0: one
  *                           thread per pair throughout
  *   CC_TUNE_TRAVERSE_BLOCK  threads per block of the BVH traversal (32..1024)
@@ -279,7 +281,7 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           each query walks its scene with one warp (a
  *                           shared-memory stack, up to 32 nodes per round);
  *                           0: one thread along the ropes. Same results
- *   CC_TUNE_ROBUST_ROOTS    1 (default): the mixed path's FP64 sub-tests
+ *   CC_TUNE_ROBUST_ROOTS    1 (default): the FP64 sub-tests after a filter
  *                           form a coplanarity root again with correctly
  *                           rounded functions only where a decision can
  *                           depend on it (not for roots well inside the time
