@@ -191,16 +191,10 @@ __device__ __forceinline__ void zone_omega(const double (*I)[3], const double* L
     }
 }
 
-// With `run` set, the zones are movable bodies (updateImpactZoneVelocityForRG,
-// dcollid.cpp:267-288, called from updateAverageVelocity when dt > 0): only
-// those of scenes in a pass, and of more than one point, move.
 __device__ void zone_motion(const int* __restrict__ members, int i, int end, const uint8_t* __restrict__ fixed,
                             const double4_32a* __restrict__ xo, double4_32a* av, const int* __restrict__ vscene,
-                            const SceneDev* __restrict__ scenes, PassCounters* ctr,
-                            const SceneRun* __restrict__ run, const PassStamp& ps) {
-    const int zs = vscene[members[i]];
-    const Params prm = scenes[zs].p;
-    if (run && (run[zs].mode == kSceneIdle || !(prm.dt > 0.0) || end - i < 2 || (ctr->err & kErrRetry))) return;
+                            const SceneDev* __restrict__ scenes, PassCounters* ctr, const PassStamp& ps) {
+    const Params prm = scenes[vscene[members[i]]].p;
     const double m = prm.m, dt = prm.dt;
     double x_cm[3] = {0.0, 0.0, 0.0}, v_cm[3] = {0.0, 0.0, 0.0};
     double L[3] = {0.0, 0.0, 0.0}, I[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}}, tmp[3][3];
@@ -259,23 +253,19 @@ __device__ __forceinline__ int zone_warp_min(int nzones, int few) { return nzone
 constexpr int kZoneWarpBlock = 128;
 constexpr int kZoneCtaThreads = 256;
 
-// Zone z's members are members[zone_off[z] .. zone_off[z+1]), or with
-// zone_rng members[zone_rng[z].x .. zone_rng[z].y); dnz (may be null): the
+// Zone z's members are members[zone_rng[z].x .. zone_rng[z].y); dnz: the
 // zone count in device memory, at most nzones.
-__global__ void k_zone_solve(const int* __restrict__ members, const int* __restrict__ zone_off,
-                             const int2* __restrict__ zone_rng, int nzones, const int* __restrict__ dnz,
-                             const uint8_t* __restrict__ fixed, const double4_32a* __restrict__ xo, double4_32a* av,
-                             const int* __restrict__ vscene, const SceneDev* __restrict__ scenes,
-                             PassCounters* ctr, const SceneRun* __restrict__ run, PassStamp ps, int few) {
-    if (dnz) {
-        if (ctr->err & kErrRetry) return;
-        if (*dnz < nzones) nzones = *dnz;
-    }
+__global__ void k_zone_solve(const int* __restrict__ members, const int2* __restrict__ zone_rng, int nzones,
+                             const int* __restrict__ dnz, const uint8_t* __restrict__ fixed,
+                             const double4_32a* __restrict__ xo, double4_32a* av, const int* __restrict__ vscene,
+                             const SceneDev* __restrict__ scenes, PassCounters* ctr, PassStamp ps, int few) {
+    if (ctr->err & kErrRetry) return;
+    if (*dnz < nzones) nzones = *dnz;
     const int warp_min = zone_warp_min(nzones, few);
     for (int z = blockIdx.x * blockDim.x + threadIdx.x; z < nzones; z += gridDim.x * blockDim.x) {
-        const int i = zone_rng ? zone_rng[z].x : zone_off[z], end = zone_rng ? zone_rng[z].y : zone_off[z + 1];
-        if (dnz && end - i >= warp_min) continue;  // k_zone_solve_warp's
-        zone_motion(members, i, end, fixed, xo, av, vscene, scenes, ctr, run, ps);
+        const int i = zone_rng[z].x, end = zone_rng[z].y;
+        if (end - i >= warp_min) continue;  // k_zone_solve_warp's
+        zone_motion(members, i, end, fixed, xo, av, vscene, scenes, ctr, ps);
     }
 }
 
@@ -378,21 +368,31 @@ __global__ void __launch_bounds__(kZoneWarpBlock) k_zone_solve_warp(
 // adding the members in list order - but every member's terms and its
 // final motion are computed by all the CTA's threads (a large zone is
 // otherwise bound by one warp's share of the SM's FP64 pipe).
+// With `run` set, the zones are the movable bodies
+// (updateImpactZoneVelocityForRG, dcollid.cpp:267-288, called from
+// updateAverageVelocity when dt > 0), zone_off their members: only those of
+// scenes in a pass, and of more than one point, move. A body of 642 points
+// took 3 ms of every pass on one thread, whose ~150 FP64 instructions per
+// member each take ~64 cycles; here the ordered sums' two per member remain.
 __global__ void __launch_bounds__(kZoneCtaThreads) k_zone_solve_cta(
-    const int* __restrict__ members, const int2* __restrict__ zone_rng, int nzones, const int* __restrict__ dnz,
-    const uint8_t* __restrict__ fixed, const double4_32a* __restrict__ xo, double4_32a* av,
-    const int* __restrict__ vscene, const SceneDev* __restrict__ scenes, PassCounters* ctr, PassStamp ps,
-    int cta_min) {
+    const int* __restrict__ members, const int* __restrict__ zone_off, const int2* __restrict__ zone_rng, int nzones,
+    const int* __restrict__ dnz, const uint8_t* __restrict__ fixed, const double4_32a* __restrict__ xo,
+    double4_32a* av, const int* __restrict__ vscene, const SceneDev* __restrict__ scenes, PassCounters* ctr,
+    const SceneRun* __restrict__ run, PassStamp ps, int cta_min) {
     __shared__ double st[kZoneCtaThreads][12];
     __shared__ double s_sum[12];
     __shared__ double s_rot[6];  // w, mag_w, sw, cw
     if (ctr->err & kErrRetry) return;
-    if (*dnz < nzones) nzones = *dnz;
+    if (dnz && *dnz < nzones) nzones = *dnz;
     const int tid = threadIdx.x;
     bool bad = false;
     for (int z = blockIdx.x; z < nzones; z += gridDim.x) {
-        const int i = zone_rng[z].x, end = zone_rng[z].y;
+        const int i = zone_rng ? zone_rng[z].x : zone_off[z], end = zone_rng ? zone_rng[z].y : zone_off[z + 1];
         if (end - i < cta_min) continue;
+        if (run) {
+            const int zs = vscene[members[i]];
+            if (run[zs].mode == kSceneIdle || !(scenes[zs].p.dt > 0.0)) continue;
+        }
         const Params prm = scenes[vscene[members[i]]].p;
         const double m = prm.m, dt = prm.dt;
         const int num_pts = end - i;
@@ -604,9 +604,10 @@ void apply_contribs(const Contrib* contrib, const PassCounters* ctr, int contrib
 void zone_solve(const int* members, const int* zone_off, int nzones, const uint8_t* fixed, const double4_32a* xo,
                 double4_32a* av, const int* vscene, const SceneDev* scenes, PassCounters* ctr, cudaStream_t s,
                 const SceneRun* run, PassStamp ps) {
+    // (a body of one point does not move)
     if (nzones > 0)
-        count_launch(), k_zone_solve<<<nblk(nzones, 128), 128, 0, s>>>(members, zone_off, nullptr, nzones, nullptr,
-                                                                       fixed, xo, av, vscene, scenes, ctr, run, ps, 0);
+        count_launch(), k_zone_solve_cta<<<nzones < 152 * 8 ? nzones : 152 * 8, kZoneCtaThreads, 0, s>>>(
+            members, zone_off, nullptr, nzones, nullptr, fixed, xo, av, vscene, scenes, ctr, run, ps, 2);
 }
 
 void zone_solve_dev(const int* members, const int2* zone_rng, const int* dnz, int zone_cap, const uint8_t* fixed,
@@ -616,8 +617,8 @@ void zone_solve_dev(const int* members, const int2* zone_rng, const int* dnz, in
     int blocks = nblk(zone_cap, 64);
     if (blocks > 152 * 8) blocks = 152 * 8;
     if (blocks > 0)
-        count_launch(), k_zone_solve<<<blocks, 64, 0, s>>>(members, nullptr, zone_rng, zone_cap, dnz, fixed, xo, av,
-                                                           vscene, scenes, ctr, nullptr, ps, few);
+        count_launch(), k_zone_solve<<<blocks, 64, 0, s>>>(members, zone_rng, zone_cap, dnz, fixed, xo, av, vscene,
+                                                           scenes, ctr, ps, few);
     int wblocks = nblk(zone_cap, kZoneWarpBlock / 32);
     if (wblocks > 152 * 4) wblocks = 152 * 4;
     if (wblocks > 0)
@@ -626,8 +627,9 @@ void zone_solve_dev(const int* members, const int2* zone_rng, const int* dnz, in
                                                                             few);
     const int cblocks = zone_cap < 152 * 2 ? zone_cap : 152 * 2;
     if (cblocks > 0)
-        count_launch(), k_zone_solve_cta<<<cblocks, kZoneCtaThreads, 0, s>>>(members, zone_rng, zone_cap, dnz, fixed,
-                                                                            xo, av, vscene, scenes, ctr, ps, cta_min);
+        count_launch(), k_zone_solve_cta<<<cblocks, kZoneCtaThreads, 0, s>>>(members, nullptr, zone_rng, zone_cap, dnz,
+                                                                            fixed, xo, av, vscene, scenes, ctr, nullptr,
+                                                                            ps, cta_min);
 }
 
 void final_rigid(const BodyBufs& b, const uint8_t* has_collsn, const double4_32a* av, cudaStream_t s) {
