@@ -831,14 +831,20 @@ __global__ void k_traverse_rope(int n, const RopeNode* __restrict__ rn, const in
 // consecutive queries with one atomic. A leaf is tested first on its 32-byte
 // FP32 record (outward-rounded box, rope, element), and only a leaf that
 // passes loads its 64-byte exact record. Same pairs as k_traverse_rope.
+// A walk longer than `budget` steps (a large element among small ones: an
+// obstacle's side over a sheet) is one long chain of dependent loads that the
+// whole pass would wait for: it is handed over, with the first sorted leaf
+// it has not reached, to k_traverse_warp. Strings over a 12-triangle box:
+// 0.94 ms per traversal without.
 __global__ void __launch_bounds__(128) k_traverse_rope_dyn(
     int n, const RopeNode* __restrict__ rn, const int* __restrict__ elem_scene, const SceneRun* __restrict__ run,
     const int* __restrict__ ev, int2* pairs, int cap, PassCounters* ctr, const Box6* __restrict__ box_static,
     const LeafRec* __restrict__ leaves, const LeafBox32* __restrict__ leaf32, const int* __restrict__ sub, int nsub,
-    const int* __restrict__ dnsub, int* qnext, int refill) {
+    const int* __restrict__ dnsub, int* qnext, int refill, int budget, int2* heavy,
+    const int* __restrict__ range_lo) {
     const int nq = sub ? (dnsub ? *dnsub : nsub) : n - 1;
     const unsigned lane_lt = (1u << (threadIdx.x & 31)) - 1u;
-    int x = kRopeEnd, ei = -1, steps = 0;
+    int x = kRopeEnd, ei = -1, steps = 0, qi = -1;
     int pi0 = -1, pi1 = -1, pi2 = -1;
     BoxOrd qo, qs;
     Box32 q32;
@@ -878,14 +884,18 @@ __global__ void __launch_bounds__(128) k_traverse_rope_dyn(
                         if (box_static) qs = box_ord(box_static[ei]);
                         x = __float_as_int(__ldg(reinterpret_cast<const float*>(&leaf32[i]) + 6));
                         steps = 0;
+                        qi = i;
                     }
                 }
             }
         }
         if (!more && __all_sync(0xffffffffu, x == kRopeEnd)) break;
         if (x == kRopeEnd) continue;
-        if (++steps > 2 * n) {
-            atomicOr(&ctr->err, kErrIndexNode);
+        if (++steps > budget) {  // one entry per query: fits
+            if (x < n - 1 && ~x < n)
+                heavy[atomicAdd(qnext + 1, 1)] = make_int2(qi, x >= 0 ? range_lo[x] : ~x);
+            else
+                atomicOr(&ctr->err, kErrIndexNode);
             x = kRopeEnd;
             continue;
         }
@@ -1042,26 +1052,68 @@ __global__ void k_traverse_rope_full(int n, const RopeNode* __restrict__ rn, con
     }
 }
 
-// The pruned traversal with one warp per dirty element: the walk from the
-// scene's root keeps its pending nodes in a shared-memory stack, and each
-// round the lanes take up to 32 of them at once, test both children of each
-// (the node record holds their FP32 boxes), test the overlapping leaves
-// exactly and push the overlapping internal children. A walk then takes
-// about as many rounds as the tree is deep, instead of one dependent load
-// per visited node. Same pairs as k_traverse_rope_full.
+// Walks with one warp per query: pending nodes and leaves in a shared-memory
+// stack, and each round the lanes take up to 32 of them - a node's record
+// (its children's FP32 boxes) or a leaf's, 64 bytes either way - push a
+// node's overlapping children and test a leaf exactly. A walk then takes
+// about as many rounds as the tree is deep, a load each, instead of one
+// dependent load per visited node. Pairs are staged in shared memory and
+// written 32 at a time, one counter add for each batch (an add per round that
+// finds one costs as much as the round's load).
+//
+// A query's walk covers its scene's leaves from sorted leaf `first` on:
+//   kWalkAll     every leaf of the pass queries (sub, or 0 .. n - 2), from the
+//                leaf after its own: each pair once. For hierarchies of at
+//                most kWarpWalkMax leaves, where a thread's chain is what a
+//                pass waits for (sheet of 3,300 leaves: 110 us with
+//                k_traverse_rope_dyn) and the chip has the warps;
+//   kWalkHeavy   the walks k_traverse_rope_dyn handed over;
+//   kWalkPruned  the dirty elements of a pruned pass (k_dirty_queries), over
+//                all leaves of their scenes: every overlapping leaf that is
+//                not itself, shares no point with it, and is clean or dirty
+//                with a larger element id. Same pairs as k_traverse_rope_full.
 constexpr int kPrunedWarps = 4;     // warps per block
-constexpr int kWarpStack = 2048;    // pending nodes per warp
+constexpr int kWarpStack = 2048;    // pending nodes and leaves per warp
+constexpr int kWalkStage = 64;      // staged pairs per warp
+constexpr int kNoEntry = (int)0x80000000;
+enum WalkKind { kWalkAll, kWalkHeavy, kWalkPruned };
 
-__global__ void __launch_bounds__(kPrunedWarps * 32) k_traverse_warp_full(
+template <int KIND>
+__global__ void __launch_bounds__(kPrunedWarps * 32) k_traverse_warp(
     int n, const BvhNode32* __restrict__ node, const int* __restrict__ elem_scene, const SceneRun* __restrict__ run,
-    const int* __restrict__ ev, int2* pairs, int cap, PassCounters* ctr, const LeafRec* __restrict__ leaves,
-    const int* __restrict__ query, const LoopCtl* __restrict__ L, const uint8_t* __restrict__ edirty) {
+    const int* __restrict__ ev, int2* pairs, int cap, PassCounters* ctr, const Box6* __restrict__ box_static,
+    const LeafRec* __restrict__ leaves, const int* __restrict__ query, int nquery, const int* __restrict__ dnquery,
+    const int2* __restrict__ heavy, const LoopCtl* __restrict__ L, const uint8_t* __restrict__ edirty) {
     __shared__ int s_stk[kPrunedWarps][kWarpStack];
+    __shared__ int2 s_out[kPrunedWarps][kWalkStage];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned lane_lt = (1u << lane) - 1u;
     int* stk = s_stk[w];
-    const int m = L->prune ? L->nquery : 0;
+    int2* out = s_out[w];
+    const int m = KIND == kWalkPruned ? (L->prune ? L->nquery : 0) : dnquery ? *dnquery : nquery;
+    int nout = 0;  // staged pairs, the same in every lane
+    auto flush = [&](int count) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&ctr->npairs, count);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int k = lane; k < count; k += 32) {
+            if (base + k < cap)
+                pairs[base + k] = out[k];
+            else
+                atomicOr(&ctr->err, kErrPairOverflow);
+        }
+        __syncwarp();
+    };
     for (int t = blockIdx.x * kPrunedWarps + w; t < m; t += gridDim.x * kPrunedWarps) {
-        const int i = query[t];
+        int i, first = 0;
+        if (KIND == kWalkHeavy) {
+            const int2 h = heavy[t];
+            i = h.x;
+            first = h.y;
+        } else {
+            i = query ? query[t] : t;
+            if (KIND == kWalkAll) first = i + 1;
+        }
         if (i < 0 || i >= n) {
             if (lane == 0) atomicOr(&ctr->err, kErrIndexLeaf);
             continue;
@@ -1069,13 +1121,17 @@ __global__ void __launch_bounds__(kPrunedWarps * 32) k_traverse_warp_full(
         const LeafRec r = leaves[i];
         const int ei = r.e;
         if (ei < 0) continue;  // flagged by k_leaf_records
-        const SceneRun sr = run[elem_scene[ei]];
-        if (sr.mode == kSceneIdle || sr.root < 0) continue;
-        if (sr.root >= n - 1) {
+        int root = 0;
+        if (run) {
+            const SceneRun sr = run[elem_scene[ei]];
+            if (sr.mode == kSceneIdle || sr.root < 0) continue;
+            root = sr.root;
+        }
+        if (root >= n - 1) {
             if (lane == 0) atomicOr(&ctr->err, kErrIndexNode);
             continue;
         }
-        BoxOrd qo;
+        BoxOrd qo, qs;
         Box6 q;
         for (int d = 0; d < 3; ++d) {
             qo.lo[d] = r.lo[d];
@@ -1083,77 +1139,88 @@ __global__ void __launch_bounds__(kPrunedWarps * 32) k_traverse_warp_full(
             q.lo[d] = unord_double(r.lo[d]);
             q.hi[d] = unord_double(r.hi[d]);
         }
-        const int pi0 = r.p[0], pi1 = r.p[1], pi2 = r.p[2];
+        if (KIND != kWalkPruned && box_static) qs = box_ord(box_static[ei]);
+        const int pi0 = ev ? r.p[0] : -1, pi1 = ev ? r.p[1] : -1, pi2 = ev ? r.p[2] : -1;
         const Box32 q32 = box32_out(q);
         __syncwarp();
-        if (lane == 0) stk[0] = sr.root;
+        if (lane == 0) stk[0] = root;
         __syncwarp();
         int sp = 1;  // the same in every lane
         for (int rounds = 0; sp > 0; ++rounds) {
-            if (rounds >= 2 * n) {  // a valid hierarchy has fewer nodes than that
+            if (rounds >= 4 * n) {  // a valid hierarchy has fewer nodes and leaves than that
                 if (lane == 0) atomicOr(&ctr->err, kErrIndexNode);
                 break;
             }
-            const int take = sp < 32 ? sp : 32;
-            const int x = lane < take ? stk[sp - take + lane] : -1;
-            __syncwarp();
-            sp -= take;
-            int push[2] = {-1, -1};
-            if (x >= 0) {
-                const float4* r4 = reinterpret_cast<const float4*>(&node[x]);
-                Box32 cb[2];
-                unpack(__ldg(r4), __ldg(r4 + 1), __ldg(r4 + 2), cb[0], cb[1]);
-                const int4 meta = __ldg(reinterpret_cast<const int4*>(r4 + 3));
-                const int cs[2] = {meta.x, meta.y};
-                for (int k = 0; k < 2; ++k) {
-                    if (!overlap32(q32, cb[k])) continue;
-                    const int c = cs[k];
-                    if (c >= 0) {
-                        if (c >= n - 1) atomicOr(&ctr->err, kErrIndexNode);
-                        else push[k] = c;
-                        continue;
-                    }
-                    const int kl = ~c;
-                    if (kl >= n) {
-                        atomicOr(&ctr->err, kErrIndexLeaf);
-                        continue;
-                    }
-                    if (kl == i) continue;
-                    const ulonglong2* lr = reinterpret_cast<const ulonglong2*>(&leaves[kl]);
-                    const ulonglong2 u0 = __ldg(lr), u1 = __ldg(lr + 1), u2 = __ldg(lr + 2);
-                    if (!(qo.lo[0] <= u1.y && qo.hi[0] >= u0.x && qo.lo[1] <= u2.x && qo.hi[1] >= u0.y &&
-                          qo.lo[2] <= u2.y && qo.hi[2] >= u1.x))
-                        continue;
-                    const int4 pe = __ldg(reinterpret_cast<const int4*>(lr + 3));
-                    const int ej = pe.w;
-                    if (ej < 0) continue;
-                    if (ev && (pe.x == pi0 || pe.x == pi1 || pe.x == pi2 || pe.y == pi0 || pe.y == pi1 ||
-                               pe.y == pi2 || (pe.z >= 0 && (pe.z == pi0 || pe.z == pi1 || pe.z == pi2))))
-                        continue;
-                    if (edirty[ej] && ej < ei) continue;  // written by ej's query
-                    emit_pair(ei, ej, pairs, cap, ctr);
-                }
-            }
-            // push the overlapping internal children (exclusive prefix over the lanes)
-            const int cnt = (push[0] >= 0) + (push[1] >= 0);
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            if (sp + total > kWarpStack) {  // the same in every lane: the walk stops with an error
+            // a nearly full stack takes fewer (each may push two)
+            const int take = min(min(sp, 32), kWarpStack - sp);
+            if (take <= 0) {
                 if (lane == 0) atomicOr(&ctr->err, kErrStack);
                 break;
             }
-            int at = sp + incl - cnt;
-            if (push[0] >= 0) stk[at++] = push[0];
-            if (push[1] >= 0) stk[at] = push[1];
-            sp += total;
+            const int x = lane < take ? stk[sp - take + lane] : kNoEntry;
+            __syncwarp();
+            sp -= take;
+            int push[2] = {kNoEntry, kNoEntry};
+            int2 pair = make_int2(-1, -1);
+            if (x != kNoEntry) {
+                const float4* p4 = x >= 0 ? reinterpret_cast<const float4*>(&node[x])
+                                          : reinterpret_cast<const float4*>(&leaves[~x]);
+                const float4 v0 = __ldg(p4), v1 = __ldg(p4 + 1), v2 = __ldg(p4 + 2);
+                const int4 v3 = __ldg(reinterpret_cast<const int4*>(p4 + 3));
+                if (x >= 0) {
+                    Box32 cb[2];
+                    unpack(v0, v1, v2, cb[0], cb[1]);
+                    const int cs[2] = {v3.x, v3.y}, last[2] = {v3.z, v3.w};
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const int c = cs[k];
+                        if (last[k] < first || !overlap32(q32, cb[k]) || ~c == i) continue;
+                        if (c >= 0 ? c >= n - 1 : ~c >= n)
+                            atomicOr(&ctr->err, c >= 0 ? kErrIndexNode : kErrIndexLeaf);
+                        else
+                            push[k] = c;
+                    }
+                } else {
+                    auto u64 = [](float a, float b) {
+                        return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
+                    };
+                    // the exact test on the encoded boxes (lo x y z, hi x y z)
+                    if (qo.lo[0] <= u64(v1.z, v1.w) && qo.hi[0] >= u64(v0.x, v0.y) && qo.lo[1] <= u64(v2.x, v2.y) &&
+                        qo.hi[1] >= u64(v0.z, v0.w) && qo.lo[2] <= u64(v2.z, v2.w) && qo.hi[2] >= u64(v1.x, v1.y)) {
+                        const int ej = v3.w;
+                        const bool shared = ev && (v3.x == pi0 || v3.x == pi1 || v3.x == pi2 || v3.y == pi0 ||
+                                                   v3.y == pi1 || v3.y == pi2 ||
+                                                   (v3.z >= 0 && (v3.z == pi0 || v3.z == pi1 || v3.z == pi2)));
+                        if (ej >= 0 && !shared) {  // ej < 0: flagged by k_leaf_records
+                            if (KIND == kWalkPruned) {
+                                if (!(edirty[ej] && ej < ei)) pair = make_int2(ei, ej);  // else written by ej's query
+                            } else {
+                                pair = make_int2(
+                                    ei, (box_static && overlap_ord(qs, &box_static[ej])) ? (ej | kPairStatic) : ej);
+                            }
+                        }
+                    }
+                }
+            }
+            const unsigned b0 = __ballot_sync(0xffffffffu, push[0] != kNoEntry);
+            const unsigned b1 = __ballot_sync(0xffffffffu, push[1] != kNoEntry);
+            if (push[0] != kNoEntry) stk[sp + __popc(b0 & lane_lt)] = push[0];
+            if (push[1] != kNoEntry) stk[sp + __popc(b0) + __popc(b1 & lane_lt)] = push[1];
+            sp += __popc(b0) + __popc(b1);
+            const unsigned found = __ballot_sync(0xffffffffu, pair.x >= 0);
+            if (found) {
+                if (pair.x >= 0) out[nout + __popc(found & lane_lt)] = pair;
+                nout += __popc(found);
+                __syncwarp();
+                if (nout > kWalkStage - 32) {
+                    flush(nout);
+                    nout = 0;
+                }
+            }
             __syncwarp();
         }
     }
+    if (nout) flush(nout);
 }
 
 __global__ void k_brute_pairs(const Box6* __restrict__ box, int n, const int* __restrict__ elem_scene, int2* pairs,
@@ -1271,6 +1338,12 @@ void launch_stack_traverse(const Box6* box, const BvhBufs& b, int nq, int block,
                                                         b.nsub, dq);
 }
 
+// Hierarchies of at most this many leaves are walked with a warp per query;
+// larger ones with a lane per query, walks of more than kHeavySteps steps
+// handed over to a warp.
+constexpr int kWarpWalkMax = 32768;
+constexpr int kHeavySteps = 192;
+
 // Resident blocks of the dynamic-fetch traversal per SM, looked up once.
 int dyn_blocks_per_sm() {
     static int cached = 0;
@@ -1290,13 +1363,21 @@ void bvh_pairs(const Box6* box, const BvhBufs& b, int2* pairs, int cap, PassCoun
     if (n <= 1) return;
     const int nleaf = b.sub ? b.nsub : n, nq = b.sub ? b.nsub : n - 1;
     if (nq <= 0) return;
+    // the stackless traversal with dynamic query fetch, or in its place, for
+    // small hierarchies, a warp per query
     const bool dyn = b.leaf && rope && b.rnode && b.rope && b.leaf32 && b.qnext && refill > 0;
+    const bool by_warp = dyn && n <= kWarpWalkMax;
     const int* dnsub = b.sub ? b.dnsub : nullptr;
     const int* dq = b.sub ? (b.dnq ? b.dnq : b.dnsub) : nullptr;  // queries of the traversal
     if (b.leaf)
         count_launch(), k_leaf_records<<<dnsub ? dev_grid(nleaf, 256) : nblk(nleaf, 256), 256, 0, s>>>(
-            box, b.order, n, b.sub, b.nsub, dnsub, b.ev, b.leaf, b.ne_all, ctr, b.rope, dyn ? b.leaf32 : nullptr);
-    if (dyn) {
+            box, b.order, n, b.sub, b.nsub, dnsub, b.ev, b.leaf, b.ne_all, ctr, b.rope, dyn && !by_warp ? b.leaf32 : nullptr);
+    const int wblocks = dev_grid(nq, kPrunedWarps);
+    if (by_warp) {
+        count_launch(), k_traverse_warp<kWalkAll><<<wblocks, kPrunedWarps * 32, 0, s>>>(
+            n, b.node, b.elem_scene, b.run, skip_shared_ev, pairs, cap, ctr, box_static, b.leaf, b.sub, nq, dq, nullptr,
+            nullptr, nullptr);
+    } else if (dyn) {
         static int num_sms = 0;
         if (!num_sms) {
             int dev = 0;
@@ -1306,11 +1387,15 @@ void bvh_pairs(const Box6* box, const BvhBufs& b, int2* pairs, int cap, PassCoun
         int blocks = num_sms * dyn_blocks_per_sm();
         const int need = nblk(nq, 128);
         if (blocks > need) blocks = need;
-        cudaMemsetAsync(b.qnext, 0, sizeof(int), s);
+        cudaMemsetAsync(b.qnext, 0, 2 * sizeof(int), s);
         count_launch(), k_traverse_rope_dyn<<<blocks, 128, 0, s>>>(n, b.rnode, b.elem_scene, b.run, skip_shared_ev,
                                                                    pairs, cap, ctr, box_static, b.leaf, b.leaf32,
                                                                    b.sub, b.nsub, dq, b.qnext,
-                                                                   refill > 32 ? 32 : refill);
+                                                                   refill > 32 ? 32 : refill, kHeavySteps, b.heavy,
+                                                                   b.range_lo);
+        count_launch(), k_traverse_warp<kWalkHeavy><<<wblocks, kPrunedWarps * 32, 0, s>>>(
+            n, b.node, b.elem_scene, b.run, skip_shared_ev, pairs, cap, ctr, box_static, b.leaf, nullptr, 0,
+            b.qnext + 1, b.heavy, nullptr, nullptr);
     } else if (b.leaf && rope && b.rnode && b.rope) {
         count_launch(), k_traverse_rope<<<dq ? dev_grid(nq, block) : nblk(nq, block), block, 0, s>>>(
             n, b.rnode, b.rope, b.elem_scene, b.run, skip_shared_ev, pairs, cap, ctr, box_static, b.leaf, b.sub,
@@ -1336,8 +1421,9 @@ void pruned_pairs(const BvhBufs& b, const int* act_e, const int* act_l, const un
     count_launch(), k_dirty_queries<<<dev_grid(ne_cap, 256), 256, 0, s>>>(act_l, b.order, b.n, b.ne_all, ev, stamp, L,
                                                                           edirty, query, ctr);
     if (warp && b.node)
-        count_launch(), k_traverse_warp_full<<<dev_grid(ne_cap, kPrunedWarps), kPrunedWarps * 32, 0, s>>>(
-            b.n, b.node, b.elem_scene, b.run, ev, pairs, cap, ctr, b.leaf, query, L, edirty);
+        count_launch(), k_traverse_warp<kWalkPruned><<<dev_grid(ne_cap, kPrunedWarps), kPrunedWarps * 32, 0, s>>>(
+            b.n, b.node, b.elem_scene, b.run, ev, pairs, cap, ctr, nullptr, b.leaf, query, 0, nullptr, nullptr, L,
+            edirty);
     else
         count_launch(), k_traverse_rope_full<<<dev_grid(ne_cap, 128), 128, 0, s>>>(
             b.n, b.rnode, b.rope, b.elem_scene, b.run, ev, pairs, cap, ctr, b.leaf, query, L, edirty);

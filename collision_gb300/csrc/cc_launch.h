@@ -121,9 +121,12 @@ struct BvhBufs {
     RopeNode* rnode;  // n-1
     int* rope;        // n-1
     // optional: the FP32 leaf boxes of the stackless traversal with dynamic
-    // query fetch, written with the leaf records; qnext: its query counter
+    // query fetch, written with the leaf records; qnext: its query counter and
+    // that of the walks it hands over; heavy: those walks (query leaf, first
+    // leaf not reached), one per leaf at most
     LeafBox32* leaf32;
     int* qnext;
+    int2* heavy;
     // optional: for a hierarchy over all elements (act null), the sorted
     // leaves of the scenes in this pass; the refit, the leaf records and the
     // traversal then cover only those (walks never leave their scene)
@@ -174,7 +177,8 @@ void bvh_refit(const Box6* box, BvhBufs& b, cudaStream_t s, bool roots = true);
 // the leaf records and rope nodes present) stackless along the ropes.
 // refill (rope only, with leaf32 and qnext present): persistent warps whose
 // lanes take new queries from a counter once `refill` of them have finished
-// their walks (0: one thread per query). stack_depth: entries of the
+// their walks, walks of many steps continued by a warp each, and a warp per
+// query where the hierarchy is small (0: one thread per query). stack_depth: entries of the
 // per-thread stack of the stack traversal (24, 32, 48 or 64); a walk that
 // needs more sets kErrStack.
 void bvh_pairs(const Box6* box, const BvhBufs& b, int2* pairs, int cap, PassCounters* ctr, cudaStream_t s,
@@ -400,7 +404,7 @@ void pass_end(const PassCounters* c, SceneCtl* ctl, const SceneRun* run, int nsc
 // such an element is written once. act_l: the pass's sorted leaves
 // (L->nact_e of them; act_e is unused); edirty, query: ne_cap each.
 // warp: one warp per dirty element walking with a shared-memory stack
-// (k_traverse_warp_full); otherwise one thread along the ropes.
+// (k_traverse_warp); otherwise one thread along the ropes.
 void pruned_pairs(const BvhBufs& b, const int* act_e, const int* act_l, const unsigned* stamp, LoopCtl* L,
                   uint8_t* edirty, int* query, int ne_cap, int2* pairs, int cap, PassCounters* ctr, const int* ev,
                   cudaStream_t s, bool warp = true);

@@ -518,7 +518,7 @@ struct cc_solver {
         dfree(d_xold_in); dfree(d_xcand_in); dfree(d_vel); dfree(d_xout); dfree(d_hc);
         dfree(d_box); dfree(d_box_st); dfree(bvh.keys); dfree(bvh.order); dfree(bvh.range_hi);
         dfree(bvh.range_lo); dfree(bvh.parent); dfree(bvh.flags); dfree(bvh.node); dfree(bvh.bbox_enc); dfree(bvh.leaf);
-        dfree(bvh.rnode); dfree(bvh.rope); dfree(bvh.leaf32); dfree(bvh.qnext);
+        dfree(bvh.rnode); dfree(bvh.rope); dfree(bvh.leaf32); dfree(bvh.qnext); dfree(bvh.heavy);
         if (bvh.sort_temp) cudaFree(bvh.sort_temp);
         bvh = BvhBufs{};
         dfree(d_pairs); dfree(d_contrib); dfree(d_pair_hit); dfree(d_pairq); dfree(d_sub_pt); dfree(d_sub_ee);
@@ -1186,7 +1186,8 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     ok &= dalloc(&bvh.rnode, (size_t)ne) == cudaSuccess;
     ok &= dalloc(&bvh.rope, (size_t)ne) == cudaSuccess;
     ok &= dalloc(&bvh.leaf32, (size_t)ne) == cudaSuccess;
-    ok &= dalloc(&bvh.qnext, 1) == cudaSuccess;
+    ok &= dalloc(&bvh.qnext, 2) == cudaSuccess;
+    ok &= dalloc(&bvh.heavy, (size_t)ne) == cudaSuccess;
     ok &= dalloc(&bvh.bbox_enc, 6 * (size_t)n) == cudaSuccess;
     ok &= cudaMalloc(&bvh.sort_temp, radix_sort_temp_bytes(ne > 0 ? ne : 1)) == cudaSuccess;
     ok &= dalloc(&apply.cnt, (size_t)nv + nbodies) == cudaSuccess;
