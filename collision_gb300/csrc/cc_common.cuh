@@ -184,6 +184,8 @@ struct PassCounters {
     int nzones;       // impact zones listed for the zone solve (impact-zone passes)
     int nmembers;     // their members
     int nseg;         // union-record segments, one per zone the pass's unions touch
+    int ntouch;       // points and bodies with contributions
+    int nseg_used;    // contributions given to their segments so far
 };
 
 // The device-resident detection loop's own state.

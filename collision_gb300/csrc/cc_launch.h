@@ -287,11 +287,12 @@ struct BodyBufs {
     const uint8_t* fixed = nullptr;
 };
 struct ApplyBufs {
-    int* cnt;      // nv + bodies
+    int* cnt;      // nv + bodies; zero between passes
     int* off;      // nv + bodies
-    int* cur;      // nv + bodies
+    int* cur;      // nv + bodies; zero between passes
+    int* touched;  // nv + bodies: those with contributions
     int* idx;      // contrib_cap
-    void* scan_temp;
+    int* ord;      // contrib_cap
     PassStamp ps;  // stamps of the points whose velocity the pass changes
 };
 // Per-point sums of the pass's contributions in visiting order, then

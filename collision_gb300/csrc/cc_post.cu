@@ -32,13 +32,28 @@ __global__ void k_step_init(const double* __restrict__ x_old, const double* __re
     av[p] = make_double4_32a(v[0], v[1], v[2], 0.0);
 }
 
-__global__ void k_contrib_count(const Contrib* __restrict__ c, const PassCounters* ctr, int cap, int* cnt) {
+// Contributions by point: counted, with the points that have any listed ...
+__global__ void k_contrib_count(const Contrib* __restrict__ c, PassCounters* ctr, int cap, int* cnt, int* touched) {
     if (ctr->err & kErrRetry) return;
     int n = ctr->ncontrib < cap ? ctr->ncontrib : cap;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        atomicAdd(&cnt[c[i].vertex], 1);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int v = c[i].vertex;
+        if (atomicAdd(&cnt[v], 1) == 0) touched[aggregated_add(&ctr->ntouch, 1)] = v;
+    }
 }
 
+// ... given a segment each (in any order) ...
+__global__ void k_contrib_segments(PassCounters* ctr, const int* __restrict__ cnt, const int* __restrict__ touched,
+                                   int* off) {
+    if (ctr->err & kErrRetry) return;
+    const int n = ctr->ntouch;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int v = touched[t];
+        off[v] = aggregated_add(&ctr->nseg_used, cnt[v]);
+    }
+}
+
+// ... and listed there.
 __global__ void k_contrib_scatter(const Contrib* __restrict__ c, const PassCounters* ctr, int cap,
                                   const int* __restrict__ off, int* cur, int* idx) {
     if (ctr->err & kErrRetry) return;
@@ -49,63 +64,92 @@ __global__ void k_contrib_scatter(const Contrib* __restrict__ c, const PassCount
     }
 }
 
-// updateAverageVelocity, dcollid.cpp:677-751, for one point: its
-// contributions are put in visiting order and summed one by one from zero,
-// as the reference accumulates collsnImpulse and friction. Slots nv.. are
-// the movable bodies: their spread impulses are added one by one onto the
+// updateAverageVelocity, dcollid.cpp:677-751, one warp per point with
+// contributions: they are put in visiting order and summed one by one from
+// zero, as the reference accumulates collsnImpulse and friction. Slots nv..
+// are the movable bodies: their spread impulses are added one by one onto the
 // body's running collsnImpulse_RG, which the reference never clears, and
 // their count is the pass's collsn_num_RG.
-__global__ void k_apply(const Contrib* __restrict__ c, PassCounters* ctr, const int* __restrict__ cnt,
-                        const int* __restrict__ off, int* idx, int nv, double4_32a* av, uint8_t* has_collsn,
-                        double4_32a* dump, int nbodies, double4_32a* body_acc, int* body_num, PassStamp ps) {
+//
+// The order: each lane ranks its contributions' keys against all of the
+// point's, in shared memory for up to kApplyStage (one thread's insertion
+// sort loaded two dependent values per comparison: 1.7 ms for a folding
+// sheet's proximity pass, whose points meet up to hundreds of sub-tests).
+// The sums: lanes 0..2 add the impulse's components and lanes 3..5 the
+// friction's, in order. The point's counters are left zero for the next pass.
+constexpr int kApplyWarps = 4;
+constexpr int kApplyStage = 256;
+__global__ void __launch_bounds__(kApplyWarps * 32) k_apply(
+    const Contrib* __restrict__ c, PassCounters* ctr, int* cnt, int* cur, const int* __restrict__ off,
+    const int* __restrict__ touched, const int* __restrict__ idx, int* ord, int nv, double4_32a* av,
+    uint8_t* has_collsn, double4_32a* dump, double4_32a* body_acc, int* body_num, PassStamp ps) {
+    __shared__ unsigned long long s_key[kApplyWarps][kApplyStage];
+    __shared__ int s_ord[kApplyWarps][kApplyStage];
     if (ctr->err & kErrRetry) return;
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= nv + nbodies) return;
-    int n = cnt[p];
-    if (n == 0) return;
-    int* seg = idx + off[p];
-    // insertion sort of the segment by key (segments are short)
-    for (int i = 1; i < n; ++i) {
-        int x = seg[i];
-        unsigned long long kx = c[x].key;
-        int j = i - 1;
-        while (j >= 0 && c[seg[j]].key > kx) {
-            seg[j + 1] = seg[j];
-            --j;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int m = ctr->ntouch;
+    for (int t = blockIdx.x * kApplyWarps + w; t < m; t += gridDim.x * kApplyWarps) {
+        const int p = touched[t], n = cnt[p], o = off[p];
+        const bool staged = n <= kApplyStage;
+        unsigned long long* key = s_key[w];
+        int* order = staged ? s_ord[w] : ord + o;
+        __syncwarp();
+        if (lane == 0) cnt[p] = cur[p] = 0;
+        if (n == 1) {
+            if (lane == 0) order[0] = idx[o];
+        } else {
+            if (staged)
+                for (int i = lane; i < n; i += 32) key[i] = c[idx[o + i]].key;
+            __syncwarp();
+            for (int i = lane; i < n; i += 32) {
+                const int x = idx[o + i];
+                const unsigned long long kx = staged ? key[i] : c[x].key;
+                int r = 0;
+                for (int j = 0; j < n; ++j) {
+                    const unsigned long long kj = staged ? key[j] : c[idx[o + j]].key;
+                    r += kj < kx || (kj == kx && j < i);
+                }
+                order[r] = x;
+            }
         }
-        seg[j + 1] = x;
-    }
-    if (p >= nv) {
-        const int b = p - nv;
-        double4_32a a = body_acc[b];
-        double acc[3] = {a.x, a.y, a.z};
-        for (int i = 0; i < n; ++i) {
-            const Contrib& q = c[seg[i]];
-            for (int k = 0; k < 3; ++k) acc[k] += q.imp[k];
+        __syncwarp();
+        const bool body = p >= nv;
+        double acc = 0.0;
+        if (body && lane < 3) {
+            const double4_32a a = body_acc[p - nv];
+            acc = lane == 0 ? a.x : lane == 1 ? a.y : a.z;
         }
-        body_acc[b] = make_double4_32a(acc[0], acc[1], acc[2], 0.0);
-        body_num[b] = n;
-        return;
+        if (lane < (body ? 3 : 6)) {
+#pragma unroll 4
+            for (int i = 0; i < n; ++i) {
+                const Contrib& q = c[order[i]];
+                const double x = lane < 3 ? q.imp[lane] : q.fric[lane - 3];
+                if (lane < 3 || (q.flags & 1)) acc += x;
+            }
+        }
+        double imp[3], fric[3];
+        for (int k = 0; k < 3; ++k) {
+            imp[k] = __shfl_sync(0xffffffffu, acc, k);
+            fric[k] = __shfl_sync(0xffffffffu, acc, 3 + k);
+        }
+        if (lane == 0 && body) {
+            body_acc[p - nv] = make_double4_32a(imp[0], imp[1], imp[2], 0.0);
+            body_num[p - nv] = n;
+        } else if (lane == 0) {
+            double4_32a a = av[p];
+            double v[3] = {a.x, a.y, a.z};
+            bool bad = false;
+            for (int k = 0; k < 3; ++k) {
+                v[k] += (imp[k] + fric[k]) / n;
+                if (!isfinite(v[k])) bad = true;
+            }
+            if (bad) atomicOr(&ctr->err, kErrNan);
+            av[p] = make_double4_32a(v[0], v[1], v[2], 0.0);
+            has_collsn[p] = 1;
+            stamp_point(ps, p);
+            if (dump) dump[p] = make_double4_32a(imp[0], imp[1], imp[2], (double)n);  // collsnImpulse, collsn_num
+        }
     }
-    double imp[3] = {0.0, 0.0, 0.0}, fric[3] = {0.0, 0.0, 0.0};
-    for (int i = 0; i < n; ++i) {
-        const Contrib& q = c[seg[i]];
-        for (int k = 0; k < 3; ++k) imp[k] += q.imp[k];
-        if (q.flags & 1)
-            for (int k = 0; k < 3; ++k) fric[k] += q.fric[k];
-    }
-    double4_32a a = av[p];
-    double v[3] = {a.x, a.y, a.z};
-    bool bad = false;
-    for (int k = 0; k < 3; ++k) {
-        v[k] += (imp[k] + fric[k]) / n;
-        if (!isfinite(v[k])) bad = true;
-    }
-    if (bad) atomicOr(&ctr->err, kErrNan);
-    av[p] = make_double4_32a(v[0], v[1], v[2], 0.0);
-    has_collsn[p] = 1;
-    stamp_point(ps, p);
-    if (dump) dump[p] = make_double4_32a(imp[0], imp[1], imp[2], (double)n);  // collsnImpulse, collsn_num
 }
 
 // The spread part of updateAverageVelocity (dcollid.cpp:726-733), after
@@ -583,18 +627,19 @@ void apply_contribs(const Contrib* contrib, const PassCounters* ctr, int contrib
     if (dump && nv > 0) cudaMemsetAsync(dump, 0, sizeof(double4_32a) * (size_t)nv, s);
     if (nv <= 0) return;
     const int nb = bodies ? bodies->n : 0, nslot = nv + nb;
-    cudaMemsetAsync(b.cnt, 0, sizeof(int) * (size_t)nslot, s);
-    cudaMemsetAsync(b.cur, 0, sizeof(int) * (size_t)nslot, s);
     if (nb > 0) cudaMemsetAsync(bodies->num, 0, sizeof(int) * (size_t)nb, s);
     int blocks = nblk(contrib_cap, 256);
     if (blocks > 152 * 8) blocks = 152 * 8;
-    count_launch(), k_contrib_count<<<blocks, 256, 0, s>>>(contrib, ctr, contrib_cap, b.cnt);
-    exclusive_scan(b.cnt, b.off, nslot, nullptr, b.scan_temp, s);
+    PassCounters* c = const_cast<PassCounters*>(ctr);
+    count_launch(), k_contrib_count<<<blocks, 256, 0, s>>>(contrib, c, contrib_cap, b.cnt, b.touched);
+    const int sblocks = nblk(nslot, 256) < 152 * 8 ? nblk(nslot, 256) : 152 * 8;
+    count_launch(), k_contrib_segments<<<sblocks, 256, 0, s>>>(c, b.cnt, b.touched, b.off);
     count_launch(), k_contrib_scatter<<<blocks, 256, 0, s>>>(contrib, ctr, contrib_cap, b.off, b.cur, b.idx);
-    count_launch(), k_apply<<<nblk(nslot, 128), 128, 0, s>>>(contrib, const_cast<PassCounters*>(ctr), b.cnt, b.off,
-                                                             b.idx, nv, av, has_collsn, dump, nb,
-                                                             nb ? bodies->acc : nullptr, nb ? bodies->num : nullptr,
-                                                             b.ps);
+    const int ablocks = nblk(nslot, kApplyWarps) < 152 * 8 ? nblk(nslot, kApplyWarps) : 152 * 8;
+    count_launch(), k_apply<<<ablocks, kApplyWarps * 32, 0, s>>>(contrib, c, b.cnt, b.cur, b.off, b.touched, b.idx,
+                                                                 b.ord, nv, av, has_collsn, dump,
+                                                                 nb ? bodies->acc : nullptr, nb ? bodies->num : nullptr,
+                                                                 b.ps);
     if (nb > 0)
         count_launch(), k_apply_rg<<<nblk(bodies->nmembers, 128), 128, 0, s>>>(
             bodies->members, bodies->member_body, bodies->nmembers, ctr, bodies->acc, bodies->num, bodies->fixed, av,

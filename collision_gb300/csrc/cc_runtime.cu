@@ -82,7 +82,7 @@ __global__ void k_reset_counters(PassCounters* c) {
     int keep = c->err & kErrNan;
     c->npairs = 0; c->ncontrib = 0; c->nhit_pairs = 0; c->nrec = 0;
     c->nvisits = 0; c->ncontacts = 0; c->nsub = 0; c->ncr = 0; c->nunion = 0; c->nsub_pt = 0; c->nsub_ee = 0; c->npairq = 0;
-    c->nzones = 0; c->nmembers = 0; c->nseg = 0;
+    c->nzones = 0; c->nmembers = 0; c->nseg = 0; c->ntouch = 0; c->nseg_used = 0;
     c->err = keep;
 }
 
@@ -95,7 +95,7 @@ __global__ void k_reset_pass(PassCounters* c, SceneRun* run, int nscenes, int np
         int keep = c->err & kErrNan;
         c->npairs = npairs_keep >= 0 ? npairs_keep : 0; c->ncontrib = 0; c->nhit_pairs = 0; c->nrec = 0;
         c->nvisits = 0; c->ncontacts = 0; c->nsub = 0; c->ncr = 0; c->nunion = 0; c->nsub_pt = 0; c->nsub_ee = 0; c->npairq = 0;
-        c->nzones = 0; c->nmembers = 0; c->nseg = 0;
+        c->nzones = 0; c->nmembers = 0; c->nseg = 0; c->ntouch = 0; c->nseg_used = 0;
         c->err = keep;
     }
     if (i < nscenes) run[i].hits = 0;
@@ -524,8 +524,7 @@ struct cc_solver {
         dfree(d_pairs); dfree(d_contrib); dfree(d_pair_hit); dfree(d_pairq); dfree(d_sub_pt); dfree(d_sub_ee);
         sub_cap = 0;
         dfree(apply.cnt); dfree(apply.off); dfree(apply.cur); dfree(apply.idx);
-        if (apply.scan_temp) cudaFree(apply.scan_temp);
-        apply.scan_temp = nullptr;
+        dfree(apply.touched); dfree(apply.ord);
         dfree(d_rank[0]); dfree(d_rank[1]);
         dfree(d_rec); dfree(d_pbox_lo); dfree(d_pbox_hi); dfree(d_p32); dfree(d_v32);
         dfree(d_act_e); dfree(d_act_p); dfree(d_sel); dfree(d_dump); dfree(d_av_pre);
@@ -614,7 +613,9 @@ struct cc_solver {
         loop_dirty = true;
         dfree(d_contrib);
         dfree(apply.idx);
-        if (dalloc(&d_contrib, (size_t)cap) != cudaSuccess || dalloc(&apply.idx, (size_t)cap) != cudaSuccess)
+        dfree(apply.ord);
+        if (dalloc(&d_contrib, (size_t)cap) != cudaSuccess || dalloc(&apply.idx, (size_t)cap) != cudaSuccess ||
+            dalloc(&apply.ord, (size_t)cap) != cudaSuccess)
             return fail(CC_NO_MEMORY, "contribution buffer");
         contrib_cap = cap;
         return CC_OK;
@@ -1193,7 +1194,7 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     ok &= dalloc(&apply.cnt, (size_t)nv + nbodies) == cudaSuccess;
     ok &= dalloc(&apply.off, (size_t)nv + nbodies) == cudaSuccess;
     ok &= dalloc(&apply.cur, (size_t)nv + nbodies) == cudaSuccess;
-    ok &= cudaMalloc(&apply.scan_temp, scan_temp_bytes(nv + nbodies > 0 ? nv + nbodies : 1)) == cudaSuccess;
+    ok &= dalloc(&apply.touched, (size_t)nv + nbodies) == cudaSuccess;
     if (nbodies > 0) {
         const size_t nm = (size_t)h_body_visit.size();
         ok &= dalloc(&d_vbody, (size_t)nv) == cudaSuccess;
@@ -1287,6 +1288,8 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     strain_bufs.order = d_strain_order;
     strain_bufs.flags = d_strain_flags;
     strain_bufs.passes_out = d_strain_passes;
+    cudaMemsetAsync(apply.cnt, 0, sizeof(int) * (size_t)(nv + nbodies > 0 ? nv + nbodies : 1), stream);
+    cudaMemsetAsync(apply.cur, 0, sizeof(int) * (size_t)(nv + nbodies > 0 ? nv + nbodies : 1), stream);
     cudaMemsetAsync(d_av, 0, sizeof(double4_32a) * (size_t)(nv > 0 ? nv : 1), stream);
     cudaMemsetAsync(d_run, 0, sizeof(SceneRun) * (size_t)n, stream);
     cudaMemsetAsync(d_rank[0], 0, sizeof(int) * (size_t)(ne > 0 ? ne : 1), stream);
