@@ -84,7 +84,7 @@ struct __align__(8) SubRec {
     int scene;
     int p[4];
     int sub;
-    int pad;
+    int counted;  // already counted as evaluated in FP64
 };
 
 // One createImpZone(pts, 4) call of an impact-zone pass (dcollid.cpp:473-484),

@@ -242,7 +242,6 @@ struct NarrowArgs {
     // 1: both sub-test lists in one launch, a warp per sub-test in small
     // passes (k_subtests_all); 0: one launch per list, a thread per sub-test
     int sub_merge = 1;
-    int sub_counted = 0;  // the filter has counted the sub-tests evaluated in FP64 (plain passes)
     // movable rigid bodies: the body of each point (-1 none), each body's
     // mass, and the contribution slot of body 0 (the point count)
     const int* vbody;

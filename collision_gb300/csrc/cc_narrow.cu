@@ -187,10 +187,40 @@ __device__ __forceinline__ bool orient_pair(const NarrowArgs& a, int2 pr, Orient
     return true;
 }
 
+// The points of sub-test `sub` of a pair (for_each_subtest's numbering) and
+// whether it is edge-edge; false past the pair's last.
+template <bool MOVING>
+__device__ __forceinline__ bool pair_subtest(const OrientedPair& o, int sub, int* pts, bool& ee) {
+    const int npt = o.kind == 0 ? 6 : o.kind == 1 ? 2 : 0;
+    const int n = o.kind == 0 ? 15 : o.kind == 1 ? 5 : 1;
+    ee = sub >= npt;
+    if (sub >= n) return false;
+    if (!ee) {
+        // moving: the triangle is A, the point B's, then the reverse; a
+        // triangle against a bond's points only
+        const bool tri_a = o.kind == 1 || (sub < 3) == MOVING;
+        const int i = sub < 3 ? sub : sub - 3;
+        for (int k = 0; k < 3; ++k) pts[k] = tri_a ? o.A[k] : o.B[k];
+        const int* P = tri_a ? o.B : o.A;
+        pts[3] = i == 0 ? P[0] : i == 1 ? P[1] : P[2];
+        return true;
+    }
+    const int e = sub - npt;
+    const int i = o.kind == 2 ? 0 : o.kind == 1 ? e : e / 3, j = o.kind == 0 ? e - 3 * i : 0;
+    pts[0] = i == 0 ? o.A[0] : i == 1 ? o.A[1] : o.A[2];
+    pts[1] = i == 0 ? o.A[1] : i == 1 ? o.A[2] : o.A[0];
+    pts[2] = j == 0 ? o.B[0] : j == 1 ? o.B[1] : o.B[2];
+    pts[3] = j == 0 ? o.B[1] : j == 1 ? o.B[2] : o.B[0];
+    return true;
+}
+
 // Stage 1 of a split pass: per candidate pair, the visit bookkeeping of
 // k_narrow, the element-pair filter, and the box and separating-axis filter
 // of every sub-test, in sub-test order; survivors are queued with their keys,
 // and a pair with survivors is queued for stage 3.
+// Passes of at most this many pairs take filter_wide.
+constexpr int kWideFilter = 131072;
+
 template <bool MOVING>
 __device__ __forceinline__ void queue_sub(const NarrowArgs& a, const NarrowCtx& c, bool ee, unsigned long long kb,
                                           int pair, int sc, const int* pts, int sub, bool& first) {
@@ -215,8 +245,137 @@ __device__ __forceinline__ void queue_sub(const NarrowArgs& a, const NarrowCtx& 
     r.scene = sc;
     for (int i = 0; i < 4; ++i) r.p[i] = pts[i];
     r.sub = sub;
-    r.pad = 0;
+    r.counted = 0;
     (ee ? a.sub_ee : a.sub_pt)[slot] = r;
+}
+
+// Queues the sub-tests of the lanes with `queue` set, sixteen lanes (from lane
+// `group` of the warp) per pair, and once each pair that has some. counted:
+// the sub-test has been counted as evaluated in FP64.
+__device__ __forceinline__ void queue_group(const NarrowArgs& a, bool queue, bool ee, unsigned long long keybase,
+                                            int pair, int scene, const int* pts, int sub, int group, bool counted) {
+    const unsigned in_pair = __ballot_sync(0xffffffffu, queue) >> group & 0xffffu;
+    if (!queue) return;
+    int slot;  // (the lanes that add together share one counter)
+    if (ee)
+        slot = aggregated_add(&a.ctr->nsub_ee, 1);
+    else
+        slot = aggregated_add(&a.ctr->nsub_pt, 1);
+    if (slot >= a.sub_cap) {
+        atomicOr(&a.ctr->err, kErrSubOverflow);
+    } else {
+        SubRec r;
+        r.keybase = keybase;
+        r.pair = pair;
+        r.scene = scene;
+        for (int i = 0; i < 4; ++i) r.p[i] = pts[i];
+        r.sub = sub;
+        r.counted = counted ? 1 : 0;
+        (ee ? a.sub_ee : a.sub_pt)[slot] = r;
+    }
+    if ((in_pair & ((1u << sub) - 1u)) == 0) {  // the pair's first
+        a.pair_hit[pair] = 0;
+        a.pairq[aggregated_add(&a.ctr->npairq, 1)] = pair;
+    }
+}
+
+// pair_may_hit on sixteen lanes (all of the group take part): lane s forms
+// the gap along axis s of the twelve.
+template <bool MOVING>
+__device__ __forceinline__ bool pair_may_hit16(const NarrowCtx& c, const OrientedPair& o, int s) {
+    const int ia[3] = {o.A[0], o.A[1], o.n1 == 3 ? o.A[2] : o.A[1]};
+    const int ib[3] = {o.B[0], o.B[1], o.n2 == 3 ? o.B[2] : o.B[1]};
+    F3 R[6];
+    const F3 X0 = f3(c.p32[ia[0]]);
+    float M = fmaxabs(X0), L = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        F3 x = q < 3 ? f3(c.p32[ia[q]]) : f3(c.p32[ib[q - 3]]);
+        M = fmaxf(M, fmaxabs(x));
+        R[q] = fsub(x, X0);
+        L = fmaxf(L, fnorm(R[q]));
+    }
+    // axis 0 the line between the centroids; 1..4 and 5..8 each element's
+    // normal and in-plane edge normals; 9..11 the first edges' common normal
+    // and the in-plane normals of each
+    float lb = -1.f;
+    if (s < 12) {
+        F3 ax;
+        if (s == 0) {
+            F3 cA = fscale(fadd(fadd(R[0], R[1]), R[2]), 1.f / 3.f);
+            F3 cB = fscale(fadd(fadd(R[3], R[4]), R[5]), 1.f / 3.f);
+            ax = fsub(cB, cA);
+        } else {
+            const bool second = s >= 5, edges = s >= 9;
+            const F3 P0 = second ? R[3] : R[0], P1 = second ? R[4] : R[1], P2 = second ? R[5] : R[2];
+            const F3 e0 = fsub(P1, P0), e1 = fsub(P2, P1), e2 = fsub(P0, P2);
+            const F3 d1 = fsub(R[1], R[0]), d2 = fsub(R[4], R[3]);
+            const F3 nrm = edges ? fcross(d1, d2) : fcross(e0, fsub(P2, P0));
+            const int k = edges ? s - 9 : second ? s - 5 : s - 1;
+            const F3 e = edges ? (k == 1 ? d1 : d2) : k == 1 ? e0 : k == 2 ? e1 : e2;
+            ax = k == 0 ? nrm : fcross(nrm, e);
+        }
+        lb = axis_gap(ax, R);
+    }
+    for (int d = 8; d > 0; d >>= 1) lb = fmaxf(lb, __shfl_xor_sync(0xffffffffu, lb, d));
+    return pair_bound_may_hit<MOVING>(c, ia, o.n1, ib, o.n2, lb, L, M);
+}
+
+// Stage 1 with sixteen threads per pair, one per axis of the pair's bound and
+// then one per sub-test; on moving passes a sub-test that passes the FP32
+// filters is done here too when its cubic can have no root in the time window
+// (may_be_coplanar). A thread's 12 axes and 15 sub-tests in turn (below) are
+// ~36 us however few pairs a pass has.
+template <bool MOVING>
+__device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, int np, int& t_visits, int& t_sub) {
+    const int sub = threadIdx.x & 15, group = (threadIdx.x & 31) & ~15;
+    const int groups = (int)((gridDim.x * blockDim.x) >> 4);
+    const int g0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 4);
+    // every lane of a warp runs the same rounds: the pairs of its two groups
+    for (int base = 0; base < np; base += groups) {
+        const int idx = base + g0;
+        bool on = idx < np, queue = false, ee = false;
+        int pts[4] = {0, 0, 0, 0}, sc = 0;
+        OrientedPair o;
+        o.kind = 2;
+        o.n1 = o.n2 = 2;
+        o.keybase = 0;
+        for (int k = 0; k < 3; ++k) o.A[k] = o.B[k] = 0;
+        if (on) {
+            int2 pr = a.pairs[idx];
+            if (!MOVING && a.static_only && !(pr.y & kPairStatic)) on = false;
+            pr.y &= kPairIdMask;
+            if (on) on = orient_pair(a, pr, o);
+            if (on) {
+                t_visits += sub == 0;
+                sc = a.escene[pr.x];
+                bool shared = false;  // a shared point makes every test of the pair return false
+                for (int i = 0; i < o.n1; ++i)
+                    for (int j = 0; j < o.n2; ++j) shared |= o.A[i] == o.B[j];
+                on = !shared;
+            }
+        }
+        const double eps = a.scenes[sc].p.eps;
+        c.hpad = __double2float_ru(MOVING ? eps : a.scenes[sc].p.thickness);
+        c.epad = __double2float_ru(eps);
+        c.dt32 = __double2float_ru(a.scenes[sc].p.dt);
+        if (__any_sync(0xffffffffu, on)) on = pair_may_hit16<MOVING>(c, o, sub) && on;
+        if (on && pair_subtest<MOVING>(o, sub, pts, ee)) {
+            float ext, extb;
+            queue = mixed_may_hit(c, pts, ee, &ext, &extb) &&
+                    (ee ? sat_may_hit<MOVING, true>(c, pts, ext, extb) : sat_may_hit<MOVING, false>(c, pts, ext, extb));
+            if (MOVING && queue) {
+                double xo4[4][3], av4[4][3];
+                for (int q = 0; q < 4; ++q) {
+                    load3(a.xo, pts[q], xo4[q]);
+                    load3(a.av, pts[q], av4[q]);
+                }
+                ++t_sub;
+                queue = may_be_coplanar(xo4, av4, a.scenes[sc].p.dt);
+            }
+        }
+        queue_group(a, queue, ee, o.keybase, idx, sc, pts, sub, group, MOVING);
+    }
 }
 
 template <bool MOVING>
@@ -226,8 +385,10 @@ __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pai
     c.pbox_lo = a.pbox_lo; c.pbox_hi = a.pbox_hi; c.p32 = a.p32; c.v32 = a.v32;
     int np = a.ctr->npairs;
     if (np > max_pairs) np = max_pairs;
-    int t_visits = 0;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < np; idx += gridDim.x * blockDim.x) {
+    int t_visits = 0, t_sub = 0;
+    if (np <= kWideFilter) filter_wide<MOVING>(a, c, np, t_visits, t_sub);
+    for (int idx = np <= kWideFilter ? np : blockIdx.x * blockDim.x + threadIdx.x; idx < np;
+         idx += gridDim.x * blockDim.x) {
         int2 pr = a.pairs[idx];
         if (!MOVING && a.static_only && !(pr.y & kPairStatic)) continue;
         pr.y &= kPairIdMask;
@@ -249,32 +410,14 @@ __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pai
             queue_sub<MOVING>(a, c, ee, o.keybase, idx, sc, pts, sub, first);
         });
     }
-    for (int o = 16; o > 0; o >>= 1) t_visits += __shfl_xor_sync(0xffffffffu, t_visits, o);
-    if ((threadIdx.x & 31) == 0 && t_visits) atomicAdd(&a.ctr->nvisits, t_visits);
-}
-
-// The points of sub-test `sub` of a moving pair (for_each_subtest<true>'s
-// numbering) and whether it is edge-edge; false past the pair's last.
-__device__ __forceinline__ bool moving_subtest(const OrientedPair& o, int sub, int* pts, bool& ee) {
-    const int npt = o.kind == 0 ? 6 : o.kind == 1 ? 2 : 0;
-    const int n = o.kind == 0 ? 15 : o.kind == 1 ? 5 : 1;
-    ee = sub >= npt;
-    if (sub >= n) return false;
-    if (!ee) {
-        const bool first = sub < 3;  // the triangle is A, the point B's; then the reverse
-        const int i = first ? sub : sub - 3;
-        for (int k = 0; k < 3; ++k) pts[k] = first ? o.A[k] : o.B[k];
-        const int *P = first ? o.B : o.A;
-        pts[3] = i == 0 ? P[0] : i == 1 ? P[1] : P[2];
-        return true;
+    for (int o = 16; o > 0; o >>= 1) {
+        t_visits += __shfl_xor_sync(0xffffffffu, t_visits, o);
+        t_sub += __shfl_xor_sync(0xffffffffu, t_sub, o);
     }
-    const int e = sub - npt;
-    const int i = o.kind == 2 ? 0 : o.kind == 1 ? e : e / 3, j = o.kind == 0 ? e - 3 * i : 0;
-    pts[0] = i == 0 ? o.A[0] : i == 1 ? o.A[1] : o.A[2];
-    pts[1] = i == 0 ? o.A[1] : i == 1 ? o.A[2] : o.A[0];
-    pts[2] = j == 0 ? o.B[0] : j == 1 ? o.B[1] : o.B[2];
-    pts[3] = j == 0 ? o.B[1] : j == 1 ? o.B[2] : o.B[0];
-    return true;
+    if ((threadIdx.x & 31) == 0) {
+        if (t_visits) atomicAdd(&a.ctr->nvisits, t_visits);
+        if (t_sub) atomicAdd(&a.ctr->nsub, t_sub);
+    }
 }
 
 // Stage 1 of a plain FP64 moving pass: the coplanarity cubic of every
@@ -307,7 +450,7 @@ __global__ void __launch_bounds__(kPlainBlock) k_plain_filter(NarrowArgs a, int 
                 for (int i = 0; i < o.n1; ++i)
                     for (int j = 0; j < o.n2; ++j) shared |= o.A[i] == o.B[j];
                 sc = a.escene[pr.x];
-                if (!shared && moving_subtest(o, sub, pts, ee)) {
+                if (!shared && pair_subtest<true>(o, sub, pts, ee)) {
                     double xo4[4][3], av4[4][3];
                     for (int q = 0; q < 4; ++q) {
                         load3(a.xo, pts[q], xo4[q]);
@@ -318,30 +461,7 @@ __global__ void __launch_bounds__(kPlainBlock) k_plain_filter(NarrowArgs a, int 
                 }
             }
         }
-        const unsigned in_pair = __ballot_sync(0xffffffffu, queue) >> group & 0xffffu;
-        if (queue) {
-            int slot;  // (the lanes that add together share one counter)
-            if (ee)
-                slot = aggregated_add(&a.ctr->nsub_ee, 1);
-            else
-                slot = aggregated_add(&a.ctr->nsub_pt, 1);
-            if (slot >= a.sub_cap) {
-                atomicOr(&a.ctr->err, kErrSubOverflow);
-            } else {
-                SubRec r;
-                r.keybase = o.keybase;
-                r.pair = idx;
-                r.scene = sc;
-                for (int i = 0; i < 4; ++i) r.p[i] = pts[i];
-                r.sub = sub;
-                r.pad = 0;
-                (ee ? a.sub_ee : a.sub_pt)[slot] = r;
-            }
-            if ((in_pair & ((1u << sub) - 1u)) == 0) {  // the pair's first
-                a.pair_hit[idx] = 0;
-                a.pairq[aggregated_add(&a.ctr->npairq, 1)] = idx;
-            }
-        }
+        queue_group(a, queue, ee, o.keybase, idx, sc, pts, sub, group, true);
     }
     for (int o = 16; o > 0; o >>= 1) {
         t_visits += __shfl_xor_sync(0xffffffffu, t_visits, o);
@@ -418,7 +538,7 @@ __device__ __forceinline__ void one_subtest(const NarrowArgs& a, NarrowCtx& c, c
     st.ncr = 0;
     st.ncontacts = 0;
     bool hit = MOVING ? moving_test<EE>(c, st, r.p) : static_test<EE>(c, st, r.p);
-    t.sub++;
+    t.sub += r.counted == 0;
     t.cr += st.ncr;
     t.contacts += st.ncontacts;
     if (hit)
@@ -441,7 +561,7 @@ __device__ __forceinline__ void subtest_counts(const NarrowArgs& a, SubTally t) 
         if (t.hits) atomicAdd(&a.ctr->nhit_pairs, t.hits);
         if (t.cr) atomicAdd(&a.ctr->ncr, t.cr);
         if (t.contacts) atomicAdd(&a.ctr->ncontacts, t.contacts);
-        if (t.sub && !a.sub_counted) atomicAdd(&a.ctr->nsub, t.sub);
+        if (t.sub) atomicAdd(&a.ctr->nsub, t.sub);
     }
 }
 
@@ -575,10 +695,12 @@ void narrow_pass_split(const NarrowArgs& args, int moving, int max_pairs, cudaSt
         if (parts & kSplitFilter) narrow_pass(args, moving, max_pairs, s, block);
         return;
     }
-    NarrowArgs a = args;
-    a.sub_counted = mixed ? 0 : 1;
+    const NarrowArgs& a = args;
     const int cap_blocks = 152 * 16 * 128 / block;
     int blocks = (max_pairs + block - 1) / block;
+    // (sixteen threads per pair in passes of few pairs)
+    const long long wide = (16ll * (max_pairs < kWideFilter ? max_pairs : kWideFilter) + block - 1) / block;
+    if (blocks < wide) blocks = (int)wide;
     if (blocks > cap_blocks) blocks = cap_blocks;
     int sblocks = (a.sub_cap + 127) / 128;
     if (sblocks > 152 * 16) sblocks = 152 * 16;

@@ -984,45 +984,11 @@ __device__ __forceinline__ float axis_gap(F3 ax, const F3* R) {
     return fmaxf(bmin - amax, amin - bmax) / an;
 }
 
+// The pair's decision from the gap lb: ia, ib its points (a segment's last
+// one twice), L and M bounds of their distances and coordinates.
 template <bool MOVING>
-__device__ __forceinline__ bool pair_may_hit(const NarrowCtx& c, const int* A, int na, const int* B, int nb) {
-    // points relative to A's first; a segment's third point repeats its
-    // second (the same convex hull, so the same projections)
-    const int ia[3] = {A[0], A[1], na == 3 ? A[2] : A[1]};
-    const int ib[3] = {B[0], B[1], nb == 3 ? B[2] : B[1]};
-    F3 R[6];
-    const F3 X0 = f3(c.p32[ia[0]]);
-    float M = fmaxabs(X0), L = 0.f;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        F3 x = q < 3 ? f3(c.p32[ia[q]]) : f3(c.p32[ib[q - 3]]);
-        M = fmaxf(M, fmaxabs(x));
-        R[q] = fsub(x, X0);
-        L = fmaxf(L, fnorm(R[q]));
-    }
-    float lb = -1.f;
-    {
-        F3 cA = fscale(fadd(fadd(R[0], R[1]), R[2]), 1.f / 3.f);
-        F3 cB = fscale(fadd(fadd(R[3], R[4]), R[5]), 1.f / 3.f);
-        lb = fmaxf(lb, axis_gap(fsub(cB, cA), R));
-    }
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        const F3* P = R + 3 * side;
-        F3 e0 = fsub(P[1], P[0]), e1 = fsub(P[2], P[1]), e2 = fsub(P[0], P[2]);
-        F3 nrm = fcross(e0, fsub(P[2], P[0]));  // zero for a segment: skipped
-        lb = fmaxf(lb, axis_gap(nrm, R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, e0), R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, e1), R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, e2), R));
-    }
-    {
-        F3 d1 = fsub(R[1], R[0]), d2 = fsub(R[4], R[3]);
-        F3 nrm = fcross(d1, d2);
-        lb = fmaxf(lb, axis_gap(nrm, R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, d1), R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, d2), R));
-    }
+__device__ __forceinline__ bool pair_bound_may_hit(const NarrowCtx& c, const int* ia, int na, const int* ib, int nb,
+                                                   float lb, float L, float M) {
     // the largest reach of the pair's sub-tests, with the boxes' extents
     float extA, extB;
     {
@@ -1073,6 +1039,48 @@ __device__ __forceinline__ bool pair_may_hit(const NarrowCtx& c, const int* A, i
         bound = __fsub_rd(bound, __fmul_ru(c.dt32, dv));
     }
     return !(bound > reach);
+}
+
+template <bool MOVING>
+__device__ __forceinline__ bool pair_may_hit(const NarrowCtx& c, const int* A, int na, const int* B, int nb) {
+    // points relative to A's first; a segment's third point repeats its
+    // second (the same convex hull, so the same projections)
+    const int ia[3] = {A[0], A[1], na == 3 ? A[2] : A[1]};
+    const int ib[3] = {B[0], B[1], nb == 3 ? B[2] : B[1]};
+    F3 R[6];
+    const F3 X0 = f3(c.p32[ia[0]]);
+    float M = fmaxabs(X0), L = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        F3 x = q < 3 ? f3(c.p32[ia[q]]) : f3(c.p32[ib[q - 3]]);
+        M = fmaxf(M, fmaxabs(x));
+        R[q] = fsub(x, X0);
+        L = fmaxf(L, fnorm(R[q]));
+    }
+    float lb = -1.f;
+    {
+        F3 cA = fscale(fadd(fadd(R[0], R[1]), R[2]), 1.f / 3.f);
+        F3 cB = fscale(fadd(fadd(R[3], R[4]), R[5]), 1.f / 3.f);
+        lb = fmaxf(lb, axis_gap(fsub(cB, cA), R));
+    }
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const F3* P = R + 3 * side;
+        F3 e0 = fsub(P[1], P[0]), e1 = fsub(P[2], P[1]), e2 = fsub(P[0], P[2]);
+        F3 nrm = fcross(e0, fsub(P[2], P[0]));  // zero for a segment: skipped
+        lb = fmaxf(lb, axis_gap(nrm, R));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, e0), R));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, e1), R));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, e2), R));
+    }
+    {
+        F3 d1 = fsub(R[1], R[0]), d2 = fsub(R[4], R[3]);
+        F3 nrm = fcross(d1, d2);
+        lb = fmaxf(lb, axis_gap(nrm, R));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, d1), R));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, d2), R));
+    }
+    return pair_bound_may_hit<MOVING>(c, ia, na, ib, nb, lb, L, M);
 }
 
 template <bool MOVING, bool EE>

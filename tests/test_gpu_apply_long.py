@@ -15,10 +15,11 @@ def _fan(n):
     h = 1e-3
     a = np.linspace(0.0, 2.0 * np.pi, n + 1) + 0.013
     ring = np.stack([0.05 * np.cos(a), 0.05 * np.sin(a), np.full(n + 1, 0.05)], axis=1)
-    p = np.concatenate([[[0.011, 0.007, 0.4 * h]], ring])
+    # above a sloping floor (z = 0.2 x), whose box reaches the fan's
+    p = np.concatenate([[[0.011, 0.007, 0.2 * 0.011 + 0.4 * h]], ring])
     t = np.array([[0, 1 + k, 2 + k] for k in range(n)], np.int32)
     v = np.tile([0.1, 0.05, -0.3], (len(p), 1))
-    floor = np.array([[-1.0, -1.1, 0.0], [1.2, -1.0, 0.0], [0.1, 1.3, 0.0]])
+    floor = np.array([[-1.0, -1.1, -0.2], [1.2, -1.0, 0.24], [0.1, 1.3, 0.02]])
     return scenes.assemble(f"fan{n}", [(p, t, v, False), (floor, np.array([[0, 1, 2]], np.int32),
                                                          np.zeros((3, 3)), True)],
                            dict(dt=1e-3, thickness=h, lam=0.2))
