@@ -333,6 +333,12 @@ struct cc_solver {
     bool robust_roots = true;        // CC_TUNE_ROBUST_ROOTS: correctly rounded roots only where decisive
     bool sub_merge = true;           // CC_TUNE_SUBTEST_MERGE: both sub-test lists in one launch
     void* d_tree_scratch = nullptr;  // nodes, parent links and leaf counts of the trees being built
+    // Collision trees built ahead, beside the proximity trees of a step's
+    // first stop, on the swept boxes of the proximity pass: when that pass
+    // then applies nothing, they are the trees the first CCD pass asks for.
+    void* d_tree_scratch2 = nullptr;
+    std::vector<int> ahead_ids;
+    std::vector<double> ahead_vol;
     int* d_tree_jobs = nullptr;      // 3 per tree: scene, first element, elements
     int* h_tree_jobs = nullptr;      // pinned
     int* d_tree_root = nullptr;
@@ -534,6 +540,9 @@ struct cc_solver {
         dfree(d_tree_built);
         if (d_tree_scratch) cudaFree(d_tree_scratch);
         d_tree_scratch = nullptr;
+        if (d_tree_scratch2) cudaFree(d_tree_scratch2);
+        d_tree_scratch2 = nullptr;
+        ahead_ids.clear();
         dfree(d_tree_jobs); dfree(d_tree_root); dfree(d_tree_vol_out);
         if (h_tree_jobs) cudaFreeHost(h_tree_jobs);
         if (h_tree_vol_out) cudaFreeHost(h_tree_vol_out);
@@ -1229,10 +1238,10 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     ok &= dalloc(&d_tree_vol, (size_t)n) == cudaSuccess;
     ok &= dalloc(&d_tree_built, 2 * (size_t)n) == cudaSuccess;
     ok &= dalloc(&d_tree_jobs, 3 * (size_t)n) == cudaSuccess;
-    ok &= dalloc(&d_tree_root, (size_t)n) == cudaSuccess;
-    ok &= dalloc(&d_tree_vol_out, (size_t)n) == cudaSuccess;
+    ok &= dalloc(&d_tree_root, 2 * (size_t)n) == cudaSuccess;
+    ok &= dalloc(&d_tree_vol_out, 2 * (size_t)n) == cudaSuccess;
     ok &= cudaMallocHost(&h_tree_jobs, sizeof(int) * 3 * (size_t)n) == cudaSuccess;
-    ok &= cudaMallocHost(&h_tree_vol_out, sizeof(double) * (size_t)n) == cudaSuccess;
+    ok &= cudaMallocHost(&h_tree_vol_out, 2 * sizeof(double) * (size_t)n) == cudaSuccess;
     ok &= cudaMallocHost(&h_ctl, sizeof(SceneCtl) * (size_t)n) == cudaSuccess;
     ok &= cudaMallocHost(&h_loop, sizeof(LoopCtl)) == cudaSuccess;
     ok &= cudaMallocHost(&h_rebuild, sizeof(int) * (size_t)n) == cudaSuccess;
@@ -1450,11 +1459,32 @@ cc_status cc_solver::build_trees(int which, std::vector<int>& ids, const Box6* b
         }
         const int nj = (int)ids.size();
         cudaMemcpyAsync(d_tree_jobs, h_tree_jobs, sizeof(int) * 3 * (size_t)nj, cudaMemcpyHostToDevice, stream);
+        // beside few enough builds that both sets run at once, a CTA per SM
+        bool ahead = which == 0 && boxes == d_box_st && use_device_loop() && bodies.empty() && 2 * nj <= 152;
+        for (size_t i = 0; i < ids.size() && ahead; ++i) ahead = !scenes[ids[i]].built[1];
+        if (ahead && !d_tree_scratch2 && cudaMalloc(&d_tree_scratch2, tree_scratch_bytes(bvh.ne_all)) != cudaSuccess) {
+            cudaGetLastError();
+            d_tree_scratch2 = nullptr;
+            ahead = false;
+        }
+        if (ahead) {
+            cudaEventRecord(ev_pass, stream);
+            cudaStreamWaitEvent(tail_stream, ev_pass, 0);
+            tree_order_gpu(d_box, d_tree_jobs, nj, max_ne, d_tree_scratch2, bvh.ne_all, d_rank[1],
+                           d_tree_root + nscenes, d_tree_vol_out + nscenes, tail_stream);
+            cudaMemcpyAsync(h_tree_vol_out + nscenes, d_tree_vol_out + nscenes, sizeof(double) * (size_t)nj,
+                            cudaMemcpyDeviceToHost, tail_stream);
+        }
         tree_order_gpu(boxes, d_tree_jobs, nj, max_ne, d_tree_scratch, bvh.ne_all, d_rank[which], d_tree_root,
                        d_tree_vol_out, stream);
         cudaMemcpyAsync(h_tree_vol_out, d_tree_vol_out, sizeof(double) * (size_t)nj, cudaMemcpyDeviceToHost, stream);
         if (cudaStreamSynchronize(stream) != cudaSuccess) return cuda_check("tree build");
         for (int i = 0; i < nj; ++i) scenes[ids[i]].volume = h_tree_vol_out[i];
+        if (ahead) {
+            if (cudaStreamSynchronize(tail_stream) != cudaSuccess) return cuda_check("tree build");
+            ahead_ids = ids;
+            ahead_vol.assign(h_tree_vol_out + nscenes, h_tree_vol_out + nscenes + nj);
+        }
     }
     for (int s : ids) scenes[s].built[which] = scenes[s].ne > 0;
     counters[22] += std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now() - t0).count();
@@ -1488,6 +1518,19 @@ cc_status cc_solver::rebuild_flagged() {
         std::vector<int>& ids = todo[which];
         if (ids.empty()) continue;
         const Box6* boxes = (which == 0 && combined_broad) ? d_box_st : d_box;
+        if (which == 1 && ids == ahead_ids && h_loop->reuse_n >= 0) {
+            // the proximity pass applied nothing (its pairs are being reused):
+            // its swept boxes are this pass's, and their trees are built
+            for (size_t i = 0; i < ids.size(); ++i) {
+                scenes[ids[i]].volume = ahead_vol[i];
+                scenes[ids[i]].built[1] = true;
+            }
+            counters[8] += (long long)ids.size();
+            sync_tree_state(ids, 1);
+            ahead_ids.clear();
+            continue;
+        }
+        if (which == 1) ahead_ids.clear();
         const cc_status st = build_trees(which, ids, boxes);
         if (st) return st;
     }
@@ -1719,6 +1762,7 @@ cc_status cc_solver::device_passes(std::string& capped) {
         cudaMemsetAsync(d_marks + 1 + 2 * kLoopMarkSlots, 0, sizeof(unsigned long long), stream);
     cudaMemcpyAsync(d_ctl, h_ctl, sizeof(SceneCtl) * (size_t)nscenes, cudaMemcpyHostToDevice, stream);
     cudaMemcpyAsync(d_loop, h_loop, sizeof(LoopCtl), cudaMemcpyHostToDevice, stream);
+    ahead_ids.clear();
     bool need_prox = true;
     long long graph_runs = 0;
     LoopGraph* lgraph = nullptr;
