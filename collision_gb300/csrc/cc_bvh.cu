@@ -30,87 +30,125 @@ __global__ void k_bbox_init(unsigned long long* bb, int n6, const int* dn = null
     if (t < n6) bb[t] = (t % 6 < 3) ? ~0ull : 0ull;
 }
 
+// Least and greatest of a warp's encoded doubles: the high words by redux,
+// then the low words of the lanes that share it (on doubles, the reduction's
+// 30 compares per box were a third of the leaf boxes' FP64 instructions).
+__device__ __forceinline__ unsigned long long warp_min_enc(unsigned long long e) {
+    const unsigned hi = (unsigned)(e >> 32), m = __reduce_min_sync(0xffffffffu, hi);
+    return ((unsigned long long)m << 32) | __reduce_min_sync(0xffffffffu, hi == m ? (unsigned)e : 0xffffffffu);
+}
+__device__ __forceinline__ unsigned long long warp_max_enc(unsigned long long e) {
+    const unsigned hi = (unsigned)(e >> 32), m = __reduce_max_sync(0xffffffffu, hi);
+    return ((unsigned long long)m << 32) | __reduce_max_sync(0xffffffffu, hi == m ? (unsigned)e : 0u);
+}
+
 // Per-scene union of boxes into bb[6*scene ..]: reduced across the warp when
 // the whole warp lies in one scene (the common case: scenes are contiguous),
-// else one atomic per lane.
+// else one atomic per lane. A box with a NaN coordinate is left out, as it
+// would be by fmin and fmax.
 __device__ __forceinline__ void scene_bbox_accumulate(unsigned long long* bb, int scene, bool valid,
                                                       const double* lo, const double* hi) {
-    int s0 = __shfl_sync(0xffffffffu, scene, 0);
-    bool uniform = __all_sync(0xffffffffu, scene == s0);
+    // the lanes past the end of the list go with the others
+    const unsigned on = __ballot_sync(0xffffffffu, valid);
+    if (!on) return;
+    const int s0 = __shfl_sync(0xffffffffu, scene, __ffs(on) - 1);
+    const bool uniform = __all_sync(0xffffffffu, !valid || scene == s0);
     for (int d = 0; d < 3; ++d) {
-        double l = valid ? lo[d] : kBig, h = valid ? hi[d] : -kBig;
+        const unsigned long long nan = 0x7ff0000000000000ull;
+        const unsigned long long bl = (unsigned long long)__double_as_longlong(lo[d]),
+                                 bh = (unsigned long long)__double_as_longlong(hi[d]);
+        const bool okl = valid && (bl & ~(1ull << 63)) <= nan, okh = valid && (bh & ~(1ull << 63)) <= nan;
+        const unsigned long long el = okl ? enc_double(lo[d]) : ~0ull, eh = okh ? enc_double(hi[d]) : 0ull;
         if (uniform) {
-            for (int o = 16; o > 0; o >>= 1) {
-                l = fmin(l, __shfl_xor_sync(0xffffffffu, l, o));
-                h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
-            }
-            if ((threadIdx.x & 31) == 0 && l <= h && s0 >= 0) {
-                atomicMin(&bb[6 * s0 + d], enc_double(l));
-                atomicMax(&bb[6 * s0 + 3 + d], enc_double(h));
+            const unsigned long long ml = warp_min_enc(el), mh = warp_max_enc(eh);
+            if ((threadIdx.x & 31) == 0) {
+                atomicMin(&bb[6 * s0 + d], ml);
+                atomicMax(&bb[6 * s0 + 3 + d], mh);
             }
         } else if (valid) {
-            atomicMin(&bb[6 * scene + d], enc_double(l));
-            atomicMax(&bb[6 * scene + 3 + d], enc_double(h));
+            atomicMin(&bb[6 * scene + d], el);
+            atomicMax(&bb[6 * scene + 3 + d], eh);
         }
     }
 }
 
-template <int MOVING>
+// The static box of an element (kBoxStatic), its box swept over the step
+// (kBoxSwept), or both from one load of its points: the swept one's extremes
+// go on from the static one's.
+enum BoxKind { kBoxStatic = 0, kBoxSwept = 1, kBoxBoth = 2 };
+__device__ __forceinline__ Box6 padded(const double* mn, const double* mx, double* lo, double* hi) {
+    Box6 b;
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = b.lo[d] = mn[d] - kBoxPad;
+        hi[d] = b.hi[d] = mx[d] + kBoxPad;
+    }
+    return b;
+}
+template <int KIND>
 __device__ __forceinline__ void leaf_box(const int* __restrict__ ev, const int* __restrict__ act, int n, int k,
                                          const int* __restrict__ elem_scene, const SceneDev* __restrict__ scenes,
                                          const double4_32a* __restrict__ xo, const double4_32a* __restrict__ av,
-                                         Box6* __restrict__ box, unsigned long long* bb) {
+                                         Box6* __restrict__ box, unsigned long long* bb, Box6* __restrict__ box_st,
+                                         unsigned long long* bb_st) {
     bool valid = k < n;
     int e = valid ? (act ? act[k] : k) : 0;
     int scene = valid ? elem_scene[e] : -1;
     double lo[3] = {kBig, kBig, kBig}, hi[3] = {-kBig, -kBig, -kBig};
+    double mx[3] = {-kBig, -kBig, -kBig}, mn[3] = {kBig, kBig, kBig};
+    int pt[3] = {0, 0, 0}, np = 0;
     if (valid) {
-        double dt = scenes[scene].p.dt;
-        int np = (ev[3 * e + 2] >= 0) ? 3 : 2;
-        double mx[3] = {-kBig, -kBig, -kBig}, mn[3] = {kBig, kBig, kBig};
-        for (int i = 0; i < np; ++i) {
-            int p = ev[3 * e + i];
-            double4_32a x = xo[p];
-            double xs[3] = {x.x, x.y, x.z};
-            if (MOVING) {
-                double4_32a v = av[p];
-                double vs[3] = {v.x, v.y, v.z};
-                for (int d = 0; d < 3; ++d) {
-                    mx[d] = smax(mx[d], xs[d]);
-                    mx[d] = smax(mx[d], xs[d] + vs[d] * dt);
-                    mn[d] = smin(mn[d], xs[d]);
-                    mn[d] = smin(mn[d], xs[d] + vs[d] * dt);
-                }
-            } else {
+        np = (ev[3 * e + 2] >= 0) ? 3 : 2;
+        for (int i = 0; i < np; ++i) pt[i] = ev[3 * e + i];
+        if (KIND != kBoxSwept)
+            for (int i = 0; i < np; ++i) {
+                const double4_32a x = xo[pt[i]];
+                const double xs[3] = {x.x, x.y, x.z};
                 for (int d = 0; d < 3; ++d) {
                     mx[d] = smax(xs[d], mx[d]);
                     mn[d] = smin(xs[d], mn[d]);
                 }
             }
-        }
-        Box6 b;
-        for (int d = 0; d < 3; ++d) {
-            b.lo[d] = mn[d] - kBoxPad;
-            b.hi[d] = mx[d] + kBoxPad;
-            lo[d] = b.lo[d];
-            hi[d] = b.hi[d];
-        }
-        box[e] = b;
     }
-    scene_bbox_accumulate(bb, scene, valid, lo, hi);
+    if (KIND != kBoxSwept) {
+        if (valid) (KIND == kBoxBoth ? box_st : box)[e] = padded(mn, mx, lo, hi);
+        scene_bbox_accumulate(KIND == kBoxBoth ? bb_st : bb, scene, valid, lo, hi);
+    }
+    if (KIND != kBoxStatic) {
+        if (valid) {
+            const double dt = scenes[scene].p.dt;
+            for (int i = 0; i < np; ++i) {
+                const double4_32a x = xo[pt[i]], v = av[pt[i]];
+                const double xs[3] = {x.x, x.y, x.z}, vs[3] = {v.x, v.y, v.z};
+                for (int d = 0; d < 3; ++d) {
+                    const double xe = xs[d] + vs[d] * dt;
+                    if (KIND == kBoxSwept) {
+                        mx[d] = smax(mx[d], xs[d]);
+                        mn[d] = smin(mn[d], xs[d]);
+                    }
+                    mx[d] = smax(mx[d], xe);
+                    mn[d] = smin(mn[d], xe);
+                }
+            }
+            box[e] = padded(mn, mx, lo, hi);
+        }
+        scene_bbox_accumulate(bb, scene, valid, lo, hi);
+    }
 }
 
 // dn (may be null): the element count in device memory; the grid strides.
-template <int MOVING>
+// What bounds it is its FP64 min and max (a compare each, ~64 cycles a warp
+// on this GPU): both boxes at once take 36 instead of 54, the scenes' boxes
+// are reduced on integers.
+template <int KIND>
 __global__ void k_leaf_boxes(const int* __restrict__ ev, const int* __restrict__ act, int n,
                              const int* __restrict__ dn, const int* __restrict__ elem_scene,
                              const SceneDev* __restrict__ scenes, const double4_32a* __restrict__ xo,
-                             const double4_32a* __restrict__ av, Box6* __restrict__ box, unsigned long long* bb) {
+                             const double4_32a* __restrict__ av, Box6* __restrict__ box, unsigned long long* bb,
+                             Box6* __restrict__ box_st, unsigned long long* bb_st) {
     if (dn) n = *dn;
     for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x)
-        leaf_box<MOVING>(ev, act, n, base + threadIdx.x, elem_scene, scenes, xo, av, box, bb);
+        leaf_box<KIND>(ev, act, n, base + threadIdx.x, elem_scene, scenes, xo, av, box, bb, box_st, bb_st);
 }
-
 
 // Union of n given boxes into bb (encoded as for k_leaf_boxes).
 __global__ void k_boxes_bbox(const Box6* __restrict__ box, int n, unsigned long long* bb) {
@@ -1251,9 +1289,21 @@ void leaf_boxes(const int* ev, const int* act, int n, const int* elem_scene, con
     if (n <= 0) return;
     const int g = dn ? dev_grid(n, 256) : nblk(n, 256);
     if (moving)
-        count_launch(), k_leaf_boxes<1><<<g, 256, 0, s>>>(ev, act, n, dn, elem_scene, scenes, xo, av, box, bbox_enc);
+        count_launch(), k_leaf_boxes<kBoxSwept><<<g, 256, 0, s>>>(ev, act, n, dn, elem_scene, scenes, xo, av, box,
+                                                                  bbox_enc, nullptr, nullptr);
     else
-        count_launch(), k_leaf_boxes<0><<<g, 256, 0, s>>>(ev, act, n, dn, elem_scene, scenes, xo, av, box, bbox_enc);
+        count_launch(), k_leaf_boxes<kBoxStatic><<<g, 256, 0, s>>>(ev, act, n, dn, elem_scene, scenes, xo, av, box,
+                                                                   bbox_enc, nullptr, nullptr);
+}
+
+void leaf_boxes_both(const int* ev, const int* act, int n, const int* elem_scene, const SceneDev* scenes, int nscenes,
+                     const double4_32a* xo, const double4_32a* av, Box6* box, unsigned long long* bbox_enc,
+                     Box6* box_st, unsigned long long* bbox_st, cudaStream_t s) {
+    // the two bounding arrays lie one after the other
+    count_launch(), k_bbox_init<<<nblk(12 * nscenes, 256), 256, 0, s>>>(bbox_enc, 12 * nscenes);
+    if (n > 0)
+        count_launch(), k_leaf_boxes<kBoxBoth><<<nblk(n, 256), 256, 0, s>>>(ev, act, n, nullptr, elem_scene, scenes, xo,
+                                                                            av, box, bbox_enc, box_st, bbox_st);
 }
 
 // Element / point k of the selection: scene j with off[j] <= k < off[j+1].

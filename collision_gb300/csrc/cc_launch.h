@@ -154,6 +154,11 @@ struct BvhBufs {
 void leaf_boxes(const int* ev, const int* act, int n, const int* elem_scene, const SceneDev* scenes, int nscenes,
                 const double4_32a* xo, const double4_32a* av, int moving, Box6* box, unsigned long long* bbox_enc,
                 cudaStream_t s, const int* dn = nullptr);
+// Static boxes into box_st and swept ones into box in one launch, with their
+// scenes' boxes in bbox_st and bbox_enc (bbox_st = bbox_enc + 6 * nscenes).
+void leaf_boxes_both(const int* ev, const int* act, int n, const int* elem_scene, const SceneDev* scenes, int nscenes,
+                     const double4_32a* xo, const double4_32a* av, Box6* box, unsigned long long* bbox_enc,
+                     Box6* box_st, unsigned long long* bbox_st, cudaStream_t s);
 // The elements and points of the given scenes, in scene order:
 // elem_off / pt_off are the exclusive prefix sums of their counts.
 void expand_scenes(const int* scene_ids, const int* elem_off, const int* pt_off, int nsel, int n_elems, int n_pts,

@@ -73,6 +73,31 @@ __global__ void k_scan_total(const int* in, const int* out, int n, int* total) {
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Scans of up to kScanOne elements take one block, a run of consecutive
+// elements per thread: one launch instead of three (~1.2 us each). At 32,768
+// elements that serial run costs more than it saves (a build of 136,000
+// leaves 0.22 -> 0.23 ms, of 196,000 0.265 -> 0.313 ms).
+constexpr int kScanOne = 4 * kScanTile;
+__global__ void __launch_bounds__(kScanThreads) k_scan_one(const int* in, int* out, int n) {
+    __shared__ int wsum[kScanThreads / 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per = (n + kScanThreads - 1) / kScanThreads;  // consecutive elements per thread
+    const int i0 = threadIdx.x * per, i1 = i0 + per < n ? i0 + per : n;
+    int local = 0;
+    for (int i = i0; i < i1; ++i) local += in[i];
+    const int incl = warp_incl_scan(local);
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    if (warp == 0) wsum[lane] = warp_incl_scan(wsum[lane]);
+    __syncthreads();
+    int run = incl - local + (warp > 0 ? wsum[warp - 1] : 0);
+    for (int i = i0; i < i1; ++i) {
+        const int v = in[i];
+        out[i] = run;
+        run += v;
+    }
+}
+
 // Levels of block sums for an n-element scan.
 size_t scan_levels_bytes(int n) {
     size_t bytes = 0;
@@ -87,6 +112,10 @@ void scan_rec(const int* in, int* out, int n, char* temp, cudaStream_t s) {
     int nb = ceil_div(n, kScanTile);
     if (nb <= 1) {
         count_launch(), k_scan_tile<<<1, kScanThreads, 0, s>>>(in, out, n, nullptr);
+        return;
+    }
+    if (n <= kScanOne) {
+        count_launch(), k_scan_one<<<1, kScanThreads, 0, s>>>(in, out, n);
         return;
     }
     int* sums = (int*)temp;
@@ -179,7 +208,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(unsigned long long
     unsigned int* s_v = reinterpret_cast<unsigned int*>(s_k + kSmallSort);
     const int m = sort_count(dn, n);
     if (m > small_max) {
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && eff) {
             *eff = m;
             if (use_h) cudaGraphSetConditional(h, 1u);
         }
@@ -215,13 +244,25 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(unsigned long long
         keys[i] = c >> kIdxBits;
         vals[i] = s_v[c & (kSmallSort - 1)];
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && eff) {
         *eff = 0;
         if (use_h) cudaGraphSetConditional(h, 0u);
     }
 }
 
 }  // namespace
+
+// Once per process and device: the one-CTA sort's shared memory.
+static cudaError_t small_sort_attr() {
+    static bool attr = false;
+    if (!attr) {
+        cudaError_t e = cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kSmallBytes);
+        if (e != cudaSuccess) return e;
+        attr = true;
+    }
+    return cudaSuccess;
+}
 
 cudaError_t sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn, int cap, int bits,
                            void* temp, int* eff, cudaStream_t s, cudaStream_t nested, bool small) {
@@ -231,15 +272,10 @@ cudaError_t sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const i
         radix_sort_pairs_dev(keys, vals, dn, cap, bits, temp, s);
         return cudaGetLastError();
     }
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kSmallBytes);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    cudaError_t e = small_sort_attr();
+    if (e != cudaSuccess) return e;
     cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
-    cudaError_t e = cudaStreamIsCapturing(s, &cst);
+    e = cudaStreamIsCapturing(s, &cst);
     if (e != cudaSuccess) return e;
     if (cst != cudaStreamCaptureStatusActive || !nested) {
         count_launch(), k_sort_small<<<1, kSmallThreads, kSmallBytes, s>>>(keys, vals, dn, cap, small_max, eff, 0, 0);
@@ -298,6 +334,13 @@ size_t radix_sort_temp_bytes(int n) {
 }
 
 void radix_sort_pairs(unsigned long long* keys, unsigned int* vals, int n, int bits, void* temp, cudaStream_t s) {
+    // up to kSmallSort pairs in one CTA: the same stable order in one launch
+    // (a 33 x 33 sheet's build: 0.13 -> 0.10 ms)
+    if (n > 1 && n <= kSmallSort && bits <= 64 - kIdxBits && small_sort_attr() == cudaSuccess) {
+        count_launch(), k_sort_small<<<1, kSmallThreads, kSmallBytes, s>>>(keys, vals, nullptr, n, kSmallSort, nullptr,
+                                                                           0, 0);
+        return;
+    }
     radix_sort_pairs_dev(keys, vals, nullptr, n, bits, temp, s);
 }
 

@@ -1198,7 +1198,7 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     ok &= dalloc(&bvh.leaf32, (size_t)ne) == cudaSuccess;
     ok &= dalloc(&bvh.qnext, 2) == cudaSuccess;
     ok &= dalloc(&bvh.heavy, (size_t)ne) == cudaSuccess;
-    ok &= dalloc(&bvh.bbox_enc, 6 * (size_t)n) == cudaSuccess;
+    ok &= dalloc(&bvh.bbox_enc, 12 * (size_t)n) == cudaSuccess;
     ok &= cudaMalloc(&bvh.sort_temp, radix_sort_temp_bytes(ne > 0 ? ne : 1)) == cudaSuccess;
     ok &= dalloc(&apply.cnt, (size_t)nv + nbodies) == cudaSuccess;
     ok &= dalloc(&apply.off, (size_t)nv + nbodies) == cudaSuccess;
@@ -1547,11 +1547,15 @@ void cc_solver::prox_pass_async() {
     cudaMemcpyAsync(d_run, h_run, sizeof(SceneRun) * (size_t)nscenes, cudaMemcpyHostToDevice, stream);
     const bool combined = combined_broad;
     prof(kStBoxes, true);
-    leaf_boxes(d_ev, bvh.act, bvh.n, d_escene, d_scenes, nscenes, d_xo, d_av, 0, combined ? d_box_st : d_box,
-               bvh.bbox_enc, stream);
-    tree_check(d_run, nscenes, bvh.bbox_enc, d_tree_vol, d_tree_built, 0, d_rebuild, d_loop, stream);
-    if (combined)
-        leaf_boxes(d_ev, bvh.act, bvh.n, d_escene, d_scenes, nscenes, d_xo, d_av, 1, d_box, bvh.bbox_enc, stream);
+    unsigned long long* bbox_st = bvh.bbox_enc;
+    if (combined) {
+        bbox_st = bvh.bbox_enc + 6 * (size_t)nscenes;
+        leaf_boxes_both(d_ev, bvh.act, bvh.n, d_escene, d_scenes, nscenes, d_xo, d_av, d_box, bvh.bbox_enc, d_box_st,
+                        bbox_st, stream);
+    } else {
+        leaf_boxes(d_ev, bvh.act, bvh.n, d_escene, d_scenes, nscenes, d_xo, d_av, 0, d_box, bvh.bbox_enc, stream);
+    }
+    tree_check(d_run, nscenes, bbox_st, d_tree_vol, d_tree_built, 0, d_rebuild, d_loop, stream);
     prof(kStBoxes, false);
     prof(kStBvh, true);
     bvh_build(d_box, bvh, stream);
