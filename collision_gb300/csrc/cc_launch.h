@@ -35,13 +35,13 @@ void radix_sort_pairs(unsigned long long* keys, unsigned int* vals, int n, int b
 // (temp sized for cap; the arrays hold cap pairs).
 void radix_sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn, int cap, int bits, void* temp,
                           cudaStream_t s);
-// The same with counts of up to 8192 pairs sorted by one CTA in shared
-// memory (keys below 2^51); eff: a device int the two stages share. On a
-// stream that is being captured, with `nested` (a second stream) given, the
-// general sort sits behind a conditional node and runs only for larger
-// counts. small = false: always the general sort.
-cudaError_t sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn, int cap, int bits,
-                           void* temp, int* eff, cudaStream_t s, cudaStream_t nested, bool small = true);
+// The same in up to two parts, for keys below 2^51: counts of up to
+// kSmallSort pairs by one CTA in shared memory (small), larger ones by the
+// general sort (general); eff: a device int the two share.
+constexpr int kSmallSort = 8192;
+cudaError_t small_sort_ready();  // before the first one-CTA sort: its shared memory
+void sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn, int cap, int bits, void* temp,
+                    int* eff, cudaStream_t s, bool small, bool general);
 // Exclusive scan of n ints (out may alias in); total written to *total.
 size_t scan_temp_bytes(int n);
 void exclusive_scan(const int* in, int* out, int n, int* total, void* temp, cudaStream_t s);
@@ -317,9 +317,18 @@ void apply_contribs(const Contrib* contrib, const PassCounters* ctr, int contrib
 void zone_solve(const int* members, const int* zone_off, int nzones, const uint8_t* fixed, const double4_32a* xo,
                 double4_32a* av, const int* vscene, const SceneDev* scenes, PassCounters* ctr, cudaStream_t s,
                 const SceneRun* run = nullptr, PassStamp ps = PassStamp{});
-// The same with zone z's members at members[zone_rng[z].x .. .y) and the
-// zone count in device memory (*dnz, at most zone_cap).
-void zone_solve_dev(const int* members, const int2* zone_rng, const int* dnz, int zone_cap, const uint8_t* fixed,
+// The zone members of the passes, in two buffers written in turn: the one of
+// the pass is buf[*epoch & 1] (no epoch: buf[0]).
+struct ZoneMembers {
+    int* buf[2];
+    const unsigned* epoch;
+#ifdef __CUDACC__
+    __device__ __forceinline__ const int* list() const { return epoch ? buf[*epoch & 1] : buf[0]; }
+#endif
+};
+// The same with zone z's members at [zone_rng[z].x .. .y) of their list and
+// the zone count in device memory (*dnz, at most zone_cap).
+void zone_solve_dev(const ZoneMembers& members, const int2* zone_rng, const int* dnz, int zone_cap, const uint8_t* fixed,
                     const double4_32a* xo, double4_32a* av, const int* vscene, const SceneDev* scenes,
                     PassCounters* ctr, cudaStream_t s, PassStamp ps = PassStamp{}, int cta_min = 64,
                     int few = 1024);
@@ -339,16 +348,16 @@ struct ZoneBufs {
     int zone_cap = 0;                    // zones the zone arrays hold
     int2* zone_rng = nullptr;            // per zone: its run of members
     int* zone_root = nullptr;            // per zone: its root
-    int* members = nullptr;              // per point (at most one zone each)
-    // the previous zone pass's lists (k_zone_members starts from them): a
-    // copy of its member array, and per root its run and the epoch it was
-    // listed in (prev_epoch == *epoch: the pass just before); n_pts_cap
-    // bounds the members and zones of a pass (the points)
-    int* prev_members = nullptr;
+    int* members = nullptr;              // per point (at most one zone each), two halves (ZoneMembers)
+    // the previous zone pass's lists (k_zone_members starts from them): per
+    // root its run and the epoch it was listed in (prev_epoch + 1 == *epoch:
+    // the pass just before); n_pts_cap bounds the members and zones of a pass
+    // (the points)
     int* prev_off = nullptr;
     int* prev_len = nullptr;
     unsigned* prev_epoch = nullptr;
-    unsigned* epoch = nullptr;
+    unsigned* epoch = nullptr;           // zone passes so far
+    int* gen = nullptr;                  // records k_zone_join leaves to the general kernels
     int n_pts_cap = 0;
     bool small_sort = true;              // sorts of up to 8192 records in one CTA
     int zone_cta_min = 64;               // zones of this many members are solved by a CTA each
@@ -361,10 +370,10 @@ size_t zone_sort_temp_bytes(int cap);
 // scene in that mode and move it rigidly (updateImpactZoneVelocity,
 // dcollid.cpp:290-310). act_pts / n_pts: the points of the pass's scenes
 // (null: all n_pts points; dn_pts, if given, holds the count on the device).
-// nested: a second stream for conditional sorts while s is being captured
-// (null otherwise); marks (may be null): stage boundaries after the sorts,
-// the replay, the zone lists and the solve go to slots mark0..mark0+3
-// (stage_mark). Returns a launch or capture error.
+// nested: a second stream for conditional stages while s is being captured
+// (null otherwise); marks (may be null): stage boundaries after the
+// one-CTA join, the general kernels, the zone lists and the solve go to slots
+// mark0..mark0+3 (stage_mark). Returns a launch or capture error.
 cudaError_t zone_pass(const ZoneBufs& z, const PassCounters* ctr, const uint8_t* fixed, const int* act_pts, int n_pts,
                       const int* dn_pts, const int* vscene, const SceneRun* run, const SceneDev* scenes,
                       double4_32a* av, const double4_32a* xo, cudaStream_t s, PassStamp ps = PassStamp{},

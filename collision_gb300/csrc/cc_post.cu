@@ -299,11 +299,12 @@ constexpr int kZoneCtaThreads = 256;
 
 // Zone z's members are members[zone_rng[z].x .. zone_rng[z].y); dnz: the
 // zone count in device memory, at most nzones.
-__global__ void k_zone_solve(const int* __restrict__ members, const int2* __restrict__ zone_rng, int nzones,
+__global__ void k_zone_solve(ZoneMembers mem, const int2* __restrict__ zone_rng, int nzones,
                              const int* __restrict__ dnz, const uint8_t* __restrict__ fixed,
                              const double4_32a* __restrict__ xo, double4_32a* av, const int* __restrict__ vscene,
                              const SceneDev* __restrict__ scenes, PassCounters* ctr, PassStamp ps, int few) {
     if (ctr->err & kErrRetry) return;
+    const int* __restrict__ members = mem.list();
     if (*dnz < nzones) nzones = *dnz;
     const int warp_min = zone_warp_min(nzones, few);
     for (int z = blockIdx.x * blockDim.x + threadIdx.x; z < nzones; z += gridDim.x * blockDim.x) {
@@ -323,12 +324,13 @@ __global__ void k_zone_solve(const int* __restrict__ members, const int2* __rest
 // the same operands as the one-thread form. The final per-member motion is
 // spread over the lanes.
 __global__ void __launch_bounds__(kZoneWarpBlock) k_zone_solve_warp(
-    const int* __restrict__ members, const int2* __restrict__ zone_rng, int nzones, const int* __restrict__ dnz,
+    ZoneMembers mem, const int2* __restrict__ zone_rng, int nzones, const int* __restrict__ dnz,
     const uint8_t* __restrict__ fixed, const double4_32a* __restrict__ xo, double4_32a* av,
     const int* __restrict__ vscene, const SceneDev* __restrict__ scenes, PassCounters* ctr, PassStamp ps,
     int cta_min, int few) {
     __shared__ double stage[kZoneWarpBlock / 32][32][12];
     if (ctr->err & kErrRetry) return;
+    const int* __restrict__ members = mem.list();
     if (*dnz < nzones) nzones = *dnz;
     const int warp_min = zone_warp_min(nzones, few);
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -419,7 +421,7 @@ __global__ void __launch_bounds__(kZoneWarpBlock) k_zone_solve_warp(
 // took 3 ms of every pass on one thread, whose ~150 FP64 instructions per
 // member each take ~64 cycles; here the ordered sums' two per member remain.
 __global__ void __launch_bounds__(kZoneCtaThreads) k_zone_solve_cta(
-    const int* __restrict__ members, const int* __restrict__ zone_off, const int2* __restrict__ zone_rng, int nzones,
+    ZoneMembers mem, const int* __restrict__ zone_off, const int2* __restrict__ zone_rng, int nzones,
     const int* __restrict__ dnz, const uint8_t* __restrict__ fixed, const double4_32a* __restrict__ xo,
     double4_32a* av, const int* __restrict__ vscene, const SceneDev* __restrict__ scenes, PassCounters* ctr,
     const SceneRun* __restrict__ run, PassStamp ps, int cta_min) {
@@ -427,6 +429,7 @@ __global__ void __launch_bounds__(kZoneCtaThreads) k_zone_solve_cta(
     __shared__ double s_sum[12];
     __shared__ double s_rot[6];  // w, mag_w, sw, cw
     if (ctr->err & kErrRetry) return;
+    const int* __restrict__ members = mem.list();
     if (dnz && *dnz < nzones) nzones = *dnz;
     const int tid = threadIdx.x;
     bool bad = false;
@@ -652,10 +655,11 @@ void zone_solve(const int* members, const int* zone_off, int nzones, const uint8
     // (a body of one point does not move)
     if (nzones > 0)
         count_launch(), k_zone_solve_cta<<<nzones < 152 * 8 ? nzones : 152 * 8, kZoneCtaThreads, 0, s>>>(
-            members, zone_off, nullptr, nzones, nullptr, fixed, xo, av, vscene, scenes, ctr, run, ps, 2);
+            ZoneMembers{{const_cast<int*>(members), nullptr}, nullptr}, zone_off, nullptr, nzones, nullptr, fixed, xo,
+            av, vscene, scenes, ctr, run, ps, 2);
 }
 
-void zone_solve_dev(const int* members, const int2* zone_rng, const int* dnz, int zone_cap, const uint8_t* fixed,
+void zone_solve_dev(const ZoneMembers& members, const int2* zone_rng, const int* dnz, int zone_cap, const uint8_t* fixed,
                     const double4_32a* xo, double4_32a* av, const int* vscene, const SceneDev* scenes,
                     PassCounters* ctr, cudaStream_t s, PassStamp ps, int cta_min, int few) {
     if (cta_min < kZoneWarpMin) cta_min = kZoneWarpMin;

@@ -193,25 +193,20 @@ __global__ void k_radix_scatter(const unsigned long long* keys, const unsigned i
 // Small sorts in one CTA: up to kSmallSort pairs, each key extended by its
 // input position (so the keys are distinct and a bitonic network gives the
 // stable order), sorted in shared memory.
-constexpr int kSmallSort = 8192;
 constexpr int kSmallThreads = 1024;
-constexpr int kIdxBits = 13;  // 2^13 = kSmallSort
+constexpr int kIdxBits = 13;
+static_assert(1 << kIdxBits == kSmallSort, "an index per pair");
 constexpr size_t kSmallBytes = (size_t)kSmallSort * (sizeof(unsigned long long) + sizeof(unsigned int));
 
-// Sorts the first m = min(*dn, n) pairs when m <= small_max (<= kSmallSort) and sets *eff
-// to 0; otherwise leaves them and sets *eff = m. In a graph, also sets the
-// conditional handle h (if use_h) to whether the general sort must run.
+// Sorts the first m = min(*dn, n) pairs when m <= kSmallSort and sets *eff
+// to 0; otherwise leaves them and sets *eff = m.
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(unsigned long long* keys, unsigned int* vals,
-                                                             const int* dn, int n, int small_max, int* eff,
-                                                             cudaGraphConditionalHandle h, int use_h) {
+                                                             const int* dn, int n, int* eff) {
     extern __shared__ unsigned long long s_k[];
     unsigned int* s_v = reinterpret_cast<unsigned int*>(s_k + kSmallSort);
     const int m = sort_count(dn, n);
-    if (m > small_max) {
-        if (threadIdx.x == 0 && eff) {
-            *eff = m;
-            if (use_h) cudaGraphSetConditional(h, 1u);
-        }
+    if (m > kSmallSort) {
+        if (threadIdx.x == 0 && eff) *eff = m;
         return;
     }
     int P = 1;
@@ -244,71 +239,21 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(unsigned long long
         keys[i] = c >> kIdxBits;
         vals[i] = s_v[c & (kSmallSort - 1)];
     }
-    if (threadIdx.x == 0 && eff) {
-        *eff = 0;
-        if (use_h) cudaGraphSetConditional(h, 0u);
-    }
+    if (threadIdx.x == 0 && eff) *eff = 0;
 }
 
 }  // namespace
 
-// Once per process and device: the one-CTA sort's shared memory.
-static cudaError_t small_sort_attr() {
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kSmallBytes);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
-    return cudaSuccess;
+cudaError_t small_sort_ready() {
+    return cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallBytes);
 }
 
-cudaError_t sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn, int cap, int bits,
-                           void* temp, int* eff, cudaStream_t s, cudaStream_t nested, bool small) {
-    const int small_max = small ? kSmallSort : -1;
-    if (cap <= 1 || bits <= 0) return cudaSuccess;
-    if (bits > 64 - kIdxBits) {
-        radix_sort_pairs_dev(keys, vals, dn, cap, bits, temp, s);
-        return cudaGetLastError();
-    }
-    cudaError_t e = small_sort_attr();
-    if (e != cudaSuccess) return e;
-    cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
-    e = cudaStreamIsCapturing(s, &cst);
-    if (e != cudaSuccess) return e;
-    if (cst != cudaStreamCaptureStatusActive || !nested) {
-        count_launch(), k_sort_small<<<1, kSmallThreads, kSmallBytes, s>>>(keys, vals, dn, cap, small_max, eff, 0, 0);
-        radix_sort_pairs_dev(keys, vals, eff, cap, bits, temp, s);
-        return cudaGetLastError();
-    }
-    // in a graph: the general sort behind an IF node that the small sort sets
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, &deps, nullptr, &ndeps);
-    cudaGraphConditionalHandle h;
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess) return e;
-    count_launch(), k_sort_small<<<1, kSmallThreads, kSmallBytes, s>>>(keys, vals, dn, cap, small_max, eff, h, 1);
-    e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, &deps, nullptr, &ndeps);
-    cudaGraphNodeParams ip = {};
-    cudaGraphNode_t node;
-    if (e == cudaSuccess) {
-        ip.type = cudaGraphNodeTypeConditional;
-        ip.conditional.handle = h;
-        ip.conditional.type = cudaGraphCondTypeIf;
-        ip.conditional.size = 1;
-        e = cudaGraphAddNode(&node, g, deps, nullptr, ndeps, &ip);
-    }
-    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
-    if (e == cudaSuccess)
-        e = cudaStreamBeginCaptureToGraph(nested, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return e;
-    radix_sort_pairs_dev(keys, vals, eff, cap, bits, temp, nested);
-    cudaGraph_t body = nullptr;
-    return cudaStreamEndCapture(nested, &body);
+void sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn, int cap, int bits, void* temp,
+                    int* eff, cudaStream_t s, bool small, bool general) {
+    if (cap <= 1 || bits <= 0) return;
+    if (small)
+        count_launch(), k_sort_small<<<1, kSmallThreads, kSmallBytes, s>>>(keys, vals, dn, cap, eff);
+    if (general) radix_sort_pairs_dev(keys, vals, small ? eff : dn, cap, bits, temp, s);
 }
 
 size_t scan_temp_bytes(int n) { return scan_levels_bytes(n) + 256; }
@@ -336,9 +281,8 @@ size_t radix_sort_temp_bytes(int n) {
 void radix_sort_pairs(unsigned long long* keys, unsigned int* vals, int n, int bits, void* temp, cudaStream_t s) {
     // up to kSmallSort pairs in one CTA: the same stable order in one launch
     // (a 33 x 33 sheet's build: 0.13 -> 0.10 ms)
-    if (n > 1 && n <= kSmallSort && bits <= 64 - kIdxBits && small_sort_attr() == cudaSuccess) {
-        count_launch(), k_sort_small<<<1, kSmallThreads, kSmallBytes, s>>>(keys, vals, nullptr, n, kSmallSort, nullptr,
-                                                                           0, 0);
+    if (n > 1 && n <= kSmallSort && bits <= 64 - kIdxBits && small_sort_ready() == cudaSuccess) {
+        count_launch(), k_sort_small<<<1, kSmallThreads, kSmallBytes, s>>>(keys, vals, nullptr, n, nullptr);
         return;
     }
     radix_sort_pairs_dev(keys, vals, nullptr, n, bits, temp, s);

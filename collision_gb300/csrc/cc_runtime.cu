@@ -200,7 +200,6 @@ struct cc_solver {
     int urec_cap = 0;
     ZoneBufs zb;
     UfNode* d_uf0 = nullptr;  // the union-find every step starts from
-    int* d_cc0 = nullptr;
     bool uf_on_device = false;  // the host arrays are stale: the device holds the last step's zones
     // staging for host-buffer calls
     double* d_xold_in = nullptr;
@@ -510,8 +509,8 @@ struct cc_solver {
         dfree(d_urec);
         urec_cap = 0;
         dfree(zb.keys); dfree(zb.vals); dfree(zb.seg); dfree(zb.noop); dfree(zb.cc); dfree(zb.uf); dfree(zb.zone_rng);
-        dfree(zb.zone_root); dfree(zb.members); dfree(d_uf0); dfree(d_cc0);
-        dfree(zb.prev_members); dfree(zb.prev_off); dfree(zb.prev_len); dfree(zb.prev_epoch); dfree(zb.epoch);
+        dfree(zb.zone_root); dfree(zb.members); dfree(d_uf0);
+        dfree(zb.gen); dfree(zb.prev_off); dfree(zb.prev_len); dfree(zb.prev_epoch); dfree(zb.epoch);
         if (zb.sort_temp) cudaFree(zb.sort_temp);
         const bool small_sort = zb.small_sort;  // settings, not buffers
         const int zone_cta_min = zb.zone_cta_min, replay_cta_min = zb.replay_cta_min, zone_few = zb.zone_few;
@@ -662,7 +661,6 @@ struct cc_solver {
     void start_zones() {
         if (nv == 0) return;
         cudaMemcpyAsync(zb.uf, d_uf0, sizeof(UfNode) * (size_t)nv, cudaMemcpyDeviceToDevice, stream);
-        cudaMemcpyAsync(zb.cc, d_cc0, sizeof(int) * (size_t)nv, cudaMemcpyDeviceToDevice, stream);
         // the lists of the last step's zones no longer hold
         if (zb.prev_epoch) cudaMemsetAsync(zb.prev_epoch, 0xff, sizeof(unsigned) * (size_t)nv, stream);
         uf_on_device = true;
@@ -1361,10 +1359,9 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
         // bodies' unions (reset_zones above, when there are bodies)
         const int nz = nv / 2 + 1;
         bool zok = dalloc(&zb.cc, (size_t)nv) == cudaSuccess && dalloc(&zb.uf, (size_t)nv) == cudaSuccess &&
-                   dalloc(&d_cc0, (size_t)nv) == cudaSuccess && dalloc(&d_uf0, (size_t)nv) == cudaSuccess &&
+                   dalloc(&d_uf0, (size_t)nv) == cudaSuccess &&
                    dalloc(&zb.zone_rng, (size_t)nz) == cudaSuccess && dalloc(&zb.zone_root, (size_t)nz) == cudaSuccess &&
-                   dalloc(&zb.members, (size_t)nv) == cudaSuccess &&
-                   dalloc(&zb.prev_members, (size_t)nv) == cudaSuccess &&
+                   dalloc(&zb.members, 2 * (size_t)nv) == cudaSuccess && dalloc(&zb.gen, 1) == cudaSuccess &&
                    dalloc(&zb.prev_off, (size_t)nv) == cudaSuccess && dalloc(&zb.prev_len, (size_t)nv) == cudaSuccess &&
                    dalloc(&zb.prev_epoch, (size_t)nv) == cudaSuccess && dalloc(&zb.epoch, 1) == cudaSuccess;
         if (!zok) return fail(CC_NO_MEMORY, "zone buffers");
@@ -1372,15 +1369,8 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
         zb.n_pts_cap = nv;
         cudaMemsetAsync(zb.epoch, 0, sizeof(unsigned), stream);
         std::vector<UfNode> u0((size_t)nv);
-        std::vector<int> c0((size_t)nv);
-        for (int p = 0; p < nv; ++p) {
-            u0[p] = UfNode{uf_root[p], uf_next[p], uf_tail[p], uf_w[p]};
-            c0[p] = find_set(p);
-        }
-        if (nv) {
-            cudaMemcpy(d_uf0, u0.data(), sizeof(UfNode) * (size_t)nv, cudaMemcpyHostToDevice);
-            cudaMemcpy(d_cc0, c0.data(), sizeof(int) * (size_t)nv, cudaMemcpyHostToDevice);
-        }
+        for (int p = 0; p < nv; ++p) u0[p] = UfNode{uf_root[p], uf_next[p], uf_tail[p], uf_w[p]};
+        if (nv) cudaMemcpy(d_uf0, u0.data(), sizeof(UfNode) * (size_t)nv, cudaMemcpyHostToDevice);
         uf_on_device = false;
     }
     if (grow_unions(1024)) return CC_NO_MEMORY;

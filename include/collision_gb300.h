@@ -273,10 +273,10 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           built on the GPU (the insertions pipelined, one
  *                           CTA per tree); 1: on host threads, one tree per
  *                           thread. Same ranks and volumes
- *   CC_TUNE_SMALL_SORT      1 (default): an impact-zone pass sorts up to
- *                           8,192 union records in one CTA (in the device
- *                           loop the general radix sort then does not run);
- *                           0: always the general sort. Same results
+ *   CC_TUNE_SMALL_SORT      1 (default): an impact-zone pass joins up to
+ *                           2,048 union records in one CTA, and larger ones
+ *                           sort up to 8,192 in one; 0: always the general
+ *                           kernels and the general sort. Same results
  *   CC_TUNE_PRUNED_WARP     1 (default): in the device loop's pruned passes
  *                           each query walks its scene with one warp (a
  *                           shared-memory stack, up to 32 nodes per round);
@@ -294,8 +294,9 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           warp, the rest a thread). Same results
  *   CC_TUNE_REPLAY_CTA_MIN  union records from which a final impact zone's
  *                           unions are replayed by a CTA in shared memory
- *                           (0, the default: every zone by one thread from
- *                           global memory, measured faster). Same results
+ *                           (0, the default: a pass of up to 2,048 records
+ *                           in one CTA, a warp per zone; larger ones a thread
+ *                           per zone from global memory). Same results
  *   CC_TUNE_REFIT_UP        1 (default): the hierarchy refit's walk up takes
  *                           one acquire-release arrival per level, carries
  *                           its box in registers and ends at its scene's
