@@ -287,234 +287,253 @@ __device__ void zone_motion(const int* __restrict__ members, int i, int end, con
     if (bad) atomicOr(&ctr->err, kErrNan);
 }
 
-// Zones of at least this many members are solved one warp per zone
-// (k_zone_solve_warp) where the zone list is built on the device; in a pass
-// with at most `few` zones (a knob), every zone of two or more members is:
-// one thread per zone keeps the FP64 pipe busiest when zones are many, one
-// warp per zone gives the shortest chain when they are few.
+// Zones of at least this many members are solved one warp per zone where the
+// zone list is built on the device; in a pass with at most `few` zones (a
+// knob), every zone of two or more members is: one thread per zone keeps the
+// FP64 pipe busiest when zones are many, one warp per zone gives the shortest
+// chain when they are few.
 constexpr int kZoneWarpMin = 16;
 __device__ __forceinline__ int zone_warp_min(int nzones, int few) { return nzones <= few ? 2 : kZoneWarpMin; }
-constexpr int kZoneWarpBlock = 128;
-constexpr int kZoneCtaThreads = 256;
+constexpr int kZoneSums = 9;  // summed components: L, then the six of I that differ
+constexpr int kZoneWarps = 8, kZoneThreads = kZoneWarps * 32;
+constexpr int kZoneCtas = 152;  // blocks of each role: with both, two per SM
 
-// Zone z's members are members[zone_rng[z].x .. zone_rng[z].y); dnz: the
-// zone count in device memory, at most nzones.
-__global__ void k_zone_solve(ZoneMembers mem, const int2* __restrict__ zone_rng, int nzones,
-                             const int* __restrict__ dnz, const uint8_t* __restrict__ fixed,
-                             const double4_32a* __restrict__ xo, double4_32a* av, const int* __restrict__ vscene,
-                             const SceneDev* __restrict__ scenes, PassCounters* ctr, PassStamp ps, int few) {
-    if (ctr->err & kErrRetry) return;
-    const int* __restrict__ members = mem.list();
-    if (*dnz < nzones) nzones = *dnz;
-    const int warp_min = zone_warp_min(nzones, few);
-    for (int z = blockIdx.x * blockDim.x + threadIdx.x; z < nzones; z += gridDim.x * blockDim.x) {
-        const int i = zone_rng[z].x, end = zone_rng[z].y;
-        if (end - i >= warp_min) continue;  // k_zone_solve_warp's
-        zone_motion(members, i, end, fixed, xo, av, vscene, scenes, ctr, ps);
-    }
+// A member's terms of the sums after the centre of mass: m (dx x dv), and the
+// upper triangle of m (|dx|^2 delta - dx dx) - the lower one is the same
+// products with their factors swapped, so its sums are the same.
+__device__ __forceinline__ void zone_terms(const double* xs, const double* vs, const double* x_cm, const double* v_cm,
+                                           double m, double* t) {
+    double dx[3], dv[3], Li[3];
+    for (int d = 0; d < 3; ++d) { dx[d] = xs[d] - x_cm[d]; dv[d] = vs[d] - v_cm[d]; }
+    cross3(dx, dv, Li);
+    for (int d = 0; d < 3; ++d) t[d] = m * Li[d];
+    const double mag_dx = mag3(dx);
+    const double mag2 = mag_dx * mag_dx;
+    int k = 3;
+    for (int r = 0; r < 3; ++r)
+        for (int q = r; q < 3; ++q) {
+            double v = -dx[r] * dx[q];
+            if (r == q) v += mag2;
+            t[k++] = v * m;
+        }
+}
+__device__ __forceinline__ void zone_inertia(const double* u, double (*I)[3]) {
+    I[0][0] = u[0], I[0][1] = I[1][0] = u[1], I[0][2] = I[2][0] = u[2];
+    I[1][1] = u[3], I[1][2] = I[2][1] = u[4], I[2][2] = u[5];
 }
 
-// Zones of at least kZoneWarpMin members: one warp per zone. The sums of
-// updateImpactListVelocity (centre of mass and velocity, angular momentum,
-// inertia) must be formed member by member in list order to round as the
-// reference's do, and GB300's FP64 pipe makes such a chain slow on one
-// thread: here the lanes load 32 members at a time and form every per-member
-// term in parallel (offsets, m * (dx x dv), m * (|dx|^2 delta - dx dx)),
-// and lane 0 only adds the staged terms in order - the same additions on
-// the same operands as the one-thread form. The final per-member motion is
-// spread over the lanes.
-__global__ void __launch_bounds__(kZoneWarpBlock) k_zone_solve_warp(
-    ZoneMembers mem, const int2* __restrict__ zone_rng, int nzones, const int* __restrict__ dnz,
-    const uint8_t* __restrict__ fixed, const double4_32a* __restrict__ xo, double4_32a* av,
-    const int* __restrict__ vscene, const SceneDev* __restrict__ scenes, PassCounters* ctr, PassStamp ps,
-    int cta_min, int few) {
-    __shared__ double stage[kZoneWarpBlock / 32][32][12];
-    if (ctr->err & kErrRetry) return;
-    const int* __restrict__ members = mem.list();
-    if (*dnz < nzones) nzones = *dnz;
-    const int warp_min = zone_warp_min(nzones, few);
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    double(*st)[12] = stage[wib];
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+struct ZoneArgs {
+    const int* members;
+    const uint8_t* fixed;
+    const double4_32a* xo;
+    double4_32a* av;
+    const int* vscene;
+    const SceneDev* scenes;
+    PassCounters* ctr;
+    PassStamp ps;
+};
+
+// A zone of at least kZoneWarpMin members (or any, in a pass of few zones) by
+// a warp. The sums of updateImpactListVelocity (centre of mass and velocity,
+// angular momentum, inertia) must be formed member by member in list order to
+// round as the reference's do, and GB300's FP64 pipe makes such a chain slow
+// on one thread: here the lanes load 32 members at a time and form every
+// per-member term in parallel, and a lane per component adds the staged terms
+// in order - the same additions on the same operands as the one-thread form.
+// The final per-member motion is spread over the lanes.
+__device__ bool zone_by_warp(const ZoneArgs& z, int i, int end, double (*st)[kZoneSums]) {
+    const int lane = threadIdx.x & 31;
+    const Params prm = z.scenes[z.vscene[z.members[i]]].p;
+    const double m = prm.m, dt = prm.dt;
+    const int num_pts = end - i;
+    double x_cm[3], v_cm[3], L[3], u[6], I[3][3];
+    double acc = 0.0;  // this lane's component of the current sum
+    for (int c = i; c < end; c += 32) {
+        const int q = c + lane;
+        if (q < end) {
+            const int p = z.members[q];
+            double xs[3], vs[3];
+            load3(z.xo, p, xs);
+            load3(z.av, p, vs);
+            for (int d = 0; d < 3; ++d) st[lane][d] = xs[d], st[lane][3 + d] = vs[d];
+        }
+        __syncwarp();
+        if (lane < 6) {  // lane d sums component d over the members in list order
+            const int k1 = end - c < 32 ? end - c : 32;
+            for (int k = 0; k < k1; ++k) acc += st[k][lane];
+        }
+        __syncwarp();
+    }
+    acc = acc / num_pts;
+    for (int d = 0; d < 3; ++d) {
+        x_cm[d] = __shfl_sync(0xffffffffu, acc, d);
+        v_cm[d] = __shfl_sync(0xffffffffu, acc, 3 + d);
+    }
+    acc = 0.0;
+    for (int c = i; c < end; c += 32) {
+        const int q = c + lane;
+        if (q < end) {
+            const int p = z.members[q];
+            double xs[3], vs[3];
+            load3(z.xo, p, xs);
+            load3(z.av, p, vs);
+            zone_terms(xs, vs, x_cm, v_cm, m, st[lane]);
+        }
+        __syncwarp();
+        if (lane < kZoneSums) {
+            const int k1 = end - c < 32 ? end - c : 32;
+            for (int k = 0; k < k1; ++k) acc = st[k][lane] + acc;
+        }
+        __syncwarp();
+    }
+    for (int d = 0; d < 3; ++d) L[d] = __shfl_sync(0xffffffffu, acc, d);
+    for (int k = 0; k < 6; ++k) u[k] = __shfl_sync(0xffffffffu, acc, 3 + k);
+    zone_inertia(u, I);
+    // every lane forms the same rotation (sin and cos on two lanes)
+    double w[3];
+    zone_omega(I, L, w);
+    const double mag_w = mag3(w);
+    double sn, cs;
+    cr::sincos_warp(dt * mag_w, &sn, &cs);
+    const double sw = mag_w < kRoundEps ? 0.0 : sn / mag_w;
+    const double cw = cs;
     bool bad = false;
-    for (int z = gw; z < nzones; z += nw) {
-        const int i = zone_rng[z].x, end = zone_rng[z].y;
-        if (end - i < warp_min || end - i >= cta_min) continue;
-        const Params prm = scenes[vscene[members[i]]].p;
-        const double m = prm.m, dt = prm.dt;
-        const int num_pts = end - i;
-        double x_cm[3], v_cm[3], L[3], I[3][3];
-        double acc = 0.0;  // this lane's component of the current sum
-        for (int c = i; c < end; c += 32) {
-            const int q = c + lane;
-            if (q < end) {
-                const int p = members[q];
-                double xs[3], vs[3];
-                load3(xo, p, xs);
-                load3(av, p, vs);
-                for (int d = 0; d < 3; ++d) st[lane][d] = xs[d], st[lane][3 + d] = vs[d];
-            }
-            __syncwarp();
-            if (lane < 6) {  // lane d sums component d over the members in list order
-                const int k1 = end - c < 32 ? end - c : 32;
-                for (int k = 0; k < k1; ++k) acc += st[k][lane];
-            }
-            __syncwarp();
+    for (int q = i + lane; q < end; q += 32)
+        bad |= zone_member_motion(z.members[q], z.fixed, z.xo, z.av, x_cm, v_cm, w, mag_w, sw, cw, dt, z.ps);
+    __syncwarp();
+    return bad;
+}
+
+// A large zone by a CTA: the same sums in the same order, a lane of warp 0 per
+// component, but every member's terms and its final motion by all the CTA's
+// threads. What bounds it is the 2 n additions in order (~64 cycles each on
+// this FP64 pipe: 41 us of 640 members). A movable body of 642 points on one
+// thread took 3 ms of every pass.
+__device__ bool zone_by_cta(const ZoneArgs& z, int i, int end, double (*st)[kZoneSums]) {
+    __shared__ double s_sum[kZoneSums];
+    __shared__ double s_rot[6];  // w, mag_w, sw, cw
+    const int tid = threadIdx.x;
+    const Params prm = z.scenes[z.vscene[z.members[i]]].p;
+    const double m = prm.m, dt = prm.dt;
+    const int num_pts = end - i;
+    double acc = 0.0;  // this thread's component of the current sum
+    for (int c = i; c < end; c += kZoneThreads) {
+        const int q = c + tid;
+        if (q < end) {
+            const int p = z.members[q];
+            double xs[3], vs[3];
+            load3(z.xo, p, xs);
+            load3(z.av, p, vs);
+            for (int d = 0; d < 3; ++d) st[tid][d] = xs[d], st[tid][3 + d] = vs[d];
         }
-        for (int d = 0; d < 3; ++d) {
-            x_cm[d] = __shfl_sync(0xffffffffu, acc / num_pts, d);
-            v_cm[d] = __shfl_sync(0xffffffffu, acc / num_pts, 3 + d);
+        __syncthreads();
+        if (tid < 6) {
+            const int k1 = end - c < kZoneThreads ? end - c : kZoneThreads;
+            for (int k = 0; k < k1; ++k) acc += st[k][tid];
         }
-        acc = 0.0;
-        for (int c = i; c < end; c += 32) {
-            const int q = c + lane;
-            if (q < end) {
-                const int p = members[q];
-                double xs[3], vs[3], dx[3], dv[3], Li[3];
-                load3(xo, p, xs);
-                load3(av, p, vs);
-                for (int d = 0; d < 3; ++d) { dx[d] = xs[d] - x_cm[d]; dv[d] = vs[d] - v_cm[d]; }
-                cross3(dx, dv, Li);
-                for (int d = 0; d < 3; ++d) st[lane][d] = m * Li[d];
-                const double mag_dx = mag3(dx);
-                for (int r = 0; r < 3; ++r)
-                    for (int s = 0; s < 3; ++s) {
-                        double t = -dx[r] * dx[s];
-                        if (r == s) t += mag_dx * mag_dx;
-                        st[lane][3 + 3 * r + s] = t * m;
-                    }
-            }
-            __syncwarp();
-            if (lane < 12) {  // lane c sums component c (L, then I row by row) in list order
-                const int k1 = end - c < 32 ? end - c : 32;
-                for (int k = 0; k < k1; ++k) acc = st[k][lane] + acc;
-            }
-            __syncwarp();
+        __syncthreads();
+    }
+    if (tid < 6) s_sum[tid] = acc / num_pts;
+    __syncthreads();
+    double x_cm[3], v_cm[3];
+    for (int d = 0; d < 3; ++d) x_cm[d] = s_sum[d], v_cm[d] = s_sum[3 + d];
+    acc = 0.0;
+    for (int c = i; c < end; c += kZoneThreads) {
+        const int q = c + tid;
+        if (q < end) {
+            const int p = z.members[q];
+            double xs[3], vs[3];
+            load3(z.xo, p, xs);
+            load3(z.av, p, vs);
+            zone_terms(xs, vs, x_cm, v_cm, m, st[tid]);
         }
-        for (int d = 0; d < 3; ++d) L[d] = __shfl_sync(0xffffffffu, acc, d);
-        for (int r = 0; r < 3; ++r)
-            for (int q = 0; q < 3; ++q) I[r][q] = __shfl_sync(0xffffffffu, acc, 3 + 3 * r + q);
-        // every lane forms the same rotation (sin and cos on two lanes)
-        double w[3];
+        __syncthreads();
+        if (tid < kZoneSums) {
+            const int k1 = end - c < kZoneThreads ? end - c : kZoneThreads;
+            for (int k = 0; k < k1; ++k) acc = st[k][tid] + acc;
+        }
+        __syncthreads();
+    }
+    if (tid < kZoneSums) s_sum[tid] = acc;
+    __syncthreads();
+    if (tid < 32) {  // warp 0: the same rotation in every lane, sin and cos on two lanes
+        double L[3], u[6], I[3][3], w[3];
+        for (int d = 0; d < 3; ++d) L[d] = s_sum[d];
+        for (int k = 0; k < 6; ++k) u[k] = s_sum[3 + k];
+        zone_inertia(u, I);
         zone_omega(I, L, w);
         const double mag_w = mag3(w);
         double sn, cs;
         cr::sincos_warp(dt * mag_w, &sn, &cs);
-        const double sw = mag_w < kRoundEps ? 0.0 : sn / mag_w;
-        const double cw = cs;
-        for (int q = i + lane; q < end; q += 32)
-            bad |= zone_member_motion(members[q], fixed, xo, av, x_cm, v_cm, w, mag_w, sw, cw, dt, ps);
-        __syncwarp();
+        if (tid == 0) {
+            for (int d = 0; d < 3; ++d) s_rot[d] = w[d];
+            s_rot[3] = mag_w;
+            s_rot[4] = mag_w < kRoundEps ? 0.0 : sn / mag_w;
+            s_rot[5] = cs;
+        }
     }
-    if (bad) atomicOr(&ctr->err, kErrNan);
+    __syncthreads();
+    const double w[3] = {s_rot[0], s_rot[1], s_rot[2]};
+    bool bad = false;
+    for (int q = i + tid; q < end; q += kZoneThreads)
+        bad |= zone_member_motion(z.members[q], z.fixed, z.xo, z.av, x_cm, v_cm, w, s_rot[3], s_rot[4], s_rot[5], dt,
+                                  z.ps);
+    __syncthreads();  // the next zone reuses the shared arrays
+    return bad;
 }
 
-// Zones of at least cta_min members: one CTA per zone. The same sums
-// as k_zone_solve_warp, in the same order - one thread per summed component
-// adding the members in list order - but every member's terms and its
-// final motion are computed by all the CTA's threads (a large zone is
-// otherwise bound by one warp's share of the SM's FP64 pipe).
-// With `run` set, the zones are the movable bodies
-// (updateImpactZoneVelocityForRG, dcollid.cpp:267-288, called from
-// updateAverageVelocity when dt > 0), zone_off their members: only those of
-// scenes in a pass, and of more than one point, move. A body of 642 points
-// took 3 ms of every pass on one thread, whose ~150 FP64 instructions per
-// member each take ~64 cycles; here the ordered sums' two per member remain.
-__global__ void __launch_bounds__(kZoneCtaThreads) k_zone_solve_cta(
-    ZoneMembers mem, const int* __restrict__ zone_off, const int2* __restrict__ zone_rng, int nzones,
-    const int* __restrict__ dnz, const uint8_t* __restrict__ fixed, const double4_32a* __restrict__ xo,
-    double4_32a* av, const int* __restrict__ vscene, const SceneDev* __restrict__ scenes, PassCounters* ctr,
-    const SceneRun* __restrict__ run, PassStamp ps, int cta_min) {
-    __shared__ double st[kZoneCtaThreads][12];
-    __shared__ double s_sum[12];
-    __shared__ double s_rot[6];  // w, mag_w, sw, cw
-    if (ctr->err & kErrRetry) return;
-    const int* __restrict__ members = mem.list();
-    if (dnz && *dnz < nzones) nzones = *dnz;
-    const int tid = threadIdx.x;
+// Every zone of a pass in one launch (zone z's members: zone_rng[z], their
+// count *dnz, at most nzones): the first kZoneCtas blocks take the zones of at
+// least cta_min members, the others the rest, a warp or a thread each.
+__global__ void __launch_bounds__(kZoneThreads, 2) k_zone_solve(ZoneArgs z, ZoneMembers mem,
+                                                                const int2* __restrict__ zone_rng, int nzones,
+                                                                const int* __restrict__ dnz, int cta_min, int few) {
+    __shared__ double st[kZoneThreads][kZoneSums];
+    if (z.ctr->err & kErrRetry) return;
+    z.members = mem.list();
+    if (*dnz < nzones) nzones = *dnz;
     bool bad = false;
-    for (int z = blockIdx.x; z < nzones; z += gridDim.x) {
-        const int i = zone_rng ? zone_rng[z].x : zone_off[z], end = zone_rng ? zone_rng[z].y : zone_off[z + 1];
-        if (end - i < cta_min) continue;
-        if (run) {
-            const int zs = vscene[members[i]];
-            if (run[zs].mode == kSceneIdle || !(scenes[zs].p.dt > 0.0)) continue;
+    if (blockIdx.x < kZoneCtas) {
+        for (int k = blockIdx.x; k < nzones; k += kZoneCtas) {
+            const int2 r = zone_rng[k];
+            if (r.y - r.x >= cta_min) bad |= zone_by_cta(z, r.x, r.y, st);
         }
-        const Params prm = scenes[vscene[members[i]]].p;
-        const double m = prm.m, dt = prm.dt;
-        const int num_pts = end - i;
-        double acc = 0.0;  // this thread's component of the current sum (threads 0..11)
-        for (int c = i; c < end; c += kZoneCtaThreads) {
-            const int q = c + tid;
-            if (q < end) {
-                const int p = members[q];
-                double xs[3], vs[3];
-                load3(xo, p, xs);
-                load3(av, p, vs);
-                for (int d = 0; d < 3; ++d) st[tid][d] = xs[d], st[tid][3 + d] = vs[d];
-            }
-            __syncthreads();
-            if (tid < 6) {
-                const int k1 = end - c < kZoneCtaThreads ? end - c : kZoneCtaThreads;
-                for (int k = 0; k < k1; ++k) acc += st[k][tid];
-            }
-            __syncthreads();
+    } else {
+        const int b = blockIdx.x - kZoneCtas, nb = gridDim.x - kZoneCtas;
+        const int warp_min = zone_warp_min(nzones, few);
+        const int wib = threadIdx.x >> 5;
+        for (int k = b + nb * wib; k < nzones; k += nb * kZoneWarps) {
+            const int2 r = zone_rng[k];
+            if (r.y - r.x >= warp_min && r.y - r.x < cta_min) bad |= zone_by_warp(z, r.x, r.y, st + 32 * wib);
         }
-        if (tid < 6) s_sum[tid] = acc / num_pts;
-        __syncthreads();
-        double x_cm[3], v_cm[3];
-        for (int d = 0; d < 3; ++d) x_cm[d] = s_sum[d], v_cm[d] = s_sum[3 + d];
-        acc = 0.0;
-        for (int c = i; c < end; c += kZoneCtaThreads) {
-            const int q = c + tid;
-            if (q < end) {
-                const int p = members[q];
-                double xs[3], vs[3], dx[3], dv[3], Li[3];
-                load3(xo, p, xs);
-                load3(av, p, vs);
-                for (int d = 0; d < 3; ++d) { dx[d] = xs[d] - x_cm[d]; dv[d] = vs[d] - v_cm[d]; }
-                cross3(dx, dv, Li);
-                for (int d = 0; d < 3; ++d) st[tid][d] = m * Li[d];
-                const double mag_dx = mag3(dx);
-                for (int r = 0; r < 3; ++r)
-                    for (int s2 = 0; s2 < 3; ++s2) {
-                        double t = -dx[r] * dx[s2];
-                        if (r == s2) t += mag_dx * mag_dx;
-                        st[tid][3 + 3 * r + s2] = t * m;
-                    }
+        if (warp_min > 2)
+            for (int k = b + nb * (int)threadIdx.x; k < nzones; k += nb * kZoneThreads) {
+                const int2 r = zone_rng[k];
+                if (r.y - r.x < warp_min)
+                    zone_motion(z.members, r.x, r.y, z.fixed, z.xo, z.av, z.vscene, z.scenes, z.ctr, z.ps);
             }
-            __syncthreads();
-            if (tid < 12) {
-                const int k1 = end - c < kZoneCtaThreads ? end - c : kZoneCtaThreads;
-                for (int k = 0; k < k1; ++k) acc = st[k][tid] + acc;
-            }
-            __syncthreads();
-        }
-        if (tid < 12) s_sum[tid] = acc;
-        __syncthreads();
-        if (tid < 32) {  // warp 0: the same rotation in every lane, sin and cos on two lanes
-            double L[3], I[3][3], w[3];
-            for (int d = 0; d < 3; ++d) L[d] = s_sum[d];
-            for (int r = 0; r < 3; ++r)
-                for (int q = 0; q < 3; ++q) I[r][q] = s_sum[3 + 3 * r + q];
-            zone_omega(I, L, w);
-            const double mag_w = mag3(w);
-            double sn, cs;
-            cr::sincos_warp(dt * mag_w, &sn, &cs);
-            if (tid == 0) {
-                for (int d = 0; d < 3; ++d) s_rot[d] = w[d];
-                s_rot[3] = mag_w;
-                s_rot[4] = mag_w < kRoundEps ? 0.0 : sn / mag_w;
-                s_rot[5] = cs;
-            }
-        }
-        __syncthreads();
-        const double w[3] = {s_rot[0], s_rot[1], s_rot[2]};
-        for (int q = i + tid; q < end; q += kZoneCtaThreads)
-            bad |= zone_member_motion(members[q], fixed, xo, av, x_cm, v_cm, w, s_rot[3], s_rot[4], s_rot[5], dt, ps);
-        __syncthreads();  // the next zone reuses the shared arrays
     }
-    if (bad) atomicOr(&ctr->err, kErrNan);
+    if (bad) atomicOr(&z.ctr->err, kErrNan);
+}
+
+// The movable bodies (updateImpactZoneVelocityForRG, dcollid.cpp:267-288,
+// called from updateAverageVelocity when dt > 0), zone_off their members: only
+// those of scenes in a pass (run), and of more than one point, move.
+__global__ void __launch_bounds__(kZoneThreads, 2) k_body_solve(ZoneArgs z, const int* __restrict__ zone_off,
+                                                                int nzones, const SceneRun* __restrict__ run) {
+    __shared__ double st[kZoneThreads][kZoneSums];
+    if (z.ctr->err & kErrRetry) return;
+    bool bad = false;
+    for (int k = blockIdx.x; k < nzones; k += gridDim.x) {
+        const int i = zone_off[k], end = zone_off[k + 1];
+        if (end - i < 2) continue;
+        if (run) {
+            const int zs = z.vscene[z.members[i]];
+            if (run[zs].mode == kSceneIdle || !(z.scenes[zs].p.dt > 0.0)) continue;
+        }
+        bad |= zone_by_cta(z, i, end, st);
+    }
+    if (bad) atomicOr(&z.ctr->err, kErrNan);
 }
 
 // detectDomainBoundaryCollision (dcollid.cpp:116-158) then
@@ -654,31 +673,17 @@ void zone_solve(const int* members, const int* zone_off, int nzones, const uint8
                 const SceneRun* run, PassStamp ps) {
     // (a body of one point does not move)
     if (nzones > 0)
-        count_launch(), k_zone_solve_cta<<<nzones < 152 * 8 ? nzones : 152 * 8, kZoneCtaThreads, 0, s>>>(
-            ZoneMembers{{const_cast<int*>(members), nullptr}, nullptr}, zone_off, nullptr, nzones, nullptr, fixed, xo,
-            av, vscene, scenes, ctr, run, ps, 2);
+        count_launch(), k_body_solve<<<nzones < 152 * 8 ? nzones : 152 * 8, kZoneThreads, 0, s>>>(
+            ZoneArgs{members, fixed, xo, av, vscene, scenes, ctr, ps}, zone_off, nzones, run);
 }
 
 void zone_solve_dev(const ZoneMembers& members, const int2* zone_rng, const int* dnz, int zone_cap, const uint8_t* fixed,
                     const double4_32a* xo, double4_32a* av, const int* vscene, const SceneDev* scenes,
                     PassCounters* ctr, cudaStream_t s, PassStamp ps, int cta_min, int few) {
     if (cta_min < kZoneWarpMin) cta_min = kZoneWarpMin;
-    int blocks = nblk(zone_cap, 64);
-    if (blocks > 152 * 8) blocks = 152 * 8;
-    if (blocks > 0)
-        count_launch(), k_zone_solve<<<blocks, 64, 0, s>>>(members, zone_rng, zone_cap, dnz, fixed, xo, av, vscene,
-                                                           scenes, ctr, ps, few);
-    int wblocks = nblk(zone_cap, kZoneWarpBlock / 32);
-    if (wblocks > 152 * 4) wblocks = 152 * 4;
-    if (wblocks > 0)
-        count_launch(), k_zone_solve_warp<<<wblocks, kZoneWarpBlock, 0, s>>>(members, zone_rng, zone_cap, dnz, fixed,
-                                                                            xo, av, vscene, scenes, ctr, ps, cta_min,
-                                                                            few);
-    const int cblocks = zone_cap < 152 * 2 ? zone_cap : 152 * 2;
-    if (cblocks > 0)
-        count_launch(), k_zone_solve_cta<<<cblocks, kZoneCtaThreads, 0, s>>>(members, nullptr, zone_rng, zone_cap, dnz,
-                                                                            fixed, xo, av, vscene, scenes, ctr, nullptr,
-                                                                            ps, cta_min);
+    if (zone_cap > 0)
+        count_launch(), k_zone_solve<<<2 * kZoneCtas, kZoneThreads, 0, s>>>(
+            ZoneArgs{nullptr, fixed, xo, av, vscene, scenes, ctr, ps}, members, zone_rng, zone_cap, dnz, cta_min, few);
 }
 
 void final_rigid(const BodyBufs& b, const uint8_t* has_collsn, const double4_32a* av, cudaStream_t s) {
