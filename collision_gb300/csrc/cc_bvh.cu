@@ -8,6 +8,7 @@
 // per axis) are sorted by the hand-written radix sort; the hierarchy is the
 // Karras (2012) construction; refit walks up with arrival counters.
 #include "cc_launch.h"
+#include "cc_point_box.cuh"
 
 namespace ccg {
 
@@ -84,6 +85,25 @@ __device__ __forceinline__ Box6 padded(const double* mn, const double* mx, doubl
     }
     return b;
 }
+// Extremes of an element's points over the step: of its ends, and of its
+// starts too where they are not in mn, mx yet.
+template <bool STARTS>
+__device__ __forceinline__ void sweep_extremes(const int* pt, int np, double dt, const double4_32a* __restrict__ xo,
+                                               const double4_32a* __restrict__ av, double* mn, double* mx) {
+    for (int i = 0; i < np; ++i) {
+        const double4_32a x = xo[pt[i]], v = av[pt[i]];
+        const double xs[3] = {x.x, x.y, x.z}, vs[3] = {v.x, v.y, v.z};
+        for (int d = 0; d < 3; ++d) {
+            const double xe = xs[d] + vs[d] * dt;
+            if (STARTS) {
+                mx[d] = smax(mx[d], xs[d]);
+                mn[d] = smin(mn[d], xs[d]);
+            }
+            mx[d] = smax(mx[d], xe);
+            mn[d] = smin(mn[d], xe);
+        }
+    }
+}
 template <int KIND>
 __device__ __forceinline__ void leaf_box(const int* __restrict__ ev, const int* __restrict__ act, int n, int k,
                                          const int* __restrict__ elem_scene, const SceneDev* __restrict__ scenes,
@@ -115,20 +135,7 @@ __device__ __forceinline__ void leaf_box(const int* __restrict__ ev, const int* 
     }
     if (KIND != kBoxStatic) {
         if (valid) {
-            const double dt = scenes[scene].p.dt;
-            for (int i = 0; i < np; ++i) {
-                const double4_32a x = xo[pt[i]], v = av[pt[i]];
-                const double xs[3] = {x.x, x.y, x.z}, vs[3] = {v.x, v.y, v.z};
-                for (int d = 0; d < 3; ++d) {
-                    const double xe = xs[d] + vs[d] * dt;
-                    if (KIND == kBoxSwept) {
-                        mx[d] = smax(mx[d], xs[d]);
-                        mn[d] = smin(mn[d], xs[d]);
-                    }
-                    mx[d] = smax(mx[d], xe);
-                    mn[d] = smin(mn[d], xe);
-                }
-            }
+            sweep_extremes<KIND == kBoxSwept>(pt, np, scenes[scene].p.dt, xo, av, mn, mx);
             box[e] = padded(mn, mx, lo, hi);
         }
         scene_bbox_accumulate(bb, scene, valid, lo, hi);
@@ -1017,6 +1024,106 @@ __global__ void k_dirty_queries(const int* __restrict__ act_l, const unsigned in
     }
 }
 
+// Grows a child's box in its parent's record to hold b, float by float
+// (integer atomics on the ordered bits); false if it held b already.
+__device__ __forceinline__ void atomic_min_float(float* p, float x) {
+    x += 0.0f;  // -0 as +0
+    if (x >= 0.0f)
+        atomicMin(reinterpret_cast<int*>(p), __float_as_int(x));
+    else
+        atomicMax(reinterpret_cast<unsigned*>(p), __float_as_uint(x));
+}
+__device__ __forceinline__ void atomic_max_float(float* p, float x) {
+    x += 0.0f;
+    if (x >= 0.0f)
+        atomicMax(reinterpret_cast<int*>(p), __float_as_int(x));
+    else
+        atomicMin(reinterpret_cast<unsigned*>(p), __float_as_uint(x));
+}
+__device__ __forceinline__ bool grow_child(BvhNode32* nd, int side, const Box32& c, const Box32& b) {
+    float* f = reinterpret_cast<float*>(nd) + (side ? 6 : 0);  // lo, then hi
+    bool grew = false;
+    for (int d = 0; d < 3; ++d) {
+        if (b.lo[d] < c.lo[d]) {
+            atomic_min_float(f + d, b.lo[d]);
+            grew = true;
+        }
+        if (b.hi[d] > c.hi[d]) {
+            atomic_max_float(f + 3 + d, b.hi[d]);
+            grew = true;
+        }
+    }
+    return grew;
+}
+
+// The boxes of a pruned pass. Between two passes only the points stamped by
+// the earlier one have moved, so only the elements that hold one (the dirty
+// ones, the pass's queries) have another box: this kernel finds them, writes
+// their boxes and leaf records, adds the boxes to the scenes' and climbs from
+// each leaf while a record above does not hold its box, and forms the
+// filters' data of the stamped points. Records and scenes' boxes only grow
+// from the step's last full refit on: the walks test leaves exactly, and
+// tree_bound_reset looks again where the grown box would rebuild a tree. A
+// full pass instead boxes every element and climbs every level of the tree.
+// 48 sheets in contact: boxes, refit and full walks of a step 5.9 -> 2.6 ms (68
+// passes).
+template <bool POINTS>
+__global__ void __launch_bounds__(256) k_dirty_update(
+    const int* __restrict__ act_l, const int* __restrict__ act_p, const unsigned int* __restrict__ order, int n,
+    int ne_all, const int* __restrict__ ev, const unsigned* __restrict__ stamp, LoopCtl* L, uint8_t* edirty, int* query,
+    PassCounters* ctr, const int* __restrict__ elem_scene, const SceneDev* __restrict__ scenes,
+    const SceneRun* __restrict__ run, const double4_32a* __restrict__ xo, const double4_32a* __restrict__ av, Box6* box,
+    unsigned long long* bb, LeafRec* leaf, BvhNode32* node, const int* __restrict__ parent,
+    const int* __restrict__ vscene, float4* plo, float4* phi, float4* p32, float4* v32) {
+    const int ne = L->nact_e, m = ne + (POINTS ? L->npts : 0);
+    const unsigned prev = L->serial - 1u, cur = L->serial;  // see k_dirty_queries
+    auto stamped = [&](int p) {
+        const unsigned s = stamp[p];
+        return s == prev || s == cur;
+    };
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
+        if (k >= ne) {
+            const int p = act_p[k - ne];
+            if (stamped(p)) point_box<true>(xo, av, vscene, scenes, p, plo, phi, p32, v32);
+            continue;
+        }
+        const int j = act_l[k];
+        const int e = (j >= 0 && j < n) ? (int)order[j] : -1;
+        if (e < 0 || e >= ne_all) {
+            atomicOr(&ctr->err, kErrIndexLeaf);
+            continue;
+        }
+        const int pt[3] = {ev[3 * e], ev[3 * e + 1], ev[3 * e + 2]};
+        const bool dirty = stamped(pt[0]) || stamped(pt[1]) || (pt[2] >= 0 && stamped(pt[2]));
+        edirty[e] = dirty ? 1 : 0;
+        if (!dirty) continue;
+        query[aggregated_add(&L->nquery, 1)] = j;
+        const int scene = elem_scene ? elem_scene[e] : 0;
+        double mx[3] = {-kBig, -kBig, -kBig}, mn[3] = {kBig, kBig, kBig}, lo[3], hi[3];
+        sweep_extremes<true>(pt, pt[2] >= 0 ? 3 : 2, scenes[scene].p.dt, xo, av, mn, mx);
+        const Box6 b = padded(mn, mx, lo, hi);
+        box[e] = b;
+        const BoxOrd o = box_ord(b);
+        for (int d = 0; d < 3; ++d) {
+            leaf[j].lo[d] = o.lo[d];
+            leaf[j].hi[d] = o.hi[d];
+            unsigned long long* w = bb + 6 * scene + d;
+            if (lo[d] == lo[d] && enc_double(lo[d]) < __ldcg(w)) atomicMin(w, enc_double(lo[d]));
+            if (hi[d] == hi[d] && enc_double(hi[d]) > __ldcg(w + 3)) atomicMax(w + 3, enc_double(hi[d]));
+        }
+        const int root = run ? run[scene].root : 0;
+        if (root < 0) continue;  // a scene of one element: no nodes
+        const Box32 b32 = box32_out(b);
+        int child = ~j, nd = parent[n - 1 + j];
+        for (int level = 0; level < n && nd >= 0 && nd < n - 1; ++level) {
+            const int side = node[nd].meta.x == child ? 0 : 1, up = parent[nd];
+            if (!grow_child(&node[nd], side, get_child_cg(&node[nd], side), b32) || nd == root) break;
+            child = nd;
+            nd = up;
+        }
+    }
+}
+
 // The pruned traversal: each dirty element walks its whole scene along the
 // ropes from the scene's root and writes every overlapping leaf that is not
 // itself, shares no point with it, and is clean or dirty with a larger
@@ -1471,12 +1578,31 @@ void pruned_pairs(const BvhBufs& b, const int* act_e, const int* act_l, const un
     count_launch(), k_dirty_queries<<<dev_grid(ne_cap, 256), 256, 0, s>>>(act_l, b.order, b.n, b.ne_all, ev, stamp, L,
                                                                           edirty, query, ctr);
     if (warp && b.node)
-        count_launch(), k_traverse_warp<kWalkPruned><<<dev_grid(ne_cap, kPrunedWarps), kPrunedWarps * 32, 0, s>>>(
-            b.n, b.node, b.elem_scene, b.run, ev, pairs, cap, ctr, nullptr, b.leaf, query, 0, nullptr, nullptr, L,
-            edirty);
+        dirty_pairs(b, L, edirty, query, ne_cap, pairs, cap, ctr, ev, s);
     else
         count_launch(), k_traverse_rope_full<<<dev_grid(ne_cap, 128), 128, 0, s>>>(
             b.n, b.rnode, b.rope, b.elem_scene, b.run, ev, pairs, cap, ctr, b.leaf, query, L, edirty);
+}
+
+void dirty_pairs_update(const BvhBufs& b, const int* act_l, const int* act_p, const unsigned* stamp, LoopCtl* L,
+                        uint8_t* edirty, int* query, int ne_cap, int nv_cap, PassCounters* ctr, const int* ev,
+                        const double4_32a* xo, const double4_32a* av, Box6* box, const PointBufs* pts,
+                        cudaStream_t s) {
+    const int g = dev_grid(ne_cap + nv_cap, 256);
+    if (pts)
+        count_launch(), k_dirty_update<true><<<g, 256, 0, s>>>(
+            act_l, act_p, b.order, b.n, b.ne_all, ev, stamp, L, edirty, query, ctr, b.elem_scene, b.scenes, b.run, xo,
+            av, box, b.bbox_enc, b.leaf, b.node, b.parent, pts->vscene, pts->lo, pts->hi, pts->p32, pts->v32);
+    else
+        count_launch(), k_dirty_update<false><<<g, 256, 0, s>>>(
+            act_l, act_p, b.order, b.n, b.ne_all, ev, stamp, L, edirty, query, ctr, b.elem_scene, b.scenes, b.run, xo,
+            av, box, b.bbox_enc, b.leaf, b.node, b.parent, nullptr, nullptr, nullptr, nullptr, nullptr);
+}
+
+void dirty_pairs(const BvhBufs& b, LoopCtl* L, const uint8_t* edirty, const int* query, int ne_cap, int2* pairs, int cap,
+                 PassCounters* ctr, const int* ev, cudaStream_t s) {
+    count_launch(), k_traverse_warp<kWalkPruned><<<dev_grid(ne_cap, kPrunedWarps), kPrunedWarps * 32, 0, s>>>(
+        b.n, b.node, b.elem_scene, b.run, ev, pairs, cap, ctr, nullptr, b.leaf, query, 0, nullptr, nullptr, L, edirty);
 }
 
 void brute_pairs(const Box6* box, int ne, const int* elem_scene, int2* pairs, int cap, PassCounters* ctr,

@@ -193,7 +193,7 @@ enum LoopHost { kHostRebuild = 1, kHostRetry = 2, kHostFatal = 4 };
 enum LoopAcc {
     kAccPasses, kAccCcd, kAccZone, kAccPairs, kAccVisits, kAccHits, kAccContacts, kAccSub, kAccMovingVisits,
     kAccCr, kAccLeaves, kAccBroadPairs, kAccPathBytes, kAccZonePasses, kAccIters, kAccProxPairs, kAccQueries,
-    kAccUnions, kNumAcc
+    kAccUnions, kAccDirty, kNumAcc
 };
 struct LoopCtl {
     int host;       // LoopHost bits: the loop stopped for the host

@@ -385,10 +385,12 @@ cudaError_t zone_pass(const ZoneBufs& z, const PassCounters* ctr, const uint8_t*
 // (eoff, poff: nscenes + 1 each); loop_expand writes the pass's elements,
 // their sorted leaves in the step's hierarchy and points; tree_check flags
 // scenes whose tree `which` must be rebuilt on the host; loop_reset opens
-// the pass; pass_end closes it and, in the graph, decides whether the loop
+// the pass; h_form: the switch between a pass's two broad phases, 1 where a
+// pruned pass may box its dirty elements only (dirty_only); pass_end closes it and, in the graph, decides whether the loop
 // goes on.
 void loop_plan(SceneCtl* ctl, SceneRun* run, const SceneDev* scenes, int nscenes, LoopCtl* L, int* sel, int* eoff,
-               int* poff, cudaGraphConditionalHandle h_zone, cudaStream_t s);
+               int* poff, cudaGraphConditionalHandle h_zone, cudaGraphConditionalHandle h_form, int dirty_only,
+               cudaStream_t s);
 void loop_expand(const int* sel, const int* eoff, const int* poff, const SceneDev* scenes, const SceneCtl* ctl,
                  const LoopCtl* L, int cap, int* act_e, int* act_l, int* act_p, cudaStream_t s);
 void tree_check(const SceneRun* run, int nscenes, const unsigned long long* bbox_enc, const double* vol,
@@ -398,6 +400,12 @@ void loop_reset(PassCounters* c, SceneRun* run, int nscenes, LoopCtl* L, cudaStr
 // above 4,096 scenes).
 void tree_check_reset(SceneRun* run, int nscenes, const unsigned long long* bbox_enc, const double* vol,
                       const int* built, int which, int* rebuild, LoopCtl* L, PassCounters* c, cudaStream_t s);
+// The same for scenes' boxes that have only grown since they were exact: a
+// scene whose grown box would rebuild its tree gets its exact box first (from
+// all its elements' boxes), and is tested on that.
+void tree_bound_reset(SceneRun* run, const SceneDev* scenes, int nscenes, unsigned long long* bbox_enc, const Box6* box,
+                      const double* vol, const int* built, int which, int* rebuild, LoopCtl* L, PassCounters* c,
+                      cudaStream_t s);
 // Stage profiling inside the loop graph: acc[0] the last boundary's time,
 // then (ns, count) for each of kLoopMarkSlots slots 1.. - the time since the
 // previous boundary - then a per-pass log (the row count, then
@@ -422,6 +430,20 @@ void pass_end(const PassCounters* c, SceneCtl* ctl, const SceneRun* run, int nsc
 void pruned_pairs(const BvhBufs& b, const int* act_e, const int* act_l, const unsigned* stamp, LoopCtl* L,
                   uint8_t* edirty, int* query, int ne_cap, int2* pairs, int cap, PassCounters* ctr, const int* ev,
                   cudaStream_t s, bool warp = true);
+
+// The same with the boxes of the pass brought up to date first, for the dirty
+// elements and stamped points only (k_dirty_update, in place of leaf_boxes,
+// bvh_refit, point_boxes and k_dirty_queries); the walks, a warp each, after
+// tree_bound_reset. pts: the mixed filters' data (null: none).
+struct PointBufs {
+    const int* vscene;
+    float4 *lo, *hi, *p32, *v32;
+};
+void dirty_pairs_update(const BvhBufs& b, const int* act_l, const int* act_p, const unsigned* stamp, LoopCtl* L,
+                        uint8_t* edirty, int* query, int ne_cap, int nv_cap, PassCounters* ctr, const int* ev,
+                        const double4_32a* xo, const double4_32a* av, Box6* box, const PointBufs* pts, cudaStream_t s);
+void dirty_pairs(const BvhBufs& b, LoopCtl* L, const uint8_t* edirty, const int* query, int ne_cap, int2* pairs, int cap,
+                 PassCounters* ctr, const int* ev, cudaStream_t s);
 
 // updateFinalForRG's device part: per body, the first point in element
 // order with has_collsn and its average velocity (into b.out).

@@ -60,7 +60,8 @@ __device__ __forceinline__ int3 block_scan3(int3 v, int3* tot) {
 __global__ void __launch_bounds__(kPlanThreads) k_loop_plan(SceneCtl* ctl, SceneRun* run,
                                                             const SceneDev* __restrict__ scenes, int nscenes,
                                                             LoopCtl* L, int* sel, int* eoff, int* poff,
-                                                            cudaGraphConditionalHandle h_zone) {
+                                                            cudaGraphConditionalHandle h_zone,
+                                                            cudaGraphConditionalHandle h_form, int dirty_only) {
     if (L->host) {
         // a pass before this one stopped for the host: nothing runs
         if (threadIdx.x == 0) {
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_loop_plan(SceneCtl* ctl, Scene
             L->nq_full = L->nquery = 0;
             L->any_zone = 0;
             cudaGraphSetConditional(h_zone, 0u);
+            if (dirty_only) cudaGraphSetConditional(h_form, 0u);
         }
         return;
     }
@@ -162,6 +164,10 @@ __global__ void __launch_bounds__(kPlanThreads) k_loop_plan(SceneCtl* ctl, Scene
         L->npts = carry.y;
         L->pending = 0;
         cudaGraphSetConditional(h_zone, any_zone ? 1u : 0u);
+        if (dirty_only) {
+            cudaGraphSetConditional(h_form, L->prune ? 1u : 0u);
+            if (L->prune) L->acc[kAccDirty] += 1;
+        }
     }
 }
 
@@ -191,6 +197,10 @@ __global__ void k_loop_expand(const int* __restrict__ sel, const int* __restrict
     }
 }
 
+__device__ __forceinline__ unsigned long long enc_double(double x) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
+}
 __device__ __forceinline__ double dec_double(unsigned long long e) {
     unsigned long long u = (e & 0x8000000000000000ull) ? (e & 0x7fffffffffffffffull) : ~e;
     return __longlong_as_double((long long)u);
@@ -200,10 +210,9 @@ __device__ __forceinline__ double dec_double(unsigned long long e) {
 // every scene of the pass: its tree `which` is unbuilt, or the root volume of
 // this pass's boxes has grown by more than 20% over the volume both trees
 // share. Such a scene is flagged for the host, and the pass stops.
-__device__ __forceinline__ void tree_check_one(const SceneRun* __restrict__ run, int s,
-                                               const unsigned long long* bbox_enc, const double* __restrict__ vol,
-                                               const int* __restrict__ built, int which, int* rebuild, LoopCtl* L) {
-    if (run[s].mode == kSceneIdle || run[s].leaf0 < 0) return;
+__device__ __forceinline__ bool tree_grown(const SceneRun* __restrict__ run, int s, const unsigned long long* bbox_enc,
+                                           const double* __restrict__ vol, const int* __restrict__ built) {
+    if (run[s].mode == kSceneIdle || run[s].leaf0 < 0) return false;
     double lo[3], hi[3];
     for (int d = 0; d < 3; ++d) {
         lo[d] = dec_double(bbox_enc[6 * s + d]);
@@ -211,7 +220,12 @@ __device__ __forceinline__ void tree_check_one(const SceneRun* __restrict__ run,
     }
     const double v = (hi[0] - lo[0]) * (hi[1] - lo[1]) * (hi[2] - lo[2]);
     const double sv = vol[s];
-    if (!built[s] || (v - sv) > 0.2 * sv) {
+    return !built[s] || (v - sv) > 0.2 * sv;
+}
+__device__ __forceinline__ void tree_check_one(const SceneRun* __restrict__ run, int s,
+                                               const unsigned long long* bbox_enc, const double* __restrict__ vol,
+                                               const int* __restrict__ built, int which, int* rebuild, LoopCtl* L) {
+    if (tree_grown(run, s, bbox_enc, vol, built)) {
         rebuild[s] = which + 1;
         atomicOr(&L->host, kHostRebuild);
     }
@@ -225,11 +239,13 @@ __global__ void k_tree_check(const SceneRun* __restrict__ run, int nscenes, cons
     tree_check_one(run, s, bbox_enc, vol, built, which, rebuild, L);
 }
 
+constexpr int kErrIndex = kErrIndexNode | kErrIndexLeaf | kErrIndexElem;
+
 // Counters and hit counts of a pass about to run. A pass stopped for the
 // host keeps the error bit kErrHost (nothing of it is applied) and covers no
 // elements or points.
-__device__ __forceinline__ void loop_reset_counters(PassCounters* c, LoopCtl* L) {
-    const int keep = c->err & kErrNan;
+__device__ __forceinline__ void loop_reset_counters(PassCounters* c, LoopCtl* L, int keep_bits = kErrNan) {
+    const int keep = c->err & keep_bits;
     const bool stop = L->host != 0;
     c->npairs = (!stop && L->reuse_n >= 0) ? L->reuse_n : 0;
     c->ncontrib = 0; c->nhit_pairs = 0; c->nrec = 0; c->nvisits = 0; c->ncontacts = 0; c->nsub = 0;
@@ -264,6 +280,62 @@ __global__ void __launch_bounds__(1024) k_tree_check_reset(SceneRun* run, int ns
     __syncthreads();
     if (threadIdx.x == 0) loop_reset_counters(c, L);
     for (int s = threadIdx.x; s < nscenes; s += blockDim.x) run[s].hits = 0;
+}
+
+// k_tree_check_reset on boxes that have only grown (k_dirty_update). The test
+// is on growth, so a scene it passes on the grown box it passes on the exact
+// one; the others (a sheet's outermost elements moving in again are rare)
+// get their exact box from their elements' boxes, the whole block on one.
+// The index errors k_dirty_update may have found stay.
+__global__ void __launch_bounds__(1024) k_tree_bound_reset(SceneRun* run, const SceneDev* __restrict__ scenes,
+                                                            int nscenes, unsigned long long* bbox_enc,
+                                                            const Box6* __restrict__ box,
+                                                            const double* __restrict__ vol,
+                                                            const int* __restrict__ built, int which, int* rebuild,
+                                                            LoopCtl* L, PassCounters* c) {
+    __shared__ unsigned long long s_bb[6];
+    __shared__ int s_list[1024], s_n;
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int base = 0; base < nscenes && L->nact != 0; base += blockDim.x) {
+        __syncthreads();
+        if (tid == 0) s_n = 0;
+        __syncthreads();
+        const int mine = base + tid;
+        if (mine < nscenes && tree_grown(run, mine, bbox_enc, vol, built)) s_list[atomicAdd(&s_n, 1)] = mine;
+        __syncthreads();
+        for (int q = 0; q < s_n; ++q) {
+            const int s = s_list[q];
+            if (tid < 6) s_bb[tid] = tid < 3 ? ~0ull : 0ull;
+            __syncthreads();
+            unsigned long long b[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
+            const int e0 = scenes[s].e0, ne = scenes[s].ne;
+            for (int e = tid; e < ne; e += blockDim.x)
+                for (int d = 0; d < 3; ++d) {
+                    const double lo = box[e0 + e].lo[d], hi = box[e0 + e].hi[d];
+                    if (lo == lo && enc_double(lo) < b[d]) b[d] = enc_double(lo);
+                    if (hi == hi && enc_double(hi) > b[3 + d]) b[3 + d] = enc_double(hi);
+                }
+            for (int d = 0; d < 6; ++d) {
+                for (int o = 16; o > 0; o >>= 1) {
+                    const unsigned long long x = __shfl_xor_sync(0xffffffffu, b[d], o);
+                    b[d] = d < 3 ? (x < b[d] ? x : b[d]) : (x > b[d] ? x : b[d]);
+                }
+                if (lane == 0) {
+                    if (d < 3)
+                        atomicMin(&s_bb[d], b[d]);
+                    else
+                        atomicMax(&s_bb[d], b[d]);
+                }
+            }
+            __syncthreads();
+            if (tid < 6) bbox_enc[6 * s + tid] = s_bb[tid];
+            __syncthreads();
+            if (tid == 0) tree_check_one(run, s, bbox_enc, vol, built, which, rebuild, L);
+        }
+    }
+    __syncthreads();
+    if (tid == 0) loop_reset_counters(c, L, kErrNan | kErrIndex);
+    for (int s = tid; s < nscenes; s += blockDim.x) run[s].hits = 0;
 }
 
 // Closes a pass. A pass that stopped or failed stops the loop (the host
@@ -361,8 +433,10 @@ __global__ void __launch_bounds__(kPlanThreads) k_pass_end(const PassCounters* _
 }  // namespace
 
 void loop_plan(SceneCtl* ctl, SceneRun* run, const SceneDev* scenes, int nscenes, LoopCtl* L, int* sel, int* eoff,
-               int* poff, cudaGraphConditionalHandle h_zone, cudaStream_t s) {
-    count_launch(), k_loop_plan<<<1, kPlanThreads, 0, s>>>(ctl, run, scenes, nscenes, L, sel, eoff, poff, h_zone);
+               int* poff, cudaGraphConditionalHandle h_zone, cudaGraphConditionalHandle h_form, int dirty_only,
+               cudaStream_t s) {
+    count_launch(), k_loop_plan<<<1, kPlanThreads, 0, s>>>(ctl, run, scenes, nscenes, L, sel, eoff, poff, h_zone,
+                                                           h_form, dirty_only);
 }
 
 void loop_expand(const int* sel, const int* eoff, const int* poff, const SceneDev* scenes, const SceneCtl* ctl,
@@ -388,6 +462,14 @@ void tree_check_reset(SceneRun* run, int nscenes, const unsigned long long* bbox
     }
     const int t = nscenes < 32 ? 32 : (nscenes < 1024 ? (nscenes + 31) / 32 * 32 : 1024);
     count_launch(), k_tree_check_reset<<<1, t, 0, s>>>(run, nscenes, bbox_enc, vol, built, which, rebuild, L, c);
+}
+
+void tree_bound_reset(SceneRun* run, const SceneDev* scenes, int nscenes, unsigned long long* bbox_enc, const Box6* box,
+                      const double* vol, const int* built, int which, int* rebuild, LoopCtl* L, PassCounters* c,
+                      cudaStream_t s) {
+    const int t = nscenes <= 256 ? 256 : 1024;
+    count_launch(), k_tree_bound_reset<<<1, t, 0, s>>>(run, scenes, nscenes, bbox_enc, box, vol, built, which, rebuild,
+                                                       L, c);
 }
 
 void loop_reset(PassCounters* c, SceneRun* run, int nscenes, LoopCtl* L, cudaStream_t s) {

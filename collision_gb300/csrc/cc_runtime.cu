@@ -352,7 +352,8 @@ struct cc_solver {
         cudaGraphExec_t exec = nullptr;
         unsigned gen = 0;
         int key_n = -1;
-        long long body_launches = 0, zone_launches = 0;
+        long long body_launches = 0, zone_launches = 0;  // per pass, and per pass with zones
+        long long full_launches = 0, dirty_launches = 0;  // of its broad phase, in one of its forms
     };
     LoopGraph loop_graphs[2];
     unsigned loop_gen = 1;   // bumped whenever a buffer or setting a graph holds changes
@@ -1597,7 +1598,7 @@ cc_status cc_solver::build_loop_graph(int n_hier) {
         return cuda_check("capture streams");
     cudaGraph_t g = nullptr;
     if (cudaGraphCreate(&g, 0) != cudaSuccess) return cuda_check("loop graph");
-    cudaGraphConditionalHandle h_loop_c, h_zone;
+    cudaGraphConditionalHandle h_loop_c, h_zone, h_form = 0;
     cudaGraphNodeParams wp = {};
     cudaGraphNode_t wnode;
     cudaError_t e = cudaGraphConditionalHandleCreate(&h_loop_c, g, 1, cudaGraphCondAssignDefault);
@@ -1610,6 +1611,16 @@ cc_status cc_solver::build_loop_graph(int n_hier) {
     }
     cudaGraph_t body = e == cudaSuccess ? wp.conditional.phGraph_out[0] : nullptr;
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h_zone, body, 0, cudaGraphCondAssignDefault);
+    BvhBufs lb = bvh;  // the step's hierarchy, over the pass's scenes' leaves
+    lb.n = n_hier;
+    lb.act = nullptr;
+    lb.sub = d_act_l;
+    lb.nsub = ne;
+    lb.dnsub = &d_loop->nbroad;
+    // pruned passes box their dirty elements only (a handle needs its node)
+    const bool dirty_only = prune && pruned_warp && lb.node && lb.leaf && n_hier > 1;
+    if (e == cudaSuccess && dirty_only)
+        e = cudaGraphConditionalHandleCreate(&h_form, body, 0, cudaGraphCondAssignDefault);
     if (e == cudaSuccess)
         e = cudaStreamBeginCaptureToGraph(cap_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) {
@@ -1621,35 +1632,88 @@ cc_status cc_solver::build_loop_graph(int n_hier) {
     int* sel = d_lsel;
     int* eoff = d_lsel + (nscenes + 1);
     int* poff = d_lsel + 2 * (nscenes + 1);
-    BvhBufs lb = bvh;  // the step's hierarchy, over the pass's scenes' leaves
-    lb.n = n_hier;
-    lb.act = nullptr;
-    lb.sub = d_act_l;
-    lb.nsub = ne;
-    lb.dnsub = &d_loop->nbroad;
     const int m0 = kStLoopPlan - 1;  // mark slot of stage st: st - m0
     mark(0, cs);
-    loop_plan(d_ctl, d_run, d_scenes, nscenes, d_loop, sel, eoff, poff, h_zone, cs);
+    loop_plan(d_ctl, d_run, d_scenes, nscenes, d_loop, sel, eoff, poff, h_zone, h_form, dirty_only ? 1 : 0, cs);
     loop_expand(sel, eoff, poff, d_scenes, d_ctl, d_loop, ne + nv, d_act_e, d_act_l, d_act_p, cs);
     mark(kStLoopPlan - m0, cs);
-    leaf_boxes(d_ev, d_act_e, ne, d_escene, d_scenes, nscenes, d_xo, d_av, 1, d_box, bvh.bbox_enc, cs,
-               &d_loop->nbroad);
-    tree_check_reset(d_run, nscenes, bvh.bbox_enc, d_tree_vol, d_tree_built + nscenes, 1, d_rebuild, d_loop, d_ctr,
-                     cs);
-    mark(kStLoopBoxes - m0, cs);
-    bvh_refit(d_box, lb, cs, false);  // the roots of the proximity pass's build stand
-    if (mode == 1)
-        point_boxes(d_xo, d_av, d_vscene, d_scenes, d_act_p, nv, 1, d_pbox_lo, d_pbox_hi, d_p32, d_v32, cs,
-                    &d_loop->npts);
-    mark(kStLoopRefit - m0, cs);
-    // the full traversal (first CCD pass) or the pruned one (later passes)
-    lb.dnq = &d_loop->nq_full;
-    bvh_pairs(d_box, lb, d_pairs, pair_cap, d_ctr, cs, d_ev, tune.traverse_block, nullptr, false, tune.rope_traverse,
-              tune.traverse_refill, tune.stack_depth);
-    mark(kStLoopTraverse - m0, cs);
-    pruned_pairs(lb, d_act_e, d_act_l, d_pstamp, d_loop, d_edirty, d_query, ne, d_pairs, pair_cap, d_ctr, d_ev, cs,
-                 pruned_warp);
-    mark(kStLoopPruned - m0, cs);
+    // the broad phase of a pass over all its elements
+    auto full_broad = [&](cudaStream_t fs) {
+        leaf_boxes(d_ev, d_act_e, ne, d_escene, d_scenes, nscenes, d_xo, d_av, 1, d_box, bvh.bbox_enc, fs,
+                   &d_loop->nbroad);
+        tree_check_reset(d_run, nscenes, bvh.bbox_enc, d_tree_vol, d_tree_built + nscenes, 1, d_rebuild, d_loop, d_ctr,
+                         fs);
+        mark(kStLoopBoxes - m0, fs);
+        bvh_refit(d_box, lb, fs, false);  // the roots of the proximity pass's build stand
+        if (mode == 1)
+            point_boxes(d_xo, d_av, d_vscene, d_scenes, d_act_p, nv, 1, d_pbox_lo, d_pbox_hi, d_p32, d_v32, fs,
+                        &d_loop->npts);
+        mark(kStLoopRefit - m0, fs);
+        // the full traversal (first CCD pass) or, without dirty_only, the pruned one (later passes)
+        lb.dnq = &d_loop->nq_full;
+        bvh_pairs(d_box, lb, d_pairs, pair_cap, d_ctr, fs, d_ev, tune.traverse_block, nullptr, false,
+                  tune.rope_traverse, tune.traverse_refill, tune.stack_depth);
+        mark(kStLoopTraverse - m0, fs);
+        if (!dirty_only)
+            pruned_pairs(lb, d_act_e, d_act_l, d_pstamp, d_loop, d_edirty, d_query, ne, d_pairs, pair_cap, d_ctr, d_ev,
+                         fs, pruned_warp);
+        mark(kStLoopPruned - m0, fs);
+    };
+    // and of a pruned pass
+    auto dirty_broad = [&](cudaStream_t fs) {
+        const PointBufs pb{d_vscene, d_pbox_lo, d_pbox_hi, d_p32, d_v32};
+        dirty_pairs_update(lb, d_act_l, d_act_p, d_pstamp, d_loop, d_edirty, d_query, ne, nv, d_ctr, d_ev, d_xo, d_av,
+                           d_box, mode == 1 ? &pb : nullptr, fs);
+        mark(kStLoopRefit - m0, fs);
+        tree_bound_reset(d_run, d_scenes, nscenes, bvh.bbox_enc, d_box, d_tree_vol, d_tree_built + nscenes, 1,
+                         d_rebuild, d_loop, d_ctr, fs);
+        mark(kStLoopBoxes - m0, fs);
+        mark(kStLoopTraverse - m0, fs);  // every pass has one
+        dirty_pairs(lb, d_loop, d_edirty, d_query, ne, d_pairs, pair_cap, d_ctr, d_ev, fs);
+        mark(kStLoopPruned - m0, fs);
+    };
+    long long full_launches = 0, dirty_launches = 0;
+    if (!dirty_only) {
+        full_broad(cs);
+    } else {
+        cudaStreamCaptureStatus st;
+        cudaGraph_t cg = nullptr;
+        const cudaGraphNode_t* deps = nullptr;
+        size_t ndeps = 0;
+        cudaGraphNodeParams sp = {};
+        cudaGraphNode_t snode;
+        e = cudaStreamGetCaptureInfo(cs, &st, nullptr, &cg, &deps, nullptr, &ndeps);
+        if (e == cudaSuccess) {
+            sp.type = cudaGraphNodeTypeConditional;
+            sp.conditional.handle = h_form;
+            sp.conditional.type = cudaGraphCondTypeSwitch;
+            sp.conditional.size = 2;
+            e = cudaGraphAddNode(&snode, cg, deps, nullptr, ndeps, &sp);
+        }
+        if (e == cudaSuccess)
+            e = cudaStreamUpdateCaptureDependencies(cs, &snode, nullptr, 1, cudaStreamSetCaptureDependencies);
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+            e = cudaStreamBeginCaptureToGraph(cap_stream2, sp.conditional.phGraph_out[k], nullptr, nullptr, 0,
+                                              cudaStreamCaptureModeThreadLocal);
+            if (e != cudaSuccess) break;
+            const long long b0 = g_kernel_launches;
+            if (k == 0)
+                full_broad(cap_stream2);
+            else
+                dirty_broad(cap_stream2);
+            (k == 0 ? full_launches : dirty_launches) = g_kernel_launches - b0;
+            g_kernel_launches = b0;
+            cudaGraph_t bg = nullptr;
+            e = cudaStreamEndCapture(cap_stream2, &bg);
+        }
+        if (e != cudaSuccess) {
+            cudaGraph_t bg = nullptr;
+            cudaStreamEndCapture(cs, &bg);
+            cudaGraphDestroy(g);
+            cudaGetLastError();
+            return fail(CC_CUDA_ERROR, std::string("loop graph: ") + cudaGetErrorString(e));
+        }
+    }
     NarrowArgs a = narrow_args(1, false);
     a.ps = loop_stamp();
     if (split_narrow) {
@@ -1704,6 +1768,8 @@ cc_status cc_solver::build_loop_graph(int n_hier) {
     cudaError_t e2 = cudaStreamEndCapture(cs, &bg);
     lg.body_launches = (l1 - l0) + (g_kernel_launches - l2);
     lg.zone_launches = l2 - l1;
+    lg.full_launches = full_launches;
+    lg.dirty_launches = dirty_launches;
     g_kernel_launches = l0;
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&lg.exec, g, 0);
@@ -1840,7 +1906,9 @@ cc_status cc_solver::device_passes(std::string& capped) {
     const long long loop_iters = (long long)a[kAccIters] - 1;
     counters[21] += loop_iters;
     if (pass_log && loop_marks && d_marks) print_pass_log();
+    const long long dirty = (long long)a[kAccDirty];
     count_launch((int)(lgraph->body_launches * (loop_iters + graph_runs) +
+                       lgraph->full_launches * (loop_iters + graph_runs - dirty) + lgraph->dirty_launches * dirty +
                        lgraph->zone_launches * (long long)a[kAccZonePasses]));
     for (int s = 0; s < nscenes; ++s) {
         SceneHost& sh = scenes[s];
@@ -2682,6 +2750,7 @@ cc_status cc_set_tuning(cc_solver* s, int knob, int value) {
             return CC_OK;
         case CC_TUNE_PRUNE:
             s->prune = value != 0;
+            s->loop_dirty = true;
             return CC_OK;
         case CC_TUNE_HOST_TREE:
             s->host_tree = value != 0;
