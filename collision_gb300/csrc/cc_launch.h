@@ -241,11 +241,8 @@ struct NarrowArgs {
     int* pairq;     // candidate pairs with a queued sub-test (capacity: the pair buffer's)
     int static_only;  // proximity pass over swept-box pairs: only those with kPairStatic
     PassStamp ps;     // stamps of the points of every sub-test that hits
-    // the split sub-tests form a root again with correctly rounded functions
-    // only where a decision can depend on it (is_coplanar's rb); 0: always
-    int robust_roots = 1;
     // 1: both sub-test lists in one launch, a warp per sub-test in small
-    // passes (k_subtests_all); 0: one launch per list, a thread per sub-test
+    // passes (k_subtests_all); 0: a thread per sub-test, blocks by list
     int sub_merge = 1;
     // movable rigid bodies: the body of each point (-1 none), each body's
     // mass, and the contribution slot of body 0 (the point count)

@@ -26,7 +26,6 @@ __global__ void __launch_bounds__(128) k_narrow(NarrowArgs a, int max_pairs) {
     c.rec = a.rec; c.rec_cap = a.rec_cap;
     c.pbox_lo = a.pbox_lo; c.pbox_hi = a.pbox_hi; c.p32 = a.p32; c.v32 = a.v32;
     c.check = a.check;
-    c.robust_roots = 0;
     int np = a.ctr->npairs;
     if (np > max_pairs) np = max_pairs;
     // counters summed per thread, added once per warp at the end
@@ -382,7 +381,6 @@ __device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, i
 template <bool MOVING>
 __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pairs) {
     NarrowCtx c;
-    c.robust_roots = 0;
     c.pbox_lo = a.pbox_lo; c.pbox_hi = a.pbox_hi; c.p32 = a.p32; c.v32 = a.v32;
     int np = a.ctr->npairs;
     if (np > max_pairs) np = max_pairs;
@@ -520,7 +518,6 @@ __device__ __forceinline__ NarrowCtx subtest_ctx(const NarrowArgs& a) {
     c.rec = nullptr; c.rec_cap = 0;
     c.pbox_lo = nullptr; c.pbox_hi = nullptr; c.p32 = nullptr; c.v32 = nullptr;
     c.check = a.check;
-    c.robust_roots = a.robust_roots;
     c.zone = 0;
     return c;
 }
@@ -566,28 +563,27 @@ __device__ __forceinline__ void subtest_counts(const NarrowArgs& a, SubTally t) 
     }
 }
 
-// Passes with more sub-tests than this run them as two launches, one per
-// kind (k_subtests): measured faster than one launch for both kinds when the
-// pass is large, where the FP64 pipes are full either way (each kind's
-// kernel keeps a smaller body).
+// Passes with more sub-tests than this give each kind blocks of its own
+// (k_subtests): measured faster than both kinds in a warp when the pass is
+// large, where the FP64 pipes are full either way.
 constexpr int kSubMergeMax = 65536;
 
-// One list (point-triangle or edge-edge), one sub-test per thread. merged:
-// k_subtests_all takes the passes of at most kSubMergeMax sub-tests.
-template <bool MOVING, bool EE>
+// One list per block (point-triangle in the even ones, edge-edge in the odd
+// ones), one sub-test per thread. merged: k_subtests_all takes the passes of
+// at most kSubMergeMax sub-tests.
+template <bool MOVING>
 __global__ void __launch_bounds__(128, 4) k_subtests(NarrowArgs a, int merged) {
-    const SubRec* list = EE ? a.sub_ee : a.sub_pt;
-    int n = EE ? a.ctr->nsub_ee : a.ctr->nsub_pt;
-    if (n > a.sub_cap) n = a.sub_cap;
-    if (merged) {
-        const int npt = a.ctr->nsub_pt < a.sub_cap ? a.ctr->nsub_pt : a.sub_cap;
-        const int nee = a.ctr->nsub_ee < a.sub_cap ? a.ctr->nsub_ee : a.sub_cap;
-        if (npt + nee <= kSubMergeMax) return;
-    }
+    const int npt = a.ctr->nsub_pt < a.sub_cap ? a.ctr->nsub_pt : a.sub_cap;
+    const int nee = a.ctr->nsub_ee < a.sub_cap ? a.ctr->nsub_ee : a.sub_cap;
+    if (merged && npt + nee <= kSubMergeMax) return;
     NarrowCtx c = subtest_ctx(a);
     SubTally t;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        one_subtest<MOVING, EE>(a, c, list[i], t);
+    const int first = (blockIdx.x >> 1) * blockDim.x + threadIdx.x, stride = (gridDim.x >> 1) * blockDim.x;
+    if (blockIdx.x & 1) {
+        for (int i = first; i < nee; i += stride) one_subtest<MOVING, true>(a, c, a.sub_ee[i], t);
+    } else {
+        for (int i = first; i < npt; i += stride) one_subtest<MOVING, false>(a, c, a.sub_pt[i], t);
+    }
     subtest_counts(a, t);
 }
 
@@ -697,16 +693,14 @@ void narrow_pass_split(const NarrowArgs& args, int moving, int max_pairs, cudaSt
         }
         if (parts & kSplitSubtests) {
             if (a.sub_merge) count_launch(), k_subtests_all<true><<<mblocks, 128, 0, s>>>(a);
-            count_launch(), k_subtests<true, false><<<sblocks, 128, 0, s>>>(a, a.sub_merge);
-            count_launch(), k_subtests<true, true><<<sblocks, 128, 0, s>>>(a, a.sub_merge);
+            count_launch(), k_subtests<true><<<2 * sblocks, 128, 0, s>>>(a, a.sub_merge);
             if (zone) count_launch(), k_zone_unions<<<blocks, 128, 0, s>>>(a);
         }
     } else {
         if (parts & kSplitFilter) count_launch(), k_narrow_filter<false><<<blocks, block, 0, s>>>(a, max_pairs);
         if (parts & kSplitSubtests) {
             if (a.sub_merge) count_launch(), k_subtests_all<false><<<mblocks, 128, 0, s>>>(a);
-            count_launch(), k_subtests<false, false><<<sblocks, 128, 0, s>>>(a, a.sub_merge);
-            count_launch(), k_subtests<false, true><<<sblocks, 128, 0, s>>>(a, a.sub_merge);
+            count_launch(), k_subtests<false><<<2 * sblocks, 128, 0, s>>>(a, a.sub_merge);
         }
     }
 }

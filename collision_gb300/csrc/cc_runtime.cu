@@ -329,7 +329,7 @@ struct cc_solver {
     bool host_tree = false;          // CC_TUNE_HOST_TREE: emulate the insertions on host threads instead
     bool pruned_warp = true;         // CC_TUNE_PRUNED_WARP: one warp per pruned query
     bool refit_up = true;            // CC_TUNE_REFIT_UP: the refit walk with one arrival per level
-    bool robust_roots = true;        // CC_TUNE_ROBUST_ROOTS: correctly rounded roots only where decisive
+    bool robust_roots = true;        // CC_TUNE_ROBUST_ROOTS (without effect)
     bool sub_merge = true;           // CC_TUNE_SUBTEST_MERGE: both sub-test lists in one launch
     void* d_tree_scratch = nullptr;  // nodes, parent links and leaf counts of the trees being built
     // Collision trees built ahead, beside the proximity trees of a step's
@@ -377,7 +377,6 @@ struct cc_solver {
     bool use_device_loop() const { return device_loop && !record && vtk_dir.empty() && !overlap_tails; }
     NarrowArgs narrow_args(int moving, bool combined) const {
         NarrowArgs a{};
-        a.robust_roots = robust_roots ? 1 : 0;
         a.sub_merge = sub_merge ? 1 : 0;
         a.xo = d_xo; a.av = d_av; a.fixed = d_fixed; a.ev = d_ev; a.esurf = d_esurf; a.erigid = d_erigid;
         a.vbody = d_vbody; a.body_mass = d_body_mass; a.body_slot0 = nv;
@@ -1998,7 +1997,6 @@ cc_status cc_solver::detect_pass(int moving, bool any_zone) {
             }
         }
         NarrowArgs a;
-        a.robust_roots = robust_roots ? 1 : 0;
         a.sub_merge = sub_merge ? 1 : 0;
         a.xo = d_xo; a.av = d_av; a.fixed = d_fixed; a.ev = d_ev; a.esurf = d_esurf; a.erigid = d_erigid;
         a.vbody = d_vbody; a.body_mass = d_body_mass; a.body_slot0 = nv;
@@ -2349,7 +2347,6 @@ cc_status cc_solver::check_ccd(const double* x_old, const double* x_new, long lo
         bvh_pairs(d_box, bvh, d_pairs, pair_cap, d_ctr, stream, d_ev, tune.traverse_block, nullptr,
                   tune.packet_traverse, tune.rope_traverse, tune.traverse_refill, kTraversalStack);
         NarrowArgs a{};
-        a.robust_roots = robust_roots ? 1 : 0;
         a.sub_merge = sub_merge ? 1 : 0;
         a.xo = d_xo; a.av = d_av; a.fixed = d_fixed; a.ev = d_ev; a.esurf = d_esurf; a.erigid = d_erigid;
         a.vbody = d_vbody; a.body_mass = d_body_mass; a.body_slot0 = nv;
@@ -2429,7 +2426,6 @@ cc_status cc_solver::autotune(double* best_ms) {
             bvh_pairs(d_box, bvh, d_pairs, pair_cap, d_ctr, stream, d_ev, t.traverse_block, nullptr,
                       t.packet_traverse, t.rope_traverse, t.traverse_refill, t.stack_depth);
             NarrowArgs a{};
-            a.robust_roots = robust_roots ? 1 : 0;
             a.sub_merge = sub_merge ? 1 : 0;
             a.xo = d_xo; a.av = d_av; a.fixed = d_fixed; a.ev = d_ev; a.esurf = d_esurf; a.erigid = d_erigid;
         a.vbody = d_vbody; a.body_mass = d_body_mass; a.body_slot0 = nv;

@@ -281,13 +281,8 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           each query walks its scene with one warp (a
  *                           shared-memory stack, up to 32 nodes per round);
  *                           0: one thread along the ropes. Same results
- *   CC_TUNE_ROBUST_ROOTS    1 (default): the FP64 sub-tests after a filter
- *                           form a coplanarity root again with correctly
- *                           rounded functions only where a decision can
- *                           depend on it (not for roots well inside the time
- *                           window at which the test misses with a margin
- *                           covering the root's error); 0: every root near
- *                           the window. Same results
+ *   CC_TUNE_ROBUST_ROOTS    accepted, without effect: every coplanarity root
+ *                           is formed with correctly rounded functions
  *   CC_TUNE_ZONE_CTA_MIN    members from which an impact zone's rigid
  *                           motion is computed by a CTA of its own (>= 16,
  *                           default 64; smaller zones of 16+ members get a
@@ -310,8 +305,8 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           and edge-edge FP64 sub-tests of a pass with at
  *                           most 65,536 of them in one launch, a warp per
  *                           sub-test where there are at most 1,216 (larger
- *                           passes: one launch per kind); 0: one launch per
- *                           kind, a thread per sub-test. Same results
+ *                           passes: blocks of one kind each); 0: always such
+ *                           blocks, a thread per sub-test. Same results
  * cc_get_tuning returns the current value, or -1 for an unknown knob. */
 enum {
     CC_TUNE_SPLIT_NARROW = 0,
