@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include <cmath>
+#include <cstring>
 
 #ifdef __CUDACC__
 #include <cooperative_groups.h>
@@ -126,6 +127,7 @@ struct Params {
 struct SceneDev {
     Params p;
     double lo[3], hi[3];  // domain box
+    double inv_dt;        // 1 / p.dt
     int v0, nv, e0, ne;   // point and element ranges
     int strain_hdr0;      // first level of its strain schedule (index into the level headers)
     int strain_levels;
@@ -250,7 +252,60 @@ __device__ __forceinline__ float cut32(double x) {
     if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);
     return (float)x;
 }
+// The same rounded down and up.
+__device__ __forceinline__ float cut32_step(double x, bool away_if_negative) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned m = (hi & 0x7fffffffu) - 0x38000000u;
+    if (m - 0x00100000u < 0x0fe00000u) {
+        const bool away = (lo & 0x1fffffffu) != 0u && ((hi >> 31) != 0u) == away_if_negative;
+        return __uint_as_float(((hi & 0x80000000u) | __funnelshift_l(lo, m, 3)) + (away ? 1u : 0u));
+    }
+    if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);
+    return away_if_negative ? __double2float_rd(x) : __double2float_ru(x);
+}
+__device__ __forceinline__ float cut32_down(double x) { return cut32_step(x, true); }
+__device__ __forceinline__ float cut32_up(double x) { return cut32_step(x, false); }
+
+// Doubles as signed integers of the same order (-0 below +0), and back: an
+// FP64 compare takes a warp ~64 cycles, a 64-bit integer one a few.
+__device__ __forceinline__ long long order_of(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double of_order(long long o) {
+    return __longlong_as_double(o ^ ((o >> 63) & 0x7fffffffffffffffll));
+}
 #endif
+
+#ifdef __CUDACC__
+#define CC_HD __host__ __device__ __forceinline__
+#else
+#define CC_HD inline
+#endif
+// a / b for inv = 1 / b rounded: two corrections of a * inv by its exact
+// remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990: the first gives a quotient within an ulp,
+// the second the correctly rounded one), 5 FP64 instructions. Outside the
+// range where the remainders are exact, the division itself.
+CC_HD double quotient(double a, double b, double inv) {
+#ifdef __CUDA_ARCH__
+    const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu, hb = (unsigned)__double2hiint(b) & 0x7fffffffu;
+    const bool zero = (ha | (unsigned)__double2loint(a)) == 0u;
+#else
+    unsigned long long ua, ub;
+    std::memcpy(&ua, &a, 8);
+    std::memcpy(&ub, &b, 8);
+    const unsigned ha = (unsigned)(ua >> 32) & 0x7fffffffu, hb = (unsigned)(ub >> 32) & 0x7fffffffu;
+    const bool zero = (ua << 1) == 0;
+#endif
+    // 2^-400 <= |a|, |b| < 2^400
+    const bool in = ha - 0x26f00000u < 0x32000000u || zero;
+    if (!in || hb - 0x26f00000u >= 0x32000000u) return a / b;
+    double q = a * inv;
+    if (zero) return q;
+    q = fma(fma(-b, q, a), inv, q);
+    return fma(fma(-b, q, a), inv, q);
+}
 
 __device__ __forceinline__ double dot3(const double* a, const double* b) {
     return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];

@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(128) k_narrow(NarrowArgs a, int max_pairs) {
         c.pass = run.pass;
         // h of the sub-tests (thickness for proximity, eps for CCD) and the
         // barycentric tolerance eps, rounded up to FP32
-        c.hpad = __double2float_ru(MOVING ? c.p.eps : c.p.thickness);
-        c.epad = __double2float_ru(c.p.eps);
-        c.dt32 = __double2float_ru(c.p.dt);
+        c.hpad = cut32_up(MOVING ? c.p.eps : c.p.thickness);
+        c.epad = cut32_up(c.p.eps);
+        c.dt32 = cut32_up(c.p.dt);
         int ri = c.rank ? c.rank[pr.x] : pr.x, rj = c.rank ? c.rank[pr.y] : pr.y;
         int ea = ri > rj ? pr.x : pr.y;  // found leaf
         int eb = ri > rj ? pr.y : pr.x;  // query leaf
@@ -356,9 +356,9 @@ __device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, i
             }
         }
         const double eps = a.scenes[sc].p.eps;
-        c.hpad = __double2float_ru(MOVING ? eps : a.scenes[sc].p.thickness);
-        c.epad = __double2float_ru(eps);
-        c.dt32 = __double2float_ru(a.scenes[sc].p.dt);
+        c.hpad = cut32_up(MOVING ? eps : a.scenes[sc].p.thickness);
+        c.epad = cut32_up(eps);
+        c.dt32 = cut32_up(a.scenes[sc].p.dt);
         if (__any_sync(0xffffffffu, on)) on = pair_may_hit16<MOVING>(c, o, sub) && on;
         if (on && pair_subtest<MOVING>(o, sub, pts, ee)) {
             float ext, extb;
@@ -396,9 +396,9 @@ __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pai
         t_visits++;
         int sc = a.escene[pr.x];
         const double eps = a.scenes[sc].p.eps;
-        c.hpad = __double2float_ru(MOVING ? eps : a.scenes[sc].p.thickness);
-        c.epad = __double2float_ru(eps);
-        c.dt32 = __double2float_ru(a.scenes[sc].p.dt);
+        c.hpad = cut32_up(MOVING ? eps : a.scenes[sc].p.thickness);
+        c.epad = cut32_up(eps);
+        c.dt32 = cut32_up(a.scenes[sc].p.dt);
         // a shared point makes every test of the pair return false
         bool shared = false;
         for (int i = 0; i < o.n1; ++i)

@@ -183,21 +183,26 @@ static __device__ void point_to_tri_impulse(const NarrowCtx& c, CallState& st, c
         return;
     }
     int has_fric = fabs(vt) > kRoundEps;
-    double imp[3], fric[3];
+    const double inv_vt = 1.0 / vt;
+    double imp[3], fric[3], slide[3];
+    for (int j = 0; j < 3; ++j) slide[j] = v_rel[j] - vn * nor[j];
     for (int i = 0; i < 3; ++i) {
         if (tri_static[i]) continue;
         double t_impulse = mv[i] ? rigid_impulse[0] : m_impulse;
+        const double share = w[i] * t_impulse;
+        const double f = has_fric ? smax(-fabs(quotient(lambda * w[i] * t_impulse, vt, inv_vt)), -1.0) : 0.0;
         for (int j = 0; j < 3; ++j) {
-            imp[j] = w[i] * t_impulse * nor[j];
-            fric[j] = has_fric ? smax(-fabs(lambda * w[i] * t_impulse / vt), -1.0) * (v_rel[j] - vn * nor[j]) : 0.0;
+            imp[j] = share * nor[j];
+            fric[j] = has_fric ? f * slide[j] : 0.0;
         }
         emit(c, st, pts[i], imp, fric, has_fric);
     }
     if (!st3) {
         double t_impulse = mv[3] ? rigid_impulse[1] : m_impulse;
+        const double f = has_fric ? smax(-fabs(quotient(lambda * t_impulse, vt, inv_vt)), -1.0) : 0.0;
         for (int j = 0; j < 3; ++j) {
             imp[j] = -(t_impulse * nor[j]);
-            fric[j] = has_fric ? smax(-fabs(lambda * t_impulse / vt), -1.0) * (v_rel[j] - vn * nor[j]) : 0.0;
+            fric[j] = has_fric ? f * slide[j] : 0.0;
         }
         emit(c, st, pts[3], imp, fric, has_fric);
     }
@@ -271,20 +276,30 @@ static __device__ void edge_to_edge_impulse(const NarrowCtx& c, CallState& st, c
     }
     int has_fric = fabs(vt) > kRoundEps;
     const double wgt[4] = {wa[0], wa[1], wb[0], wb[1]};
-    double imp[3], fric[3];
+    const double inv_vt = 1.0 / vt;
+    double imp[3], fric[3], slide[3];
+    for (int j = 0; j < 3; ++j) slide[j] = v_rel[j] - vn * nor[j];
     for (int q = 0; q < 4; ++q) {
         if (sq[q]) continue;
         double t_impulse = mv[q] ? rigid_impulse[q < 2 ? 0 : 1] : m_impulse;
+        const double share = wgt[q] * t_impulse;
+        const double f = has_fric ? smax(-fabs(quotient(lambda * wgt[q] * t_impulse, vt, inv_vt)), -1.0) : 0.0;
         for (int j = 0; j < 3; ++j) {
-            double d = wgt[q] * t_impulse * nor[j];
+            double d = share * nor[j];
             imp[j] = (q < 2) ? d : -d;
-            fric[j] = has_fric ? smax(-fabs(lambda * wgt[q] * t_impulse / vt), -1.0) * (v_rel[j] - vn * nor[j]) : 0.0;
+            fric[j] = has_fric ? f * slide[j] : 0.0;
         }
         emit(c, st, pts[q], imp, fric, has_fric);
     }
 }
 
 // ------------------------------------------------------- point / edge tests
+// v / d, each component as rounded by the division.
+__device__ __forceinline__ void divide3(double* v, double d) {
+    const double inv = 1.0 / d;
+    for (int i = 0; i < 3; ++i) v[i] = quotient(v[i], d, inv);
+}
+
 // PointToTri, dcollid3d.cpp:778-922. pts[0..2] the triangle, pts[3] the
 // point; X holds the four positions the reference keeps in Coords.
 static __device__ bool point_to_tri(const NarrowCtx& c, CallState& st, const int* pts, const double (*X)[3], double h) {
@@ -305,10 +320,11 @@ static __device__ bool point_to_tri(const NarrowCtx& c, CallState& st, const int
     double x43_old[3];
     for (int i = 0; i < 3; ++i) x43_old[i] = xo[3][i] - xo[2][i];
     dist = dot3(x43_old, nor);
-    for (int i = 0; i < 3; ++i) nor[i] /= nor_mag * ((dist >= 0) ? 1.0 : -1.0);
+    divide3(nor, nor_mag * ((dist >= 0) ? 1.0 : -1.0));
     dist = fabs(dot3(x43, nor));
-    w[0] = (dot3(x13, x43) * dot3(x23, x23) - dot3(x23, x43) * dot3(x13, x23)) / det;
-    w[1] = (dot3(x13, x13) * dot3(x23, x43) - dot3(x13, x23) * dot3(x13, x43)) / det;
+    const double inv_det = 1.0 / det;
+    w[0] = quotient(dot3(x13, x43) * dot3(x23, x23) - dot3(x23, x43) * dot3(x13, x23), det, inv_det);
+    w[1] = quotient(dot3(x13, x13) * dot3(x23, x43) - dot3(x13, x23) * dot3(x13, x43), det, inv_det);
     w[2] = 1 - w[0] - w[1];
     if (fabs(w[0]) < kRoundEps || fabs(w[1]) < kRoundEps || fabs(w[2]) < kRoundEps) {
         double vec[3];
@@ -321,7 +337,7 @@ static __device__ bool point_to_tri(const NarrowCtx& c, CallState& st, const int
     }
     nor_mag = mag3(nor);
     if (nor_mag > kRoundEps) {
-        for (int i = 0; i < 3; ++i) nor[i] /= nor_mag;
+        divide3(nor, nor_mag);
     } else {
         atomicOr(&c.ctr->err, kErrNan);  // "nan nor vec": the reference exits
         return false;
@@ -348,8 +364,9 @@ static __device__ bool edge_to_edge(const NarrowCtx& c, CallState& st, const int
     if (mag3(tmp) < kRoundEps) return false;
     double d4343 = dot3(x43, x43), d2131 = dot3(x21, x31), d2143 = dot3(x21, x43), d4331 = dot3(x43, x31),
            d2121 = dot3(x21, x21);
-    a = (d4343 * d2131 - d2143 * d4331) / (d2121 * d4343 - d2143 * d2143);
-    b = (d2143 * d2131 - d2121 * d4331) / (d2121 * d4343 - d2143 * d2143);
+    const double den = d2121 * d4343 - d2143 * d2143, inv_den = 1.0 / den;
+    a = quotient(d4343 * d2131 - d2143 * d4331, den, inv_den);
+    b = quotient(d2143 * d2131 - d2121 * d4331, den, inv_den);
     a = smax(smin(a, 1.0), 0.0);
     b = smax(smin(b, 1.0), 0.0);
     for (int i = 0; i < 3; ++i) {
@@ -362,6 +379,8 @@ static __device__ bool edge_to_edge(const NarrowCtx& c, CallState& st, const int
     }
     for (int i = 0; i < 3; ++i) nor[i] = v2[i] - v1[i];
     nor_mag = mag3(nor);
+    // the distance: the same squares in the same order
+    dist = nor_mag;
     if (nor_mag < 1000 * kMachEps) {
         double xo[4][3];
         for (int q = 0; q < 4; ++q) load3(c.xo, pts[q], xo[q]);
@@ -369,17 +388,14 @@ static __device__ bool edge_to_edge(const NarrowCtx& c, CallState& st, const int
             nor[j] = (1.0 - b) * xo[2][j] + b * xo[3][j];
             nor[j] -= (1.0 - a) * xo[0][j] + a * xo[1][j];
         }
+        nor_mag = mag3(nor);
     }
-    double s = 0.0;
-    for (int i = 0; i < 3; ++i) s += sqr(v1[i] - v2[i]);
-    dist = sqrt(s);
     if (dist > h) return false;
-    nor_mag = mag3(nor);
     if (nor_mag < kMachEps) {
         atomicOr(&c.ctr->err, kErrNan);  // "Normal vector is nan": the reference exits
         return false;
     }
-    for (int i = 0; i < 3; ++i) nor[i] /= nor_mag;
+    divide3(nor, nor_mag);
     if (c.check) return true;
     st.ncontacts++;
     edge_to_edge_impulse(c, st, pts, nor, a, b, dist);
@@ -510,7 +526,8 @@ static __device__ bool is_coplanar(const Cubic& q, double dt, double* roots, int
         return window_roots(roots, dt);
     }
     if (no_root_in_window(q, dt)) return false;
-    const double a = q.b / q.a, b = q.c / q.a, c = q.d / q.a;
+    const double inv_a = 1.0 / q.a;
+    const double a = quotient(q.b, q.a, inv_a), b = quotient(q.c, q.a, inv_a), c = quotient(q.d, q.a, inv_a);
     double Q = (a * a - 3 * b) / 9;
     double R = (2 * a * a * a - 9 * a * b + 27 * c) / 54;
     double Q3 = Q * Q * Q;

@@ -959,6 +959,7 @@ struct cc_solver {
     }
     void set_scene_params(int i, const cc_params& p) {
         h_scenes[i].p = Params{p.dt, p.thickness, p.eps, p.k, p.m, p.lambda, p.cr};
+        h_scenes[i].inv_dt = 1.0 / p.dt;
         scenes_dirty = true;
     }
     void set_scene_domain(int i, const double* l, const double* h) {

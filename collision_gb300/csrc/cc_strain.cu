@@ -267,13 +267,13 @@ __device__ __forceinline__ float4 cut32x3(double x, double y, double z) {
 
 // The strain decision of one edge in FP32: 1 over the limit, 0 within it, -1
 // too close to tell. With u = 2^-24 and b the sum over the components of
-// |dx| + dt (|v0| + |v1|), the inputs' roundings (velocities 2u, dx u, dt
+// |dx| + dt (|v0| + |v1|), the inputs' roundings (velocities and dx 2u, dt
 // 2u) and the operations' put each component of dx + dt (v0 - v1) within
-// 7 u b_k and s within 19 u b^2 of its exact value; the margin is 40 u b^2,
-// whose remaining 20 u b^2 > 16 u s covers the rounding of the margin and
-// the bounds' own: u for the FP32 rounding, and the 1e-9 beyond the exact
-// threshold that a decision has to keep (the exact test rounds by less than
-// 1e-15).
+// 8 u b_k and s within 21 u b^2 of its exact value; the margin is 40 u b^2,
+// whose remaining 19 u b^2 > 15 u s covers the rounding of the margin and of
+// its sum with s (2 u), and the bounds' own: 10 u (lengths cut 2u, squared,
+// summed and scaled), and the 1e-9 beyond the exact threshold that a decision
+// has to keep (the exact test rounds by less than 1e-15).
 constexpr float kSweepMargin = 40.0f * 5.9604645e-8f;
 __device__ __forceinline__ int sweep_decide(float s, float b, float2 limit) {
     const float err = b * b * kSweepMargin;
@@ -307,7 +307,8 @@ __device__ __noinline__ bool sweep_exact(int p0, int p1, double len0, const doub
     return strain_flag_vals(strain_step(p0, p1, len0, xo), v0, v1, dt, &n);
 }
 
-// Per step: every element's record.
+// Per step: every element's record. Only the differences are formed in FP64:
+// 1,420,000 elements 162 -> 41 us.
 __global__ void k_sweep_setup(const SweepElem* __restrict__ elems, int m, const double4_32a* __restrict__ xo,
                               SweepRec* __restrict__ out) {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -320,21 +321,14 @@ __global__ void k_sweep_setup(const SweepElem* __restrict__ elems, int m, const 
     r.s2n = el.s2n;
     for (int j = 0; j < 3; ++j) {
         const double *a = x[j], *b = x[(j + 1) % 3];
-        double so = 0.0;
-        float sum = 0.f;
-        for (int k = 0; k < 3; ++k) {
-            so += sqr(a[k] - b[k]);
-            const float d = (float)(a[k] - b[k]);
-            (k == 0 ? r.dx[j].x : k == 1 ? r.dx[j].y : r.dx[j].z) = d;
-            sum += fabsf(d);
-        }
-        r.dx[j].w = sum;
+        const float dx = cut32(a[0] - b[0]), dy = cut32(a[1] - b[1]), dz = cut32(a[2] - b[2]);
+        r.dx[j] = make_float4(dx, dy, dz, fabsf(dx) + fabsf(dy) + fabsf(dz));
         // over the limit above 1.1 times the shorter, below 0.9 times the
         // longer of the rest and the start-of-step length
-        const double L = el.len0[j], l2 = L * L;
-        const bool degenerate = !(so > 1e-12 && L > 1e-6);
-        r.limit[j].x = degenerate ? __int_as_float(0x7fffffff) : (float)(1.21 * fmin(l2, so));
-        r.limit[j].y = degenerate ? __int_as_float(0x7fffffff) : (float)(0.81 * fmax(l2, so));
+        const float so = dx * dx + dy * dy + dz * dz, L = cut32(el.len0[j]), l2 = L * L;
+        const bool degenerate = !(so > 1e-12f && L > 1e-6f);
+        r.limit[j].x = degenerate ? __int_as_float(0x7fffffff) : 1.21f * fminf(l2, so);
+        r.limit[j].y = degenerate ? __int_as_float(0x7fffffff) : 0.81f * fmaxf(l2, so);
     }
     out[e] = r;
 }
