@@ -251,10 +251,9 @@ struct NarrowArgs {
     int body_slot0;
 };
 void narrow_pass(const NarrowArgs& a, int moving, int max_pairs, cudaStream_t s, int block = 128);
-// The same pass in stages (no recording): the filters - FP32 ones per pair
-// with the point data of mode 1, else, for moving passes, each sub-test's
-// coplanarity cubic in FP64 - then the FP64 sub-tests that pass them, one thread
-// each, then - for scenes in impact-zone mode - the createImpZone calls of
+// The same pass in stages (no recording): the filters - per pair and per
+// sub-test with the point data of mode 1, else per sub-test on points cut to
+// FP32 (k_plain_filter) - then the FP64 sub-tests that pass them, then - for scenes in impact-zone mode - the createImpZone calls of
 // every pair that hit. parts selects the filters (kSplitFilter), the rest
 // (kSplitSubtests) or both, so that the two can be timed apart.
 enum { kSplitFilter = 1, kSplitSubtests = 2, kSplitAll = 3 };

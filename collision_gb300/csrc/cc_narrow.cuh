@@ -800,26 +800,26 @@ __device__ __forceinline__ bool mixed_may_hit(const NarrowCtx& c, const int* pts
 // points within h are points of the segments, so the segments are within
 // h + 2^-20*ext. Sub-tests whose bound exceeds the reach return false in
 // FP64 too and are skipped.
+// On given points (rounded to FP32, or cut to it by cut32, which is within
+// the same bound) and velocities; ext, extb: the extents of the elements'
+// boxes over the window.
 template <bool MOVING, bool EE>
-__device__ __forceinline__ bool sat_may_hit(const NarrowCtx& c, const int* pts, float ext, float extb) {
-    F3 X[4];
-    for (int q = 0; q < 4; ++q) X[q] = f3(c.p32[pts[q]]);
+__device__ __forceinline__ bool gap_may_hit(const F3* X, const F3* V, float ext, float extb, float hpad, float epad,
+                                            float dt32) {
     float M = fmaxf(fmaxf(fmaxabs(X[0]), fmaxabs(X[1])), fmaxf(fmaxabs(X[2]), fmaxabs(X[3])));
     float lb, L, reach;
     if (!EE) {
         // triangle X0 X1 X2, point X3; origin X0
         lb = triangle_gap(fsub(X[3], X[0]), fsub(X[1], X[0]), fsub(X[2], X[0]), &L);
-        reach = __fadd_ru(c.hpad, __fmul_ru(ext, __fmul_ru(8.0f, __fadd_ru(c.epad, 0x1p-10f))));
+        reach = __fadd_ru(hpad, __fmul_ru(ext, __fmul_ru(8.0f, __fadd_ru(epad, 0x1p-10f))));
     } else {
         // segments S1 = X0 X1, S2 = X2 X3; origin X2
         lb = segment_gap(fsub(X[1], X[0]), fsub(X[3], X[2]), fsub(X[0], X[2]), &L);
-        reach = __fadd_ru(c.hpad, __fmul_ru(__fadd_ru(ext, extb), 0x1p-20f));
+        reach = __fadd_ru(hpad, __fmul_ru(__fadd_ru(ext, extb), 0x1p-20f));
     }
     float err = __fmul_ru(32.0f * 0x1p-24f, __fadd_ru(L, M));
     float bound = __fsub_rd(lb, err);
     if (MOVING) {
-        F3 V[4];
-        for (int q = 0; q < 4; ++q) V[q] = f3(c.v32[pts[q]]);
         // reference velocity: the first point's
         float D1, D2;
         if (!EE) {
@@ -832,9 +832,18 @@ __device__ __forceinline__ bool sat_may_hit(const NarrowCtx& c, const int* pts, 
         float Vm = fmaxf(fmaxf(fmaxabs(V[0]), fmaxabs(V[1])), fmaxf(fmaxabs(V[2]), fmaxabs(V[3])));
         // FP32 rounding of the velocities and of the sums above
         float dv = __fadd_ru(__fmul_ru(__fadd_ru(D1, D2), 1.0f + 0x1p-16f), __fmul_ru(Vm, 32.0f * 0x1p-24f));
-        bound = __fsub_rd(bound, __fmul_ru(c.dt32, dv));
+        bound = __fsub_rd(bound, __fmul_ru(dt32, dv));
     }
     return !(bound > reach);
+}
+
+template <bool MOVING, bool EE>
+__device__ __forceinline__ bool sat_may_hit(const NarrowCtx& c, const int* pts, float ext, float extb) {
+    F3 X[4], V[4];
+    for (int q = 0; q < 4; ++q) X[q] = f3(c.p32[pts[q]]);
+    if (MOVING)
+        for (int q = 0; q < 4; ++q) V[q] = f3(c.v32[pts[q]]);
+    return gap_may_hit<MOVING, EE>(X, V, ext, extb, c.hpad, c.epad, c.dt32);
 }
 
 __device__ __forceinline__ F3 fcross(F3 a, F3 b) {

@@ -1565,7 +1565,7 @@ void cc_solver::prox_pass_async() {
     prof(kStNarrowProx, true);
     NarrowArgs a = narrow_args(0, combined);
     a.ps = loop_stamp();
-    if (mode == 1 && split_narrow)
+    if (split_narrow)
         narrow_pass_split(a, 0, pair_cap, stream, tune.narrow_block, false);
     else
         narrow_pass(a, 0, pair_cap, stream, tune.narrow_block);
