@@ -185,6 +185,7 @@ struct PassCounters {
     int npairq;       // pairs with a queued sub-test (split passes)
     int nzones;       // impact zones listed for the zone solve (impact-zone passes)
     int nmembers;     // their members
+    int nlive_pt, nlive_ee;  // sub-tests listed by k_subtests_cubic
     int nseg;         // union-record segments, one per zone the pass's unions touch
     int ntouch;       // points and bodies with contributions
     int nseg_used;    // contributions given to their segments so far

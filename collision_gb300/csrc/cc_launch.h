@@ -237,6 +237,8 @@ struct NarrowArgs {
     SubRec* sub_pt;
     SubRec* sub_ee;
     int sub_cap;
+    int* live_pt;   // the sub-tests whose cubic may have a root (sub_cap each)
+    int* live_ee;
     int* pair_hit;  // per candidate pair: bit s set when sub-test s hit
     int* pairq;     // candidate pairs with a queued sub-test (capacity: the pair buffer's)
     int static_only;  // proximity pass over swept-box pairs: only those with kPairStatic
@@ -253,8 +255,9 @@ struct NarrowArgs {
 void narrow_pass(const NarrowArgs& a, int moving, int max_pairs, cudaStream_t s, int block = 128);
 // The same pass in stages (no recording): the filters - per pair and per
 // sub-test with the point data of mode 1, else per sub-test on points cut to
-// FP32 (k_plain_filter) - then the FP64 sub-tests that pass them, then - for scenes in impact-zone mode - the createImpZone calls of
-// every pair that hit. parts selects the filters (kSplitFilter), the rest
+// FP32 (k_plain_filter) - then the FP64 sub-tests that pass them, then - for
+// scenes in impact-zone mode - the createImpZone calls of every pair that
+// hit. parts selects the filters (kSplitFilter), the rest
 // (kSplitSubtests) or both, so that the two can be timed apart.
 enum { kSplitFilter = 1, kSplitSubtests = 2, kSplitAll = 3 };
 void narrow_pass_split(const NarrowArgs& a, int moving, int max_pairs, cudaStream_t s, int block = 128,

@@ -250,7 +250,7 @@ __device__ __forceinline__ void loop_reset_counters(PassCounters* c, LoopCtl* L,
     c->npairs = (!stop && L->reuse_n >= 0) ? L->reuse_n : 0;
     c->ncontrib = 0; c->nhit_pairs = 0; c->nrec = 0; c->nvisits = 0; c->ncontacts = 0; c->nsub = 0;
     c->ncr = 0; c->nunion = 0; c->nsub_pt = 0; c->nsub_ee = 0; c->npairq = 0; c->nzones = 0; c->nmembers = 0;
-    c->nseg = 0; c->ntouch = 0; c->nseg_used = 0;
+    c->nseg = 0; c->ntouch = 0; c->nseg_used = 0; c->nlive_pt = 0; c->nlive_ee = 0;
     c->err = keep | (stop ? kErrHost : 0);
     if (stop) {
         L->nbroad = 0;

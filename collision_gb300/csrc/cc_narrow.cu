@@ -322,12 +322,10 @@ __device__ __forceinline__ bool pair_may_hit16(const NarrowCtx& c, const Oriente
 }
 
 // Stage 1 with sixteen threads per pair, one per axis of the pair's bound and
-// then one per sub-test; on moving passes a sub-test that passes the FP32
-// filters is done here too when its cubic can have no root in the time window
-// (may_be_coplanar). A thread's 12 axes and 15 sub-tests in turn (below) are
-// ~36 us however few pairs a pass has.
+// then one per sub-test. A thread's 12 axes and 15 sub-tests in turn (below)
+// are ~36 us however few pairs a pass has.
 template <bool MOVING>
-__device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, int np, int& t_visits, int& t_sub) {
+__device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, int np, int& t_visits) {
     const int sub = threadIdx.x & 15, group = (threadIdx.x & 31) & ~15;
     const int groups = (int)((gridDim.x * blockDim.x) >> 4);
     const int g0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 4);
@@ -364,17 +362,8 @@ __device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, i
             float ext, extb;
             queue = mixed_may_hit(c, pts, ee, &ext, &extb) &&
                     (ee ? sat_may_hit<MOVING, true>(c, pts, ext, extb) : sat_may_hit<MOVING, false>(c, pts, ext, extb));
-            if (MOVING && queue) {
-                double xo4[4][3], av4[4][3];
-                for (int q = 0; q < 4; ++q) {
-                    load3(a.xo, pts[q], xo4[q]);
-                    load3(a.av, pts[q], av4[q]);
-                }
-                ++t_sub;
-                queue = may_be_coplanar(xo4, av4, a.scenes[sc].p.dt);
-            }
         }
-        queue_group(a, queue, ee, o.keybase, idx, sc, pts, sub, group, MOVING);
+        queue_group(a, queue, ee, o.keybase, idx, sc, pts, sub, group, false);
     }
 }
 
@@ -384,8 +373,8 @@ __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pai
     c.pbox_lo = a.pbox_lo; c.pbox_hi = a.pbox_hi; c.p32 = a.p32; c.v32 = a.v32;
     int np = a.ctr->npairs;
     if (np > max_pairs) np = max_pairs;
-    int t_visits = 0, t_sub = 0;
-    if (np <= kWideFilter) filter_wide<MOVING>(a, c, np, t_visits, t_sub);
+    int t_visits = 0;
+    if (np <= kWideFilter) filter_wide<MOVING>(a, c, np, t_visits);
     for (int idx = np <= kWideFilter ? np : blockIdx.x * blockDim.x + threadIdx.x; idx < np;
          idx += gridDim.x * blockDim.x) {
         int2 pr = a.pairs[idx];
@@ -409,14 +398,8 @@ __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pai
             queue_sub<MOVING>(a, c, ee, o.keybase, idx, sc, pts, sub, first);
         });
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        t_visits += __shfl_xor_sync(0xffffffffu, t_visits, o);
-        t_sub += __shfl_xor_sync(0xffffffffu, t_sub, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (t_visits) atomicAdd(&a.ctr->nvisits, t_visits);
-        if (t_sub) atomicAdd(&a.ctr->nsub, t_sub);
-    }
+    for (int o = 16; o > 0; o >>= 1) t_visits += __shfl_xor_sync(0xffffffffu, t_visits, o);
+    if ((threadIdx.x & 31) == 0 && t_visits) atomicAdd(&a.ctr->nvisits, t_visits);
 }
 
 // The extents of n points' box over the window, for gap_may_hit.
@@ -437,10 +420,8 @@ __device__ __forceinline__ float swept_extent(const F3* X, const F3* V, int n, f
 
 // Stage 1 of a plain FP64 pass, sixteen threads per pair: a sub-test whose
 // elements stay farther apart than a hit allows (gap_may_hit, on the points
-// cut to FP32) is done; on moving passes of few pairs, so is one whose cubic
-// can have no root in the time window (may_be_coplanar, FP64; in large passes
-// the sub-tests themselves find that, a full warp at a time). The others are
-// queued for the full test. Every sub-test counts as evaluated. An FP64 test
+// cut to FP32) is done, the others are queued for the full test. Every
+// sub-test counts as evaluated. An FP64 test
 // of each of a pair's fifteen sub-tests took a static pass over 24 sheets
 // 2.07 ms, and the moving passes of their step 2.0 ms; now 0.28 and 0.63 ms.
 constexpr int kPlainBlock = 128;
@@ -488,14 +469,6 @@ __global__ void __launch_bounds__(kPlainBlock) k_plain_filter(NarrowArgs a, int 
                     const float hpad = cut32_up(MOVING ? prm.eps : prm.thickness), epad = cut32_up(prm.eps);
                     queue = ee ? gap_may_hit<MOVING, true>(X, V, ext, extb, hpad, epad, dt32)
                                : gap_may_hit<MOVING, false>(X, V, ext, extb, hpad, epad, dt32);
-                    if (MOVING && queue && np <= kWideFilter) {
-                        double xo4[4][3], av4[4][3];
-                        for (int q = 0; q < 4; ++q) {
-                            load3(a.xo, pts[q], xo4[q]);
-                            load3(a.av, pts[q], av4[q]);
-                        }
-                        queue = may_be_coplanar(xo4, av4, prm.dt);
-                    }
                 }
             }
         }
@@ -563,8 +536,10 @@ __device__ __forceinline__ NarrowCtx subtest_ctx(const NarrowArgs& a) {
 
 // One sub-test: its test, the stamps of its points and its pair's hit flag
 // when it hits, the scene's hit count when it is the pair's first.
+// counted: the sub-test has been counted (k_subtests_cubic).
 template <bool MOVING, bool EE>
-__device__ __forceinline__ void one_subtest(const NarrowArgs& a, NarrowCtx& c, const SubRec& r, SubTally& t) {
+__device__ __forceinline__ void one_subtest(const NarrowArgs& a, NarrowCtx& c, const SubRec& r, bool counted,
+                                            SubTally& t) {
     c.p = a.scenes[r.scene].p;
     c.pass = 0;
     CallState st;
@@ -575,7 +550,7 @@ __device__ __forceinline__ void one_subtest(const NarrowArgs& a, NarrowCtx& c, c
     st.ncr = 0;
     st.ncontacts = 0;
     bool hit = MOVING ? moving_test<EE>(c, st, r.p) : static_test<EE>(c, st, r.p);
-    t.sub += r.counted == 0;
+    t.sub += !counted && r.counted == 0;
     t.cr += st.ncr;
     t.contacts += st.ncontacts;
     if (hit)
@@ -602,6 +577,57 @@ __device__ __forceinline__ void subtest_counts(const NarrowArgs& a, SubTally t) 
     }
 }
 
+// Moving passes of more sub-tests than kSubSparse first form every cubic, a
+// sub-test per thread, and list those that may have a root in the time window
+// (may_be_coplanar); the tests then run on the lists. Most of a filter's
+// survivors end here, and one lane's roots and tests otherwise hold up its
+// warp. 257 x 257 points in contact: filters and sub-tests of a step 1.48 ->
+// 1.09 ms (the filter formed the cubics of its survivors before, with almost
+// every warp holding one).
+constexpr int kSubSparse = 1216;
+struct SubLists {
+    int npt, nee;
+    bool listed;
+};
+template <bool MOVING>
+__device__ __forceinline__ SubLists sub_lists(const NarrowArgs& a) {
+    SubLists l;
+    l.npt = a.ctr->nsub_pt < a.sub_cap ? a.ctr->nsub_pt : a.sub_cap;
+    l.nee = a.ctr->nsub_ee < a.sub_cap ? a.ctr->nsub_ee : a.sub_cap;
+    l.listed = MOVING && l.npt + l.nee > kSubSparse;
+    if (l.listed) {
+        l.npt = a.ctr->nlive_pt;
+        l.nee = a.ctr->nlive_ee;
+    }
+    return l;
+}
+
+__global__ void __launch_bounds__(128) k_subtests_cubic(NarrowArgs a) {
+    const int npt = a.ctr->nsub_pt < a.sub_cap ? a.ctr->nsub_pt : a.sub_cap;
+    const int nee = a.ctr->nsub_ee < a.sub_cap ? a.ctr->nsub_ee : a.sub_cap;
+    const int n = npt + nee;
+    if (n <= kSubSparse) return;
+    int t_sub = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const bool ee = i >= npt;
+        const int k = ee ? i - npt : i;
+        const SubRec& r = (ee ? a.sub_ee : a.sub_pt)[k];
+        double xo4[4][3], av4[4][3];
+        for (int q = 0; q < 4; ++q) {
+            load3(a.xo, r.p[q], xo4[q]);
+            load3(a.av, r.p[q], av4[q]);
+        }
+        t_sub += r.counted == 0;
+        if (!may_be_coplanar(xo4, av4, a.scenes[r.scene].p.dt)) continue;
+        if (ee)  // (the lanes that add together share one counter)
+            a.live_ee[aggregated_add(&a.ctr->nlive_ee, 1)] = k;
+        else
+            a.live_pt[aggregated_add(&a.ctr->nlive_pt, 1)] = k;
+    }
+    for (int o = 16; o > 0; o >>= 1) t_sub += __shfl_xor_sync(0xffffffffu, t_sub, o);
+    if ((threadIdx.x & 31) == 0 && t_sub) atomicAdd(&a.ctr->nsub, t_sub);
+}
+
 // Passes with more sub-tests than this give each kind blocks of its own
 // (k_subtests): measured faster than both kinds in a warp when the pass is
 // large, where the FP64 pipes are full either way.
@@ -612,16 +638,17 @@ constexpr int kSubMergeMax = 65536;
 // at most kSubMergeMax sub-tests.
 template <bool MOVING>
 __global__ void __launch_bounds__(128, 4) k_subtests(NarrowArgs a, int merged) {
-    const int npt = a.ctr->nsub_pt < a.sub_cap ? a.ctr->nsub_pt : a.sub_cap;
-    const int nee = a.ctr->nsub_ee < a.sub_cap ? a.ctr->nsub_ee : a.sub_cap;
-    if (merged && npt + nee <= kSubMergeMax) return;
+    const SubLists l = sub_lists<MOVING>(a);
+    if (merged && l.npt + l.nee <= kSubMergeMax) return;
     NarrowCtx c = subtest_ctx(a);
     SubTally t;
     const int first = (blockIdx.x >> 1) * blockDim.x + threadIdx.x, stride = (gridDim.x >> 1) * blockDim.x;
     if (blockIdx.x & 1) {
-        for (int i = first; i < nee; i += stride) one_subtest<MOVING, true>(a, c, a.sub_ee[i], t);
+        for (int i = first; i < l.nee; i += stride)
+            one_subtest<MOVING, true>(a, c, a.sub_ee[l.listed ? a.live_ee[i] : i], l.listed, t);
     } else {
-        for (int i = first; i < npt; i += stride) one_subtest<MOVING, false>(a, c, a.sub_pt[i], t);
+        for (int i = first; i < l.npt; i += stride)
+            one_subtest<MOVING, false>(a, c, a.sub_pt[l.listed ? a.live_pt[i] : i], l.listed, t);
     }
     subtest_counts(a, t);
 }
@@ -636,12 +663,10 @@ __global__ void __launch_bounds__(128, 4) k_subtests(NarrowArgs a, int merged) {
 // sub-test per thread, which keeps the FP64 pipe's issue slots full.
 // Two blocks per SM: one warp per SM sub-partition already keeps its FP64
 // pipe issuing, and the registers then hold both tests without spills.
-constexpr int kSubSparse = 1216;
 template <bool MOVING>
 __global__ void __launch_bounds__(128, 2) k_subtests_all(NarrowArgs a) {
-    const int npt = a.ctr->nsub_pt < a.sub_cap ? a.ctr->nsub_pt : a.sub_cap;
-    const int nee = a.ctr->nsub_ee < a.sub_cap ? a.ctr->nsub_ee : a.sub_cap;
-    const int n = npt + nee;
+    const SubLists l = sub_lists<MOVING>(a);
+    const int n = l.npt + l.nee;
     if (n > kSubMergeMax) return;  // k_subtests's
     NarrowCtx c = subtest_ctx(a);
     SubTally t;
@@ -650,10 +675,10 @@ __global__ void __launch_bounds__(128, 2) k_subtests_all(NarrowArgs a) {
     if (!sparse || (threadIdx.x & 31) == 0) {
         const int first = sparse ? g >> 5 : g, stride = sparse ? threads >> 5 : threads;
         for (int i = first; i < n; i += stride) {
-            if (i < npt)
-                one_subtest<MOVING, false>(a, c, a.sub_pt[i], t);
+            if (i < l.npt)
+                one_subtest<MOVING, false>(a, c, a.sub_pt[l.listed ? a.live_pt[i] : i], l.listed, t);
             else
-                one_subtest<MOVING, true>(a, c, a.sub_ee[i - npt], t);
+                one_subtest<MOVING, true>(a, c, a.sub_ee[l.listed ? a.live_ee[i - l.npt] : i - l.npt], l.listed, t);
         }
     }
     subtest_counts(a, t);
@@ -727,6 +752,7 @@ void narrow_pass_split(const NarrowArgs& args, int moving, int max_pairs, cudaSt
             }
         }
         if (parts & kSplitSubtests) {
+            count_launch(), k_subtests_cubic<<<sblocks < 152 * 8 ? sblocks : 152 * 8, 128, 0, s>>>(a);
             if (a.sub_merge) count_launch(), k_subtests_all<true><<<mblocks, 128, 0, s>>>(a);
             count_launch(), k_subtests<true><<<2 * sblocks, 128, 0, s>>>(a, a.sub_merge);
             if (zone) count_launch(), k_zone_unions<<<blocks, 128, 0, s>>>(a);

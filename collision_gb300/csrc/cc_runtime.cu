@@ -82,7 +82,7 @@ __global__ void k_reset_counters(PassCounters* c) {
     int keep = c->err & kErrNan;
     c->npairs = 0; c->ncontrib = 0; c->nhit_pairs = 0; c->nrec = 0;
     c->nvisits = 0; c->ncontacts = 0; c->nsub = 0; c->ncr = 0; c->nunion = 0; c->nsub_pt = 0; c->nsub_ee = 0; c->npairq = 0;
-    c->nzones = 0; c->nmembers = 0; c->nseg = 0; c->ntouch = 0; c->nseg_used = 0;
+    c->nzones = 0; c->nmembers = 0; c->nseg = 0; c->ntouch = 0; c->nseg_used = 0; c->nlive_pt = 0; c->nlive_ee = 0;
     c->err = keep;
 }
 
@@ -95,7 +95,7 @@ __global__ void k_reset_pass(PassCounters* c, SceneRun* run, int nscenes, int np
         int keep = c->err & kErrNan;
         c->npairs = npairs_keep >= 0 ? npairs_keep : 0; c->ncontrib = 0; c->nhit_pairs = 0; c->nrec = 0;
         c->nvisits = 0; c->ncontacts = 0; c->nsub = 0; c->ncr = 0; c->nunion = 0; c->nsub_pt = 0; c->nsub_ee = 0; c->npairq = 0;
-        c->nzones = 0; c->nmembers = 0; c->nseg = 0; c->ntouch = 0; c->nseg_used = 0;
+        c->nzones = 0; c->nmembers = 0; c->nseg = 0; c->ntouch = 0; c->nseg_used = 0; c->nlive_pt = 0; c->nlive_ee = 0;
         c->err = keep;
     }
     if (i < nscenes) run[i].hits = 0;
@@ -225,6 +225,7 @@ struct cc_solver {
     int pair_cap = 0;
     SubRec* d_sub_pt = nullptr;
     SubRec* d_sub_ee = nullptr;
+    int* d_live = nullptr;  // 2 * sub_cap: k_subtests_cubic's lists
     int sub_cap = 0;
     Contrib* d_contrib = nullptr;
     int contrib_cap = 0;
@@ -388,7 +389,7 @@ struct cc_solver {
         a.pbox_hi = mode == 1 ? d_pbox_hi : nullptr;
         a.p32 = d_p32; a.v32 = d_v32;
         a.check = 0;
-        a.sub_pt = d_sub_pt; a.sub_ee = d_sub_ee; a.sub_cap = sub_cap;
+        a.sub_pt = d_sub_pt; a.sub_ee = d_sub_ee; a.sub_cap = sub_cap; a.live_pt = d_live; a.live_ee = d_live + sub_cap;
         a.pair_hit = d_pair_hit; a.pairq = d_pairq;
         a.static_only = combined ? 1 : 0;
         return a;
@@ -526,7 +527,7 @@ struct cc_solver {
         dfree(bvh.rnode); dfree(bvh.rope); dfree(bvh.leaf32); dfree(bvh.qnext); dfree(bvh.heavy);
         if (bvh.sort_temp) cudaFree(bvh.sort_temp);
         bvh = BvhBufs{};
-        dfree(d_pairs); dfree(d_contrib); dfree(d_pair_hit); dfree(d_pairq); dfree(d_sub_pt); dfree(d_sub_ee);
+        dfree(d_pairs); dfree(d_contrib); dfree(d_pair_hit); dfree(d_pairq); dfree(d_sub_pt); dfree(d_sub_ee); dfree(d_live);
         sub_cap = 0;
         dfree(apply.cnt); dfree(apply.off); dfree(apply.cur); dfree(apply.idx);
         dfree(apply.touched); dfree(apply.ord);
@@ -633,7 +634,9 @@ struct cc_solver {
         loop_dirty = true;
         dfree(d_sub_pt);
         dfree(d_sub_ee);
-        if (dalloc(&d_sub_pt, (size_t)cap) != cudaSuccess || dalloc(&d_sub_ee, (size_t)cap) != cudaSuccess)
+        dfree(d_live);
+        if (dalloc(&d_sub_pt, (size_t)cap) != cudaSuccess || dalloc(&d_sub_ee, (size_t)cap) != cudaSuccess ||
+            dalloc(&d_live, 2 * (size_t)cap) != cudaSuccess)
             return fail(CC_NO_MEMORY, "sub-test queues");
         sub_cap = cap;
         return CC_OK;
@@ -2012,7 +2015,7 @@ cc_status cc_solver::detect_pass(int moving, bool any_zone) {
         a.check = 0;
         a.sub_pt = d_sub_pt;
         a.sub_ee = d_sub_ee;
-        a.sub_cap = sub_cap;
+        a.sub_cap = sub_cap; a.live_pt = d_live; a.live_ee = d_live + sub_cap;
         a.pair_hit = d_pair_hit;
         a.pairq = d_pairq;
         a.static_only = combined ? 1 : 0;
@@ -2358,7 +2361,7 @@ cc_status cc_solver::check_ccd(const double* x_old, const double* x_new, long lo
         a.check = 1;
         a.sub_pt = d_sub_pt;
         a.sub_ee = d_sub_ee;
-        a.sub_cap = sub_cap;
+        a.sub_cap = sub_cap; a.live_pt = d_live; a.live_ee = d_live + sub_cap;
         a.pair_hit = d_pair_hit;
         a.pairq = d_pairq;
         if (split_narrow)  // in FP64 throughout: no FP32 point data
@@ -2436,7 +2439,7 @@ cc_status cc_solver::autotune(double* best_ms) {
             a.pbox_lo = mode == 1 ? d_pbox_lo : nullptr;
             a.pbox_hi = mode == 1 ? d_pbox_hi : nullptr;
             a.p32 = d_p32; a.v32 = d_v32;
-            a.sub_pt = d_sub_pt; a.sub_ee = d_sub_ee; a.sub_cap = sub_cap; a.pair_hit = d_pair_hit;
+            a.sub_pt = d_sub_pt; a.sub_ee = d_sub_ee; a.sub_cap = sub_cap; a.live_pt = d_live; a.live_ee = d_live + sub_cap; a.pair_hit = d_pair_hit;
             a.pairq = d_pairq;
             if (split)
                 narrow_pass_split(a, 1, pair_cap, stream, t.narrow_block);
