@@ -678,8 +678,8 @@ def run_gpu(args):
     ms, calls = prof.get("strain", (0.0, 0))
     if calls:
         per = tot["strain_bytes"] / calls
-        kern["strain"] = {"kernel": "strain stage: k_strain_setup, k_strain_check and k_strain_window sweeps "
-                          "(one CTA per scene), one launch = one step's tail graph", "bytes_per_launch": per,
+        kern["strain"] = {"kernel": "strain stage: k_sweep_setup, k_sweep_check and k_strain_sweeps "
+                          "(one CTA per scene and sweep), one launch = one step's tail graph", "bytes_per_launch": per,
                           "ms_per_launch": ms / calls, "achieved": per / (ms / calls / 1e3) / 1e9}
     kp = mixed["kprof"]
     if kp:
@@ -690,7 +690,7 @@ def run_gpu(args):
         if t_sub > 0 and kc.get("fp64_subtests"):
             flops = SUBTEST_FP64_FLOPS * kc["fp64_subtests"]
             kern["ccd_subtests"] = {
-                "kernel": "k_subtests_all (the FP64 sub-tests that pass the FP32 filters, both kinds in one launch)",
+                "kernel": "k_subtests (the FP64 sub-tests that pass the FP32 filters, both kinds in one launch)",
                 "bound": "fp64",
                 "flops": flops, "s": t_sub, "achieved_tflops": flops / t_sub / 1e12, "peak_tflops": FP64_PEAK_TFLOPS,
                 "frac": flops / t_sub / 1e12 / FP64_PEAK_TFLOPS, "peak_source": "nominal",

@@ -244,7 +244,7 @@ struct NarrowArgs {
     int static_only;  // proximity pass over swept-box pairs: only those with kPairStatic
     PassStamp ps;     // stamps of the points of every sub-test that hits
     // 1: both sub-test lists in one launch, a warp per sub-test in small
-    // passes (k_subtests_all); 0: a thread per sub-test, blocks by list
+    // passes; 0: a thread per sub-test, blocks of one kind each
     int sub_merge = 1;
     // movable rigid bodies: the body of each point (-1 none), each body's
     // mass, and the contribution slot of body 0 (the point count)

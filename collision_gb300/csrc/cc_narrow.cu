@@ -628,34 +628,15 @@ __global__ void __launch_bounds__(128) k_subtests_cubic(NarrowArgs a) {
     if ((threadIdx.x & 31) == 0 && t_sub) atomicAdd(&a.ctr->nsub, t_sub);
 }
 
-// Passes with more sub-tests than this give each kind blocks of its own
-// (k_subtests): measured faster than both kinds in a warp when the pass is
-// large, where the FP64 pipes are full either way.
+// Passes with more sub-tests than this give each kind blocks of its own:
+// measured faster than both kinds in a warp when the pass is large, where the
+// FP64 pipes are full either way.
 constexpr int kSubMergeMax = 65536;
 
-// One list per block (point-triangle in the even ones, edge-edge in the odd
-// ones), one sub-test per thread. merged: k_subtests_all takes the passes of
-// at most kSubMergeMax sub-tests.
-template <bool MOVING>
-__global__ void __launch_bounds__(128, 4) k_subtests(NarrowArgs a, int merged) {
-    const SubLists l = sub_lists<MOVING>(a);
-    if (merged && l.npt + l.nee <= kSubMergeMax) return;
-    NarrowCtx c = subtest_ctx(a);
-    SubTally t;
-    const int first = (blockIdx.x >> 1) * blockDim.x + threadIdx.x, stride = (gridDim.x >> 1) * blockDim.x;
-    if (blockIdx.x & 1) {
-        for (int i = first; i < l.nee; i += stride)
-            one_subtest<MOVING, true>(a, c, a.sub_ee[l.listed ? a.live_ee[i] : i], l.listed, t);
-    } else {
-        for (int i = first; i < l.npt; i += stride)
-            one_subtest<MOVING, false>(a, c, a.sub_pt[l.listed ? a.live_pt[i] : i], l.listed, t);
-    }
-    subtest_counts(a, t);
-}
-
-// Both lists in one launch (passes of at most kSubMergeMax sub-tests),
-// point-triangle sub-tests first, so that a small pass's two lists run side
-// by side. A warp pays for an FP64 instruction the
+// Both lists in one launch. Up to kSubMergeMax sub-tests, point-triangle ones
+// first, so that a small pass's two lists run side by side; above (and with
+// merged = 0 throughout) point-triangle ones in the even blocks and edge-edge
+// ones in the odd. A warp pays for an FP64 instruction the
 // same whatever the number of its lanes that execute it, and the lanes of a
 // warp running different sub-tests follow the union of their paths: a pass
 // with at most kSubSparse sub-tests (two warps per SM sub-partition) gives
@@ -664,17 +645,18 @@ __global__ void __launch_bounds__(128, 4) k_subtests(NarrowArgs a, int merged) {
 // Two blocks per SM: one warp per SM sub-partition already keeps its FP64
 // pipe issuing, and the registers then hold both tests without spills.
 template <bool MOVING>
-__global__ void __launch_bounds__(128, 2) k_subtests_all(NarrowArgs a) {
+__global__ void __launch_bounds__(128, 2) k_subtests(NarrowArgs a, int merged) {
     const SubLists l = sub_lists<MOVING>(a);
     const int n = l.npt + l.nee;
-    if (n > kSubMergeMax) return;  // k_subtests's
     NarrowCtx c = subtest_ctx(a);
     SubTally t;
-    const int g = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
-    const bool sparse = n <= kSubSparse;
+    const bool by_kind = !merged || n > kSubMergeMax, sparse = !by_kind && n <= kSubSparse;
     if (!sparse || (threadIdx.x & 31) == 0) {
-        const int first = sparse ? g >> 5 : g, stride = sparse ? threads >> 5 : threads;
-        for (int i = first; i < n; i += stride) {
+        // this thread's place among those that share its list, of `end` sub-tests from `i` on
+        const int per = sparse ? (int)(blockDim.x >> 5) : (int)blockDim.x;
+        const int block = by_kind ? blockIdx.x >> 1 : blockIdx.x, blocks = by_kind ? gridDim.x >> 1 : gridDim.x;
+        const int first = by_kind && (blockIdx.x & 1) ? l.npt : 0, end = by_kind && !(blockIdx.x & 1) ? l.npt : n;
+        for (int i = first + block * per + (sparse ? threadIdx.x >> 5 : threadIdx.x); i < end; i += blocks * per) {
             if (i < l.npt)
                 one_subtest<MOVING, false>(a, c, a.sub_pt[l.listed ? a.live_pt[i] : i], l.listed, t);
             else
@@ -737,12 +719,12 @@ void narrow_pass_split(const NarrowArgs& args, int moving, int max_pairs, cudaSt
     if (blocks > cap_blocks) blocks = cap_blocks;
     int sblocks = (a.sub_cap + 127) / 128;
     if (sblocks > 152 * 16) sblocks = 152 * 16;
-    // both lists of a pass of at most kSubMergeMax in one grid, at least one
-    // warp per sub-test of a sparse pass
+    // one grid for any number of sub-tests, strided above kSubMergeMax, with at
+    // least one warp per sub-test of a sparse pass and an even block count
     long long mb = (2ll * a.sub_cap + 127) / 128;
     if (mb > (kSubMergeMax + 127) / 128) mb = (kSubMergeMax + 127) / 128;
     if (mb < (kSubSparse + 3) / 4) mb = (kSubSparse + 3) / 4;
-    const int mblocks = (int)mb;
+    const int mblocks = (int)(mb + 1) & ~1;
     if (moving) {
         if (parts & kSplitFilter) {
             if (mixed) {
@@ -753,8 +735,7 @@ void narrow_pass_split(const NarrowArgs& args, int moving, int max_pairs, cudaSt
         }
         if (parts & kSplitSubtests) {
             count_launch(), k_subtests_cubic<<<sblocks < 152 * 8 ? sblocks : 152 * 8, 128, 0, s>>>(a);
-            if (a.sub_merge) count_launch(), k_subtests_all<true><<<mblocks, 128, 0, s>>>(a);
-            count_launch(), k_subtests<true><<<2 * sblocks, 128, 0, s>>>(a, a.sub_merge);
+            count_launch(), k_subtests<true><<<mblocks, 128, 0, s>>>(a, a.sub_merge);
             if (zone) count_launch(), k_zone_unions<<<blocks, 128, 0, s>>>(a);
         }
     } else {
@@ -765,8 +746,7 @@ void narrow_pass_split(const NarrowArgs& args, int moving, int max_pairs, cudaSt
                 count_launch(), k_plain_filter<false><<<(int)pb, kPlainBlock, 0, s>>>(a, max_pairs);
         }
         if (parts & kSplitSubtests) {
-            if (a.sub_merge) count_launch(), k_subtests_all<false><<<mblocks, 128, 0, s>>>(a);
-            count_launch(), k_subtests<false><<<2 * sblocks, 128, 0, s>>>(a, a.sub_merge);
+            count_launch(), k_subtests<false><<<mblocks, 128, 0, s>>>(a, a.sub_merge);
         }
     }
 }

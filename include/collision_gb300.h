@@ -195,11 +195,10 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
 
 /* Tuning knobs (none changes results):
  *   CC_TUNE_SPLIT_NARROW    1 (default): passes without recording filter
- *                           first (mixed: in FP32 per pair; plain moving
- *                           passes and cc_check_ccd: each sub-test's
- *                           coplanarity cubic in FP64), then run the FP64
- *                           sub-tests that pass, one thread each; 0: one
- *                           thread per pair throughout
+ *                           first (mixed: in FP32 per pair and sub-test;
+ *                           plain passes and cc_check_ccd: per sub-test on
+ *                           points cut to FP32), then run the FP64 sub-tests
+ *                           that pass; 0: one thread per pair throughout
  *   CC_TUNE_TRAVERSE_BLOCK  threads per block of the BVH traversal (32..1024)
  *   CC_TUNE_NARROW_BLOCK    threads per block of the per-pair filter stage
  *                           of split passes (32..512)
@@ -278,9 +277,10 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           sort up to 8,192 in one; 0: always the general
  *                           kernels and the general sort. Same results
  *   CC_TUNE_PRUNED_WARP     1 (default): in the device loop's pruned passes
- *                           each query walks its scene with one warp (a
- *                           shared-memory stack, up to 32 nodes per round);
- *                           0: one thread along the ropes. Same results
+ *                           only touched elements are boxed again, and each
+ *                           walks its scene with one warp (a shared-memory
+ *                           stack, up to 32 nodes per round); 0: every box,
+ *                           one thread along the ropes. Same results
  *   CC_TUNE_ROBUST_ROOTS    accepted, without effect: every coplanarity root
  *                           is formed with correctly rounded functions
  *   CC_TUNE_ZONE_CTA_MIN    members from which an impact zone's rigid
