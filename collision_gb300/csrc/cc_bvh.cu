@@ -222,9 +222,11 @@ __device__ __forceinline__ int delta(const unsigned long long* keys, int n, int 
 // With rope given, the node that splits sorted leaves gamma and gamma+1
 // (every boundary has exactly one) records its right child as the rope of
 // that boundary, or kRopeEnd where the two leaves' scenes differ (the scene
-// id sits above the 30 Morton bits of the keys).
+// id sits above the 30 Morton bits of the keys). With run given, the node
+// whose leaves are exactly a scene's records itself as the scene's root (a
+// climb from the scene's first leaf took 10 us of a small step).
 __global__ void k_karras(const unsigned long long* __restrict__ keys, int n, BvhNode32* node, int* range_hi,
-                         int* range_lo, int* parent, int* rope) {
+                         int* range_lo, int* parent, int* rope, SceneRun* run) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -254,6 +256,11 @@ __global__ void k_karras(const unsigned long long* __restrict__ keys, int n, Bvh
     if (right >= 0) parent[right] = i; else parent[n - 1 + ~right] = i;
     if (i == 0) parent[0] = -1;
     if (rope) rope[gamma] = ((keys[gamma] ^ keys[gamma + 1]) >> 30) ? kRopeEnd : right;
+    if (run) {
+        const unsigned long long sc = keys[lo] >> 30;
+        if (sc == keys[hi] >> 30 && (lo == 0 || keys[lo - 1] >> 30 != sc) && (hi == n - 1 || keys[hi + 1] >> 30 != sc))
+            run[sc].root = i;
+    }
 }
 
 // Each internal node's first child and rope: a node covering sorted leaves
@@ -1459,12 +1466,8 @@ void bvh_build(const Box6* box, BvhBufs& b, cudaStream_t s) {
     radix_sort_pairs(b.keys, b.order, n, bits, b.sort_temp, s);
     const bool ropes = b.rnode && b.rope;
     count_launch(), k_karras<<<nblk(n - 1, 256), 256, 0, s>>>(b.keys, n, b.node, b.range_hi, b.range_lo, b.parent,
-                                                              ropes ? b.rope : nullptr);
+                                                              ropes ? b.rope : nullptr, b.run);
     if (ropes) count_launch(), k_ropes<<<nblk(n - 1, 256), 256, 0, s>>>(b.node, b.rope, n, b.rnode);
-    // the scenes' roots first: the refit's walks end there
-    if (b.run)
-        count_launch(), k_scene_roots<<<nblk(b.nscenes, 128), 128, 0, s>>>(b.scenes, b.run, b.nscenes, n, b.parent,
-                                                                          b.range_lo, b.range_hi);
     cudaMemsetAsync(b.flags, 0, sizeof(int) * (size_t)(n - 1), s);
     launch_refit(box, b, n, nullptr, 0, nullptr, nblk(n, 256), ropes ? b.rnode : nullptr, s);
 }
