@@ -960,9 +960,12 @@ struct cc_solver {
         cudaStreamSynchronize(stream);  // the vectors are pageable
         return cuda_check("strain edge schedule");
     }
+    static void put_params(SceneDev& sd, const cc_params& p) {
+        sd.p = Params{p.dt, p.thickness, p.eps, p.k, p.m, p.lambda, p.cr};
+        sd.inv_dt = 1.0 / p.dt;
+    }
     void set_scene_params(int i, const cc_params& p) {
-        h_scenes[i].p = Params{p.dt, p.thickness, p.eps, p.k, p.m, p.lambda, p.cr};
-        h_scenes[i].inv_dt = 1.0 / p.dt;
+        put_params(h_scenes[i], p);
         scenes_dirty = true;
     }
     void set_scene_domain(int i, const double* l, const double* h) {
@@ -1024,7 +1027,7 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
         SceneHost& sh = scenes[si];
         sh.v0 = v0; sh.nv = snv; sh.e0 = e0; sh.ne = sne; sh.nt = nt;
         SceneDev& sd = h_scenes[si];
-        sd.p = Params{prm.dt, prm.thickness, prm.eps, prm.k, prm.m, prm.lambda, prm.cr};
+        put_params(sd, prm);
         for (int d = 0; d < 3; ++d) {
             sd.lo[d] = lo[d];
             sd.hi[d] = hi[d];
