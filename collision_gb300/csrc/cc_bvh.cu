@@ -879,7 +879,7 @@ __global__ void k_traverse_rope(int n, const RopeNode* __restrict__ rn, const in
 // consecutive queries with one atomic. A leaf is tested first on its 32-byte
 // FP32 record (outward-rounded box, rope, element), and only a leaf that
 // passes loads its 64-byte exact record. Same pairs as k_traverse_rope.
-// A walk longer than `budget` steps (a large element among small ones: an
+// A walk longer than `longest` steps (a large element among small ones: an
 // obstacle's side over a sheet) is one long chain of dependent loads that the
 // whole pass would wait for: it is handed over, with the first sorted leaf
 // it has not reached, to k_traverse_warp. Strings over a 12-triangle box:
@@ -888,7 +888,7 @@ __global__ void __launch_bounds__(128) k_traverse_rope_dyn(
     int n, const RopeNode* __restrict__ rn, const int* __restrict__ elem_scene, const SceneRun* __restrict__ run,
     const int* __restrict__ ev, int2* pairs, int cap, PassCounters* ctr, const Box6* __restrict__ box_static,
     const LeafRec* __restrict__ leaves, const LeafBox32* __restrict__ leaf32, const int* __restrict__ sub, int nsub,
-    const int* __restrict__ dnsub, int* qnext, int refill, int budget, int2* heavy,
+    const int* __restrict__ dnsub, int* qnext, int refill, int longest, int2* heavy,
     const int* __restrict__ range_lo) {
     const int nq = sub ? (dnsub ? *dnsub : nsub) : n - 1;
     const unsigned lane_lt = (1u << (threadIdx.x & 31)) - 1u;
@@ -939,7 +939,7 @@ __global__ void __launch_bounds__(128) k_traverse_rope_dyn(
         }
         if (!more && __all_sync(0xffffffffu, x == kRopeEnd)) break;
         if (x == kRopeEnd) continue;
-        if (++steps > budget) {  // one entry per query: fits
+        if (++steps > longest) {  // one entry per query: fits
             if (x < n - 1 && ~x < n)
                 heavy[atomicAdd(qnext + 1, 1)] = make_int2(qi, x >= 0 ? range_lo[x] : ~x);
             else
