@@ -195,12 +195,14 @@ __global__ void k_morton(const Box6* __restrict__ box, const int* __restrict__ a
     Box6 b = box[e];
     int sc = elem_scene ? elem_scene[e] : 0;
     const unsigned long long* sb = bb + 6 * sc;
-    // (in FP32: the codes order the leaves, no result depends on them)
+    // in FP32 from the scene's corner (the codes order the leaves, no result
+    // depends on them)
     unsigned int q[3];
     for (int d = 0; d < 3; ++d) {
-        const float lo = cut32(dec_double(sb[d])), ext = cut32(dec_double(sb[3 + d])) - lo;
-        const float c = 0.5f * (cut32(b.lo[d]) + cut32(b.hi[d]));
-        const float t = ext > 0.f ? fminf(fmaxf((c - lo) / ext, 0.f), 1.f) : 0.f;
+        const double lo = dec_double(sb[d]);
+        const float ext = cut32(dec_double(sb[3 + d]) - lo);
+        const float c = 0.5f * (cut32(b.lo[d] - lo) + cut32(b.hi[d] - lo));
+        const float t = ext > 0.f ? fminf(fmaxf(c / ext, 0.f), 1.f) : 0.f;
         unsigned int v = (unsigned int)(t * 1023.f);
         q[d] = v > 1023u ? 1023u : v;
     }
