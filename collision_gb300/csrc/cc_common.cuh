@@ -242,31 +242,6 @@ __device__ __forceinline__ int aggregated_add(int* p, int n) {
     return base + incl - n;
 }
 
-// x in FP32 by cutting the mantissa (error below 2^-23 |x|): the double's
-// bits re-biased and shifted on the integer pipe, where a conversion takes
-// the FP64 pipe's 64 cycles. Zeros keep their sign; values outside FP32's
-// normal range take the conversion.
-__device__ __forceinline__ float cut32(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const unsigned m = (hi & 0x7fffffffu) - 0x38000000u;  // exponent bias 1023 -> 127
-    if (m - 0x00100000u < 0x0fe00000u) return __uint_as_float((hi & 0x80000000u) | __funnelshift_l(lo, m, 3));
-    if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);
-    return (float)x;
-}
-// The same rounded down and up.
-__device__ __forceinline__ float cut32_step(double x, bool away_if_negative) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const unsigned m = (hi & 0x7fffffffu) - 0x38000000u;
-    if (m - 0x00100000u < 0x0fe00000u) {
-        const bool away = (lo & 0x1fffffffu) != 0u && ((hi >> 31) != 0u) == away_if_negative;
-        return __uint_as_float(((hi & 0x80000000u) | __funnelshift_l(lo, m, 3)) + (away ? 1u : 0u));
-    }
-    if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);
-    return away_if_negative ? __double2float_rd(x) : __double2float_ru(x);
-}
-__device__ __forceinline__ float cut32_down(double x) { return cut32_step(x, true); }
-__device__ __forceinline__ float cut32_up(double x) { return cut32_step(x, false); }
-
 // Doubles as signed integers of the same order (-0 below +0), and back: an
 // FP64 compare takes a warp ~64 cycles, a 64-bit integer one a few.
 __device__ __forceinline__ long long order_of(double x) {
@@ -283,22 +258,74 @@ __device__ __forceinline__ double of_order(long long o) {
 #else
 #define CC_HD inline
 #endif
+// The words of a double, and a float's bits.
+CC_HD unsigned hi_word(double x) {
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2hiint(x);
+#else
+    unsigned long long u;
+    std::memcpy(&u, &x, 8);
+    return (unsigned)(u >> 32);
+#endif
+}
+CC_HD unsigned lo_word(double x) {
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2loint(x);
+#else
+    unsigned long long u;
+    std::memcpy(&u, &x, 8);
+    return (unsigned)u;
+#endif
+}
+CC_HD float float_of_bits(unsigned u) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float x;
+    std::memcpy(&x, &u, 4);
+    return x;
+#endif
+}
+
+// x in FP32 by cutting the mantissa (error below 2^-23 |x|): the double's
+// bits re-biased and shifted on the integer pipe, where a conversion takes
+// the FP64 pipe's 64 cycles. Zeros keep their sign; values outside FP32's
+// normal range take the conversion.
+CC_HD float cut32(double x) {
+    const unsigned hi = hi_word(x), lo = lo_word(x);
+    const unsigned m = (hi & 0x7fffffffu) - 0x38000000u;  // exponent bias 1023 -> 127
+    if (m - 0x00100000u < 0x0fe00000u) return float_of_bits((hi & 0x80000000u) | ((m << 3) | (lo >> 29)));
+    if (((hi << 1) | lo) == 0u) return float_of_bits(hi);
+    return (float)x;
+}
+// The same rounded down and up.
+CC_HD float cut32_step(double x, bool away_if_negative) {
+    const unsigned hi = hi_word(x), lo = lo_word(x);
+    const unsigned m = (hi & 0x7fffffffu) - 0x38000000u;
+    if (m - 0x00100000u < 0x0fe00000u) {
+        const bool away = (lo & 0x1fffffffu) != 0u && ((hi >> 31) != 0u) == away_if_negative;
+        return float_of_bits(((hi & 0x80000000u) | ((m << 3) | (lo >> 29))) + (away ? 1u : 0u));
+    }
+    if (((hi << 1) | lo) == 0u) return float_of_bits(hi);
+#ifdef __CUDA_ARCH__
+    return away_if_negative ? __double2float_rd(x) : __double2float_ru(x);
+#else
+    const float f = (float)x;
+    return away_if_negative ? ((double)f > x ? nextafterf(f, -INFINITY) : f)
+                            : ((double)f < x ? nextafterf(f, INFINITY) : f);
+#endif
+}
+CC_HD float cut32_down(double x) { return cut32_step(x, true); }
+CC_HD float cut32_up(double x) { return cut32_step(x, false); }
+
 // a / b for inv = 1 / b rounded: two corrections of a * inv by its exact
 // remainder (Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990: the first gives a quotient within an ulp,
 // the second the correctly rounded one), 5 FP64 instructions. Outside the
 // range where the remainders are exact, the division itself.
 CC_HD double quotient(double a, double b, double inv) {
-#ifdef __CUDA_ARCH__
-    const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu, hb = (unsigned)__double2hiint(b) & 0x7fffffffu;
-    const bool zero = (ha | (unsigned)__double2loint(a)) == 0u;
-#else
-    unsigned long long ua, ub;
-    std::memcpy(&ua, &a, 8);
-    std::memcpy(&ub, &b, 8);
-    const unsigned ha = (unsigned)(ua >> 32) & 0x7fffffffu, hb = (unsigned)(ub >> 32) & 0x7fffffffu;
-    const bool zero = (ua << 1) == 0;
-#endif
+    const unsigned ha = hi_word(a) & 0x7fffffffu, hb = hi_word(b) & 0x7fffffffu;
+    const bool zero = (ha | lo_word(a)) == 0u;
     // 2^-400 <= |a|, |b| < 2^400
     const bool in = ha - 0x26f00000u < 0x32000000u || zero;
     if (!in || hb - 0x26f00000u >= 0x32000000u) return a / b;

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(128) k_narrow(NarrowArgs a, int max_pairs) {
         c.pass = run.pass;
         // h of the sub-tests (thickness for proximity, eps for CCD) and the
         // barycentric tolerance eps, rounded up to FP32
-        c.hpad = cut32_up(MOVING ? c.p.eps : c.p.thickness);
+        c.hpad = filter_reach(MOVING ? c.p.eps : c.p.thickness);
         c.epad = cut32_up(c.p.eps);
         c.dt32 = cut32_up(c.p.dt);
         int ri = c.rank ? c.rank[pr.x] : pr.x, rj = c.rank ? c.rank[pr.y] : pr.y;
@@ -223,10 +223,12 @@ constexpr int kWideFilter = 131072;
 
 template <bool MOVING>
 __device__ __forceinline__ void queue_sub(const NarrowArgs& a, const NarrowCtx& c, bool ee, unsigned long long kb,
-                                          int pair, int sc, const int* pts, int sub, bool& first) {
+                                          int pair, int sc, const int* pts, int sub, bool thin, bool& first) {
     float ext, extb;
-    if (!mixed_may_hit(c, pts, ee, &ext, &extb)) return;
-    if (ee ? !sat_may_hit<MOVING, true>(c, pts, ext, extb) : !sat_may_hit<MOVING, false>(c, pts, ext, extb)) return;
+    if (ee || !thin) {
+        if (!mixed_may_hit(c, pts, ee, &ext, &extb)) return;
+        if (ee ? !sat_may_hit<MOVING, true>(c, pts, ext, extb) : !sat_may_hit<MOVING, false>(c, pts, ext, extb)) return;
+    }
     int* cnt = ee ? &a.ctr->nsub_ee : &a.ctr->nsub_pt;
     int slot = aggregated_add(cnt, 1);
     if (slot >= a.sub_cap) {
@@ -282,7 +284,7 @@ __device__ __forceinline__ void queue_group(const NarrowArgs& a, bool queue, boo
 // pair_may_hit on sixteen lanes (all of the group take part): lane s forms
 // the gap along axis s of the twelve.
 template <bool MOVING>
-__device__ __forceinline__ bool pair_may_hit16(const NarrowCtx& c, const OrientedPair& o, int s) {
+__device__ __forceinline__ int pair_may_hit16(const NarrowCtx& c, const OrientedPair& o, int s) {
     const int ia[3] = {o.A[0], o.A[1], o.n1 == 3 ? o.A[2] : o.A[1]};
     const int ib[3] = {o.B[0], o.B[1], o.n2 == 3 ? o.B[2] : o.B[1]};
     F3 R[6];
@@ -298,7 +300,7 @@ __device__ __forceinline__ bool pair_may_hit16(const NarrowCtx& c, const Oriente
     // axis 0 the line between the centroids; 1..4 and 5..8 each element's
     // normal and in-plane edge normals; 9..11 the first edges' common normal
     // and the in-plane normals of each
-    float lb = -1.f;
+    float lb = -1.f, an = 0.f;
     if (s < 12) {
         F3 ax;
         if (s == 0) {
@@ -315,10 +317,12 @@ __device__ __forceinline__ bool pair_may_hit16(const NarrowCtx& c, const Oriente
             const F3 e = edges ? (k == 1 ? d1 : d2) : k == 1 ? e0 : k == 2 ? e1 : e2;
             ax = k == 0 ? nrm : fcross(nrm, e);
         }
-        lb = axis_gap(ax, R);
+        lb = axis_gap(ax, R, an);
     }
     for (int d = 8; d > 0; d >>= 1) lb = fmaxf(lb, __shfl_xor_sync(0xffffffffu, lb, d));
-    return pair_bound_may_hit<MOVING>(c, ia, o.n1, ib, o.n2, lb, L, M);
+    // the normals' lengths, from lanes 1 and 5
+    return pair_bound<MOVING>(c, ia, o.n1, ib, o.n2, lb, L, M, __shfl_sync(0xffffffffu, an, 1, 16),
+                              __shfl_sync(0xffffffffu, an, 5, 16));
 }
 
 // Stage 1 with sixteen threads per pair, one per axis of the pair's bound and
@@ -354,21 +358,27 @@ __device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, i
             }
         }
         const double eps = a.scenes[sc].p.eps;
-        c.hpad = cut32_up(MOVING ? eps : a.scenes[sc].p.thickness);
+        c.hpad = filter_reach(MOVING ? eps : a.scenes[sc].p.thickness);
         c.epad = cut32_up(eps);
         c.dt32 = cut32_up(a.scenes[sc].p.dt);
-        if (__any_sync(0xffffffffu, on)) on = pair_may_hit16<MOVING>(c, o, sub) && on;
+        int bound = kPairNear;
+        if (__any_sync(0xffffffffu, on)) bound = pair_may_hit16<MOVING>(c, o, sub);
+        if (bound == kPairFar) on = false;
         if (on && pair_subtest<MOVING>(o, sub, pts, ee)) {
             float ext, extb;
-            queue = mixed_may_hit(c, pts, ee, &ext, &extb) &&
-                    (ee ? sat_may_hit<MOVING, true>(c, pts, ext, extb) : sat_may_hit<MOVING, false>(c, pts, ext, extb));
+            queue = (!ee && bound == kPairThin) ||
+                    (mixed_may_hit(c, pts, ee, &ext, &extb) &&
+                     (ee ? sat_may_hit<MOVING, true>(c, pts, ext, extb) : sat_may_hit<MOVING, false>(c, pts, ext, extb)));
         }
         queue_group(a, queue, ee, o.keybase, idx, sc, pts, sub, group, false);
     }
 }
 
+// Registers held to 64 and 96, which let a block of 128 threads run eight and
+// five times on an SM: with the moving kernel's own choice of 108 a step of 48
+// sheets in contact took 29.2 ms against 28.8.
 template <bool MOVING>
-__global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pairs) {
+__global__ void __maxnreg__(MOVING ? 96 : 64) k_narrow_filter(NarrowArgs a, int max_pairs) {
     NarrowCtx c;
     c.pbox_lo = a.pbox_lo; c.pbox_hi = a.pbox_hi; c.p32 = a.p32; c.v32 = a.v32;
     int np = a.ctr->npairs;
@@ -385,37 +395,22 @@ __global__ void __launch_bounds__(512) k_narrow_filter(NarrowArgs a, int max_pai
         t_visits++;
         int sc = a.escene[pr.x];
         const double eps = a.scenes[sc].p.eps;
-        c.hpad = cut32_up(MOVING ? eps : a.scenes[sc].p.thickness);
+        c.hpad = filter_reach(MOVING ? eps : a.scenes[sc].p.thickness);
         c.epad = cut32_up(eps);
         c.dt32 = cut32_up(a.scenes[sc].p.dt);
         // a shared point makes every test of the pair return false
         bool shared = false;
         for (int i = 0; i < o.n1; ++i)
             for (int j = 0; j < o.n2; ++j) shared |= o.A[i] == o.B[j];
-        if (shared || !pair_may_hit<MOVING>(c, o.A, o.n1, o.B, o.n2)) continue;
+        const int bound = shared ? kPairFar : pair_may_hit<MOVING>(c, o.A, o.n1, o.B, o.n2);
+        if (bound == kPairFar) continue;
         bool first = true;
         for_each_subtest<MOVING>(o.kind, o.A, o.B, [&](int sub, const int* pts, bool ee) {
-            queue_sub<MOVING>(a, c, ee, o.keybase, idx, sc, pts, sub, first);
+            queue_sub<MOVING>(a, c, ee, o.keybase, idx, sc, pts, sub, bound == kPairThin, first);
         });
     }
     for (int o = 16; o > 0; o >>= 1) t_visits += __shfl_xor_sync(0xffffffffu, t_visits, o);
     if ((threadIdx.x & 31) == 0 && t_visits) atomicAdd(&a.ctr->nvisits, t_visits);
-}
-
-// The extents of n points' box over the window, for gap_may_hit.
-template <bool MOVING>
-__device__ __forceinline__ float swept_extent(const F3* X, const F3* V, int n, float dt) {
-    F3 lo = X[0], hi = X[0];
-    auto take = [&](F3 p) {
-        lo = F3{fminf(lo.x, p.x), fminf(lo.y, p.y), fminf(lo.z, p.z)};
-        hi = F3{fmaxf(hi.x, p.x), fmaxf(hi.y, p.y), fmaxf(hi.z, p.z)};
-    };
-    for (int i = 0; i < n; ++i) {
-        take(X[i]);
-        if (MOVING) take(fadd(X[i], fscale(V[i], dt)));
-    }
-    const F3 d = fsub(hi, lo);
-    return (d.x + d.y + d.z) * 1.001f;
 }
 
 // Stage 1 of a plain FP64 pass, sixteen threads per pair: a sub-test whose
@@ -450,39 +445,8 @@ __global__ void __launch_bounds__(kPlainBlock) k_plain_filter(NarrowArgs a, int 
                     for (int j = 0; j < o.n2; ++j) shared |= o.A[i] == o.B[j];
                 sc = a.escene[pr.x];
                 if (!shared && pair_subtest<MOVING>(o, sub, pts, ee)) {
-                    const Params& prm = a.scenes[sc].p;
-                    const float dt32 = cut32_up(prm.dt);
-                    F3 X[4], V[4];
-                    for (int q = 0; q < 4; ++q) {
-                        double x[3];
-                        load3(a.xo, pts[q], x);
-                        X[q] = cut_f3(x);
-                        if (MOVING) {
-                            load3(a.av, pts[q], x);
-                            V[q] = cut_f3(x);
-                        }
-                    }
                     ++t_sub;
-                    float hpad = cut32_up(MOVING ? prm.eps : prm.thickness), epad = cut32_up(prm.eps);
-                    const float most = fmaxf(fmaxf(fmaxabs(X[0]), fmaxabs(X[1])), fmaxf(fmaxabs(X[2]), fmaxabs(X[3])));
-                    if (most * 0x1p-13f > fmaxabs(fsub(X[1], X[0]))) {
-                        // far from the origin for its size: positions from the first
-                        // point's, and the tests' own rounding on the reach
-                        double x0[3], x[3];
-                        load3(a.xo, pts[0], x0);
-                        X[0] = F3{0.f, 0.f, 0.f};
-                        for (int q = 1; q < 4; ++q) {
-                            load3(a.xo, pts[q], x);
-                            for (int k = 0; k < 3; ++k) x[k] -= x0[k];
-                            X[q] = cut_f3(x);
-                        }
-                        hpad += most * 0x1p-44f;
-                    }
-                    const int na = ee ? 2 : 3;
-                    const float ext = swept_extent<MOVING>(X, V, na, dt32);
-                    const float extb = swept_extent<MOVING>(X + na, V + na, 4 - na, dt32);
-                    queue = ee ? gap_may_hit<MOVING, true>(X, V, ext, extb, hpad, epad, dt32)
-                               : gap_may_hit<MOVING, false>(X, V, ext, extb, hpad, epad, dt32);
+                    queue = plain_may_hit<MOVING>(a.xo, a.av, pts, ee, a.scenes[sc].p);
                 }
             }
         }

@@ -39,7 +39,7 @@ struct NarrowCtx {
     const float4* pbox_hi;
     const float4* p32;    // x_old rounded to FP32
     const float4* v32;    // avgVel rounded to FP32 (moving passes)
-    float hpad;   // h of the sub-tests, rounded up
+    float hpad;   // h of the sub-tests, padded (filter_reach)
     float epad;   // eps (barycentric tolerance), rounded up
     int check;    // decide hits only: no impulses, contacts or zones
     float dt32;   // dt rounded up to FP32
@@ -572,6 +572,9 @@ __device__ __forceinline__ F3 fadd(F3 a, F3 b) { return F3{a.x + b.x, a.y + b.y,
 __device__ __forceinline__ F3 fscale(F3 a, float s) { return F3{a.x * s, a.y * s, a.z * s}; }
 __device__ __forceinline__ F3 cut_f3(const double* a) { return F3{cut32(a[0]), cut32(a[1]), cut32(a[2])}; }
 __device__ __forceinline__ float fdot(F3 a, F3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ F3 fcross(F3 a, F3 b) {
+    return F3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+}
 __device__ __forceinline__ float fnorm(F3 a) { return sqrtf(fdot(a, a)); }
 __device__ __forceinline__ float fmaxabs(F3 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)); }
 __device__ __forceinline__ float clamp01(float x) { return fminf(fmaxf(x, 0.f), 1.f); }
@@ -641,6 +644,32 @@ __device__ __forceinline__ float triangle_gap(F3 ap, F3 ab, F3 ac, float* len) {
     return (fdot(n, ap) - fmaxf(0.f, fmaxf(fdot(n, ab), fdot(n, ac)))) / nn;
 }
 
+// Whether a point that PointToTri (dcollid3d.cpp:778-922) calls a hit is
+// certainly near the triangle, as every bound here assumes. Its coordinates
+// come from det = |a|^2 |b|^2 - (a . b)^2 of two edges a, b: with u = 2^-53,
+// det and the numerators round by at most 15 u |a|^2 |b|^2 (and |q| / |a| or
+// |q| / |b| times that, q the point from the edges' corner), so a hit lies
+// within r (2 |q| + 3 S) of where its coordinates put it, r = 15 u |a|^2
+// |b|^2 / det and S the longest edge. The reach allows 2^-7 of the box's
+// extents and 2^-10 of h, which holds for r <= 2^-12:
+//  - extents up to 0.35 in all (|a| |b| <= 0.35^2), where the test's own cut
+//    det >= 1000 MACH_EPS gives r < 2^-13; or
+//  - an area |a x b| of at least 2^-16 of the extents squared: r < 2^-16.
+// Of a thinner large triangle the test may call a point several lengths away
+// a hit. ab, ac: its edges, up to err of them off at some time in the window;
+// ext: its box's extents over the window, a bound on each edge.
+__device__ __forceinline__ bool area_near(float area, float ext, float err) {
+    return ext <= 0.35f || area - 4.0f * ext * err > ext * ext * 0x1p-16f;
+}
+__device__ __forceinline__ bool tri_near(F3 ab, F3 ac, float ext, float err) {
+    return area_near(fnorm(fcross(ab, ac)), ext, err);
+}
+// err for points rounded to FP32 of magnitude up to M, whose velocities V
+// differ by D at most and have magnitude up to Vm.
+__device__ __forceinline__ float edge_error(float ext, float M, float D, float Vm, float dt32) {
+    return (M + ext) * 0x1p-20f + dt32 * (D + Vm * 0x1p-18f) * 1.001f;
+}
+
 // Whether the static test at time t of a moving one certainly misses, in FP32
 // on the points' positions x and velocities v from the first point's (cut
 // from their FP64 differences, so that the error is relative to the
@@ -672,6 +701,7 @@ __device__ __forceinline__ bool misses_at(const F3* x, const F3* v, float t, flo
                           (fmaxf(0.f, fmaxf(P[1].y, P[2].y)) - fminf(0.f, fminf(P[1].y, P[2].y))) +
                           (fmaxf(0.f, fmaxf(P[1].z, P[2].z)) - fminf(0.f, fminf(P[1].z, P[2].z)));
         reach = h * 1.001f + (ext * 1.001f + S * 0x1p-16f) * (8.0f * eps + 0x1p-10f) * 1.001f;
+        if (!tri_near(P[1], P[2], ext * 1.001f + S * 0x1p-16f, S * 0x1p-18f)) return false;
     }
     return gap - (S * 0x1p-15f + 8.0f * slack) > reach;
 }
@@ -719,6 +749,21 @@ __device__ __forceinline__ bool static_test(const NarrowCtx& c, CallState& st, c
     return EE ? edge_to_edge(c, st, pts, X, c.p.thickness) : point_to_tri(c, st, pts, X, c.p.thickness);
 }
 
+// tri_near of points a, b, c on the filters' FP32 data (v32 null: at rest).
+// Only large triangles come here.
+static __device__ bool points_near(const float4* p32, const float4* v32, int a, int b, int c, float ext,
+                                   float dt32) {
+    const F3 x0 = f3(p32[a]), x1 = f3(p32[b]), x2 = f3(p32[c]);
+    float D = 0.f, Vm = 0.f;
+    if (v32) {
+        const F3 v0 = f3(v32[a]), v1 = f3(v32[b]), v2 = f3(v32[c]);
+        D = fmaxf(fnorm(fsub(v1, v0)), fnorm(fsub(v2, v0)));
+        Vm = fmaxf(fmaxabs(v0), fmaxf(fmaxabs(v1), fmaxabs(v2)));
+    }
+    const float M = fmaxf(fmaxabs(x0), fmaxf(fmaxabs(x1), fmaxabs(x2)));
+    return tri_near(fsub(x1, x0), fsub(x2, x0), ext, edge_error(ext, M, D, Vm, dt32));
+}
+
 // Mixed-precision filter. Every position an FP64 test evaluates lies in its
 // point's box (x_old and x_old + dt*avgVel, both rounded outward to FP32):
 // the roots are in [0, dt] and x_old + t*avgVel rounds monotonically in t.
@@ -728,10 +773,9 @@ __device__ __forceinline__ bool static_test(const NarrowCtx& c, CallState& st, c
 //  - Point-triangle (dcollid3d.cpp:778-922): a hit needs the point within h
 //    of the plane and barycentric coordinates in [-eps, 1+eps], so its
 //    projection is within 4*eps*diameter of the triangle. The computed
-//    coordinates carry a solve error of about 1e-16/sin^2 of the smallest
-//    angle, which the reference's determinant cut (|det| >= 1000*MACH_EPS)
-//    keeps below 2^-10 for triangles up to unit size: the reach is padded by
-//    (8*eps + 2^-10) times the triangle's box extent.
+//    coordinates carry a solve error; where tri_near holds, the reach padded
+//    by (8*eps + 2^-10) times the triangle's box extent covers it, and no
+//    other triangle is filtered.
 // When the padded boxes do not overlap, the FP64 test returns false and is
 // skipped; every other sub-test runs unchanged, so the results are the plain
 // FP64 path's.
@@ -795,14 +839,15 @@ __device__ __forceinline__ bool mixed_may_hit(const NarrowCtx& c, const int* pts
 //    corners), dt*(D1 + D2) with D the largest |v - v_ref| of each side.
 // A hit needs the distance within reach: for PT the plane distance <= h and
 // barycentric coordinates >= -eps - dw (dw <= 2^-10, the solve error the
-// box stage allows too) put the point within h + 6*(eps + dw)*diam of the
-// triangle (padded to 8*(eps + 2^-10)*ext); for EE the clamped closest
+// box stage allows too; see tri_near) put the point within h + 6*(eps +
+// dw)*diam of the triangle (padded to 8*(eps + 2^-10)*ext); for EE the clamped closest
 // points within h are points of the segments, so the segments are within
 // h + 2^-20*ext. Sub-tests whose bound exceeds the reach return false in
 // FP64 too and are skipped.
 // On given points (rounded to FP32, or cut to it by cut32, which is within
 // the same bound) and velocities; ext, extb: the extents of the elements'
 // boxes over the window.
+// (The caller has seen to tri_near.)
 template <bool MOVING, bool EE>
 __device__ __forceinline__ bool gap_may_hit(const F3* X, const F3* V, float ext, float extb, float hpad, float epad,
                                             float dt32) {
@@ -837,6 +882,71 @@ __device__ __forceinline__ bool gap_may_hit(const F3* X, const F3* V, float ext,
     return !(bound > reach);
 }
 
+// h as the filters take it: rounded up, with 2^-10 of it for the error of a
+// hit's coordinates where h is much larger than the triangle (tri_near).
+__device__ __forceinline__ float filter_reach(double h) { return cut32_up(h) * (1.0f + 0x1p-10f); }
+
+// The extents of n points' box over the window, for gap_may_hit.
+template <bool MOVING>
+__device__ __forceinline__ float swept_extent(const F3* X, const F3* V, int n, float dt) {
+    F3 lo = X[0], hi = X[0];
+    auto take = [&](F3 p) {
+        lo = F3{fminf(lo.x, p.x), fminf(lo.y, p.y), fminf(lo.z, p.z)};
+        hi = F3{fmaxf(hi.x, p.x), fmaxf(hi.y, p.y), fmaxf(hi.z, p.z)};
+    };
+    for (int i = 0; i < n; ++i) {
+        take(X[i]);
+        if (MOVING) take(fadd(X[i], fscale(V[i], dt)));
+    }
+    const F3 d = fsub(hi, lo);
+    return (d.x + d.y + d.z) * 1.001f;
+}
+
+// The gap bound of one sub-test on its points cut to FP32 (plain passes).
+template <bool MOVING>
+__device__ __forceinline__ bool plain_may_hit(const double4_32a* __restrict__ xo, const double4_32a* __restrict__ av,
+                                              const int* pts, bool ee, const Params& prm) {
+    const float dt32 = cut32_up(prm.dt);
+    F3 X[4], V[4];
+    for (int q = 0; q < 4; ++q) {
+        double x[3];
+        load3(xo, pts[q], x);
+        X[q] = cut_f3(x);
+        if (MOVING) {
+            load3(av, pts[q], x);
+            V[q] = cut_f3(x);
+        }
+    }
+    float hpad = filter_reach(MOVING ? prm.eps : prm.thickness), epad = cut32_up(prm.eps);
+    const float most = fmaxf(fmaxf(fmaxabs(X[0]), fmaxabs(X[1])), fmaxf(fmaxabs(X[2]), fmaxabs(X[3])));
+    if (most * 0x1p-13f > fmaxabs(fsub(X[1], X[0]))) {
+        // far from the origin for its size: positions from the first
+        // point's, and the tests' own rounding on the reach
+        double x0[3], x[3];
+        load3(xo, pts[0], x0);
+        X[0] = F3{0.f, 0.f, 0.f};
+        for (int q = 1; q < 4; ++q) {
+            load3(xo, pts[q], x);
+            for (int k = 0; k < 3; ++k) x[k] -= x0[k];
+            X[q] = cut_f3(x);
+        }
+        hpad += most * 0x1p-44f;
+    }
+    const int na = ee ? 2 : 3;
+    const float ext = swept_extent<MOVING>(X, V, na, dt32);
+    const float extb = swept_extent<MOVING>(X + na, V + na, 4 - na, dt32);
+    if (ee) return gap_may_hit<MOVING, true>(X, V, ext, extb, hpad, epad, dt32);
+    if (ext > 0.35f) {
+        float M = 0.f, D = 0.f, Vm = 0.f;
+        for (int q = 0; q < 3; ++q) {
+            M = fmaxf(M, fmaxabs(X[q]));
+            if (MOVING) Vm = fmaxf(Vm, fmaxabs(V[q])), D = fmaxf(D, fnorm(fsub(V[q], V[0])));
+        }
+        if (!tri_near(fsub(X[1], X[0]), fsub(X[2], X[0]), ext, edge_error(ext, M, D, Vm, dt32))) return true;
+    }
+    return gap_may_hit<MOVING, false>(X, V, ext, extb, hpad, epad, dt32);
+}
+
 template <bool MOVING, bool EE>
 __device__ __forceinline__ bool sat_may_hit(const NarrowCtx& c, const int* pts, float ext, float extb) {
     F3 X[4], V[4];
@@ -844,10 +954,6 @@ __device__ __forceinline__ bool sat_may_hit(const NarrowCtx& c, const int* pts, 
     if (MOVING)
         for (int q = 0; q < 4; ++q) V[q] = f3(c.v32[pts[q]]);
     return gap_may_hit<MOVING, EE>(X, V, ext, extb, c.hpad, c.epad, c.dt32);
-}
-
-__device__ __forceinline__ F3 fcross(F3 a, F3 b) {
-    return F3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 
 // Element-pair stage of the mixed-precision filter: one lower bound on the
@@ -861,9 +967,9 @@ __device__ __forceinline__ F3 fcross(F3 a, F3 b) {
 // those separates them), for two segments their common normal and the
 // in-plane normals of each, and the line between the centroids.
 // Gap between the projections of two point sets (3 points each) onto ax,
-// divided by |ax|: a lower bound on their distance (-1 for a zero axis).
-__device__ __forceinline__ float axis_gap(F3 ax, const F3* R) {
-    float an = fnorm(ax);
+// divided by |ax| (an): a lower bound on their distance (-1 for a zero axis).
+__device__ __forceinline__ float axis_gap(F3 ax, const F3* R, float& an) {
+    an = fnorm(ax);
     if (!(an > 0.f)) return -1.f;
     float amin = fdot(ax, R[0]), amax = amin, bmin = fdot(ax, R[3]), bmax = bmin;
 #pragma unroll
@@ -878,10 +984,13 @@ __device__ __forceinline__ float axis_gap(F3 ax, const F3* R) {
 }
 
 // The pair's decision from the gap lb: ia, ib its points (a segment's last
-// one twice), L and M bounds of their distances and coordinates.
+// one twice), L and M bounds of their distances and coordinates, areaA and
+// areaB the lengths of the triangles' normals. kPairThin: it holds a triangle
+// outside tri_near, whose point-triangle sub-tests no bound rules out.
+enum PairBound { kPairFar = 0, kPairNear = 1, kPairThin = 2 };
 template <bool MOVING>
-__device__ __forceinline__ bool pair_bound_may_hit(const NarrowCtx& c, const int* ia, int na, const int* ib, int nb,
-                                                   float lb, float L, float M) {
+__device__ __forceinline__ int pair_bound(const NarrowCtx& c, const int* ia, int na, const int* ib, int nb, float lb,
+                                          float L, float M, float areaA, float areaB) {
     // the largest reach of the pair's sub-tests, with the boxes' extents
     float extA, extB;
     {
@@ -913,9 +1022,10 @@ __device__ __forceinline__ bool pair_bound_may_hit(const NarrowCtx& c, const int
     float reach = __fadd_ru(c.hpad, fmaxf(reach_pt, reach_ee));
     float err = __fmul_ru(32.0f * 0x1p-24f, __fadd_ru(L, M));
     float bound = __fsub_rd(lb, err);
+    float DA = 0.f, DB = 0.f, Vm = 0.f;  // (DB from A's first point)
     if (MOVING) {
         F3 v0 = f3(c.v32[ia[0]]);
-        float DA = 0.f, DB = 0.f, Vm = fmaxabs(v0);
+        Vm = fmaxabs(v0);
 #pragma unroll
         for (int q = 1; q < 3; ++q) {
             F3 v = f3(c.v32[ia[q]]);
@@ -931,11 +1041,16 @@ __device__ __forceinline__ bool pair_bound_may_hit(const NarrowCtx& c, const int
         float dv = __fadd_ru(__fmul_ru(__fadd_ru(DA, DB), 1.0f + 0x1p-16f), __fmul_ru(Vm, 32.0f * 0x1p-24f));
         bound = __fsub_rd(bound, __fmul_ru(c.dt32, dv));
     }
-    return !(bound > reach);
+    if (ext_tri > 0.35f) {
+        if (na == 3 && extA > 0.35f && !area_near(areaA, extA, edge_error(extA, M, DA, Vm, c.dt32))) return kPairThin;
+        if (nb == 3 && extB > 0.35f && !area_near(areaB, extB, edge_error(extB, M, 2.0f * DB, Vm, c.dt32)))
+            return kPairThin;
+    }
+    return bound > reach ? kPairFar : kPairNear;
 }
 
 template <bool MOVING>
-__device__ __forceinline__ bool pair_may_hit(const NarrowCtx& c, const int* A, int na, const int* B, int nb) {
+__device__ __forceinline__ int pair_may_hit(const NarrowCtx& c, const int* A, int na, const int* B, int nb) {
     // points relative to A's first; a segment's third point repeats its
     // second (the same convex hull, so the same projections)
     const int ia[3] = {A[0], A[1], na == 3 ? A[2] : A[1]};
@@ -950,38 +1065,39 @@ __device__ __forceinline__ bool pair_may_hit(const NarrowCtx& c, const int* A, i
         R[q] = fsub(x, X0);
         L = fmaxf(L, fnorm(R[q]));
     }
-    float lb = -1.f;
+    float lb = -1.f, an, area[2];
     {
         F3 cA = fscale(fadd(fadd(R[0], R[1]), R[2]), 1.f / 3.f);
         F3 cB = fscale(fadd(fadd(R[3], R[4]), R[5]), 1.f / 3.f);
-        lb = fmaxf(lb, axis_gap(fsub(cB, cA), R));
+        lb = fmaxf(lb, axis_gap(fsub(cB, cA), R, an));
     }
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
         const F3* P = R + 3 * side;
         F3 e0 = fsub(P[1], P[0]), e1 = fsub(P[2], P[1]), e2 = fsub(P[0], P[2]);
         F3 nrm = fcross(e0, fsub(P[2], P[0]));  // zero for a segment: skipped
-        lb = fmaxf(lb, axis_gap(nrm, R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, e0), R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, e1), R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, e2), R));
+        lb = fmaxf(lb, axis_gap(nrm, R, area[side]));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, e0), R, an));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, e1), R, an));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, e2), R, an));
     }
     {
         F3 d1 = fsub(R[1], R[0]), d2 = fsub(R[4], R[3]);
         F3 nrm = fcross(d1, d2);
-        lb = fmaxf(lb, axis_gap(nrm, R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, d1), R));
-        lb = fmaxf(lb, axis_gap(fcross(nrm, d2), R));
+        lb = fmaxf(lb, axis_gap(nrm, R, an));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, d1), R, an));
+        lb = fmaxf(lb, axis_gap(fcross(nrm, d2), R, an));
     }
-    return pair_bound_may_hit<MOVING>(c, ia, na, ib, nb, lb, L, M);
+    return pair_bound<MOVING>(c, ia, na, ib, nb, lb, L, M, area[0], area[1]);
 }
 
 template <bool MOVING, bool EE>
 __device__ __forceinline__ bool sub_test(const NarrowCtx& c, CallState& st, const int* pts) {
     if (c.pbox_lo) {
         float ext, extb;
-        if (!mixed_may_hit(c, pts, EE, &ext, &extb)) return false;
-        if (!sat_may_hit<MOVING, EE>(c, pts, ext, extb)) return false;
+        const bool out = !mixed_may_hit(c, pts, EE, &ext, &extb) || !sat_may_hit<MOVING, EE>(c, pts, ext, extb);
+        if (out && (EE || ext <= 0.35f || points_near(c.p32, MOVING ? c.v32 : nullptr, pts[0], pts[1], pts[2], ext, c.dt32)))
+            return false;
     }
     st.nsub++;
     if (MOVING) return moving_test<EE>(c, st, pts);
