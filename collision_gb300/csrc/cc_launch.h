@@ -484,6 +484,7 @@ struct SweepElem {
 // element's record of the step, levels of records staged ahead.
 constexpr int kSweepSlotBytes = 48, kSweepRecBytes = 80, kSweepRing = 8;
 constexpr int kSweepMaxEpoch = 4;
+constexpr int kSweepPolls = 1 << 21;  // about a second
 constexpr size_t kSweepMaxBytes = 224 * 1024;    // within the 227 KB a CTA may hold
 constexpr size_t kSweepSharedBytes = 110 * 1024;  // lets two CTAs share an SM
 inline size_t sweep_smem(int slots, int width, int ring) {
@@ -520,6 +521,7 @@ struct StrainPlan {
     bool any_global;   // some scene is swept by k_strain
     int workers;       // warps taking a level's elements
     size_t smem;       // dynamic shared memory of a sweep CTA
+    int polls;         // polls without progress before a sweep gives up on those before it
 };
 size_t strain_edge_step_bytes(int nedges);
 int strain_state_ints(int nscenes);

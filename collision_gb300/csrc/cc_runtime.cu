@@ -444,6 +444,7 @@ struct cc_solver {
     bool split_narrow = true;  // staged narrow phase
     bool strain_warp = false;  // a sweep CTA's elements on one warp
     bool strain_roles = true;  // CC_TUNE_STRAIN_ROLES, without effect
+    int strain_wait = kSweepPolls;  // CC_TUNE_STRAIN_WAIT
     LaunchTuning tune;
     int host_threads = 0;  // tree emulation threads (0: hardware concurrency)
     const bool pass_log = std::getenv("CC_PASS_LOG") != nullptr;
@@ -815,7 +816,7 @@ struct cc_solver {
     // strain settings, then replayed.
     struct TailGraph {
         const void* key[4];
-        int block, window, warp;
+        int block, window, warp, wait;
         cudaGraphExec_t exec;
         long long launches;
     };
@@ -830,7 +831,7 @@ struct cc_solver {
         TailGraph* hit = nullptr;
         for (auto& g : tail_graphs)
             if (std::equal(key, key + 4, g.key) && g.block == tune.strain_block && g.window == (int)strain_window &&
-                g.warp == (int)strain_warp) {
+                g.warp == (int)strain_warp && g.wait == strain_wait) {
                 hit = &g;
                 break;
             }
@@ -853,6 +854,7 @@ struct cc_solver {
             tg.block = tune.strain_block;
             tg.window = (int)strain_window;
             tg.warp = (int)strain_warp;
+            tg.wait = strain_wait;
             tg.launches = n;
             e = cudaGraphInstantiate(&tg.exec, g, 0);
             cudaGraphDestroy(g);
@@ -914,7 +916,7 @@ struct cc_solver {
     }
 
     StrainPlan strain_plan() const {
-        StrainPlan pl{strain_window, false, 1, 0};
+        StrainPlan pl{strain_window, false, 1, 0, strain_wait};
         int width = 1;
         for (int s = 0; s < nscenes; ++s) {
             const SceneDev& sd = h_scenes[s];
@@ -2273,6 +2275,8 @@ cc_status cc_solver::resolve_impl(const double* x_old, const double* x_cand, dou
                         stream);
     }
     if (cudaStreamSynchronize(stream) != cudaSuccess) return cuda_check("finalize");
+    for (int s = 0; s < nscenes; ++s)
+        if (h_strain_passes[3 * s] < 0) return fail(CC_CUDA_ERROR, "strain sweeps gave up waiting for one another");
     // updateFinalForRG (dcollid.cpp:626-675): a body with a collided point
     // takes that point's velocity, and its centre of mass moves from the
     // remembered one (if that point is the body's first) or the current one
@@ -2298,8 +2302,6 @@ cc_status cc_solver::resolve_impl(const double* x_old, const double* x_cand, dou
         }
         std::copy(B.com, B.com + 3, B.mrg_com);
     }
-    for (int s = 0; s < nscenes; ++s)
-        if (h_strain_passes[3 * s] < 0) return fail(CC_CUDA_ERROR, "strain sweeps gave up waiting for one another");
     for (int s = 0; s < nscenes; ++s) {
         // algorithmic bytes of the sweep: per pass, each edge's 48-byte
         // record and one 32-byte read and write of each point it touches
@@ -2780,6 +2782,10 @@ cc_status cc_set_tuning(cc_solver* s, int knob, int value) {
             s->zb.replay_cta_min = value;
             s->loop_dirty = true;
             return CC_OK;
+        case CC_TUNE_STRAIN_WAIT:
+            if (value < 0 || value > kSweepPolls) return CC_BAD_INPUT;
+            s->strain_wait = value;
+            return CC_OK;
         case CC_TUNE_SUBTEST_MERGE:
             s->sub_merge = value != 0;
             s->loop_dirty = true;
@@ -2848,6 +2854,7 @@ int cc_get_tuning(cc_solver* s, int knob) {
         case CC_TUNE_REFIT_UP: return s->refit_up ? 1 : 0;
         case CC_TUNE_ZONE_FEW: return s->zb.zone_few;
         case CC_TUNE_SUBTEST_MERGE: return s->sub_merge ? 1 : 0;
+        case CC_TUNE_STRAIN_WAIT: return s->strain_wait;
         case CC_TUNE_STACK_DEPTH: return s->tune.stack_depth;
         case CC_TUNE_PAIR_CAPACITY: return s->pair_cap;
         default: return -1;

@@ -541,9 +541,7 @@ constexpr int kSweepWorkers = 16;                // most warps taking a level's 
 constexpr int kSweepHelpers = 4;                 // warps for copy-ins and write-backs
 constexpr int kSweepService = kSweepHelpers + 3; // with the record, the publishing and the polling warp
 constexpr int kSweepStop = 1 << 30;  // progress of a sweep after which nothing changes (or that failed)
-// polls without progress (about half a microsecond each) before a sweep
-// gives up on the one before, and tries before a level's records are given up
-constexpr int kSweepPolls = 1 << 21;
+// Tries (about 50 ns each) before a level's records are given up.
 constexpr int kSweepTries = 1 << 16;
 
 struct SweepArgs {
@@ -563,6 +561,7 @@ struct SweepArgs {
     int* stat;      // per scene and sweep: averaged edges, exact tests
     int* failed;    // per scene
     int workers;    // worker warps of the block
+    int polls;      // polls without progress before a sweep gives up on the one before (kSweepPolls)
 };
 
 // One CTA per scene and sweep. The sweeps of a scene are a pipeline through
@@ -575,7 +574,8 @@ struct SweepArgs {
 //
 // CTAs take (scene, sweep) pairs from a ticket counter, a scene's sweeps in
 // order, so a CTA waits only for one that has already started. The wait is
-// bounded (kSweepPolls); after it the sweep and its successors end and the
+// bounded (kSweepPolls). A sweep that gives up, or finds a level's records
+// missing, ends at the end of its step in all its warps together, and the
 // scene is reported as failed.
 //
 // What bounds a level is its chain: barrier, slot loads, three FP32
@@ -591,7 +591,7 @@ struct SweepArgs {
 // before, both at their own pace through flags in shared memory.
 //
 // Slots are for a point's live time only (cc_sweep_plan.h): a 129 x 129
-// sheet takes 1,074 slots and 107 KB with its record ring.
+// sheet takes 903 slots and 96 KB with its record ring.
 //
 // Measured (strain loop of one step, ten sweeps; before: one CTA per scene,
 // sweep after sweep, edges on levels of their own): folded 129 x 129 sheet
@@ -641,15 +641,17 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
         const double dt = sd.p.dt;
         const float dt32 = (float)dt;
         int n_avg = 0, n_exact = 0;
-        // the level's first element and count (x < 0: waited in vain, the
-        // sweep fails)
+        // the level's first element and count; none for a warp that waits in
+        // vain: its lanes decide as one, and it goes on meeting the barriers
+        // until the sweep ends (the vote goes while the level is loaded)
         auto level = [&](int l) {
-            for (int tries = 0; !mbar_try(&s_full[l % kSweepRing], (l / kSweepRing) & 1);)
-                if (++tries > kSweepTries) {
-                    s_fail = 1;
-                    return make_int2(0, 0);
-                }
-            return s_level[l % kSweepRing];
+            bool got = false;
+            for (int tries = 0; !got && tries < kSweepTries; ++tries)
+                got = mbar_try(&s_full[l % kSweepRing], (l / kSweepRing) & 1);
+            const int2 lv = s_level[l % kSweepRing];
+            const bool ok = __all_sync(0xffffffffu, got);
+            if (!ok) flag_store(&s_fail, 1);
+            return make_int2(ok ? lv.x : 0, ok ? lv.y : 0);
         };
         auto record = [&](int l, int2 lv, int i, SweepLane& r) {
             const int k = i < lv.y ? i : 0;  // lanes without an element read the level's first
@@ -757,7 +759,7 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
                 SweepSlot& w = win[ps.y];
                 *reinterpret_cast<float4*>(w.f) = cut32x3(w.d[0], w.d[1], w.d[2]);
             }
-            if (h == 0) s_stop[t & 1] = seen >= kSweepStop ? 1 : 0;
+            if (h == 0) s_stop[t & 1] = seen >= kSweepStop || flag_load(&s_fail) ? 1 : 0;
             bar_sync(2, stepped);
             if (s_stop[t & 1]) break;
             out = cur;
@@ -845,8 +847,8 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
                 flag_store(&s_seen, now);
                 seen = now;
                 polls = 0;
-            } else if (++polls > kSweepPolls) {
-                s_fail = 1;
+            } else if (++polls > A.polls) {
+                flag_store(&s_fail, 1);
                 flag_store(&s_seen, kSweepStop);
                 break;
             } else {
@@ -933,7 +935,7 @@ void strain_limit(const StrainBufs& b, const SceneDev* scenes, int nscenes, cons
     check(0);
     if (plan.window) {
         SweepArgs a{b.elems, recs, b.lev, b.epoch, b.need, b.load, b.wb, scenes, b.order, xo, av, b.flags,
-                    ticket, progress, stat, failed, plan.workers};
+                    ticket, progress, stat, failed, plan.workers, plan.polls};
         count_launch(), k_strain_sweeps<<<nscenes * kStrainMaxIter, (plan.workers + kSweepService) * 32, plan.smem,
                                           s>>>(a);
         count_launch(), k_sweep_count<<<nblk(nscenes, 128), 128, 0, s>>>(scenes, nscenes, b.flags, stat, failed,

@@ -307,6 +307,10 @@ cc_status cc_set_scene_enabled(cc_solver* s, int scene, int on);
  *                           sub-test where there are at most 1,216 (larger
  *                           passes: blocks of one kind each); 0: always such
  *                           blocks, a thread per sub-test. Same results
+ *   CC_TUNE_STRAIN_WAIT     0..2^21 (default): times a strain sweep looks for
+ *                           the sweeps before it to move before it gives up
+ *                           (about a second) and the call returns
+ *                           CC_CUDA_ERROR; the solver stays usable
  * cc_get_tuning returns the current value, or -1 for an unknown knob. */
 enum {
     CC_TUNE_SPLIT_NARROW = 0,
@@ -334,7 +338,8 @@ enum {
     CC_TUNE_REPLAY_CTA_MIN = 22,
     CC_TUNE_REFIT_UP = 23,
     CC_TUNE_ZONE_FEW = 24,
-    CC_TUNE_SUBTEST_MERGE = 25
+    CC_TUNE_SUBTEST_MERGE = 25,
+    CC_TUNE_STRAIN_WAIT = 26
 };
 cc_status cc_set_tuning(cc_solver* s, int knob, int value);
 int cc_get_tuning(cc_solver* s, int knob);
