@@ -541,8 +541,11 @@ constexpr int kSweepWorkers = 16;                // most warps taking a level's 
 constexpr int kSweepHelpers = 4;                 // warps for copy-ins and write-backs
 constexpr int kSweepService = kSweepHelpers + 3; // with the record, the publishing and the polling warp
 constexpr int kSweepStop = 1 << 30;  // progress of a sweep after which nothing changes (or that failed)
-// Tries (about 50 ns each) before a level's records are given up.
+// Tries (about 50 ns each) before a level's records are given up; and tries
+// (100 ns and more) of the warp that brings them while neither the workers
+// nor any earlier sweep move, several times what the polls take to notice.
 constexpr int kSweepTries = 1 << 16;
+constexpr int kSweepRecordTries = 1 << 26;
 
 struct SweepArgs {
     const SweepElem* elems;
@@ -561,7 +564,7 @@ struct SweepArgs {
     int* stat;      // per scene and sweep: averaged edges, exact tests
     int* failed;    // per scene
     int workers;    // worker warps of the block
-    int polls;      // polls without progress before a sweep gives up on the one before (kSweepPolls)
+    int polls;      // polls without progress before a sweep gives up on the ones before (kSweepPolls)
 };
 
 // One CTA per scene and sweep. The sweeps of a scene are a pipeline through
@@ -574,9 +577,11 @@ struct SweepArgs {
 //
 // CTAs take (scene, sweep) pairs from a ticket counter, a scene's sweeps in
 // order, so a CTA waits only for one that has already started. The wait is
-// bounded (kSweepPolls). A sweep that gives up, or finds a level's records
-// missing, ends at the end of its step in all its warps together, and the
-// scene is reported as failed.
+// bounded: a sweep gives up when none of those before it has moved for
+// kSweepPolls polls (on a closed string the sweeps follow one another whole,
+// so the one before may itself be waiting). A sweep that gives up, or finds a
+// level's records missing, ends at the end of its step in all its warps
+// together, and the scene is reported as failed.
 //
 // What bounds a level is its chain: barrier, slot loads, three FP32
 // decisions, and where an edge averages its FP64 sums (~64 cycles each on
@@ -605,12 +610,13 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
     __shared__ int s_ticket, s_avg, s_exact, s_fail;
     __shared__ int s_stop[2];             // step t's in s_stop[t & 1]: everyone ends after it
     __shared__ int s_seen, s_wrote, s_quit;  // epochs the sweep before has published; helper warps' write-back steps
+    __shared__ int s_moves;                  // times an earlier sweep was seen to move while the one before did not
     __shared__ unsigned long long s_full[kSweepRing], s_empty[kSweepRing];  // the record ring's levels
     __shared__ int2 s_level[kSweepRing];  // their first elements and counts
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         s_ticket = atomicAdd(A.ticket, 1);
-        s_avg = s_exact = s_fail = s_stop[0] = s_stop[1] = s_wrote = s_quit = 0;
+        s_avg = s_exact = s_fail = s_stop[0] = s_stop[1] = s_wrote = s_quit = s_moves = 0;
         // the first sweep waits for nothing
         s_seen = s_ticket % kStrainMaxIter == 0 ? kSweepStop - 1 : 0;
         for (int i = 0; i < kSweepRing; ++i) {
@@ -815,13 +821,17 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
             const int slot = l % kSweepRing;
             bool go = true;
             if (l >= kSweepRing)
-                for (int tries = 0; !mbar_try(&s_empty[slot], (l / kSweepRing - 1) & 1);)
-                    if (flag_load(&s_quit) || ++tries > kSweepPolls) {  // (the workers may wait for another sweep)
+                for (int tries = 0, last = 0; !mbar_try(&s_empty[slot], (l / kSweepRing - 1) & 1);) {
+                    // (the workers may wait for another sweep, and that one for others)
+                    const int moved = flag_load(&s_seen) + flag_load(&s_moves);
+                    if (moved != last) tries = 0;
+                    last = moved;
+                    if (flag_load(&s_quit) || ++tries > kSweepRecordTries) {
                         go = false;
                         break;
-                    } else {
-                        __nanosleep(100);
                     }
+                    __nanosleep(100);
+                }
             if (!__all_sync(0xffffffffu, go)) break;
             if (lane == 0) {
                 s_level[slot] = make_int2(o0, n);
@@ -840,7 +850,8 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
         return;
     }
     // ---- follows the sweep before
-    if (lane == 0 && k > 0)
+    if (lane == 0 && k > 0) {
+        unsigned others = 0;  // epochs of the sweeps before that one
         for (int seen = 0, polls = 0; seen < E && !flag_load(&s_quit);) {
             const int now = ld_acquire(mine - 1);
             if (now > seen) {
@@ -848,13 +859,21 @@ __global__ void __launch_bounds__((kSweepWorkers + kSweepService) * 32) k_strain
                 seen = now;
                 polls = 0;
             } else if (++polls > A.polls) {
-                flag_store(&s_fail, 1);
-                flag_store(&s_seen, kSweepStop);
-                break;
+                unsigned sum = 0;  // (an ended sweep's kSweepStop cut so that nine fit)
+                for (int j = 2; j <= k; ++j) sum += (unsigned)min(ld_acquire(mine - j), kSweepStop >> 2);
+                if (sum == others) {
+                    flag_store(&s_fail, 1);
+                    flag_store(&s_seen, kSweepStop);
+                    break;
+                }
+                others = sum;
+                polls = 0;
+                flag_add(&s_moves, 1);
             } else {
                 __nanosleep(40);
             }
         }
+    }
     bar_sync(3, all);
 }
 

@@ -1,7 +1,7 @@
-"""A strain sweep whose wait for the one before runs out ends the call with an
-error and leaves the solver usable. The scene is a closed string, whose first
+"""The strain sweeps' waits for one another: a closed string, whose first
 point's last element is its last, so that every sweep waits for the whole of
-the one before."""
+the one before while that one waits for others; and a wait that runs out,
+which ends the call with an error and leaves the solver usable."""
 import numpy as np
 import pytest
 
@@ -28,6 +28,25 @@ def _loop(n, dt=1e-3):
 
 def _step(s, sc):
     return s.resolveCollision(sc.x, scenes.candidate(sc, sc.x, sc.v), sc.v, np.zeros(sc.nv, np.uint8))
+
+
+# 2,000 polls are about a millisecond: a sweep of 20,000 levels takes a dozen
+@pytest.mark.parametrize("n,wait", [(3, None), (100, None), (20000, None), (20000, 2000)])
+def test_closed_string_equals_global_path(n, wait):
+    from collision_gb300.solver import CollisionSolver3d
+    sc = _loop(n)
+    got = []
+    for window in (True, False):
+        s = CollisionSolver3d(0)
+        s.assembleFromScene(sc)
+        s.setStrainWindow(window)
+        if wait:
+            s.setTuning(s.TUNE_STRAIN_WAIT, wait)
+        got.append((_step(s, sc), s.counters()["strain_averaged"]))
+        s.close()
+    assert got[0][1] == got[1][1] and (got[0][1] > 0 or n < 100)
+    for a, b in zip(got[0][0], got[1][0]):
+        assert np.array_equal(a, b)
 
 
 def test_wait_that_runs_out():
