@@ -985,6 +985,12 @@ struct cc_solver {
     }
 
     cc_status assemble(const cc_mesh* meshes, int n);
+    cc_status fill_mesh(const cc_mesh* meshes, int n, int tot_v, int tot_e);
+    // the last assemble call failed after the mesh before it was released
+    bool assemble_failed = false;
+    cc_status check_mesh() {
+        return assemble_failed ? fail(CC_BAD_INPUT, "no mesh: the last assemble call failed") : CC_OK;
+    }
     cc_status resolve(const double* x_old, const double* x_cand, double* vel, uint8_t* hc, double* x_out,
                       int* has_collision);
     cc_status resolve_impl(const double* x_old, const double* x_cand, double* vel, uint8_t* hc, double* x_out,
@@ -1013,9 +1019,16 @@ cc_status cc_solver::assemble(const cc_mesh* meshes, int n) {
     if (tot_v >= kMaxTotal || tot_e >= kMaxTotal) return fail(CC_BAD_INPUT, "more than 2^28 points or elements");
     cudaSetDevice(device);
     release_mesh();
+    const cc_status st = fill_mesh(meshes, n, (int)tot_v, (int)tot_e);
+    assemble_failed = st != CC_OK;
+    if (assemble_failed) release_mesh();  // no half of a mesh is left to be stepped
+    return st;
+}
+
+cc_status cc_solver::fill_mesh(const cc_mesh* meshes, int n, int tot_v, int tot_e) {
     nscenes = n;
-    nv = (int)tot_v;
-    ne = (int)tot_e;
+    nv = tot_v;
+    ne = tot_e;
     scenes.resize((size_t)n);
     h_scenes.assign((size_t)n, SceneDev{});
     std::vector<int> ev((size_t)ne * 3, -1), esurf((size_t)ne, -1), vscene((size_t)nv), escene((size_t)ne);
@@ -2137,6 +2150,7 @@ cc_status cc_solver::detect_pass(int moving, bool any_zone) {
 
 cc_status cc_solver::resolve(const double* x_old, const double* x_cand, double* vel, uint8_t* hc, double* x_out,
                              int* has_collision) {
+    if (cc_status st = check_mesh()) return st;
     long long l0 = g_kernel_launches;
     cc_status st0 = resolve_impl(x_old, x_cand, vel, hc, x_out, has_collision);
     launches_last = g_kernel_launches - l0;
@@ -2337,6 +2351,7 @@ cc_status cc_solver::check_ccd(const double* x_old, const double* x_new, long lo
     if (hits) *hits = 0;
     if (scene_hits)
         for (int s = 0; s < nscenes; ++s) scene_hits[s] = 0;
+    if (cc_status st = check_mesh()) return st;
     if (ne == 0) return CC_OK;
     upload_scenes();
     count_launch(), k_reset_counters<<<1, 1, 0, stream>>>(d_ctr);
@@ -2409,6 +2424,7 @@ cc_status cc_solver::check_ccd(const double* x_old, const double* x_new, long lo
 // quarter, so that the passes that follow do not overflow and retry.
 cc_status cc_solver::autotune(double* best_ms) {
     if (best_ms) *best_ms = 0.0;
+    if (cc_status st = check_mesh()) return st;
     if (ne == 0) return CC_OK;
     upload_scenes();
     for (int s = 0; s < nscenes; ++s)
