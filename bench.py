@@ -68,20 +68,14 @@ PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 # The traversal's DRAM traffic (bytes read + written) per query leaf and
 # its threads active per instruction, from one ncu capture of each kernel on
 # the batched workload cut to 96 scenes, each a full traversal of all
-# 1,298,248 elements: k_traverse_rope_dyn 257.1 MB and k_traverse_rope
+# 1,298,248 elements: k_traverse_rope_dyn 255.9 MB and k_traverse_rope
 # 215.8 MB (the first traversal of the run, the proximity pass of step 1),
 # k_traverse (a stack per thread) 221 MB (a free-fall step)
-TRAVERSE_DRAM_BYTES_PER_LEAF = {"dyn": 198.0, "rope": 166.2, "stack": 170.4}
-TRAVERSE_LANES_ACTIVE = {"dyn": 7.8, "rope": 6.2, "stack": 7.4}
+TRAVERSE_DRAM_BYTES_PER_LEAF = {"dyn": 197.1, "rope": 166.2, "stack": 170.4}
+TRAVERSE_LANES_ACTIVE = {"dyn": 7.4, "rope": 6.2, "stack": 7.4}
 TRAVERSE_KERNEL = {"dyn": "k_traverse_rope_dyn (LBVH broad phase, stackless, persistent warps refilling lanes)",
                    "rope": "k_traverse_rope (LBVH broad phase, stackless along ropes, one thread per query)",
                    "stack": "k_traverse (LBVH broad phase, a stack per thread)"}
-# FP64 operations (dadd + dmul + 2 dfma) per queued FP64 sub-test, from one
-# ncu capture of both k_subtests launches of a CCD pass of the same 96
-# scenes: 85.6 MFLOP for 123,752 point-triangle and 44,900 edge-edge
-# sub-tests; GB300's FP64 peak is 1.25 TFLOP/s (nominal: none measured)
-SUBTEST_FP64_FLOPS = 507.6
-FP64_PEAK_TFLOPS = 1.25
 # the CCD filter's algorithmic bytes per visited pair: the pair, two ranks,
 # the two elements' point ids, FP32 x_old and avgVel of six points
 FILTER_BYTES_PER_VISIT = 8 + 8 + 24 + 6 * 32
@@ -688,15 +682,12 @@ def run_gpu(args):
         kc, kpr = kp["counters"], kp["prof"]
         t_sub = (kpr.get("loop_subtests", (0.0, 0))[0] + kpr.get("ccd_subtests", (0.0, 0))[0]) / 1e3
         if t_sub > 0 and kc.get("fp64_subtests"):
-            flops = SUBTEST_FP64_FLOPS * kc["fp64_subtests"]
+            # no rate: a queued sub-test ends after its cubic, at an FP32
+            # bound or in the FP64 test, and the counters do not say which
             kern["ccd_subtests"] = {
-                "kernel": "k_subtests (the FP64 sub-tests that pass the FP32 filters, both kinds in one launch)",
-                "bound": "fp64",
-                "flops": flops, "s": t_sub, "achieved_tflops": flops / t_sub / 1e12, "peak_tflops": FP64_PEAK_TFLOPS,
-                "frac": flops / t_sub / 1e12 / FP64_PEAK_TFLOPS, "peak_source": "nominal",
-                "flops_per_subtest": SUBTEST_FP64_FLOPS, "cr_roots": kc.get("cr_roots"),
-                "note": "FP64 pipe 77% busy in the ncu capture: most FP64 issue slots are compares, selects and "
-                        "conversions, run at the FP64 rate"}
+                "kernel": "k_subtests_cubic and k_subtests (the sub-tests that pass the FP32 filters)",
+                "bound": "fp64", "subtests": kc["fp64_subtests"], "s": t_sub,
+                "ns_per_subtest": t_sub * 1e9 / kc["fp64_subtests"], "cubics_with_a_root": kc.get("cr_roots")}
         t_f = kpr.get("loop_filter", (0.0, 0))[0] / 1e3
         if t_f > 0 and kc.get("moving_visits"):
             b = FILTER_BYTES_PER_VISIT * kc["moving_visits"]
