@@ -4,7 +4,8 @@
 // reference's order of evaluation and compiled with --fmad=false, so that
 // each a*b+c rounds twice exactly as the reference's x86 build does; the
 // only results that can differ from the reference are those that pass
-// through acos/cos/pow/sin (CUDA's libdevice versus glibc, an ulp or so).
+// through acos/cos/pow/sin, correctly rounded here (cc_crmath.cuh), where
+// glibc misrounds the argument at hand.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -134,7 +135,6 @@ struct SceneDev {
     int strain_slots;     // shared-memory slots of its window sweep
     int wb_final0, wb_final1;  // write-backs after its last level
     int enabled;          // 0: left out of resolve calls (candidates pass through)
-    int strain_e0, strain_ne;  // its strain edges
     int nt;               // triangles (its first nt elements)
     // schedule of its strain sweeps in shared memory (cc_sweep_plan.h): first
     // level offset, levels, first epoch, epochs, levels per epoch, elements
@@ -177,8 +177,9 @@ struct PassCounters {
     int err;          // ErrBits
     int nvisits;      // narrow-phase calls (pairs not skipped as same-rigid-surface)
     int ncontacts;    // sub-tests that applied an impulse
-    int nsub;         // sub-tests evaluated in FP64 (not rejected by a filter)
-    int ncr;          // coplanarity cubics whose roots were formed again correctly rounded
+    int nsub;         // mixed passes: sub-tests the filters left; plain passes: every sub-test visited, those the
+                      // gap bound rules out among them
+    int ncr;          // coplanarity cubics with a root in the time window
     int nunion;       // union records written (impact-zone passes)
     int nsub_pt;      // point-triangle sub-tests queued by a split pass
     int nsub_ee;      // edge-edge sub-tests queued by a split pass

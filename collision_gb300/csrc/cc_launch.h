@@ -42,9 +42,9 @@ constexpr int kSmallSort = 8192;
 cudaError_t small_sort_ready();  // before the first one-CTA sort: its shared memory
 void sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn, int cap, int bits, void* temp,
                     int* eff, cudaStream_t s, bool small, bool general);
-// Exclusive scan of n ints (out may alias in); total written to *total.
+// Exclusive scan of n ints (out may alias in).
 size_t scan_temp_bytes(int n);
-void exclusive_scan(const int* in, int* out, int n, int* total, void* temp, cudaStream_t s);
+void exclusive_scan(const int* in, int* out, int n, void* temp, cudaStream_t s);
 
 // ------------------------------------------------------------- broad phase
 struct __align__(16) Box6 {
@@ -308,11 +308,10 @@ void apply_contribs(const Contrib* contrib, const PassCounters* ctr, int contrib
                     uint8_t* has_collsn, ApplyBufs& b, cudaStream_t s, double4_32a* dump = nullptr,
                     const BodyBufs* bodies = nullptr);
 
-// updateImpactZoneVelocity (dcollid.cpp:290-310): rigid motion of every
-// zone, one thread per zone over members[zone_off[z] .. zone_off[z+1]) in
-// the order of the reference's member list, with its scene's parameters.
-// With run set, the zones are movable bodies and move only in scenes that
-// are in a pass (updateImpactZoneVelocityForRG).
+// Rigid motion of the movable bodies (updateImpactZoneVelocityForRG,
+// dcollid.cpp:267-288), a CTA each over members[zone_off[z] ..
+// zone_off[z+1]) in the order of the reference's member list, with its
+// scene's parameters. With run set, only in scenes that are in a pass.
 void zone_solve(const int* members, const int* zone_off, int nzones, const uint8_t* fixed, const double4_32a* xo,
                 double4_32a* av, const int* vscene, const SceneDev* scenes, PassCounters* ctr, cudaStream_t s,
                 const SceneRun* run = nullptr, PassStamp ps = PassStamp{});
@@ -325,7 +324,8 @@ struct ZoneMembers {
     __device__ __forceinline__ const int* list() const { return epoch ? buf[*epoch & 1] : buf[0]; }
 #endif
 };
-// The same with zone z's members at [zone_rng[z].x .. .y) of their list and
+// Rigid motion of every impact zone (updateImpactZoneVelocity,
+// dcollid.cpp:290-310), zone z's members at [zone_rng[z].x .. .y) of their list and
 // the zone count in device memory (*dnz, at most zone_cap).
 void zone_solve_dev(const ZoneMembers& members, const int2* zone_rng, const int* dnz, int zone_cap, const uint8_t* fixed,
                     const double4_32a* xo, double4_32a* av, const int* vscene, const SceneDev* scenes,

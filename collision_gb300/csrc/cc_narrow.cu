@@ -214,13 +214,8 @@ __device__ __forceinline__ bool pair_subtest(const OrientedPair& o, int sub, int
     return true;
 }
 
-// Stage 1 of a split pass: per candidate pair, the visit bookkeeping of
-// k_narrow, the element-pair filter, and the box and separating-axis filter
-// of every sub-test, in sub-test order; survivors are queued with their keys,
-// and a pair with survivors is queued for stage 3.
-// Passes of at most this many pairs take filter_wide.
-constexpr int kWideFilter = 131072;
-
+// One sub-test of a pair through the box and separating-axis filters; a
+// survivor is queued with its key, and its pair, with its first, for stage 3.
 template <bool MOVING>
 __device__ __forceinline__ void queue_sub(const NarrowArgs& a, const NarrowCtx& c, bool ee, unsigned long long kb,
                                           int pair, int sc, const int* pts, int sub, bool thin, bool& first) {
@@ -325,6 +320,13 @@ __device__ __forceinline__ int pair_may_hit16(const NarrowCtx& c, const Oriented
                               __shfl_sync(0xffffffffu, an, 5, 16));
 }
 
+// Passes of at most this many pairs take filter_wide. Moving filters of a
+// step, with a thread per pair throughout / this line / sixteen threads
+// throughout: sheet of 3,300 elements 0.032 / 0.015 / 0.015 ms, 48 sheets in
+// contact (68 passes, the first of 1.46M pairs) 2.97 / 2.11 / 2.11, sheet of
+// 136,000 elements 0.36 / 0.45 / 0.58 (0.34 with the line at 16,384 pairs).
+constexpr int kWideFilter = 131072;
+
 // Stage 1 with sixteen threads per pair, one per axis of the pair's bound and
 // then one per sub-test. A thread's 12 axes and 15 sub-tests in turn (below)
 // are ~36 us however few pairs a pass has.
@@ -374,6 +376,11 @@ __device__ __forceinline__ void filter_wide(const NarrowArgs& a, NarrowCtx& c, i
     }
 }
 
+// Stage 1 of a split mixed pass: per candidate pair, the visit bookkeeping of
+// k_narrow, the element-pair filter, and the box and separating-axis filter
+// of every sub-test; survivors are queued, and pairs with survivors for
+// stage 3. Sixteen threads per pair in passes of at most kWideFilter pairs,
+// in larger ones, which fill the chip either way, a thread per pair.
 // Registers held to 64 and 96, which let a block of 128 threads run eight and
 // five times on an SM: with the moving kernel's own choice of 108 a step of 48
 // sheets in contact took 29.2 ms against 28.8.
@@ -562,6 +569,11 @@ __device__ __forceinline__ void subtest_counts(const NarrowArgs& a, SubTally t) 
 // warp. 257 x 257 points in contact: filters and sub-tests of a step 1.48 ->
 // 1.09 ms (the filter formed the cubics of its survivors before, with almost
 // every warp holding one).
+// Passes of fewer give each sub-test its own warp (k_subtests) and need no
+// list: two warps on each of the 608 SM sub-partitions. Sub-tests of a step
+// without such passes / with this line / at 9,728 of them: 64 strings 0.25 /
+// 0.14 / 0.15 ms, 48 sheets in contact 4.38 / 3.41 / 5.52, 24 FP64 sheets
+// 0.51 / 0.40 / 0.52, sheet of 136,000 elements 0.67 / 0.67 / 0.74.
 constexpr int kSubSparse = 1216;
 struct SubLists {
     int npt, nee;

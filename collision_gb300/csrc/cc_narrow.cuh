@@ -52,7 +52,7 @@ struct CallState {
     int dcount[6];
     int sub;
     int nsub;   // sub-tests evaluated in FP64
-    int ncr;    // cubics whose roots were formed again correctly rounded
+    int ncr;    // cubics with a root in the time window
     int ncontacts;
 };
 

@@ -64,13 +64,6 @@ __global__ void k_scan_add(int* out, int n, const int* block_off) {
     }
 }
 
-__global__ void k_scan_total(const int* in, const int* out, int n, int* total) {
-    if (n > 0)
-        *total = out[n - 1] + in[n - 1];
-    else
-        *total = 0;
-}
-
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Scans of up to kScanOne elements take one block, a run of consecutive
@@ -311,16 +304,8 @@ void sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const int* dn,
 
 size_t scan_temp_bytes(int n) { return scan_levels_bytes(n) + 256; }
 
-void exclusive_scan(const int* in, int* out, int n, int* total, void* temp, cudaStream_t s) {
-    if (n <= 0) {
-        if (total) cudaMemsetAsync(total, 0, sizeof(int), s);
-        return;
-    }
-    // The last input is needed for the total after an in-place scan.
-    int* last = (int*)((char*)temp + scan_levels_bytes(n));
-    if (total) cudaMemcpyAsync(last, in + (n - 1), sizeof(int), cudaMemcpyDeviceToDevice, s);
-    scan_rec(in, out, n, (char*)temp, s);
-    if (total) count_launch(), k_scan_total<<<1, 1, 0, s>>>(last, out + (n - 1), 1, total);
+void exclusive_scan(const int* in, int* out, int n, void* temp, cudaStream_t s) {
+    if (n > 0) scan_rec(in, out, n, (char*)temp, s);
 }
 
 size_t radix_sort_temp_bytes(int n) {
@@ -365,7 +350,7 @@ void radix_sort_pairs_dev(unsigned long long* keys, unsigned int* vals, const in
     for (int ps = 0; ps < passes; ++ps) {
         int shift = ps * 8;
         count_launch(), k_radix_hist<<<nb, kSortThreads, 0, s>>>(ka, n, shift, hist, nb, dn);
-        exclusive_scan(hist, off, (int)hist_n, nullptr, stemp, s);
+        exclusive_scan(hist, off, (int)hist_n, stemp, s);
         count_launch(), k_radix_scatter<<<nb, kSortThreads, 0, s>>>(ka, va, kb, vb, n, shift, off, nb, dn);
         unsigned long long* tk = ka; ka = kb; kb = tk;
         unsigned int* tv = va; va = vb; vb = tv;

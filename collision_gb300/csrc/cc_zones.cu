@@ -10,8 +10,7 @@
 // A concurrent union-find gives the same partition but another order, so the
 // unions of a pass are replayed in the reference's visiting order - but only
 // where order matters: the unions of different final zones touch disjoint
-// points, so every final zone replays its own unions, one thread per zone,
-// all zones at once.
+// points, so every final zone replays its own unions, all zones at once.
 //
 // A pass of few records does all of it in one CTA in shared memory
 // (k_zone_join). In larger ones:

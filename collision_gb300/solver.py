@@ -354,6 +354,10 @@ class CollisionSolver3d:
                      "tree_build_us", "pruned_queries", "zone_unions")
 
     def counters(self) -> dict:
+        """Counters of the last step (cc_get_counters). fp64_subtests: in mixed
+        mode the sub-tests the FP32 filters left, in plain mode every one
+        visited, also where an FP32 bound decided it; cr_roots: coplanarity
+        cubics with a root in the time window."""
         n_all = len(self.COUNTER_NAMES)
         out = (C.c_longlong * n_all)()
         n = self._lib.cc_get_counters(self._h, out, n_all)

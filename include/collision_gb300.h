@@ -385,11 +385,11 @@ cc_status cc_set_strain_window(cc_solver* s, int on);
  * order: detection passes, CCD passes, impact-zone passes, candidate pairs
  * (all passes), narrow-phase visits, pairs that hit, contacts (sub-tests
  * that applied an impulse), strain passes, tree builds, kernel launches,
- * strain edges averaged, strain tests taken the exact way, sub-tests
- * evaluated in FP64, narrow-phase visits of CCD and impact-zone passes,
- * algorithmic bytes of the strain sweeps, coplanarity cubics whose roots
- * were formed again with correctly rounded functions, leaves traversed by
- * the broad phase (summed over its traversals), candidate pairs those
+ * strain edges averaged, strain tests taken the exact way, sub-tests (mixed
+ * passes: those the FP32 filters left; plain passes: every one visited,
+ * also where an FP32 bound decided it), narrow-phase visits of CCD and
+ * impact-zone passes, algorithmic bytes of the strain sweeps, coplanarity
+ * cubics with a root in the time window, leaves traversed by the broad phase (summed over its traversals), candidate pairs those
  * traversals wrote, the step's algorithmic bytes (below), the leaves and
  * pairs of the traversals launched from the host (those the "traverse" stage
  * of cc_get_profile times: every traversal in the host loop, the proximity
