@@ -1400,6 +1400,7 @@ cc_status cc_solver::fill_mesh(const cc_mesh* meshes, int n, int tot_v, int tot_
     h_strain_passes.assign(3 * (size_t)n, 0);
     scenes_dirty = true;
     strain_configure();
+    tree_configure();
     upload_scenes();  // synchronises: the host vectors above are pageable
     return cuda_check("assemble");
 }

@@ -250,6 +250,12 @@ size_t tree_scratch_bytes(long long ne) {
     return (size_t)(ne + 1) * (sizeof(TreeNode) + sizeof(TreeChild) + 3 * sizeof(int));
 }
 
+void tree_configure() {
+    cudaFuncAttributes a;
+    cudaFuncGetAttributes(&a, k_tree_build);
+    cudaFuncGetAttributes(&a, k_tree_ranks);
+}
+
 void tree_order_gpu(const Box6* boxes, const int* jobs, int njobs, int max_ne, void* scratch, long long ne_total,
                     int* rank, int* root_out, double* vol_out, cudaStream_t s) {
     if (njobs <= 0) return;
