@@ -29,7 +29,14 @@ namespace ccg {
 namespace {
 
 constexpr int kTreeThreads = 1024;
-constexpr int kTreeGroups = kTreeThreads / 4;  // insertions in flight
+constexpr int kTreeGroups = kTreeThreads / 4;  // insertions in flight, by lanes
+// Trees of at most this many leaves by lanes, larger ones by threads. One
+// tree by lanes / by threads: 97 x 97 sheet on two obstacles (39,000 leaves)
+// 45 / 67 ms, 85,000 leaves 173 / 198, 126,000 322 / 331, 152,000 443 / 435,
+// 280,000 1,137 / 1,052, 545,000 3,218 / 2,777, 2.1 million 24.6 / 20.4 s.
+// Two or more insertions per group in registers (512 and 1,024 in flight) are
+// slower than either: 3.6 s and more for the 545,000.
+constexpr int kTreeLaneMax = 131072;
 
 // Box coordinates are kept as order-preserving integer keys: key(a) <
 // key(b) exactly when a < b for doubles that are not NaN, except that -0
@@ -68,6 +75,19 @@ __device__ __forceinline__ double volume_k(const TreeChild& c) {
                      __dsub_rn(odec(c.zhi), odec(c.zlo)));
 }
 
+// A child's box with another's (volume and id left out), and whether it holds
+// the other already.
+__device__ __forceinline__ TreeChild joined(const TreeChild& a, const TreeChild& b) {
+    TreeChild c;
+    c.xlo = kmin(a.xlo, b.xlo); c.xhi = kmax(a.xhi, b.xhi);
+    c.ylo = kmin(a.ylo, b.ylo); c.yhi = kmax(a.yhi, b.yhi);
+    c.zlo = kmin(a.zlo, b.zlo); c.zhi = kmax(a.zhi, b.zhi);
+    return c;
+}
+__device__ __forceinline__ bool holds(const TreeChild& a, const TreeChild& b) {
+    return a.xlo <= b.xlo && a.ylo <= b.ylo && a.zlo <= b.zlo && b.xhi <= a.xhi && b.yhi <= a.yhi && b.zhi <= a.zhi;
+}
+
 // One lane's half of a child: lane h = 0 xlo, xhi, ylo, yhi; h = 1 zlo, zhi,
 // the volume's bits, the id.
 struct Half {
@@ -84,51 +104,18 @@ __device__ __forceinline__ void store_half(TreeChild* p, int h, const Half& x) {
     q[1] = make_longlong2(x.c, x.d);
 }
 
-// One CTA per tree, four lanes per insertion (lane 2 s + h: half h of child
-// s). What bounds a build is the time of a step, one level of every
-// insertion in flight: with a thread per insertion it was ~14 FP64
-// instructions of each warp (GB300 takes ~64 cycles for one however many
-// lanes it serves, and 32 insertions' lanes rarely all skip them), two
-// dependent loads (the child ids, then the children) and the barrier. Here
-// both children's unions are formed side by side, x and z too, which leaves
-// five FP64 instructions; a node's record holds both children, so a level is
-// one round of loads; a new leaf's record is loaded an insertion ahead; and
-// the leaf counts are adds that nothing waits for.
-__global__ void __launch_bounds__(kTreeThreads) k_tree_build(const Box6* __restrict__ boxes, const int* __restrict__ jobs,
-                                                            TreeNode* nodes_all, TreeChild* leaves_all, int* parent_all,
-                                                            int* extra_all, int* root_out, double* vol_out) {
-    const int e0 = jobs[3 * blockIdx.x + 1], n = jobs[3 * blockIdx.x + 2];
-    TreeNode* nd = nodes_all + e0;         // internal node q is nd[q - n]
-    TreeChild* leaf = leaves_all + e0;
-    int* parent = parent_all + 2 * (size_t)e0;
-    int* extra = extra_all + e0;           // node q has 2 + extra[q - n] leaves
+// Insertions 2 .. n - 1, four lanes each (lane 2 s + h: half h of child s).
+// What bounds a build is the time of a step, one level of every insertion in
+// flight: with a thread per insertion it was ~14 FP64 instructions of each
+// warp (GB300 takes ~64 cycles for one however many lanes it serves, and 32
+// insertions' lanes rarely all skip them), two dependent loads (the child ids,
+// then the children) and the barrier. Here both children's unions are formed
+// side by side, x and z too, which leaves five FP64 instructions; a node's
+// record holds both children, so a level is one round of loads; a new leaf's
+// record is loaded an insertion ahead; and the leaf counts are adds that
+// nothing waits for.
+__device__ void insert_by_lanes(TreeNode* nd, const TreeChild* leaf, int* parent, int* extra, int n) {
     const int tid = threadIdx.x;
-    for (int e = tid; e < n; e += kTreeThreads) {
-        const Box6 b = boxes[e0 + e];
-        TreeChild L;
-        L.xlo = okey(b.lo[0]); L.xhi = okey(b.hi[0]);
-        L.ylo = okey(b.lo[1]); L.yhi = okey(b.hi[1]);
-        L.zlo = okey(b.lo[2]); L.zhi = okey(b.hi[2]);
-        L.vol = volume_k(L);
-        L.id = e;
-        leaf[e] = L;
-        parent[e] = -1;
-        extra[e] = 0;
-    }
-    __syncthreads();
-    if (n < 2) {
-        if (tid == 0) {
-            root_out[blockIdx.x] = n - 1;
-            vol_out[blockIdx.x] = n == 1 ? leaf[0].vol : 0.0;
-        }
-        return;
-    }
-    if (tid == 0) {  // insertion 1 splits the root leaf 0 into node n
-        nd[0].child[0] = leaf[1];
-        nd[0].child[1] = leaf[0];
-        parent[n] = -1;
-        parent[0] = parent[1] = n;
-    }
     const int g = tid >> 2, side = (tid >> 1) & 1, h = tid & 1;
     const int lane = tid & 31, base = lane & ~3;  // the group's first lane in its warp
     const Half none{0, 0, 0, 0};
@@ -216,14 +203,122 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_build(const Box6* __restr
         next += __syncthreads_or(start) ? 1 : 0;
         if (next >= n && !__syncthreads_or(my_e >= 0)) break;
     }
+}
+
+// The same, a thread each: four times as many in flight, for trees so deep
+// (a flat sheet's are ~1.4 times its side) that insertions wait for a free
+// group more than shorter steps make up for.
+__device__ void insert_by_threads(TreeNode* nd, const TreeChild* leaf, int* parent, int* extra, int n) {
+    const int tid = threadIdx.x;
+    int my_e = -1, p = n;
+    TreeChild mine;
+    int next = 2;
+    __syncthreads();
+    for (;;) {
+        const bool start = next < n && my_e < 0 && next % kTreeThreads == tid;
+        if (start) {
+            my_e = next;
+            p = n;
+            mine = leaf[my_e];
+        }
+        if (my_e >= 0) {
+            TreeNode* at = &nd[p - n];
+            const TreeChild l = at->child[0], r = at->child[1];
+            // a box that holds the new leaf's does not grow (the same
+            // doubles), and a growth is never below 0
+            bool go_left, grows;
+            double vol;  // the chosen child's with the new leaf
+            if (holds(r, mine)) {
+                go_left = false;  // the right one's growth is 0
+                grows = false;
+                vol = r.vol;
+            } else {
+                const double vr = volume_k(joined(r, mine));
+                if (holds(l, mine)) {
+                    go_left = __dsub_rn(l.vol, l.vol) < __dsub_rn(vr, r.vol);  // (0, or NaN if it is infinite)
+                    grows = !go_left;
+                    vol = go_left ? l.vol : vr;
+                } else {
+                    const double vl = volume_k(joined(l, mine));
+                    go_left = __dsub_rn(vl, l.vol) < __dsub_rn(vr, r.vol);
+                    grows = true;
+                    vol = go_left ? vl : vr;
+                }
+            }
+            const TreeChild was = go_left ? l : r;
+            const int c = (int)was.id;
+            const bool split = c < n;
+            const int q = n + my_e - 1;
+            if (grows || split) {
+                TreeChild w = joined(was, mine);
+                w.vol = vol;
+                w.id = split ? q : c;
+                at->child[go_left ? 0 : 1] = w;
+            }
+            if (split) {
+                // new leaf left, old leaf right
+                mine.id = my_e;  // (needs no register until here)
+                nd[q - n].child[0] = mine;
+                nd[q - n].child[1] = was;
+                parent[q] = p;
+                parent[my_e] = q;
+                parent[c] = q;
+                my_e = -1;
+            } else {
+                p = c;
+                atomicAdd(&extra[c - n], 1);
+            }
+        }
+        next += __syncthreads_or(start) ? 1 : 0;
+        if (next >= n && !__syncthreads_or(my_e >= 0)) break;
+    }
+}
+
+// One CTA per tree, of those that are inserted by threads or by lanes.
+template <bool BY_THREADS>
+__global__ void __launch_bounds__(kTreeThreads) k_tree_build(const Box6* __restrict__ boxes, const int* __restrict__ jobs,
+                                                            TreeNode* nodes_all, TreeChild* leaves_all, int* parent_all,
+                                                            int* extra_all, int* root_out, double* vol_out) {
+    const int e0 = jobs[3 * blockIdx.x + 1], n = jobs[3 * blockIdx.x + 2];
+    if ((n > kTreeLaneMax) != BY_THREADS) return;
+    TreeNode* nd = nodes_all + e0;         // internal node q is nd[q - n]
+    TreeChild* leaf = leaves_all + e0;
+    int* parent = parent_all + 2 * (size_t)e0;
+    int* extra = extra_all + e0;           // node q has 2 + extra[q - n] leaves
+    const int tid = threadIdx.x;
+    for (int e = tid; e < n; e += kTreeThreads) {
+        const Box6 b = boxes[e0 + e];
+        TreeChild L;
+        L.xlo = okey(b.lo[0]); L.xhi = okey(b.hi[0]);
+        L.ylo = okey(b.lo[1]); L.yhi = okey(b.hi[1]);
+        L.zlo = okey(b.lo[2]); L.zhi = okey(b.hi[2]);
+        L.vol = volume_k(L);
+        L.id = e;
+        leaf[e] = L;
+        parent[e] = -1;
+        extra[e] = 0;
+    }
+    __syncthreads();
+    if (n < 2) {
+        if (tid == 0) {
+            root_out[blockIdx.x] = n - 1;
+            vol_out[blockIdx.x] = n == 1 ? leaf[0].vol : 0.0;
+        }
+        return;
+    }
+    if (tid == 0) {  // insertion 1 splits the root leaf 0 into node n
+        nd[0].child[0] = leaf[1];
+        nd[0].child[1] = leaf[0];
+        parent[n] = -1;
+        parent[0] = parent[1] = n;
+    }
+    if (BY_THREADS)
+        insert_by_threads(nd, leaf, parent, extra, n);
+    else
+        insert_by_lanes(nd, leaf, parent, extra, n);
     if (tid == 0) {
-        const TreeChild a = nd[0].child[0], b = nd[0].child[1];
-        TreeChild r;
-        r.xlo = kmin(a.xlo, b.xlo); r.xhi = kmax(a.xhi, b.xhi);
-        r.ylo = kmin(a.ylo, b.ylo); r.yhi = kmax(a.yhi, b.yhi);
-        r.zlo = kmin(a.zlo, b.zlo); r.zhi = kmax(a.zhi, b.zhi);
         root_out[blockIdx.x] = n;
-        vol_out[blockIdx.x] = volume_k(r);
+        vol_out[blockIdx.x] = volume_k(joined(nd[0].child[0], nd[0].child[1]));
     }
 }
 
@@ -252,7 +347,8 @@ size_t tree_scratch_bytes(long long ne) {
 
 void tree_configure() {
     cudaFuncAttributes a;
-    cudaFuncGetAttributes(&a, k_tree_build);
+    cudaFuncGetAttributes(&a, k_tree_build<false>);
+    cudaFuncGetAttributes(&a, k_tree_build<true>);
     cudaFuncGetAttributes(&a, k_tree_ranks);
 }
 
@@ -263,7 +359,9 @@ void tree_order_gpu(const Box6* boxes, const int* jobs, int njobs, int max_ne, v
     TreeChild* leaves = reinterpret_cast<TreeChild*>(nodes + ne_total + 1);
     int* parent = reinterpret_cast<int*>(leaves + ne_total + 1);
     int* extra = parent + 2 * (ne_total + 1);
-    k_tree_build<<<njobs, kTreeThreads, 0, s>>>(boxes, jobs, nodes, leaves, parent, extra, root_out, vol_out);
+    k_tree_build<false><<<njobs, kTreeThreads, 0, s>>>(boxes, jobs, nodes, leaves, parent, extra, root_out, vol_out);
+    if (max_ne > kTreeLaneMax)
+        k_tree_build<true><<<njobs, kTreeThreads, 0, s>>>(boxes, jobs, nodes, leaves, parent, extra, root_out, vol_out);
     const int bx = std::max(1, std::min((max_ne + 255) / 256, 1024));
     k_tree_ranks<<<dim3(bx, njobs), 256, 0, s>>>(jobs, nodes, parent, extra, rank);
 }
